@@ -148,7 +148,7 @@ int ttg_zbfun3(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1, ttg
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1 && A && phi2 && x && y && nvec > 0, "null pointer or nvec <= 0");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  size_t bytes = 2 * bfun3_f64_scratch(L, (int)nvec);
+  size_t bytes = bfun3_z_scratch(L, (int)nvec);
   c->ws.reset();
   c->ws.reserve(bytes);
   double2* scr = (double2*)c->ws.take(bytes);
@@ -165,7 +165,7 @@ int ttg_zbfun3_transp(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int r
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1 && A && phi2 && x && y && nvec > 0, "null pointer or nvec <= 0");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  size_t bytes = (size_t)(rx1 * ra1 * n * ry2 + rx1 * m * ra2 * ry2) * nvec * sizeof(double2);
+  size_t bytes = bfun3_z_scratch(L, (int)nvec);
   c->ws.reset();
   c->ws.reserve(bytes);
   double2* scr = (double2*)c->ws.take(bytes);
@@ -210,8 +210,8 @@ int ttg_zphi_left(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1, 
   TTG_REQUIRE(phi1_old && A && x && y && phi1_new, "null pointer");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
   c->ws.reset();
-  c->ws.reserve(phi_f64_scratch(L) * 2);
-  double2* scr = (double2*)c->ws.take(phi_f64_scratch(L) * 2);
+  c->ws.reserve(phi_z_scratch(L));
+  double2* scr = (double2*)c->ws.take(phi_z_scratch(L));
   phi_left_z(L, (const double2*)phi1_old, (const double2*)A, (const double2*)x,
              (const double2*)y, (double2*)phi1_new, scr, c->stream);
   TTG_API_END(c)
@@ -225,8 +225,8 @@ int ttg_zphi_right(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1,
   TTG_REQUIRE(phi2_old && A && x && y && phi2_new, "null pointer");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
   c->ws.reset();
-  c->ws.reserve(phi_f64_scratch(L) * 2);
-  double2* scr = (double2*)c->ws.take(phi_f64_scratch(L) * 2);
+  c->ws.reserve(phi_z_scratch(L));
+  double2* scr = (double2*)c->ws.take(phi_z_scratch(L));
   phi_right_z(L, (const double2*)phi2_old, (const double2*)A, (const double2*)x,
               (const double2*)y, (double2*)phi2_new, scr, c->stream);
   TTG_API_END(c)

@@ -264,6 +264,33 @@ struct GemmZ {
 void gemm_z(const GemmZ& g, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
+// The same products on the tensor cores by error-free splitting (ttg_oz.cu):
+//   C[m,n] = sum_k A[m,k] B[k,n], element (m,k) of A at A[map(am, m) + k*ak]
+//   (B by n, C by m and n), map(i) = i / d * s2 + i % d * s1; sizes, strides
+//   and pointers in complex elements when cplx.
+// ---------------------------------------------------------------------------
+struct OzMap {
+  int d;
+  i64 s1, s2;
+};
+struct OzGemm {
+  int M = 0, N = 0, K = 0;
+  const double* A = nullptr; OzMap am{1, 0, 0}; i64 ak = 0;
+  const double* B = nullptr; OzMap bn{1, 0, 0}; i64 bk = 0;
+  double* C = nullptr;       OzMap cm{1, 0, 0}, cn{1, 0, 0};
+  bool cplx = false, conjA = false, conjB = false;
+};
+constexpr double kOzMinMNK = 2.0e6;              // below: never split
+constexpr size_t kOzMaxBytes = (size_t)4 << 30;  // workspace limit: larger products stay FP64
+size_t oz_bytes(i64 M, i64 N, i64 K, bool cplx); // workspace, non-decreasing in every size
+bool oz_fits(i64 M, i64 N, i64 K, bool cplx);    // within both limits
+double oz_us(i64 M, i64 N, i64 K, bool cplx);    // estimated time
+void oz_gemm(const OzGemm& g, void* ws, cudaStream_t s);
+// runs g as a split product when it has the form for it and that is faster
+bool oz_try(const GemmF64& g, void* ws, cudaStream_t s);
+bool oz_try(const GemmZ& g, void* ws, cudaStream_t s);
+
+// ---------------------------------------------------------------------------
 // Local operator kernels (ttg_local.cu)
 // ---------------------------------------------------------------------------
 struct LocalDims {
@@ -275,10 +302,16 @@ struct LocalDims {
 };
 
 // bfun3 for nvec vectors (x: xsize*nvec contiguous, y: ysize*nvec).
-// scratch: (t1size + t2size) * nvec doubles.
+// scratch: bfun3_f64_scratch bytes, or (t1size + t2size) * nvec doubles with
+// split = false (FP64 kernels only).
 void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
-               const double* x, double* y, int nvec, double* scratch, cudaStream_t s);
+               const double* x, double* y, int nvec, double* scratch, cudaStream_t s,
+               bool split = true);
+// Bytes; non-decreasing in every size, so a sweep may size for its largest
+// ranks and hand the same scratch to every smaller problem.
 size_t bfun3_f64_scratch(const LocalDims& L, int nvec);
+size_t bfun3_z_scratch(const LocalDims& L, int nvec);   // bfun3_z and bfun3_transp_z
+size_t phi_z_scratch(const LocalDims& L);
 
 void phi_left_f64(const LocalDims& L, const double* phi1_old, const double* A,
                   const double* x, const double* y, double* phi1_new, double* scratch,

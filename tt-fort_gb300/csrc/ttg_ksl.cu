@@ -210,8 +210,8 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
     capmax = std::max(capmax, c);
     Nmax = std::max(Nmax, c);
     LocalDims L{Rc[i], n[i], Rc[i + 1], Rc[i], n[i], Rc[i + 1], P.ra[i], P.ra[i + 1]};
-    scr = std::max<i64>(scr, (i64)(phi_f64_scratch(L) / sizeof(double)) + 1);
-    scr = std::max<i64>(scr, (L.t1size() + L.t2size()) * 4 + 16);
+    scr = std::max<i64>(scr, (i64)(phi_z_scratch(L) / sizeof(double2)) + 16);
+    scr = std::max<i64>(scr, (i64)(bfun3_z_scratch(L, 4) / sizeof(double2)) + 16);   // norm estimate: 4 vectors
     scr = std::max<i64>(scr, (Rc[i] * P.ra[i] * n[i] * Rc[i + 1] + Rc[i] * n[i] * P.ra[i + 1] * Rc[i + 1]) * 4 + 16);
     rmx = std::max(rmx, Rc[i]);
   }

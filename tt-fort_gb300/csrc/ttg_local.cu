@@ -13,19 +13,73 @@
 //   T1[b1, j, a2, c2]   = x * Phi2              (rx1*m  x ra2*ry2)
 //   T2[b1, a1, i, c2]   = A (x) T1, one GEMM per c2
 //   y [c1, i, c2]       = Phi1 * T2             (ry1 x n*ry2)
-// so the transposes cost nothing.  All GEMMs go through gemm_f64 / gemm_z.
+// so the transposes cost nothing.  Large products run on the tensor cores
+// (ttg_oz.cu: FP64 by error-free splitting), the others through gemm_f64 / gemm_z.
 #include "ttg_common.cuh"
+#include <algorithm>
 
 namespace ttg {
 
+// Scratch layout: two FP64 (or complex) intermediates, then the workspace of
+// the split products (ttg_oz.cu) that the sizes can reach.
+static size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
+// rows of Q = A Phi2 (see bfun3_f64): only for small modes, and only where a
+// split product can follow
+static i64 q_size(const LocalDims& L, int nvec) {
+  if (L.n * L.m > 4 || oz_bytes(L.rx1 * nvec, L.n * L.ry2 * L.ra1, L.m * L.rx2, false) == 0) return 0;
+  return L.n * L.ry2 * L.ra1 * L.m * L.rx2;
+}
+static size_t bfun3_oz_bytes(const LocalDims& L, int nvec, bool cplx) {
+  size_t b = std::max({oz_bytes(L.rx1 * L.m * nvec, L.ra2 * L.ry2, L.rx2, cplx),
+                       oz_bytes(L.rx1 * L.ry2 * nvec, L.ra1 * L.n, L.m * L.ra2, cplx),
+                       oz_bytes(L.ry1, L.n * L.ry2 * nvec, L.rx1 * L.ra1, cplx)});
+  if (!cplx && L.n * L.m <= 4)
+    b = std::max(b, oz_bytes(L.rx1 * nvec, L.n * L.ry2 * L.ra1, L.m * L.rx2, false));
+  if (cplx)   // the adjoint's products
+    b = std::max({b, oz_bytes(L.rx1 * L.ra1, L.n * L.ry2 * nvec, L.ry1, true),
+                  oz_bytes(L.rx1 * L.ry2 * nvec, L.m * L.ra2, L.ra1 * L.n, true),
+                  oz_bytes(L.rx1 * L.m * nvec, L.rx2, L.ra2 * L.ry2, true)});
+  return b;
+}
+static size_t bfun3_t_bytes(const LocalDims& L, int nvec) {
+  return al256((size_t)(std::max(L.t1size() * nvec, q_size(L, nvec)) + L.t2size() * nvec) * sizeof(double));
+}
 size_t bfun3_f64_scratch(const LocalDims& L, int nvec) {
-  return (size_t)(L.t1size() + L.t2size()) * nvec * sizeof(double);
+  return bfun3_t_bytes(L, nvec) + bfun3_oz_bytes(L, nvec, false);
+}
+static size_t bfun3_z_t_bytes(const LocalDims& L, int nvec) {
+  return al256((size_t)(L.t1size() + L.t2size()) * nvec * sizeof(double2));
+}
+size_t bfun3_z_scratch(const LocalDims& L, int nvec) {
+  return bfun3_z_t_bytes(L, nvec) + bfun3_oz_bytes(L, nvec, true);
 }
 
-size_t phi_f64_scratch(const LocalDims& L) {
+static size_t phi_t_bytes(const LocalDims& L, size_t elem) {
   i64 a = std::max(L.t1size(), L.rx1 * L.ra1 * L.n * L.ry2);
   i64 b = std::max(L.t2size(), L.rx1 * L.m * L.ra2 * L.ry2);
-  return (size_t)(a + b) * sizeof(double) * 2;   // room for complex too
+  return al256((size_t)(a + b) * elem);
+}
+static size_t phi_oz_bytes(const LocalDims& L, bool cplx) {
+  return std::max({bfun3_oz_bytes(L, 1, cplx),
+                   oz_bytes(L.rx1 * L.ra1, L.n * L.ry2, L.ry1, cplx),
+                   oz_bytes(L.rx1 * L.ry2, L.m * L.ra2, L.ra1 * L.n, cplx),
+                   oz_bytes(L.ry2 * L.ra2, L.rx2, L.rx1 * L.m, cplx),
+                   oz_bytes(L.rx1 * L.ra1, L.ry1, L.n * L.ry2, cplx)});
+}
+size_t phi_f64_scratch(const LocalDims& L) {
+  return phi_t_bytes(L, sizeof(double)) + phi_oz_bytes(L, false);
+}
+size_t phi_z_scratch(const LocalDims& L) {
+  return phi_t_bytes(L, sizeof(double2)) + phi_oz_bytes(L, true);
+}
+
+// one product: on the tensor cores where that is faster (ws: their workspace,
+// null for the FP64 kernels only)
+static void product(const GemmF64& g, void* ws, cudaStream_t s) {
+  if (!oz_try(g, ws, s)) gemm_f64(g, s);
+}
+static void product(const GemmZ& g, void* ws, cudaStream_t s) {
+  if (!oz_try(g, ws, s)) gemm_z(g, s);
 }
 
 template <class G, class T>
@@ -63,22 +117,87 @@ static void stage3(G& g, const LocalDims& L, const T* phi1, const T* T2, T* y, i
   g.bA2 = 0; g.bB2 = L.t2size(); g.bC2 = L.ysize();
 }
 
+// Q[kq + KQ (i + n (c2 + ry2 a1))] = sum_a2 A(a1,i,j,a2) Phi2(b2,a2,c2), kq = j + m b2.
+// One block per (c2, a1): its n m ra2 core entries in shared memory, then a
+// thread per b2 forms the n m outputs of that b2 from one read of Phi2.  Bound
+// by its FP64 FMAs (m n <= 4).
+__global__ void __launch_bounds__(128) q_kernel(int m, int rx2, int n, int ry2, int ra1, int ra2,
+                                                const double* __restrict__ A,
+                                                const double* __restrict__ phi2,
+                                                double* __restrict__ Q) {
+  extern __shared__ double core[];                // [a2][i + n j]
+  pdl_wait();
+  const int c2 = blockIdx.x, a1 = blockIdx.y, nm = n * m;
+  for (int e = threadIdx.x; e < nm * ra2; e += blockDim.x)
+    core[e] = A[a1 + (i64)ra1 * e];
+  __syncthreads();
+  const double* p2 = phi2 + (i64)rx2 * ra2 * c2;
+  double* q = Q + (i64)m * rx2 * n * (c2 + (i64)ry2 * a1);
+  for (int b2 = threadIdx.x; b2 < rx2; b2 += blockDim.x) {
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int a2 = 0; a2 < ra2; ++a2) {
+      const double p = p2[b2 + (i64)rx2 * a2];
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (e < nm) v[e] = fma(core[a2 * nm + e], p, v[e]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (e < nm) q[(i64)m * rx2 * (e % n) + e / n + (i64)m * b2] = v[e];
+  }
+  pdl_trigger();
+}
+
+// Small modes (spin chains) at sizes where the products run on the tensor
+// cores: the middle contraction would then be most of the time (its K = m ra2
+// is too small to split: 105 MFLOP of FP64, 91 us, at r = 256, block of 8,
+// beside 46 us for each of the two large products).  Contracting the core into
+// Phi2 first costs K_Q times ra2 FMAs per row instead (11 us there) and makes
+// the first product n times larger.
+static bool bfun3_q(const LocalDims& L, const double* A, const double* phi2, const double* x,
+                    double* Q, double* T2, int nvec, void* ws, cudaStream_t s) {
+  const i64 M = L.rx1 * nvec, N = L.n * L.ry2 * L.ra1, K = L.m * L.rx2;
+  if (q_size(L, nvec) == 0 || !oz_fits(M, N, K, false)) return false;
+  const double core = 2.0 * (double)(L.ra1 * L.n) * (double)(L.m * L.ra2) * (double)(L.ry2 * L.rx1) * nvec / 1.0e6;
+  const double first = 2.0 * (double)(L.rx1 * L.m * nvec) * (double)(L.ra2 * L.ry2) * (double)L.rx2 / 1.0e6;
+  const double general = 8.0 + core +
+                         std::min(first, oz_us(L.rx1 * L.m * nvec, L.ra2 * L.ry2, L.rx2, false));
+  const double build = 2.0 * (double)N * (double)K * (double)L.ra2 / 1.0e6 + 4.0;
+  if (build + oz_us(M, N, K, false) >= general) return false;
+  if (L.ra1 >= 65536 || L.n * L.m * L.ra2 > 4096) return false;   // grid and shared memory
+  launch_pdl(q_kernel, dim3((unsigned)L.ry2, (unsigned)L.ra1), dim3(128),
+             sizeof(double) * L.n * L.m * L.ra2, s, (int)L.m, (int)L.rx2, (int)L.n, (int)L.ry2,
+             (int)L.ra1, (int)L.ra2, A, phi2, Q);
+  OzGemm g;   // T2[b1,a1,i,c2,v] = sum_kq X_v[b1,kq] Q[(i,c2,a1),kq]
+  g.M = (int)M; g.N = (int)N; g.K = (int)K;
+  g.A = x; g.am = {(int)L.rx1, 1, L.xsize()}; g.ak = L.rx1;
+  g.B = Q; g.bn = {(int)N, K, 0}; g.bk = 1;
+  g.C = T2; g.cm = {(int)L.rx1, 1, L.t2size()}; g.cn = {(int)(L.n * L.ry2), L.rx1 * L.ra1, L.rx1};
+  oz_gemm(g, ws, s);
+  return true;
+}
+
 void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
-               const double* x, double* y, int nvec, double* scratch, cudaStream_t s) {
+               const double* x, double* y, int nvec, double* scratch, cudaStream_t s, bool split) {
+  const i64 t1 = split ? std::max(L.t1size() * nvec, q_size(L, nvec)) : L.t1size() * nvec;
   double* T1 = scratch;
-  double* T2 = scratch + L.t1size() * nvec;
-  { GemmF64 g; stage1(g, L, x, phi2, T1, nvec); gemm_f64(g, s); }
-  { GemmF64 g; stage2(g, L, A, T1, T2, nvec); gemm_f64(g, s); }
-  { GemmF64 g; stage3(g, L, phi1, T2, y, nvec); gemm_f64(g, s); }
+  double* T2 = scratch + t1;
+  void* ws = split ? (char*)scratch + bfun3_t_bytes(L, nvec) : nullptr;
+  if (!ws || !bfun3_q(L, A, phi2, x, T1, T2, nvec, ws, s)) {
+    { GemmF64 g; stage1(g, L, x, phi2, T1, nvec); product(g, ws, s); }
+    { GemmF64 g; stage2(g, L, A, T1, T2, nvec); product(g, ws, s); }
+  }
+  { GemmF64 g; stage3(g, L, phi1, T2, y, nvec); product(g, ws, s); }
 }
 
 void bfun3_z(const LocalDims& L, const double2* phi1, const double2* A, const double2* phi2,
              const double2* x, double2* y, int nvec, double2* scratch, cudaStream_t s) {
   double2* T1 = scratch;
   double2* T2 = scratch + L.t1size() * nvec;
-  { GemmZ g; stage1(g, L, x, phi2, T1, nvec); gemm_z(g, s); }
-  { GemmZ g; stage2(g, L, A, T1, T2, nvec); gemm_z(g, s); }
-  { GemmZ g; stage3(g, L, phi1, T2, y, nvec); gemm_z(g, s); }
+  void* ws = (char*)scratch + bfun3_z_t_bytes(L, nvec);
+  { GemmZ g; stage1(g, L, x, phi2, T1, nvec); product(g, ws, s); }
+  { GemmZ g; stage2(g, L, A, T1, T2, nvec); product(g, ws, s); }
+  { GemmZ g; stage3(g, L, phi1, T2, y, nvec); product(g, ws, s); }
 }
 
 // Adjoint product (zbfun3_transp, ttals.f90:85-108): x has the y layout
@@ -90,6 +209,7 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
   const i64 p2 = L.rx1 * L.m * L.ra2 * L.ry2;     // R2[b1,j,a2,c2]
   double2* R1 = scratch;
   double2* R2 = scratch + p1 * nvec;
+  void* ws = (char*)scratch + bfun3_z_t_bytes(L, nvec);
   {
     GemmZ g;   // R1[(b1,a1),(i,c2)] = sum_c1 conj(phi1[c1,(b1,a1)]) x[c1,(i,c2)]
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)(L.n * L.ry2); g.K = (int)L.ry1;
@@ -97,7 +217,7 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
     g.B = x; g.sBk = 1; g.sBn = L.ry1;
     g.C = R1; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
     g.nb2 = nvec; g.bB2 = L.ysize(); g.bC2 = p1;
-    gemm_z(g, s);
+    product(g, ws, s);
   }
   {
     GemmZ g;   // per (c2, vec): R2[b1,(j,a2)] = sum_p conj(A[p,(j,a2)]) R1[b1,p]
@@ -108,7 +228,7 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
     g.nb1 = (int)L.ry2; g.nb2 = nvec;
     g.bB1 = L.rx1 * L.ra1 * L.n; g.bB2 = p1;
     g.bC1 = L.rx1 * L.m * L.ra2; g.bC2 = p2;
-    gemm_z(g, s);
+    product(g, ws, s);
   }
   {
     GemmZ g;   // y[(b1,j), b2] = sum_(a2,c2) R2[(b1,j),(a2,c2)] conj(phi2[b2,(a2,c2)])
@@ -117,18 +237,18 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
     g.B = phi2; g.sBk = L.rx2; g.sBn = 1; g.conjB = true;
     g.C = y; g.sCm = 1; g.sCn = L.rx1 * L.m;
     g.nb2 = nvec; g.bA2 = p2; g.bC2 = L.xsize();
-    gemm_z(g, s);
+    product(g, ws, s);
   }
 }
 
 template <class G, class T>
 static void phi_right_impl(const LocalDims& L, const T* phi2_old, const T* A, const T* x,
-                           const T* y, T* phi2_new, T* scratch, bool conj_y, cudaStream_t s,
-                           void (*gemm)(const G&, cudaStream_t)) {
+                           const T* y, T* phi2_new, T* scratch, bool conj_y, cudaStream_t s) {
   T* T1 = scratch;
   T* T2 = scratch + L.t1size();
-  { G g; stage1(g, L, x, phi2_old, T1, 1); gemm(g, s); }
-  { G g; stage2(g, L, A, T1, T2, 1); gemm(g, s); }
+  void* ws = (char*)scratch + phi_t_bytes(L, sizeof(T));
+  { G g; stage1(g, L, x, phi2_old, T1, 1); product(g, ws, s); }
+  { G g; stage2(g, L, A, T1, T2, 1); product(g, ws, s); }
   {
     // phi2_new (rx1*ra1 x ry1) = T2 (rx1*ra1 x n*ry2) * y^T (n*ry2 x ry1)
     G g;
@@ -137,17 +257,17 @@ static void phi_right_impl(const LocalDims& L, const T* phi2_old, const T* A, co
     g.B = y; g.sBk = L.ry1; g.sBn = 1;
     g.C = phi2_new; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
     if constexpr (sizeof(T) == 16) g.conjB = conj_y;
-    gemm(g, s);
+    product(g, ws, s);
   }
 }
 
 template <class G, class T>
 static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, const T* x,
-                          const T* y, T* phi1_new, T* scratch, bool conj_y, cudaStream_t s,
-                          void (*gemm)(const G&, cudaStream_t)) {
+                          const T* y, T* phi1_new, T* scratch, bool conj_y, cudaStream_t s) {
   const i64 psz = L.rx1 * L.ra1 * L.n * L.ry2;   // P[b1,a1,i,c2]
   T* P = scratch;
   T* Q = scratch + psz;                           // Q[b1,j,a2,c2]
+  void* ws = (char*)scratch + phi_t_bytes(L, sizeof(T));
   {
     G g;   // P[(b1,a1),(i,c2)] = sum_c1 phi1_old[c1,(b1,a1)] y[c1,(i,c2)]
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)(L.n * L.ry2); g.K = (int)L.ry1;
@@ -155,7 +275,7 @@ static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, con
     g.B = y; g.sBk = 1; g.sBn = L.ry1;
     g.C = P; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
     if constexpr (sizeof(T) == 16) g.conjB = conj_y;
-    gemm(g, s);
+    product(g, ws, s);
   }
   {
     G g;   // per c2: Q[b1,(j,a2)] = sum_(a1,i) A[(a1,i),(j,a2)] P[b1,(a1,i)]
@@ -164,7 +284,7 @@ static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, con
     g.B = P; g.sBk = L.rx1; g.sBn = 1;
     g.C = Q; g.sCm = L.rx1; g.sCn = 1;
     g.nb1 = (int)L.ry2; g.bB1 = L.rx1 * L.ra1 * L.n; g.bC1 = L.rx1 * L.m * L.ra2;
-    gemm(g, s);
+    product(g, ws, s);
   }
   {
     G g;   // per a2: phi1_new[c2, b2] = sum_(b1,j) Q[(b1,j), a2, c2] x[(b1,j), b2]
@@ -173,29 +293,29 @@ static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, con
     g.B = x; g.sBk = 1; g.sBn = L.rx1 * L.m;
     g.C = phi1_new; g.sCm = 1; g.sCn = L.ry2;
     g.nb1 = (int)L.ra2; g.bA1 = L.rx1 * L.m; g.bC1 = L.ry2 * L.rx2;
-    gemm(g, s);
+    product(g, ws, s);
   }
 }
 
 void phi_right_f64(const LocalDims& L, const double* phi2_old, const double* A,
                    const double* x, const double* y, double* phi2_new, double* scratch,
                    cudaStream_t s) {
-  phi_right_impl<GemmF64, double>(L, phi2_old, A, x, y, phi2_new, scratch, false, s, gemm_f64);
+  phi_right_impl<GemmF64, double>(L, phi2_old, A, x, y, phi2_new, scratch, false, s);
 }
 void phi_left_f64(const LocalDims& L, const double* phi1_old, const double* A,
                   const double* x, const double* y, double* phi1_new, double* scratch,
                   cudaStream_t s) {
-  phi_left_impl<GemmF64, double>(L, phi1_old, A, x, y, phi1_new, scratch, false, s, gemm_f64);
+  phi_left_impl<GemmF64, double>(L, phi1_old, A, x, y, phi1_new, scratch, false, s);
 }
 void phi_right_z(const LocalDims& L, const double2* phi2_old, const double2* A,
                  const double2* x, const double2* y, double2* phi2_new, double2* scratch,
                  cudaStream_t s) {
-  phi_right_impl<GemmZ, double2>(L, phi2_old, A, x, y, phi2_new, scratch, true, s, gemm_z);
+  phi_right_impl<GemmZ, double2>(L, phi2_old, A, x, y, phi2_new, scratch, true, s);
 }
 void phi_left_z(const LocalDims& L, const double2* phi1_old, const double2* A,
                 const double2* x, const double2* y, double2* phi1_new, double2* scratch,
                 cudaStream_t s) {
-  phi_left_impl<GemmZ, double2>(L, phi1_old, A, x, y, phi1_new, scratch, true, s, gemm_z);
+  phi_left_impl<GemmZ, double2>(L, phi1_old, A, x, y, phi1_new, scratch, true, s);
 }
 
 void phi2_left_f64(i64 rx1, i64 rx2, i64 ry1, i64 n, i64 ry2, const double* phi1_old,

@@ -102,7 +102,8 @@ extern "C" int ttg_dbfun3_noalloc(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx
       return TTG_ERR_ARG;
     }
     double* scr = scratch_on(c->device);
-    ttg::bfun3_f64(L, phi1, A, phi2, x, y, (int)nvec, scr, c->stream);
+    ttg::bfun3_f64(L, phi1, A, phi2, x, y, (int)nvec, scr, c->stream,
+                   /*split=*/false);   // the fixed array has no room for split operands
   } catch (const ttg::Error& e) {
     c->last_error = e.msg;
     return e.code;

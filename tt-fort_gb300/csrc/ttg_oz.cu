@@ -1,0 +1,679 @@
+// FP64 products on the tensor cores by error-free splitting.
+//
+// GB300 issues two FP64 FMAs per clock per SM (1.2 TFLOP/s) but 1.9 PFLOP/s of
+// BF16 products with FP32 accumulation, so a large FP64 product is computed as
+// a sum of exact BF16 products (the scheme of Ozaki, Ogita, Oishi and Rump,
+// "Error-free transformations of matrix multiplication by using fast routines
+// of matrix multiplication and its applications", Numer. Algorithms 59, 2012):
+//
+//   a_mk = 2^(ea_m - 55) I_mk,  |a_mk| < 2^ea_m for every k, I rounded to an
+//   integer; I = sum_p d_p 256^(6-p) with balanced digits d_0..d_6 in
+//   [-128, 128], each exact in BF16; likewise b_kn with eb_n.
+//   sum_k a_mk b_kn = 2^(ea_m + eb_n - 14) sum_g 2^(-8 g) G_g,
+//   G_g = sum_k sum_(p+q=g) d_p d'_q,  g = 0..6 (28 of the 49 digit products;
+//   the others lie below 2^-56 of the row and column maxima).
+//
+// Every G_g is an integer that FP32 accumulation in tensor memory keeps
+// exactly: |d d'| <= 2^14, so K = 256 terms of at most 4 digit products stay
+// within 2^24; the groups g >= 4 could pass 2^24 only for constant digits of
+// -128, and a rounding there lies at 2^-24 2^-32.  After 256 K the groups are
+// drained into two 64-bit integers per element (no FP64 arithmetic), which
+// sum exactly in any order, and the end result is rounded once.  The error
+// left is that of I (2^-55 of a row's largest element) and of the dropped
+// products: measured against 64-bit values below that of the FP64 FMA chain
+// (tests/test_oz_gpu.py).
+//
+// A row whose elements are not all finite, or whose largest element lies
+// outside 2^(+-400), is flagged and its outputs are formed by the plain FP64
+// FMA chain, so infinities, NaN and extreme ranges give what they give there.
+//
+// Measured on GB300, FP64 kernels -> split products: chain product r=256, block
+// of 8: 4560 -> 243 us (22.6 TFLOP/s of FP64 accuracy; its two products run at
+// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 40.3
+// us; grid interface updates r = 82, 77, n = 64: 1908 -> 170 us; complex
+// operator and adjoint r=48, n=32, block of 4: 6968 -> 408 us.  What bounds the
+// product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
+// measured against 900 of MMA), for small ones its fixed ~10 us (pipeline
+// fill, one drain, rounding); oz_us below holds both.
+//
+// Tensor memory: a 128 x 64 tile with its seven groups side by side (448 of
+// the 512 columns).  The digit planes of B sit stacked along N, so the MMA of
+// A's plane p with B's planes 0..6-p writes groups p..6 in one instruction
+// (two where N > 256): ten instructions per 16-wide K step, and A's planes are
+// read from shared memory once per step.
+#include "ttg_common.cuh"
+#include "ttg_tcgen05.cuh"
+#include <algorithm>
+#include <climits>
+
+namespace ttg {
+namespace oz {
+
+using namespace tc;
+
+constexpr int P = 7;            // digit planes
+constexpr int BM = 128, BN = 64;
+constexpr int KCHUNK = 16;      // 16-wide K steps between drains (256 K)
+constexpr int STAGES = 5;
+constexpr uint32_t A_PLANE = BM * 32, B_PLANE = BN * 32;   // bytes of a plane in one K step
+constexpr uint32_t A_BYTES = P * A_PLANE, B_BYTES = P * B_PLANE;
+constexpr uint32_t STAGE = A_BYTES + B_BYTES;              // 43,008
+constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024;
+constexpr int EPI_WARPS = 16;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;
+constexpr int SLOW = 1 << 20;   // exponent of a flagged row
+constexpr int EMAX = 400;       // largest |exponent| of the fast path
+
+struct Side {                   // one operand, element (r, k) = src[map(r) + k * sk]
+  const double* src;
+  OzMap map;
+  i64 sk;
+  int rows, R;                  // logical rows; rows of a tile (BM or BN)
+  int rtiles;
+  unsigned char* planes;        // [rtile][K step][plane][R x 16 bf16, core matrices]
+  int* expo;                    // per split row
+  int cplx;                     // 0 real, 1: rows (re, im) x K (re, im), 2: K (re, im) only
+  int conj;
+};
+
+struct Args {
+  const unsigned char *Ad, *Bd;
+  const int *ea, *eb;
+  int M, N, K;                  // product rows and columns; logical K (for the FP64 chain)
+  int kt, kper, mtiles, ntiles, nz;
+  double* C;
+  OzMap cm, cn;
+  longlong2* part;              // nz > 1: partial sums [z][n][row]
+  const double *A, *B;          // original operands (flagged rows)
+  OzMap am, bn;
+  i64 ak, bk;
+  int cplx, conjA, conjB;
+};
+
+// 32-bit division: a 64-bit one per stored element took a third of the product
+__device__ __forceinline__ i64 at(const OzMap& m, int i) {
+  const uint32_t q = (uint32_t)i / (uint32_t)m.d, r = (uint32_t)i - q * (uint32_t)m.d;
+  return (i64)q * m.s2 + (i64)r * m.s1;
+}
+
+// bf16 pair from two digit bytes u (digit = u - 128): float 2^23 + u is exact,
+// and so is the difference; its upper half is the bf16
+__device__ __forceinline__ uint32_t digit_pair(uint32_t ja, uint32_t jb, uint32_t sel) {
+  const float a = __uint_as_float(__byte_perm(ja, 0x4B000000u, sel)) - 8388736.f;
+  const float b = __uint_as_float(__byte_perm(jb, 0x4B000000u, sel)) - 8388736.f;
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+__device__ __forceinline__ uint32_t top_pair(int ta, int tb) {
+  const float a = __uint_as_float(0x4B400000u + (uint32_t)ta) - 12582912.f;
+  const float b = __uint_as_float(0x4B400000u + (uint32_t)tb) - 12582912.f;
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+
+// Splits two operands in one launch (blocks [0, nblkA) take A).  A cluster of
+// gridDim.y blocks takes 8 rows and all of K, its blocks every gridDim.y-th
+// run of 256: a first pass finds the rows' largest exponents (joined over the
+// cluster), a second writes the digits, each thread one 16-byte core-matrix
+// row (8 K) per plane.  Bound by its 8 bytes read and 14 written per element
+// (integer digits, no FP64 arithmetic).
+constexpr int SROWS = 8;
+__global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA, int K, int kt) {
+  namespace cgr = cooperative_groups;
+  cgr::cluster_group cl = cgr::this_cluster();
+  __shared__ unsigned int key_s[SROWS];
+  pdl_wait();
+  const bool isA = (int)blockIdx.x < nblkA;
+  const Side& S = isA ? a : b;
+  const int blk = isA ? blockIdx.x : blockIdx.x - nblkA;
+  const int row = threadIdx.x & 7, kg0 = (threadIdx.x >> 3) + 32 * blockIdx.y;
+  const int kgs = 32 * gridDim.y;
+  const int r = blk * SROWS + row;                   // row of src
+  const bool real = r < S.rows;
+  const double* p = S.src + (real ? at(S.map, r) * (S.cplx ? 2 : 1) : 0);
+  const int groups = 2 * kt;
+  if (threadIdx.x < SROWS) key_s[threadIdx.x] = 0u;
+  __syncthreads();
+  double v[8];
+  auto load = [&](int g) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) v[q] = 0.0;
+    if (!real) return;
+    if (S.cplx) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int k = g * 4 + q;
+        if (k < K) {
+          const double2 z = *reinterpret_cast<const double2*>(p + 2 * (i64)k * S.sk);
+          v[2 * q] = z.x;
+          v[2 * q + 1] = S.conj ? -z.y : z.y;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int k = g * 8 + q;
+        if (k < K) v[q] = p[(i64)k * S.sk];
+      }
+    }
+  };
+  unsigned int key = 0u;
+  for (int g = kg0; g < groups; g += kgs) {
+    load(g);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      key = max(key, ((unsigned)__double2hiint(v[q]) & 0x7fffffffu) | (__double2loint(v[q]) != 0 ? 1u : 0u));
+  }
+  atomicMax(&key_s[row], key);
+  if (gridDim.y > 1) {
+    cl.sync();
+    for (unsigned q = 0; q < cl.num_blocks(); ++q) key = max(key, *cl.map_shared_rank(&key_s[row], q));
+    cl.sync();   // no block leaves, or goes on, while another reads its maxima
+  } else {
+    __syncthreads();
+    key = key_s[row];
+  }
+  const int em = (int)(key >> 20);
+  const int e = em - 1022;
+  const bool slow = em == 0 ? key != 0u : (em == 0x7ff || e > EMAX || e < -EMAX);
+  const bool zero = em == 0 || slow;
+  if (kg0 == 0) {
+    const int ex = slow ? SLOW : (zero ? 0 : e);
+    if (S.cplx == 1) {
+      S.expo[2 * r] = ex;
+      S.expo[2 * r + 1] = ex;
+    } else {
+      S.expo[r] = ex;
+    }
+  }
+  for (int g = kg0; g < groups; g += kgs) {
+    if (groups > kgs) load(g);                       // one group per thread: still in registers
+    int top[8];
+    uint32_t jl[8], jh[8];                           // bytes of I + sum 128 256^i
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const unsigned hi = (unsigned)__double2hiint(v[q]), lo = (unsigned)__double2loint(v[q]);
+      const int eq = (int)((hi >> 20) & 0x7ff);
+      long long m = (long long)(((unsigned long long)(hi & 0xfffffu) << 32) | lo);
+      if (eq) m |= 1ll << 52;
+      const int sh = em - (eq ? eq : 1) - 2;         // I = m 2^-sh
+      long long I = 0;
+      if (!zero) I = sh <= 0 ? m << -sh : (sh < 55 ? (m + (1ll << (sh - 1))) >> sh : 0);
+      if (hi >> 31) I = -I;
+      const long long J = I + 0x0000808080808080ll;
+      jl[q] = (uint32_t)J;
+      jh[q] = (uint32_t)((unsigned long long)J >> 32);
+      top[q] = (int)(J >> 48);
+    }
+    auto emit = [&](int rr, int neg_odd, bool swap) {
+      // pairs (0,1) (2,3) (4,5) (6,7); neg_odd: the second of a pair negated
+      // (I -> -I digit by digit is again balanced: digits in [-128, 128])
+      const int rt = rr / S.R, ri = rr % S.R;
+      unsigned char* o = S.planes + ((size_t)rt * kt + (g >> 1)) * ((size_t)P * S.R * 32) +
+                         (size_t)((ri >> 3) * 256 + (g & 1) * 128 + (ri & 7) * 16);
+#pragma unroll
+      for (int pl = 0; pl < P; ++pl) {
+        uint32_t w[4];
+#pragma unroll
+        for (int h = 0; h < 4; ++h) {
+          uint32_t x;
+          if (pl == 0) x = top_pair(top[2 * h], top[2 * h + 1]);
+          else if (pl < 3) x = digit_pair(jh[2 * h], jh[2 * h + 1], pl == 1 ? 0x7651u : 0x7650u);
+          else x = digit_pair(jl[2 * h], jl[2 * h + 1], 0x7650u + (6 - pl));
+          if (swap) x = __byte_perm(x, x, 0x1032);
+          if (neg_odd) x = (x & 0x7fff0000u) ? x ^ 0x80000000u : x;
+          w[h] = x;
+        }
+        *reinterpret_cast<uint4*>(o + (size_t)pl * S.R * 32) = make_uint4(w[0], w[1], w[2], w[3]);
+      }
+    };
+    if (S.cplx == 1) {
+      emit(2 * r, 1, false);      // (re, -im): the real part's row
+      emit(2 * r + 1, 0, true);   // (im, re): the imaginary part's row
+    } else {
+      emit(r, 0, false);
+    }
+  }
+  pdl_trigger();
+}
+
+// hi 2^32 + lo as a double, times 2^sc, rounded once to nearest even; integer
+// arithmetic only (the exponent stays in the normal range by the row limits)
+__device__ __forceinline__ double to_double(long long hi, long long lo, int sc) {
+  hi += lo >> 32;
+  uint32_t l = (uint32_t)lo;
+  const bool neg = hi < 0;
+  if (neg) {
+    l = 0u - l;
+    hi = ~hi + (l == 0u ? 1 : 0);
+  }
+  const unsigned long long h = (unsigned long long)hi;
+  if ((h | l) == 0ull) return 0.0;
+  unsigned long long x;
+  int off = 0;
+  if (h < (1ull << 31)) {
+    x = (h << 32) | l;
+  } else {
+    const int lz = __clzll((long long)h);            // 0 < lz <= 32
+    x = (h << lz) | (lz == 32 ? (unsigned long long)l : (unsigned long long)(l >> (32 - lz)));
+    if (lz < 32 && (l << lz) != 0u) x |= 1ull;       // sticky
+    off = 32 - lz;
+  }
+  const int z = __clzll((long long)x);
+  x <<= z;
+  unsigned long long m = x >> 11;
+  const unsigned int r = (unsigned int)(x & 0x7ffull);
+  m += (r > 0x400u || (r == 0x400u && (m & 1ull))) ? 1ull : 0ull;
+  const long long ex = (long long)(63 - z + off + sc + 1023);
+  const unsigned long long bits = ((unsigned long long)ex << 52) + (m - (1ull << 52));
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
+// The FP64 FMA chain of one output (flagged rows): what gemm_kernel forms
+__device__ __noinline__ double fma_chain(const Args& g, int row, int n) {
+  if (!g.cplx) {
+    const double* a = g.A + at(g.am, row);
+    const double* b = g.B + at(g.bn, n);
+    double c = 0.0;
+    for (int k = 0; k < g.K; ++k) c = fma(a[(i64)k * g.ak], b[(i64)k * g.bk], c);
+    return c;
+  }
+  const double2* a = reinterpret_cast<const double2*>(g.A) + at(g.am, row >> 1);
+  const double2* b = reinterpret_cast<const double2*>(g.B) + at(g.bn, n);
+  double cx = 0.0, cy = 0.0;
+  for (int k = 0; k < g.K; ++k) {
+    double2 x = a[(i64)k * g.ak], y = b[(i64)k * g.bk];
+    if (g.conjA) x.y = -x.y;
+    if (g.conjB) y.y = -y.y;
+    cx = fma(x.x, y.x, cx);
+    cx = fma(-x.y, y.y, cx);
+    cy = fma(x.x, y.y, cy);
+    cy = fma(x.y, y.x, cy);
+  }
+  return (row & 1) ? cy : cx;
+}
+
+__device__ __forceinline__ i64 c_row(const Args& g, int row) {
+  return g.cplx ? 2 * at(g.cm, row >> 1) + (row & 1) : at(g.cm, row);
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(taddr));
+}
+
+__device__ __forceinline__ i64 c_col(const Args& g, int n) {
+  return at(g.cn, n) * (g.cplx ? 2 : 1);
+}
+// an output whose row or column is flagged, or whose sums are not there
+__device__ __noinline__ void slow_fix(const Args& g, i64 crow, int row, int n, int ea, bool bad) {
+  if (bad) g.C[crow + c_col(g, n)] = __longlong_as_double(0x7ff8000000000000ll);
+  else if (ea == SLOW || g.eb[n] == SLOW) g.C[crow + c_col(g, n)] = fma_chain(g, row, n);
+}
+
+constexpr float kCarry = 3221225472.f;   // 1.5 2^31: FP32 spacing 256
+// an integer |x| < 2^22 held in FP32, without the conversion unit
+__device__ __forceinline__ int small_int(float x) {
+  return (int)(__float_as_uint(__fadd_rn(x, 12582912.f)) - 0x4B400000u);
+}
+
+// Persistent and warp-specialised: one CTA per SM walks the tiles (mt fastest,
+// then nt, then the K split z).  Warp 0 issues the bulk copies into the ring
+// (one for A's seven planes of a K step, one for B's), warp 1 the MMAs, warps
+// 2-17 drain: warp w holds TMEM lanes 32 (w % 4).. and 16 of the 64 columns,
+// and keeps their two 64-bit sums in registers over the tile's drains.  Every
+// wait is bounded; a CTA whose wait ran out fills the outputs it has not
+// finished with NaN.  The outputs are scaled by 2^(ea + eb - 14): hi 2^-16 + lo 2^-48.
+__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
+  __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int fail_s;
+  volatile int* fail = &fail_s;
+  unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int per_z = g.mtiles * g.ntiles, total = per_z * g.nz;
+  if (tid == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(smem_u32(&full_bar[s]), 1);
+      mbar_init(smem_u32(&empty_bar[s]), 1);
+    }
+    mbar_init(smem_u32(&acc_full), 1);
+    mbar_init(smem_u32(&acc_empty), EPI_WARPS);
+    mbar_init(smem_u32(&done_bar), 1);
+    fail_s = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_slot), 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t taddr = tmem_slot;
+  pdl_wait();
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int it = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        const int rz = t % per_z, mt = rz % g.mtiles, nt = rz / g.mtiles, z = t / per_z;
+        const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
+        for (int k = k0; k < k1; ++k, ++it) {
+          const int s = it % STAGES;
+          if (it >= STAGES &&
+              !mbar_wait_f(smem_u32(&empty_bar[s]), (uint32_t)((it / STAGES - 1) & 1), fail)) {
+            ok = false;
+            break;
+          }
+          unsigned char* st = base + (size_t)s * STAGE;
+          const uint32_t bar = smem_u32(&full_bar[s]);
+          mbar_expect_tx(bar, STAGE);
+          bulk_g2s(smem_u32(st), g.Ad + ((size_t)mt * g.kt + k) * A_BYTES, A_BYTES, bar);
+          bulk_g2s(smem_u32(st + A_BYTES), g.Bd + ((size_t)nt * g.kt + k) * B_BYTES, B_BYTES, bar);
+        }
+      }
+      if (!ok) *fail = 1;
+      if (!ok || *fail) {
+        // the last fill of each stage may not have been consumed: let it land
+        for (int s = 0; s < STAGES; ++s) {
+          const int last = it - 1 - ((it - 1 - s) % STAGES + STAGES) % STAGES;
+          if (last >= 0 && last < it) mbar_wait(smem_u32(&full_bar[s]), (uint32_t)((last / STAGES) & 1));
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int it = 0, use = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
+        const int z = t / per_z, k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
+        for (int kc = k0; kc < k1 && ok; kc += KCHUNK, ++use) {
+          if (use > 0 && !mbar_wait_f(smem_u32(&acc_empty), (uint32_t)((use - 1) & 1), fail)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const int ke = min(k1, kc + KCHUNK);
+          for (int k = kc; k < ke; ++k, ++it) {
+            const int s = it % STAGES;
+            if (!mbar_wait_f(smem_u32(&full_bar[s]), (uint32_t)((it / STAGES) & 1), fail)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sa = smem_u32(base + (size_t)s * STAGE), sb = sa + A_BYTES;
+            const uint32_t acc0 = k > kc ? 1u : 0u;
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+              // planes 0..6-p of B against plane p of A: groups p..6
+              const int n = BN * (P - p), parts = n > 256 ? 2 : 1, w = n / parts;
+              const uint64_t da = make_desc(sa + p * A_PLANE, LBO, SBO);
+#pragma unroll
+              for (int h = 0; h < parts; ++h)
+                mma_bf16(taddr + (uint32_t)(p * BN + h * w), da,
+                         make_desc(sb + (uint32_t)(h * w * 32), LBO, SBO), make_idesc(BM, w),
+                         p > 0 ? 1u : acc0);
+            }
+            mma_commit(smem_u32(&empty_bar[s]));
+          }
+          if (ok) mma_commit(smem_u32(&acc_full));
+        }
+      }
+      if (!ok) *fail = 1;
+      mma_commit(smem_u32(&done_bar));
+      mbar_wait(smem_u32(&done_bar), 0);   // every MMA issued here has completed
+    }
+    __syncwarp();
+  } else {
+    const int q = warp & 3, cb = ((warp - 2) >> 2) * 16;
+    const uint32_t tb = taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
+    int use = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < total; t += gridDim.x) {
+      const int rz = t % per_z, mt = rz % g.mtiles, nt = rz / g.mtiles, z = t / per_z;
+      const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
+      long long hi[16];                              // sum = hi 2^32 + lo, in 2^-48
+      uint32_t lo[16];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) { hi[c] = 0; lo[c] = 0u; }
+      for (int kc = k0; kc < k1 && ok; kc += KCHUNK, ++use) {
+        ok = __all_sync(0xffffffffu, mbar_wait_f(smem_u32(&acc_full), (uint32_t)(use & 1), fail));
+        if (!ok) {
+          if (lane == 0) *fail = 1;
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int c0 = 0; c0 < 16; c0 += 4) {
+          uint32_t v[P][4];
+#pragma unroll
+          for (int p = 0; p < P; ++p) tmem_ld4(tb + (uint32_t)(p * BN + c0), v[p]);
+          tmem_ld_wait();
+          if (c0 == 12) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&acc_empty));
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            // carry the groups down to bytes in FP32 (every step exact): l is
+            // G less its nearest multiple of 256, which joins the group above
+            float G[P];
+#pragma unroll
+            for (int p = 0; p < P; ++p) G[p] = __uint_as_float(v[p][c]);
+#pragma unroll
+            for (int p = P - 1; p > 0; --p) {
+              const float h = __fsub_rn(__fadd_rn(G[p], kCarry), kCarry);
+              G[p] = __fsub_rn(G[p], h);
+              G[p - 1] = __fmaf_rn(h, 1.f / 256.f, G[p - 1]);
+            }
+            const int g12 = small_int(__fmaf_rn(G[1], 256.f, G[2]));
+            const int g34 = small_int(__fmaf_rn(G[3], 256.f, G[4]));
+            const int g56 = small_int(__fmaf_rn(G[5], 256.f, G[6]));
+            const long long l = (long long)lo[c0 + c] + (long long)g34 * 65536 + g56;
+            hi[c0 + c] += (long long)__float2int_rn(G[0]) * 65536 + g12 + (l >> 32);
+            lo[c0 + c] = (uint32_t)l;
+          }
+        }
+      }
+      const int row = mt * BM + q * 32 + lane, n0 = nt * BN + cb;
+      if (g.nz > 1) {
+        longlong2* o = g.part + ((size_t)z * g.ntiles * BN + n0) * ((size_t)g.mtiles * BM) + row;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          // a failed CTA's partials carry a mark the finishing kernel turns into NaN
+          o[(size_t)c * g.mtiles * BM] = ok ? make_longlong2(hi[c], (long long)lo[c]) : make_longlong2(LLONG_MIN, 0);
+        }
+      } else {
+        // lane c holds column c's exponent and offset
+        const int nl = n0 + (lane & 15);
+        const int my_eb = nl < g.N ? g.eb[nl] : 0;
+        const i64 my_col = nl < g.N ? c_col(g, nl) : 0;
+        const int ea = row < g.M ? g.ea[row] : 0;
+        const i64 cr = row < g.M ? c_row(g, row) : 0;
+        bool slow = ea == SLOW || !ok;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+          const int eb = __shfl_sync(0xffffffffu, my_eb, c);
+          const i64 col = __shfl_sync(0xffffffffu, my_col, c);
+          slow = slow || eb == SLOW;
+          if (row < g.M && n0 + c < g.N)
+            g.C[cr + col] = to_double(hi[c], (long long)lo[c], ea + eb - 62);
+        }
+        if (slow && row < g.M) {
+#pragma unroll 1
+          for (int n = n0; n < min(n0 + 16, g.N); ++n) slow_fix(g, cr, row, n, ea, !ok);
+        }
+      }
+    }
+  }
+  pdl_trigger();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 1) tmem_dealloc(taddr, 512);
+}
+
+// adds the K-split partials (exact integers) and rounds
+__global__ void __launch_bounds__(256) finish_kernel(const Args g) {
+  pdl_wait();
+  pdl_trigger();
+  const size_t Mp = (size_t)g.mtiles * BM, Np = (size_t)g.ntiles * BN;
+  const i64 total = (i64)Mp * g.N;
+  for (i64 e = blockIdx.x * (i64)blockDim.x + threadIdx.x; e < total; e += (i64)gridDim.x * blockDim.x) {
+    const int row = (int)(e % (i64)Mp), n = (int)(e / (i64)Mp);
+    if (row >= g.M) continue;
+    long long hi = 0, lo = 0;
+    bool bad = false;
+    for (int z = 0; z < g.nz; ++z) {
+      const longlong2 v = g.part[((size_t)z * Np + n) * Mp + row];
+      bad = bad || v.x == LLONG_MIN;
+      hi += v.x;
+      lo += v.y;
+    }
+    const i64 cr = c_row(g, row);
+    const int ea = g.ea[row], eb = g.eb[n];
+    if (bad || ea == SLOW || eb == SLOW) slow_fix(g, cr, row, n, ea, bad);
+    else g.C[cr + c_col(g, n)] = to_double(hi, lo, ea + eb - 62);
+  }
+}
+
+constexpr int SMS = 152;
+
+struct Shape {
+  i64 M, N, K;                  // split rows, columns, K
+  i64 mt, nt, kt;
+};
+static Shape shape(i64 M, i64 N, i64 K, bool cplx) {
+  Shape s{cplx ? 2 * M : M, N, cplx ? 2 * K : K, 0, 0, 0};
+  s.mt = (s.M + BM - 1) / BM;
+  s.nt = (s.N + BN - 1) / BN;
+  s.kt = (s.K + 15) / 16;
+  return s;
+}
+// K split: only where the tiles leave SMs idle; at least 8 K steps per chunk
+static int z_split(const Shape& s) {
+  const i64 tiles = s.mt * s.nt;
+  if (tiles * 2 > SMS) return 1;
+  return (int)std::max<i64>(1, std::min<i64>(SMS / tiles, s.kt / 8));
+}
+static inline size_t al(size_t b) { return (b + 255) & ~size_t(255); }
+
+}  // namespace oz
+
+double oz_us(i64 M, i64 N, i64 K, bool cplx) {
+  const oz::Shape s = oz::shape(M, N, K, cplx);
+  const int nz = oz::z_split(s);
+  const double waves = (double)((s.mt * s.nt * nz + oz::SMS - 1) / oz::SMS);
+  const double ks = (double)((s.kt + nz - 1) / nz);
+  const double mma = waves * (ks * 950.0 + (ks / oz::KCHUNK + 1) * 2500.0 + 3000.0) / 1900.0;
+  const double split = ((double)s.M + s.N) * s.K * 22.0 / 4.0e6;
+  return mma + split + 12.0 + (nz > 1 ? 4.0 : 0.0);
+}
+
+size_t oz_bytes(i64 M, i64 N, i64 K, bool cplx) {
+  if ((cplx ? 4.0 : 1.0) * (double)M * (double)N * (double)K < kOzMinMNK) return 0;
+  const oz::Shape s = oz::shape(M, N, K, cplx);
+  // rows of both operands padded to the larger tile: either may become A
+  const double rows = 128.0 * (double)((s.M + 127) / 128 + (s.N * (cplx ? 2 : 1) + 127) / 128);
+  const double need = 14.0 * 16.0 * (double)s.kt * rows + 4.0 * rows +
+                      (double)oz::SMS * oz::BM * oz::BN * 16.0 + 4096.0;
+  return need > (double)kOzMaxBytes ? kOzMaxBytes : (size_t)need;
+}
+
+bool oz_fits(i64 M, i64 N, i64 K, bool cplx) {
+  const size_t b = oz_bytes(M, N, K, cplx);
+  return b > 0 && b < kOzMaxBytes;
+}
+
+void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
+  using namespace oz;
+  const Shape s = shape(g.M, g.N, g.K, g.cplx);
+  TTG_REQUIRE(s.M < (1ll << 31) - BM && s.N < (1ll << 31) - BN && s.K < (1ll << 30), "oz: size");
+  char* p = (char*)ws;
+  auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
+  const size_t ra = (size_t)s.mt * BM, rb = (size_t)s.nt * BN;
+  unsigned char* Ad = (unsigned char*)take(14 * 16 * (size_t)s.kt * ra);
+  unsigned char* Bd = (unsigned char*)take(14 * 16 * (size_t)s.kt * rb);
+  int* ea = (int*)take(4 * ra);
+  int* eb = (int*)take(4 * rb);
+  const int nz0 = z_split(s);
+  const int kper = (int)((s.kt + nz0 - 1) / nz0), nz = (int)((s.kt + kper - 1) / kper);
+  longlong2* part = nz > 1 ? (longlong2*)take(sizeof(longlong2) * nz * ra * rb) : nullptr;
+  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, g.cplx ? 1 : 0, g.conjA};
+  const Side b{g.B, g.bn, g.bk, g.N, BN, (int)s.nt, Bd, eb, g.cplx ? 2 : 0, g.conjB};
+  const int nA = (int)(ra / (g.cplx ? 2 : 1) / SROWS), nB = (int)(rb / SROWS);
+  // few rows and a long K: K over a cluster (246 + 82 rows, K = 4928: 50 -> 17 us)
+  int ky = 1;
+  while (ky < kMaxCluster && (nA + nB) * ky < 2 * SMS && 2 * s.kt > 32 * ky) ky *= 2;
+  launch_ex(split_kernel, dim3(nA + nB, ky), dim3(256), dim3(ky > 1 ? 1 : 0, ky, 1), true, 0, st, a, b,
+            nA, g.K, (int)s.kt);
+  Args x{};
+  x.Ad = Ad; x.Bd = Bd; x.ea = ea; x.eb = eb;
+  x.M = (int)s.M; x.N = (int)s.N; x.K = g.K;
+  x.kt = (int)s.kt; x.kper = kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.nz = nz;
+  x.C = g.C; x.cm = g.cm; x.cn = g.cn; x.part = part;
+  x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
+  x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
+  static const cudaError_t attr_rc =
+      cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+  TTG_CUDA(attr_rc);
+  const int grid = (int)std::min<i64>(SMS, s.mt * s.nt * nz);
+  launch_pdl(gemm_kernel, dim3(grid), dim3(THREADS), SMEM, st, x);
+  if (nz > 1) {
+    const int fb = (int)std::min<i64>(1024, ((i64)ra * s.N + 255) / 256);
+    launch_pdl(finish_kernel, dim3(fb), dim3(256), 0, st, x);
+  }
+}
+
+// A strided batched product as one split product: a batch over which one
+// operand does not move joins the rows (or columns) of the other.  The side
+// that C stores contiguously becomes the MMA's M (a warp's TMEM lanes).
+// Returns false, with nothing launched, when the product does not have that
+// form, does not fit the workspace rule, or the FP64 kernel is the faster.
+template <class G>
+static bool oz_try_impl(const G& g, bool cplx, bool conjA, bool conjB, bool plain, void* ws,
+                        cudaStream_t s) {
+  if (!ws || !plain || g.M <= 0 || g.N <= 0 || g.K <= 0) return false;
+  i64 nb = (i64)g.nb1 * g.nb2, bA = g.bA1, bB = g.bB1, bC = g.bC1;
+  if (g.nb1 == 1) {
+    bA = g.bA2; bB = g.bB2; bC = g.bC2;
+  } else if (g.nb2 > 1 && (g.bA2 != g.nb1 * g.bA1 || g.bB2 != g.nb1 * g.bB1 || g.bC2 != g.nb1 * g.bC1)) {
+    return false;
+  }
+  i64 M = g.M, N = g.N;
+  OzMap am{g.M, g.sAm, 0}, cm{g.M, g.sCm, 0}, bn{g.N, g.sBn, 0}, cn{g.N, g.sCn, 0};
+  if (nb > 1) {
+    if (bB == 0) { am.s2 = bA; cm.s2 = bC; M *= nb; }
+    else if (bA == 0) { bn.s2 = bB; cn.s2 = bC; N *= nb; }
+    else return false;
+  }
+  const bool swap = g.sCm != 1;
+  if (swap && g.sCn != 1) return false;
+  if (M >= (1ll << 29) || N >= (1ll << 29)) return false;
+  const i64 Mo = swap ? N : M, No = swap ? M : N;
+  if (!oz_fits(Mo, No, g.K, cplx)) return false;
+  const double fp64 = (cplx ? 8.0 : 2.0) * (double)M * (double)N * g.K / 1.0e6 + 4.0;   // us
+  if (oz_us(Mo, No, g.K, cplx) >= fp64) return false;
+  OzGemm o;
+  o.M = (int)Mo; o.N = (int)No; o.K = g.K; o.cplx = cplx;
+  o.A = (const double*)(swap ? g.B : g.A); o.am = swap ? bn : am; o.ak = swap ? g.sBk : g.sAk;
+  o.B = (const double*)(swap ? g.A : g.B); o.bn = swap ? am : bn; o.bk = swap ? g.sAk : g.sBk;
+  o.C = (double*)g.C; o.cm = swap ? cn : cm; o.cn = swap ? cm : cn;
+  o.conjA = swap ? conjB : conjA; o.conjB = swap ? conjA : conjB;
+  oz_gemm(o, ws, s);
+  return true;
+}
+bool oz_try(const GemmF64& g, void* ws, cudaStream_t s) {
+  return oz_try_impl(g, false, false, false, g.alpha == 1.0 && g.beta == 0.0, ws, s);
+}
+bool oz_try(const GemmZ& g, void* ws, cudaStream_t s) {
+  const bool plain = g.alpha.x == 1.0 && g.alpha.y == 0.0 && g.beta.x == 0.0 && g.beta.y == 0.0;
+  return oz_try_impl(g, true, g.conjA, g.conjB, plain, ws, s);
+}
+
+}  // namespace ttg
