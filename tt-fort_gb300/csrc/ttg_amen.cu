@@ -362,6 +362,7 @@ class AmenSolver {
   DevTT x_, y_, z_;
   std::vector<double*> A_;
   std::vector<double*> pxax_, pxy_, pzax_, pzy_;
+  size_t tau_n_ = 0;   // elements of tau_
   double *tmpA_, *tmpB_, *tmpC_, *R_, *tau_, *rhs_, *resid_, *sol_, *xnew_, *scr_, *svU_, *svS_,
       *svVt_, *svScr_, *cand_, *candY_, *red_, *V_, *w_, *gm_, *dense_;
   double* h_ = nullptr;   // pinned
@@ -415,7 +416,7 @@ void AmenSolver::qr(DevTT& t, int k, int dir) {
     const i64 m = r[k] * n[k], rr = r[k + 1], p = n[k + 1] * r[k + 2];
     if (m >= rr) {
       TTG_CUDA(cudaMemcpyAsync(tmpA_, t.c[k], sizeof(double) * m * rr, cudaMemcpyDeviceToDevice, s_));
-      qr_householder((int)m, (int)rr, tmpA_, R_, tau_, s_);
+      qr_householder((int)m, (int)rr, tmpA_, R_, tau_, tau_n_, s_);
       TTG_CUDA(cudaMemcpyAsync(t.c[k], tmpA_, sizeof(double) * m * rr, cudaMemcpyDeviceToDevice, s_));
       gemm((int)rr, (int)p, (int)rr, R_, 1, rr, t.c[k + 1], 1, rr, tmpB_, 1, rr);
       TTG_CUDA(cudaMemcpyAsync(t.c[k + 1], tmpB_, sizeof(double) * rr * p, cudaMemcpyDeviceToDevice, s_));
@@ -431,7 +432,7 @@ void AmenSolver::qr(DevTT& t, int k, int dir) {
     const i64 m = n[k] * r[k + 1], rr = r[k], p = r[k - 1] * n[k - 1];
     transpose_f64(rr, m, t.c[k], tmpA_, s_);    // m x rr
     if (m >= rr) {
-      qr_householder((int)m, (int)rr, tmpA_, R_, tau_, s_);
+      qr_householder((int)m, (int)rr, tmpA_, R_, tau_, tau_n_, s_);
       transpose_f64(m, rr, tmpA_, t.c[k], s_);   // rr x m
       // core_{k-1} (p x rr) R^T
       gemm((int)p, (int)rr, (int)rr, t.c[k - 1], 1, p, R_, rr, 1, tmpB_, 1, p);
@@ -629,7 +630,11 @@ void AmenSolver::run(AmenOut& out) {
   for (int k = 0; k <= d; ++k)
     total += al8(x_.cap[k] * x_.cap[k] * P_.ra[k]) + al8(x_.cap[k] * P_.ry[k]) +
              al8(z_.r[k] * x_.cap[k] * P_.ra[k]) + al8(z_.r[k] * P_.ry[k]);
-  total += 2 * al8(cmax) + al8(tcap) + al8(Nmax) * 5 + al8(cmax) + al8(8192) + scr + 256;
+  {
+    const i64 rcap = *std::max_element(x_.cap.begin(), x_.cap.end());   // widest QR
+    tau_n_ = std::max<size_t>(8192, qr_work_elems(rcap, rcap));
+  }
+  total += 2 * al8(cmax) + al8(tcap) + al8(Nmax) * 5 + al8(cmax) + al8(tau_n_) + scr + 256;
   total += svds + 256 + 3 * al8(cmax) + al8(8192);
   total += 2 * al8(Nmax * kBatch) + al8(Nmax * (nr + 1)) + al8(Nmax) + al8(4096) +
            al8((size_t)std::min<i64>(P_.max_full_size, 64) * 64) + (1 << 16);
@@ -666,7 +671,7 @@ void AmenSolver::run(AmenOut& out) {
   rhs_ = mem_.take(Nmax); resid_ = mem_.take(Nmax); sol_ = mem_.take(Nmax); xnew_ = mem_.take(Nmax);
   w_ = mem_.take(Nmax);
   R_ = mem_.take(cmax);
-  tau_ = mem_.take(8192);
+  tau_ = mem_.take(tau_n_);
   scr_ = (double*)mem_.take(scr / sizeof(double) + 1);
   svScr_ = (double*)mem_.take(svds / sizeof(double) + 1);
   svU_ = mem_.take(cmax); svS_ = mem_.take(8192); svVt_ = mem_.take(cmax);
@@ -960,7 +965,7 @@ static int uchol_run(bool trans, i64 m, i64 n, const double* dA, int numvec, dou
     uchol_scale_kernel<<<eb(n), 256, 0, s>>>(n, cnt, piv, du, W.dd);
     TTG_CHECK_LAUNCH();
     const int k = cnt + 1;
-    qr_householder((int)n, k, du, Rk, W.tau, s);          // du[:, :k] = Q, Rk = R
+    qr_householder((int)n, k, du, Rk, W.tau, 16, s);          // du[:, :k] = Q, Rk = R
     uchol_dv_kernel<<<1, 256, 0, s>>>(k, Rk, lam, dv);
     TTG_CHECK_LAUNCH();
     syev_jacobi(k, dv, k, lam, V, k, W.ired + 8, s);      // ascending, as dsyev
@@ -1042,6 +1047,7 @@ class AlsSolver {
   ttg_ctx* ctx_;
   Arena mem_;
   std::vector<i64> n_, rx_, cap_;
+  size_t tau_n_ = 0;   // elements of tau_
   std::vector<double*> x_, A_, Y_, phiA_, phiy_;
   double *rhs_, *r0_, *sol_, *w_, *V_, *gm_, *red_, *kickY_, *kickB_, *tA_, *tB_, *tC_, *U_, *S_,
       *Vt_, *svScr_, *cand_, *candY_, *Um_, *Rm_, *Rq_, *tau_, *tmp_, *scr_, *du_, *dd_, *small_;
@@ -1075,7 +1081,7 @@ class AlsSolver {
     bfun3_f64(dims(k), phiA_[k], A_[k], phiA_[k + 1], x, y, nv, scr_, s_);
     nmv_ += nv;
   }
-  void qr(i64 m, i64 c, double* A, double* R) { qr_householder((int)m, (int)c, A, R, tau_, s_); }
+  void qr(i64 m, i64 c, double* A, double* R) { qr_householder((int)m, (int)c, A, R, tau_, tau_n_, s_); }
   void upd_left(int i);
   void upd_right(int i);
   int scan(int i, int rmin, const double* L, i64 ldl, const double* Rr, i64 ldr, i64 rows, i64 cols,
@@ -1201,12 +1207,16 @@ void AlsSolver::run(AmenOut& out) {
     yt += ry[k] * n_[k] * ry[k + 1];
   }
   const i64 M2 = Mmax * std::max<i64>(Mmax, 1);
+  {
+    const i64 rcap = *std::max_element(cap_.begin(), cap_.end()) + 16;
+    tau_n_ = std::max<size_t>(8192, qr_work_elems(rcap, rcap));
+  }
   size_t total = al8(at) + al8(yt);
   for (int k = 0; k < d; ++k) total += al8(cap_[k] * n_[k] * cap_[k + 1]);
   for (int k = 0; k <= d; ++k) total += al8(cap_[k] * cap_[k] * ra[k]) + al8(cap_[k] * ry[k]);
   total += 4 * al8(Nmax) + al8(Nmax * (nr + 1)) + al8(4096) + al8(64) + al8(Cmax) + al8(KB) +
            3 * al8(T) + al8(SVD) + al8(1024) + al8(SVD) + svs + 256 + 2 * al8(Nmax * kBatch) +
-           al8(M2) + 2 * al8(M2) + al8(8192) + al8(M2) + scr + 256 + al8(Mmax * 16) +
+           al8(M2) + 2 * al8(M2) + al8(tau_n_) + al8(M2) + scr + 256 + al8(Mmax * 16) +
            al8(Mmax) + al8(1024) + al8(64) + (1 << 16);
   mem_.alloc(total);
   double* dA = mem_.take(at);
@@ -1236,7 +1246,7 @@ void AlsSolver::run(AmenOut& out) {
   svScr_ = (double*)mem_.take(svs / sizeof(double) + 1);
   cand_ = mem_.take(Nmax * kBatch); candY_ = mem_.take(Nmax * kBatch);
   Um_ = mem_.take(M2); Rm_ = mem_.take(M2); Rq_ = mem_.take(M2);
-  tau_ = mem_.take(8192);
+  tau_ = mem_.take(tau_n_);
   tmp_ = mem_.take(M2);
   scr_ = (double*)mem_.take(scr / sizeof(double) + 1);
   du_ = mem_.take(Mmax * 16);
@@ -1482,6 +1492,7 @@ class MvkSolver {
   Arena mem_;
   std::vector<i64> ry_, cap_;
   std::vector<double*> y_, A_, X_, phi_;
+  size_t tau_n_ = 0;   // elements of tau_
   double *cur_, *diff_, *red_, *U_, *S_, *Vt_, *svScr_, *Um_, *Rm_, *Rq_, *tmp_, *full_, *tA_,
       *tB_, *scr_, *du_, *dd_, *small_, *tau_;
   int* ired_;
@@ -1553,6 +1564,7 @@ void MvkSolver::run(AmenOut& out) {
   for (int k = 0; k <= d; ++k) PH = std::max(PH, cap_[k] * rx[k] * ra[k]);
   const i64 M2 = std::max(Nmax, Mmax * (cmax + kpad));
   const i64 R2 = (cmax + kpad) * (cmax + kpad);
+  tau_n_ = std::max<size_t>(8192, qr_work_elems(cmax + kpad, cmax + kpad));
   i64 at = 0, xt = 0;
   for (int k = 0; k < d; ++k) {
     at += ra[k] * n[k] * m[k] * ra[k + 1];
@@ -1563,7 +1575,7 @@ void MvkSolver::run(AmenOut& out) {
   for (int k = 0; k <= d; ++k) total += al8(std::max<i64>(1, cap_[k] * rx[k] * ra[k]));
   total += 2 * al8(Nmax) + al8(64) + 2 * al8(SVDU) + al8(4096) + svs + 256 + al8(M2) +
            2 * al8(R2) + al8(M2) + al8(FB) + 2 * al8(T) + scr + 256 + al8(Mmax * 16) +
-           al8(Mmax) + al8(1024) + al8(8192) + al8(64) + (1 << 16);
+           al8(Mmax) + al8(1024) + al8(tau_n_) + al8(64) + (1 << 16);
   mem_.alloc(total);
   double* dA = mem_.take(at);
   double* dX = mem_.take(xt);
@@ -1585,7 +1597,7 @@ void MvkSolver::run(AmenOut& out) {
   full_ = mem_.take(FB); tA_ = mem_.take(T); tB_ = mem_.take(T);
   scr_ = (double*)mem_.take(scr / sizeof(double) + 1);
   du_ = mem_.take(Mmax * 16); dd_ = mem_.take(Mmax); small_ = mem_.take(1024);
-  tau_ = mem_.take(8192);
+  tau_ = mem_.take(tau_n_);
   ired_ = (int*)mem_.take(64);
   TTG_CUDA(cudaMallocHost(&h_, 4096 * sizeof(double)));
   struct HG { double* p; ~HG() { if (p) cudaFreeHost(p); } } hg{h_};
@@ -1611,7 +1623,7 @@ void MvkSolver::run(AmenOut& out) {
     const i64 m_ = ry_[i] * n[i], rr = ry_[i + 1], p = n[i + 1] * ry_[i + 2];
     const i64 rnew = std::min(m_, rr);
     TTG_CUDA(cudaMemcpyAsync(Um_, y_[i], sizeof(double) * m_ * rr, cudaMemcpyDeviceToDevice, s_));
-    qr_householder((int)m_, (int)rr, Um_, Rq_, tau_, s_);
+    qr_householder((int)m_, (int)rr, Um_, Rq_, tau_, tau_n_, s_);
     TTG_CUDA(cudaMemcpyAsync(y_[i], Um_, sizeof(double) * m_ * rnew, cudaMemcpyDeviceToDevice, s_));
     gemm((int)rnew, (int)p, (int)rr, Rq_, 1, rnew, y_[i + 1], 1, rr, tmp_, 1, rnew);
     TTG_CUDA(cudaMemcpyAsync(y_[i + 1], tmp_, sizeof(double) * rnew * p, cudaMemcpyDeviceToDevice, s_));
@@ -1646,7 +1658,7 @@ void MvkSolver::run(AmenOut& out) {
         rnew = nn;
       } else {
         TTG_CUDA(cudaMemcpyAsync(Um_, cur_, sizeof(double) * m_ * rr, cudaMemcpyDeviceToDevice, s_));
-        qr_householder((int)m_, (int)rr, Um_, Rm_, tau_, s_);
+        qr_householder((int)m_, (int)rr, Um_, Rm_, tau_, tau_n_, s_);
       }
       TTG_REQUIRE(rnew <= cap_[i + 1], "tt_mvk4: rank capacity exceeded");
       TTG_CUDA(cudaMemcpyAsync(y_[i], Um_, sizeof(double) * m_ * rnew, cudaMemcpyDeviceToDevice, s_));
@@ -1678,11 +1690,11 @@ void MvkSolver::run(AmenOut& out) {
         pad_rows_kernel<<<eb((nn + mm) * rl), 256, 0, s_>>>(nn, mm, rl, Rm_, tmp_);
         TTG_CHECK_LAUNCH();
         rnew = std::min<i64>(m_, nn + mm);
-        qr_householder((int)m_, nn + mm, Um_, Rq_, tau_, s_);
+        qr_householder((int)m_, nn + mm, Um_, Rq_, tau_, tau_n_, s_);
         gemm((int)rnew, (int)rl, nn + mm, Rq_, 1, rnew, tmp_, 1, nn + mm, Rm_, 1, rnew);
       } else {
         transpose_f64(rl, m_, cur_, Um_, s_);                            // m_ x rl
-        qr_householder((int)m_, (int)rl, Um_, Rm_, tau_, s_);
+        qr_householder((int)m_, (int)rl, Um_, Rm_, tau_, tau_n_, s_);
       }
       TTG_REQUIRE(rnew <= cap_[i], "tt_mvk4: rank capacity exceeded");
       transpose_f64(m_, rnew, Um_, y_[i], s_);                           // rnew x m_

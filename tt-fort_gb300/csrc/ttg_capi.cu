@@ -272,9 +272,10 @@ int ttg_dqr(ttg_ctx* c, ttg_int n, ttg_int m, double* A, double* R) {
   TTG_REQUIRE(n > 0 && m > 0 && A && R, "bad arguments");
   TTG_REQUIRE(n < (1ll << 31) && m < (1ll << 31), "size too large");
   c->ws.reset();
-  c->ws.reserve(sizeof(double) * std::min(n, m));
-  double* tau = c->ws.takeT<double>(std::min(n, m));
-  qr_householder((int)n, (int)m, A, R, tau, c->stream);
+  const size_t work = qr_work_elems(n, m);
+  c->ws.reserve(sizeof(double) * work);
+  double* tau = c->ws.takeT<double>(work);
+  qr_householder((int)n, (int)m, A, R, tau, work, c->stream);
   TTG_API_END(c)
 }
 
@@ -283,9 +284,10 @@ int ttg_zqr(ttg_ctx* c, ttg_int n, ttg_int m, double* A, double* R) {
   TTG_REQUIRE(n > 0 && m > 0 && A && R, "bad arguments");
   TTG_REQUIRE(n < (1ll << 31) && m < (1ll << 31), "size too large");
   c->ws.reset();
-  c->ws.reserve(sizeof(double2) * std::min(n, m));
-  double2* tau = c->ws.takeT<double2>(std::min(n, m));
-  qr_householder_z((int)n, (int)m, (double2*)A, (double2*)R, tau, c->stream);
+  const size_t work = qr_work_elems(n, m);
+  c->ws.reserve(sizeof(double2) * work);
+  double2* tau = c->ws.takeT<double2>(work);
+  qr_householder_z((int)n, (int)m, (double2*)A, (double2*)R, tau, work, c->stream);
   TTG_API_END(c)
 }
 

@@ -394,8 +394,15 @@ void syev_lowest_svd(int N, int k, double* H, double* w, double* V, double* scra
 void svd_jacobi(int p, int q, const double* M, double* U, double* sigma, double* Vt,
                 double* scratch, int* status, cudaStream_t s);
 // Householder QR with LAPACK's convention: A (n x m) -> Q (n x min), R (min x m).
-void qr_householder(int n, int m, double* A, double* R, double* tau, cudaStream_t s);
-void qr_householder_z(int n, int m, double2* A, double2* R, double2* tau, cudaStream_t s);
+// tau: work elements, at least min(n, m); with qr_work_elems(n, m) of them large
+// blocks run over the whole GPU (ttg_qr.cu)
+size_t qr_work_elems(i64 n, i64 m);
+void qr_householder(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s);
+void qr_householder_z(int n, int m, double2* A, double2* R, double2* tau, size_t work,
+                      cudaStream_t s);
+// ttg_qr.cu: false (nothing launched) when the block does not fit shared memory
+bool qr_rows(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s);
+bool qr_rows(int n, int m, double2* A, double2* R, double2* tau, size_t work, cudaStream_t s);
 
 // small helpers
 void transpose_f64(i64 rows, i64 cols, const double* in, double* out, cudaStream_t s);

@@ -225,7 +225,7 @@ static void run_eigb(ttg_ctx* ctx, EigbParams P, EigbOutput& out) {
   for (int i = 0; i < d; ++i) {
     i64 rows = ry[i] * n[i];
     i64 rnew = std::min(rows, ry[i + 1]);
-    qr_householder((int)rows, (int)ry[i + 1], cr[i], tmp, tmp2, s);
+    qr_householder((int)rows, (int)ry[i + 1], cr[i], tmp, tmp2, (size_t)capmax, s);
     if (i < d - 1) {
       GemmF64 g;   // cr[i+1] = R (rnew x ry[i+1]) * cr[i+1] (ry[i+1] x n ry[i+2])
       g.M = (int)rnew; g.N = (int)(n[i + 1] * ry[i + 2]); g.K = (int)ry[i + 1];

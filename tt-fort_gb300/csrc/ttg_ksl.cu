@@ -223,7 +223,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
   for (int i = 0; i < d; ++i) total += alz(sizeof(double2) * Rc[i] * n[i] * Rc[i + 1]);
   for (int i = 0; i <= d; ++i) total += alz(sizeof(double2) * std::max<i64>(1, Rc[i] * Rc[i] * P.ra[i]));
   total += 5 * alz(sizeof(double2) * capmax) + alz(sizeof(double2) * phimax) +
-           2 * alz(sizeof(double2) * rmx * rmx) + alz(sizeof(double2) * rmx * 2) +
+           2 * alz(sizeof(double2) * rmx * rmx) + alz(sizeof(double2) * qr_work_elems(rmx, rmx)) +
            alz(sizeof(double2) * scr) + alz(ExpWork::bytes(Nmax, P.order)) + (1 << 16);
   // chosen form: realified local operator (doubled ranks) on the tensor cores
   const bool split = P.method == TTG_METHOD_SPLIT;
@@ -270,7 +270,8 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
   double2* phitmp = mem.take<double2>(phimax);
   double2* R = mem.take<double2>(rmx * rmx);
   double2* Rt = mem.take<double2>(rmx * rmx);
-  double2* tau_ws = mem.take<double2>(rmx * 2);
+  const size_t tau_n = qr_work_elems(rmx, rmx);
+  double2* tau_ws = mem.take<double2>(tau_n);
   double2* scratch = mem.take<double2>(scr);
   void* expmem = mem.take<char>(ExpWork::bytes(Nmax, P.order));
   double *rphi1[2] = {}, *rphi2[2] = {}, *rA[2] = {}, *rx = nullptr, *ryv = nullptr;
@@ -332,7 +333,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
     for (int i = 0; i + 1 < d; ++i) {
       const i64 rows = ry[i] * n[i];
       const i64 rnew = std::min(rows, ry[i + 1]);
-      qr_householder_z((int)rows, (int)ry[i + 1], cr[i], R, tau_ws, s);
+      qr_householder_z((int)rows, (int)ry[i + 1], cr[i], R, tau_ws, tau_n, s);
       GemmZ g;
       g.M = (int)rnew; g.N = (int)(n[i + 1] * ry[i + 2]); g.K = (int)ry[i + 1];
       g.A = R; g.sAm = 1; g.sAk = rnew;
@@ -429,7 +430,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
       // QR of X (ry_i n_i x ry_{i+1}) in place, S-step of R, out = Q S
       auto left_s = [&](int i, double2* X, double2* out) {
         const i64 rows = ry[i] * n[i], r2 = ry[i + 1];
-        qr_householder_z((int)rows, (int)r2, X, R, tau_ws, s);
+        qr_householder_z((int)rows, (int)r2, X, R, tau_ws, tau_n, s);
         phi_left_z(Ld(i), phi[i], A_of(i), X, X, phitmp, scratch, s);
         sstep(r2, r2, P.ra[i + 1], r2, r2, phitmp, phi[i + 1], R);
         GemmZ g;
@@ -454,7 +455,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
         if (i > 0) {
           const i64 cols = n[i] * ry[i + 1], r1 = ry[i];
           transpose_z(r1, cols, cur, t1, s);               // cols x r1
-          qr_householder_z((int)cols, (int)r1, t1, R, tau_ws, s);
+          qr_householder_z((int)cols, (int)r1, t1, R, tau_ws, tau_n, s);
           transpose_z(cols, r1, t1, cr[i], s);             // Q^T: r1 x cols
           transpose_z(r1, r1, R, Rt, s);
           GemmZ g;   // core_{i-1} = core_{i-1} R^T
@@ -477,7 +478,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
         kstep(i);                                          // curcr
         if (i < d - 1) {
           const i64 rows = ry[i] * n[i], r2 = ry[i + 1];
-          qr_householder_z((int)rows, (int)r2, curcr, R, tau_ws, s);
+          qr_householder_z((int)rows, (int)r2, curcr, R, tau_ws, tau_n, s);
           copy(cr[i], curcr, rows * r2);
           GemmZ g;   // core_{i+1} = R core_{i+1}
           g.M = (int)r2; g.N = (int)(n[i + 1] * ry[i + 2]); g.K = (int)r2;
@@ -503,7 +504,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
           const i64 rnew = std::min(cols, ry[i]);
           TTG_REQUIRE(rnew == ry[i], "ztt_ksl: the S-step needs a rank-preserving QR");
           transpose_z(ry[i], cols, curcr, t1, s);                    // cols x ry_i
-          qr_householder_z((int)cols, (int)ry[i], t1, R, tau_ws, s); // Q: cols x rnew
+          qr_householder_z((int)cols, (int)ry[i], t1, R, tau_ws, tau_n, s); // Q: cols x rnew
           transpose_z(cols, rnew, t1, cr[i], s);                     // rnew x cols
           transpose_z(rnew, ry[i], R, Rt, s);                        // ry_i x rnew
           LocalDims Lr{rnew, n[i], ry[i + 1], rnew, n[i], ry[i + 1], P.ra[i], P.ra[i + 1]};
@@ -529,7 +530,7 @@ static void run_ksl(ttg_ctx* ctx, KslParams P, std::vector<std::complex<double>>
           const i64 rows = ry[i] * n[i];
           const i64 rnew = std::min(rows, ry[i + 1]);
           TTG_REQUIRE(rnew == ry[i + 1], "ztt_ksl: the S-step needs a rank-preserving QR");
-          qr_householder_z((int)rows, (int)ry[i + 1], curcr, R, tau_ws, s);
+          qr_householder_z((int)rows, (int)ry[i + 1], curcr, R, tau_ws, tau_n, s);
           TTG_CUDA(cudaMemcpyAsync(cr[i], curcr, sizeof(double2) * rows * rnew,
                                    cudaMemcpyDeviceToDevice, s));
           LocalDims Ll{ry[i], n[i], rnew, ry[i], n[i], rnew, P.ra[i], P.ra[i + 1]};

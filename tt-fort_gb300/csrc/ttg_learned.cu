@@ -490,7 +490,7 @@ void learned_record(ttg_ctx* ctx, const LocalDims& L, const double* phi1, const 
   double* scr = Cc + (size_t)B * B;
   int* st = (int*)(scr + svs);
   TTG_CUDA(cudaMemcpyAsync(V, X0, nb * sizeof(double), cudaMemcpyDeviceToDevice, s));
-  qr_householder((int)N, B, V, Rq, tau, s);
+  qr_householder((int)N, B, V, Rq, tau, (size_t)B * B, s);
   mv(V, W, B);
   gemm_tn_small(B, B, N, V, N, W, N, H, B, 1.0, 0.0, s);
   syev_jacobi(B, H, B, th, S, B, st, s);
