@@ -403,6 +403,8 @@ void qr_householder_z(int n, int m, double2* A, double2* R, double2* tau, size_t
 // ttg_qr.cu: false (nothing launched) when the block does not fit shared memory
 bool qr_rows(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s);
 bool qr_rows(int n, int m, double2* A, double2* R, double2* tau, size_t work, cudaStream_t s);
+// the same without Q: R on and above the diagonal of A, reflectors below it
+bool qr_rows_factor(int n, int m, double* A, double* tau, size_t work, cudaStream_t s);
 
 // small helpers
 void transpose_f64(i64 rows, i64 cols, const double* in, double* out, cudaStream_t s);

@@ -6,9 +6,9 @@
 //                 Cyclic Jacobi, round-robin parallel ordering, one CTA.
 //   svd_jacobi    truncation SVD (dgesvd, tt_eigb.f90:312,361;
 //                 ttnodeop.f90:254).  One-sided (Hestenes) Jacobi on the
-//                 columns, one warp per column pair, all pairs of a round in
-//                 parallel, rounds separated by a grid-wide barrier of one
-//                 cooperative launch.  High relative accuracy of the small
+//                 columns of the twice QR-preconditioned block, disjoint column
+//                 blocks of a round in parallel, rounds separated by a grid-wide
+//                 barrier of one cooperative launch.  High relative accuracy of the small
 //                 singular values, which my_chop3 sums.
 //   qr_householder  dgeqrf+dorgqr (dqr, matrix_util.f90:37-61) and
 //                 zgeqrf+zungqr (zqr, :64-90; ttg_qr.cu) with LAPACK's reflector
@@ -324,13 +324,7 @@ void syev_jacobi(int k, double* A, int lda, double* w, double* V, int ldv, int* 
 // ---------------------------------------------------------------------------
 // one-sided Jacobi SVD (cooperative launch, grid barrier between rounds)
 // ---------------------------------------------------------------------------
-#ifndef TTG_SVD_CT
-#define TTG_SVD_CT 128
-#endif
-// one CTA per column pair; its warps share the rows (measured on GB300, 128
-// threads: 7.6 ms at 320x128 and 54 ms at 2048x512; 64: 8.3 and 60; 32: 9.2
-// and 81)
-constexpr int SVD_CT = TTG_SVD_CT;
+constexpr int SVD_CT = 128;   // FP32 sweeps: one CTA per column pair
 constexpr int SVD_MAX_SWEEPS = 60;
 
 template <class T>
@@ -340,26 +334,401 @@ __device__ __forceinline__ T warp_sum_t(T v) {
   return v;
 }
 
-// One-sided Jacobi sweeps over the column pairs of M (p x q), rotations
+// The rotation that makes two columns with squared norms A, B and product G
+// orthogonal, as three shears: with p = tan(theta / 2) and s = sin(theta) =
+// 2 p / (1 + p^2),
+//   x <- x - p y,  y <- y + s x,  x <- x - p y
+// is x <- c x - s y, y <- s x + c y: three FMAs per element in place of two
+// products and two FMAs.  p comes from FP32 arithmetic on the leading bits (an
+// angle off by FP32 rounding leaves ~1e-7 of G for the next sweep); s is formed
+// from that p in FP64, so the rotation is orthogonal to FP64 precision whatever
+// p is: 1/(1 + p^2) by one third-order step from the FP32 quotient.  Exponents
+// are moved as integers, so no FP32 range is passed, and FP32 values become
+// FP64 ones by their bits.  A dependent FP64 operation takes about 100 clocks
+// here, and this is the serial part of every round: six of them, against about
+// forty with FP64 quotients, square roots and tests.
+__device__ __forceinline__ float lead24(double v) {   // mantissa of v in [1, 2), truncated
+  return __uint_as_float(0x3f800000u | (((unsigned)__double2hiint(v) & 0xfffffu) << 3) |
+                         ((unsigned)__double2loint(v) >> 29));
+}
+__device__ __forceinline__ int exp_bits(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+__device__ __forceinline__ double widen(float f, int e, unsigned sign) {   // f 2^e, f > 0 normal
+  const unsigned b = __float_as_uint(f);
+  const int he = (int)(b >> 23) + 896 + e;
+  return __hiloint2double((int)(((unsigned)he << 20) | ((b & 0x7fffffu) >> 3) | sign), (int)(b << 29));
+}
+__device__ __forceinline__ void jacobi_shears(double A, double Bv, double G, double& p, double& s) {
+  const double d = Bv - A;
+  const int k = exp_bits(d) - exp_bits(G) - 1;        // zeta = d / (2 G) = +-(fd / fg) 2^k
+  const float fd = lead24(d), fg = lead24(G);
+  const unsigned sg = ((unsigned)__double2hiint(d) ^ (unsigned)__double2hiint(G)) & 0x80000000u;
+  float pf = 0.41421356f;                             // |p| = pf 2^pe; here tan(pi / 8)
+  int pe = 0;
+  if (k > 30) {
+    pf = __fdividef(fg, fd);                          // 1 / (4 zeta)
+    pe = -k - 2;
+  } else if (d != 0.0 && k >= -60) {
+    const float z = __fdividef(fd, fg) * __uint_as_float((unsigned)(127 + k) << 23);
+    const float t = __fdividef(1.f, z + sqrtf(fmaf(z, z, 1.f)));
+    pf = __fdividef(t, 1.f + sqrtf(fmaf(t, t, 1.f)));
+  }
+  if (pe < -850) {                                    // no FP64 value of the columns moves
+    p = s = 0.0;
+    return;
+  }
+  p = widen(pf, pe, sg);
+  const double u = fma(p, p, 1.0);
+  const double z0 = widen(__fdividef(1.f, pe < 0 ? 1.f : fmaf(pf, pf, 1.f)), 0, 0u);
+  const double e = fma(-u, z0, 1.0);
+  const double w = fma(z0, fma(e, e, e), z0);         // 1 / (1 + p^2) in [0.85, 1]
+  s = p * __hiloint2double(__double2hiint(w) + (1 << 20), __double2loint(w));
+}
+// G^2 > tol2 A B on the leading 24 bits; false for G = 0 and anything not finite
+__device__ __forceinline__ bool above(double A, double Bv, double G, float tol2) {
+  const int ea = exp_bits(A), eb = exp_bits(Bv), eg = exp_bits(G);
+  const int k = 2 * eg - ea - eb;
+  if (eg == 0 || max(ea, max(eb, eg)) == 0x7ff || k < -124) return false;
+  const float fg = lead24(G);
+  return k > 60 || fg * fg * __uint_as_float((unsigned)(127 + k) << 23) > tol2 * (lead24(A) * lead24(Bv));
+}
+
+// lanes 0-7 return the warp's sum of a, 8-15 that of b, 16-31 that of g: values
+// change lanes as the sums halve, six additions in place of fifteen
+__device__ __forceinline__ double warp_sum3(double a, double b, double g) {
+  const int lane = threadIdx.x & 31;
+  const bool up = lane & 16, mid = lane & 8;
+  double x = up ? g : a;
+  x += __shfl_xor_sync(0xffffffffu, up ? a : g, 16);
+  const double y = b + __shfl_xor_sync(0xffffffffu, b, 16);
+  const double give = up ? x : (mid ? x : y);
+  double v = up ? x : (mid ? y : x);
+  v += __shfl_xor_sync(0xffffffffu, give, 8);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// One-sided Jacobi sweeps over the column pairs of M (p x q) in FP64, rotations
 // accumulated in V (q x q).  Cooperative launch: a round of disjoint pairs
-// (round-robin ordering) per grid barrier, one CTA per pair whose four warps
-// split the rows (so all four FP64 pipes of an SM work on it).  T = float
-// gives the cheap pre-sweeps of large matrices, T = double the polish.
-template <class T>
-__global__ void __launch_bounds__(SVD_CT) svd_sweep_kernel(int p, int q, T* M, T* V,
-                                                           int* counters, int* status, int init_v,
-                                                           T tol, T tol_count, int max_sweeps) {
+// (round-robin ordering) per grid barrier, one CTA per pair.  Warps 0-3 (one on
+// each FP64 pipe of the SM) split the rows of the pair's columns of M: products,
+// rotation, columns turned.  Warps 4-7 turn the columns of V by the rotations
+// of the round before, which nothing waits for, while warps 0-3 are in their
+// serial part.  Clocks of a round at q = 128 (512) before these two and after:
+// products 720 (1840), sum and rotation 2340 (2690) -> 1770 (3060), columns
+// turned 890 (3030) -> 400 (1360), barrier 2790 (3940) -> 2790 (3320).
+constexpr int SVD_MG = 128;                       // threads on M; as many on V
+constexpr int SVD_LAG = 16;                       // pairs of a CTA in one round
+struct GridBar {                                  // arrivals count up; bounded wait
+  unsigned int* c;
+  unsigned int target;
+  __device__ bool sync() {
+    __syncthreads();
+    target += gridDim.x;
+    __shared__ int ok_s;
+    if (threadIdx.x == 0) {
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c) : "memory");
+      unsigned int v = 0;
+      long long spin = 0;
+      do {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(c) : "memory");
+      } while ((int)(v - target) < 0 && ++spin < (1ll << 24) && ((spin & 255) || *(volatile unsigned int*)(c + 1) == 0u));
+      ok_s = (int)(v - target) >= 0;
+      if (!ok_s) atomicExch(c + 1, 1u);
+    }
+    __syncthreads();
+    return ok_s != 0;
+  }
+};
+__global__ void __launch_bounds__(2 * SVD_MG) svd_sweep64_kernel(int p, int q, double* M, double* V,
+                                                                 int* counters, int* status, int init_v,
+                                                                 float tol2, float tol2_count,
+                                                                 int max_sweeps) {
+  __shared__ double red[4][3];
+  __shared__ double rot[2][SVD_LAG][2];
+  __shared__ int act[2][SVD_LAG];
+  GridBar bar{(unsigned int*)(counters + 2), 0u};
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool on_m = tid < SVD_MG;
+  const int K = (q + 1) & ~1, npairs = K / 2;
+  // V = I, unless the pre-sweeps already supplied the rotation
+  if (!init_v)
+    for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)q * q; e += (i64)gridDim.x * blockDim.x)
+      V[e] = (e % q == e / q) ? 1.0 : 0.0;
+  if (blockIdx.x == 0 && tid == 0) { counters[0] = 0; counters[1] = 0; }
+  bool ok = bar.sync();
+  int par = 0, last_r = -1, sweep = 0;
+  auto turn = [](double* x, double* y, int n, int t0, double ps, double sn) {
+    for (int i = t0; i < n; i += SVD_MG) {
+      double u = x[i], w = y[i];
+      u = fma(-ps, w, u);
+      w = fma(sn, u, w);
+      u = fma(-ps, w, u);
+      x[i] = u;
+      y[i] = w;
+    }
+  };
+  // V by the rotations of round last_r, held in slot par ^ 1
+  auto turn_v = [&]() {
+    if (last_r < 0) return;
+    for (int pi = blockIdx.x, k = 0; pi < npairs; pi += gridDim.x, ++k) {
+      if (!act[par ^ 1][k]) continue;
+      int a, b;
+      rr_pair(K, last_r, pi, a, b);
+      turn(V + (i64)q * a, V + (i64)q * b, q, tid - SVD_MG, rot[par ^ 1][k][0], rot[par ^ 1][k][1]);
+    }
+  };
+  for (sweep = 0; sweep < max_sweeps && ok; ++sweep) {
+    int* cnt = counters + (sweep & 1);
+    for (int r = 0; r < K - 1 && ok; ++r) {
+      if (on_m) {
+        for (int pi = blockIdx.x, k = 0; pi < npairs; pi += gridDim.x, ++k) {
+          int a, b;
+          rr_pair(K, r, pi, a, b);
+          if (a >= q || b >= q) {
+            if (tid == 0) act[par][k] = 0;
+            continue;
+          }
+          double* ca = M + (i64)p * a;
+          double* cb = M + (i64)p * b;
+          double al = 0, be = 0, ga = 0;
+          for (int i = tid; i < p; i += SVD_MG) {
+            const double x = ca[i], y = cb[i];
+            al = fma(x, x, al); be = fma(y, y, be); ga = fma(x, y, ga);
+          }
+          const double v = warp_sum3(al, be, ga);
+          if ((lane & 7) == 0 && lane < 24) red[warp][lane >> 3] = v;
+          asm volatile("bar.sync 1, %0;" ::"n"(SVD_MG) : "memory");
+          if (warp == 0) {
+            // lanes 0-2 add the warps' sums of A, Bv and G
+            const int l = lane < 3 ? lane : 0;
+            const double sum = (red[0][l] + red[1][l]) + (red[2][l] + red[3][l]);
+            const double A = __shfl_sync(0xffffffffu, sum, 0), Bv = __shfl_sync(0xffffffffu, sum, 1),
+                         G = __shfl_sync(0xffffffffu, sum, 2);
+            if (lane == 0) {
+              const bool go = above(A, Bv, G, tol2);
+              if (go) {
+                jacobi_shears(A, Bv, G, rot[par][k][0], rot[par][k][1]);
+                // rotations whose cosine is within the rounding noise of a dot
+                // product of length p are applied but do not keep the sweeps going
+                if (above(A, Bv, G, tol2_count)) atomicAdd(cnt, 1);
+              }
+              act[par][k] = go;
+            }
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(SVD_MG) : "memory");
+          if (act[par][k]) turn(ca, cb, p, tid, rot[par][k][0], rot[par][k][1]);
+        }
+      } else {
+        turn_v();
+      }
+      ok = bar.sync();
+      last_r = r;
+      par ^= 1;
+    }
+    const int done = (*((volatile int*)cnt) == 0);
+    ok = bar.sync() && ok;
+    if (blockIdx.x == 0 && tid == 0) counters[(sweep + 1) & 1] = 0;
+    ok = bar.sync() && ok;
+    if (done) break;
+  }
+  if (!on_m) turn_v();
+  if (!ok)   // a wait ran out: nothing here may be taken for a result
+    for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)p * q; e += (i64)gridDim.x * blockDim.x)
+      M[e] = __longlong_as_double(0x7ff8000000000000ll);
+  if (blockIdx.x == 0 && tid == 0 && status) *status = sweep;
+}
+
+// The same sweeps for columns of at most 1024 rows, two columns to a block: a
+// CTA takes a pair of blocks, (a0 a1) and (b0 b1), holds their rows in the
+// registers of warps 0-3 (R rows a thread) and makes all four cross pairs
+// orthogonal, {a0 b0, a1 b1} then {a0 b1, a1 b0}, between two grid barriers;
+// once a sweep also {a0 a1, b0 b1}.  Half the barriers and half the traffic of
+// the kernel above; the two pairs of a step share one reduction (nine
+// additions for four norms and two products) and one lane each forms their
+// rotations.  Warps 4-7 turn V by the round before, as above.  All sweeps of a
+// 320 x 128 (2048 x 512) block: 5.6 (30) ms before, 3.75 (19.7) with the pair
+// kernel above, 2.2 (17.2) ms so.
+template <int R>
+__global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, double* M, double* V,
+                                                               int* counters, int* status, int init_v,
+                                                               float tol2, float tol2_count,
+                                                               int max_sweeps) {
+  __shared__ double red[4][8];
+  __shared__ double rot[2][3][2][2];               // [round parity][step][pair][p, s]
+  __shared__ int act[2][3];                        // either pair turns
+  GridBar bar{(unsigned int*)(counters + 2), 0u};
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool on_m = tid < SVD_MG;
+  const int KB = ((q + 1) / 2 + 1) & ~1;           // blocks, even
+  if (!init_v)
+    for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)q * q; e += (i64)gridDim.x * blockDim.x)
+      V[e] = (e % q == e / q) ? 1.0 : 0.0;
+  if (blockIdx.x == 0 && tid == 0) { counters[0] = 0; counters[1] = 0; }
+  bool ok = bar.sync();
+  int par = 0, last_r = -1, sweep = 0;
+  // columns of step st (0: a0 a1 | b0 b1, 1: a0 b0 | a1 b1, 2: a0 b1 | a1 b0) as
+  // positions in (a0, b0, a1, b1)
+  auto shear = [](double& u, double& w, double ps, double sn) {
+    u = fma(-ps, w, u);
+    w = fma(sn, u, w);
+    u = fma(-ps, w, u);
+  };
+  auto turn4 = [&](double (&x)[4], int st, const double (&rt)[2][2]) {
+    if (st == 0) {
+      shear(x[0], x[2], rt[0][0], rt[0][1]);
+      shear(x[1], x[3], rt[1][0], rt[1][1]);
+    } else if (st == 1) {
+      shear(x[0], x[1], rt[0][0], rt[0][1]);
+      shear(x[2], x[3], rt[1][0], rt[1][1]);
+    } else {
+      shear(x[0], x[3], rt[0][0], rt[0][1]);
+      shear(x[2], x[1], rt[1][0], rt[1][1]);
+    }
+  };
+  auto columns = [&](int r, int (&col)[4]) {
+    int a, b;
+    rr_pair(KB, r, blockIdx.x, a, b);
+    col[0] = 2 * a; col[1] = 2 * b; col[2] = 2 * a + 1; col[3] = 2 * b + 1;
+  };
+  auto turn_v = [&]() {
+    if (last_r < 0) return;
+    const int o = par ^ 1;
+    if (!(act[o][0] | act[o][1] | act[o][2])) return;
+    int col[4];
+    columns(last_r, col);
+    for (int i = tid - SVD_MG; i < q; i += SVD_MG) {
+      double x[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) x[c] = col[c] < q ? V[(i64)q * col[c] + i] : 0.0;
+#pragma unroll
+      for (int st = 0; st < 3; ++st)
+        if (act[o][st]) turn4(x, st, rot[o][st]);
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        if (col[c] < q) V[(i64)q * col[c] + i] = x[c];
+    }
+  };
+  for (sweep = 0; sweep < max_sweeps && ok; ++sweep) {
+    int* cnt = counters + (sweep & 1);
+    for (int r = 0; r < KB - 1 && ok; ++r) {
+      if (on_m) {
+        int col[4];
+        columns(r, col);
+        double x[R][4];
+#pragma unroll
+        for (int k = 0; k < R; ++k)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            const int i = tid + SVD_MG * k;
+            x[k][c] = (i < p && col[c] < q) ? M[(i64)p * col[c] + i] : 0.0;
+          }
+        bool any = false;
+#pragma unroll
+        for (int st = 0; st < 3; ++st) {
+          if (st == 0 && r > 0) {
+            if (tid == 0) act[par][0] = 0;
+            continue;
+          }
+          // norms of the four columns, products of the two pairs
+          double s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0, s5 = 0;
+#pragma unroll
+          for (int k = 0; k < R; ++k) {
+            const double(&v)[4] = x[k];
+            s0 = fma(v[0], v[0], s0); s1 = fma(v[1], v[1], s1);
+            s2 = fma(v[2], v[2], s2); s3 = fma(v[3], v[3], s3);
+            s4 = fma(v[0], st == 0 ? v[2] : (st == 1 ? v[1] : v[3]), s4);
+            s5 = fma(st == 0 ? v[1] : v[2], st == 2 ? v[1] : v[3], s5);
+          }
+          // lanes with bits 4, 3, 2 = b end with the sum of value b
+          const bool h4 = lane & 16, h3 = lane & 8, h2 = lane & 4;
+          double y0 = (h4 ? s4 : s0) + __shfl_xor_sync(0xffffffffu, h4 ? s0 : s4, 16);
+          double y1 = (h4 ? s5 : s1) + __shfl_xor_sync(0xffffffffu, h4 ? s1 : s5, 16);
+          double y2 = (h4 ? 0.0 : s2) + __shfl_xor_sync(0xffffffffu, h4 ? s2 : 0.0, 16);
+          double y3 = (h4 ? 0.0 : s3) + __shfl_xor_sync(0xffffffffu, h4 ? s3 : 0.0, 16);
+          y0 = (h3 ? y2 : y0) + __shfl_xor_sync(0xffffffffu, h3 ? y0 : y2, 8);
+          y1 = (h3 ? y3 : y1) + __shfl_xor_sync(0xffffffffu, h3 ? y1 : y3, 8);
+          y0 = (h2 ? y1 : y0) + __shfl_xor_sync(0xffffffffu, h2 ? y0 : y1, 4);
+          y0 += __shfl_xor_sync(0xffffffffu, y0, 2);
+          y0 += __shfl_xor_sync(0xffffffffu, y0, 1);
+          if ((lane & 3) == 0) red[warp][lane >> 2] = y0;
+          asm volatile("bar.sync 1, %0;" ::"n"(SVD_MG) : "memory");
+          if (warp == 0) {
+            const int l = lane & 7;
+            const double sum = (red[0][l] + red[1][l]) + (red[2][l] + red[3][l]);
+            // lane 0: pair 0, lane 1: pair 1
+            const int la = st == 0 ? (lane ? 1 : 0) : (lane ? 2 : 0);
+            const int lb = st == 0 ? (lane ? 3 : 2) : ((lane != 0) == (st == 1) ? 3 : 1);
+            const double A = __shfl_sync(0xffffffffu, sum, la), Bv = __shfl_sync(0xffffffffu, sum, lb),
+                         G = __shfl_sync(0xffffffffu, sum, lane ? 5 : 4);
+            const bool go = lane < 2 && above(A, Bv, G, tol2);
+            double ps = 0.0, sn = 0.0;
+            if (go) jacobi_shears(A, Bv, G, ps, sn);
+            if (lane < 2) {
+              rot[par][st][lane][0] = ps;
+              rot[par][st][lane][1] = sn;
+            }
+            // rotations whose cosine is within the rounding noise of a dot
+            // product of length p are applied but do not keep the sweeps going
+            const unsigned n = __popc(__ballot_sync(0xffffffffu, go && above(A, Bv, G, tol2_count)));
+            const unsigned g = __ballot_sync(0xffffffffu, go);
+            if (lane == 0) {
+              if (n) atomicAdd(cnt, (int)n);
+              act[par][st] = g != 0u;
+            }
+          }
+          asm volatile("bar.sync 1, %0;" ::"n"(SVD_MG) : "memory");
+          if (act[par][st]) {
+            any = true;
+            const double rt[2][2] = {{rot[par][st][0][0], rot[par][st][0][1]},
+                                     {rot[par][st][1][0], rot[par][st][1][1]}};
+#pragma unroll
+            for (int k = 0; k < R; ++k) turn4(x[k], st, rt);
+          }
+        }
+        if (any) {
+#pragma unroll
+          for (int k = 0; k < R; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int i = tid + SVD_MG * k;
+              if (i < p && col[c] < q) M[(i64)p * col[c] + i] = x[k][c];
+            }
+        }
+      } else {
+        turn_v();
+      }
+      ok = bar.sync();
+      last_r = r;
+      par ^= 1;
+    }
+    const int done = (*((volatile int*)cnt) == 0);
+    ok = bar.sync() && ok;
+    if (blockIdx.x == 0 && tid == 0) counters[(sweep + 1) & 1] = 0;
+    ok = bar.sync() && ok;
+    if (done) break;
+  }
+  if (!on_m) turn_v();
+  if (!ok)   // a wait ran out: nothing here may be taken for a result
+    for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)p * q; e += (i64)gridDim.x * blockDim.x)
+      M[e] = __longlong_as_double(0x7ff8000000000000ll);
+  if (blockIdx.x == 0 && tid == 0 && status) *status = sweep;
+}
+
+// The same sweeps in FP32: the cheap pre-sweeps of blocks of 8 to 15 columns
+// that do not fit one CTA's shared memory.
+__global__ void __launch_bounds__(SVD_CT) svd_sweep32_kernel(int p, int q, float* M, float* V,
+                                                             int* counters, int* status,
+                                                             float tol, float tol_count, int max_sweeps) {
   cg::grid_group grid = cg::this_grid();
-  __shared__ T red[3][SVD_CT / 32];
-  __shared__ T csn[2];
+  __shared__ float red[3][SVD_CT / 32];
+  __shared__ float csn[2];
   __shared__ int act;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int K = (q + 1) & ~1;
   const int npairs = K / 2;
-  // V = I, unless the pre-sweeps already supplied the rotation
-  if (!init_v)
-    for (i64 e = blockIdx.x * (i64)SVD_CT + tid; e < (i64)q * q; e += (i64)gridDim.x * SVD_CT)
-      V[e] = (e % q == e / q) ? T(1) : T(0);
+  for (i64 e = blockIdx.x * (i64)SVD_CT + tid; e < (i64)q * q; e += (i64)gridDim.x * SVD_CT)
+    V[e] = (e % q == e / q) ? 1.f : 0.f;
   if (blockIdx.x == 0 && tid == 0) { counters[0] = 0; counters[1] = 0; }
   grid.sync();
   int sweep = 0;
@@ -370,56 +739,43 @@ __global__ void __launch_bounds__(SVD_CT) svd_sweep_kernel(int p, int q, T* M, T
         int a, b;
         rr_pair(K, r, pi, a, b);
         if (a >= q || b >= q) continue;
-        T* ca = M + (i64)p * a;
-        T* cb = M + (i64)p * b;
-        T al = 0, be = 0, ga = 0;
+        float* ca = M + (i64)p * a;
+        float* cb = M + (i64)p * b;
+        float al = 0, be = 0, ga = 0;
         for (int i = tid; i < p; i += SVD_CT) {
-          const T x = ca[i], y = cb[i];
-          al = fma(x, x, al); be = fma(y, y, be); ga = fma(x, y, ga);
+          const float x = ca[i], y = cb[i];
+          al = fmaf(x, x, al); be = fmaf(y, y, be); ga = fmaf(x, y, ga);
         }
         al = warp_sum_t(al); be = warp_sum_t(be); ga = warp_sum_t(ga);
         if (lane == 0) { red[0][warp] = al; red[1][warp] = be; red[2][warp] = ga; }
         __syncthreads();
         if (tid == 0) {
-          T A = 0, Bv = 0, G = 0;
+          float A = 0, Bv = 0, G = 0;
           for (int w = 0; w < SVD_CT / 32; ++w) { A += red[0][w]; Bv += red[1][w]; G += red[2][w]; }
-          // |G| > tol sqrt(A Bv), compared in squares (no square root)
-          const T g2 = G * G, ab = A * Bv;
-          int go = (G != T(0)) && (g2 > tol * tol * ab);
+          const float g2 = G * G, ab = A * Bv;
+          const int go = (G != 0.f) && (g2 > tol * tol * ab);
           if (go) {
-            // The angle is taken in FP32 (GB300 runs FP64 square roots and
-            // divides as long dependent chains on a narrow pipe, and this is
-            // the serial part of every round); c and s are formed in T from
-            // that t, c = 1/sqrt(1 + t^2), s = c t, so the rotation is
-            // orthogonal to T's precision whatever t is.  A t off by FP32
-            // rounding leaves an off-diagonal ~1e-7 of G, which the next
-            // sweep removes like any other; the stopping test is unchanged.
-            const T zeta_t = (Bv - A) / (T(2) * G);
-            const float z = (float)zeta_t, az = fabsf(z);
-            // |zeta| beyond FP32's comfortable range: t = 1/(2 zeta) in T
-            const T t = az < 1e18f ? (T)copysignf(1.f / (az + sqrtf(1.f + z * z)), z)
-                                   : T(0.5) / zeta_t;
-            const T c = rsqrt(T(1) + t * t);
+            const float z = (Bv - A) / (2.f * G), az = fabsf(z);
+            const float t = az < 1e18f ? copysignf(1.f / (az + sqrtf(1.f + z * z)), z) : 0.5f / z;
+            const float c = rsqrtf(1.f + t * t);
             csn[0] = c;
             csn[1] = c * t;
-            // rotations whose cosine is within the rounding noise of a dot
-            // product of length p are applied but do not keep the sweeps going
             if (g2 > tol_count * tol_count * ab) atomicAdd(cnt, 1);
           }
           act = go;
         }
         __syncthreads();
         if (act) {
-          const T c = csn[0], sn = csn[1];
+          const float c = csn[0], sn = csn[1];
           for (int i = tid; i < p; i += SVD_CT) {
-            const T x = ca[i], y = cb[i];
+            const float x = ca[i], y = cb[i];
             ca[i] = c * x - sn * y;
             cb[i] = sn * x + c * y;
           }
-          T* va = V + (i64)q * a;
-          T* vb = V + (i64)q * b;
+          float* va = V + (i64)q * a;
+          float* vb = V + (i64)q * b;
           for (int i = tid; i < q; i += SVD_CT) {
-            const T x = va[i], y = vb[i];
+            const float x = va[i], y = vb[i];
             va[i] = c * x - sn * y;
             vb[i] = sn * x + c * y;
           }
@@ -446,27 +802,50 @@ __global__ void f2d_kernel(i64 n, const float* __restrict__ a, double* __restric
     b[e] = (double)a[e];
 }
 
-template <class T>
-static int svd_coop_blocks() {
-  static const int max_coop = [] {
-    int dev = 0, nsm = 0, per = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, svd_sweep_kernel<T>, SVD_CT, 0) !=
-            cudaSuccess)
-      return 0;
-    return nsm * per;
-  }();
-  TTG_REQUIRE(max_coop > 0, "svd: occupancy query failed");
-  return max_coop;
+static int coop_blocks(const void* k, int nt) {
+  int dev = 0, nsm = 0, per = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, nt, 0) != cudaSuccess)
+    return 0;
+  return nsm * per;
 }
 
-template <class T>
-static void svd_sweeps(int p, int q, T* M, T* V, int* counters, int* status, int init_v, T tol,
-                       T tol_count, int max_sweeps, cudaStream_t s) {
-  int blocks = std::max(1, std::min((q + 1) / 2, svd_coop_blocks<T>()));
-  void* args[] = {&p, &q, &M, &V, &counters, &status, &init_v, &tol, &tol_count, &max_sweeps};
-  TTG_CUDA(cudaLaunchCooperativeKernel((void*)svd_sweep_kernel<T>, dim3(blocks), dim3(SVD_CT),
+static void svd_sweeps(int p, int q, double* M, double* V, int* counters, int* status, int init_v,
+                       double tol, double tol_count, int max_sweeps, cudaStream_t s) {
+  float tol2 = (float)(tol * tol), tol2_count = (float)(tol_count * tol_count);
+  TTG_CUDA(cudaMemsetAsync(counters, 0, 4 * sizeof(int), s));
+  void* args[] = {&p, &q, &M, &V, &counters, &status, &init_v, &tol2, &tol2_count, &max_sweeps};
+  auto launch = [&](const void* k, int blocks) {
+    TTG_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(2 * SVD_MG), args, 0, s));
+    ++g_launches;
+  };
+  // two columns to a block where their rows fit registers and there are four
+  // columns to a CTA (a resident grid of q / 4 CTAs always fits)
+  const int kb = ((q + 1) / 2 + 1) & ~1;
+  if (p <= 8 * SVD_MG && q >= 4) {
+    static const int max_block = coop_blocks((const void*)svd_block_kernel<8>, 2 * SVD_MG);
+    if (kb / 2 <= max_block) {
+      if (p <= SVD_MG) launch((const void*)svd_block_kernel<1>, kb / 2);
+      else if (p <= 2 * SVD_MG) launch((const void*)svd_block_kernel<2>, kb / 2);
+      else if (p <= 4 * SVD_MG) launch((const void*)svd_block_kernel<4>, kb / 2);
+      else launch((const void*)svd_block_kernel<8>, kb / 2);
+      return;
+    }
+  }
+  static const int max_coop = coop_blocks((const void*)svd_sweep64_kernel, 2 * SVD_MG);
+  const int npairs = (q + 1) / 2, blocks = std::max(1, std::min(npairs, max_coop));
+  TTG_REQUIRE(max_coop > 0, "svd: occupancy query failed");
+  TTG_REQUIRE(ceil_div(npairs, blocks) <= SVD_LAG, "svd: too many columns");
+  launch((const void*)svd_sweep64_kernel, blocks);
+}
+static void svd_sweeps32(int p, int q, float* M, float* V, int* counters, int* status, float tol,
+                         float tol_count, int max_sweeps, cudaStream_t s) {
+  static const int max_coop = coop_blocks((const void*)svd_sweep32_kernel, SVD_CT);
+  TTG_REQUIRE(max_coop > 0, "svd: occupancy query failed");
+  int blocks = std::max(1, std::min((q + 1) / 2, max_coop));
+  void* args[] = {&p, &q, &M, &V, &counters, &status, &tol, &tol_count, &max_sweeps};
+  TTG_CUDA(cudaLaunchCooperativeKernel((const void*)svd_sweep32_kernel, dim3(blocks), dim3(SVD_CT),
                                        args, 0, s));
   ++g_launches;
 }
@@ -475,7 +854,7 @@ static void svd_sweeps(int p, int q, T* M, T* V, int* counters, int* status, int
 // accumulated rotation V (q x q) in shared memory.  FP32 runs at 64 times
 // the FP64 rate of a GB300 SM, so the sweeps that take the columns from
 // arbitrary to nearly orthogonal are cheap here; the FP64 sweeps that follow
-// (svd_rotate_kernel, started from V) only polish.  V is written as FP64.
+// (started from V) only polish.  V is written as FP64.
 constexpr int SVD32_NT = 1024;
 constexpr int SVD32_MAX_SWEEPS = 20;
 constexpr size_t SVD32_SMEM = 227 * 1024 - 1024;
@@ -565,11 +944,16 @@ __global__ void svd_finish_kernel(int p, int q, const double* M, const double* V
   }
 }
 
+// descending, ties by index, NaN first: a permutation whatever the norms are
 __global__ void svd_rank_kernel(int q, const double* nrm, int* rank) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < q; j += gridDim.x * blockDim.x) {
-    double v = nrm[j];
+    const double v = nrm[j];
     int rk = 0;
-    for (int t = 0; t < q; ++t) rk += (nrm[t] > v) || (nrm[t] == v && t < j);
+    for (int t = 0; t < q; ++t) {
+      const double w = nrm[t];
+      const bool same = w == v || (w != w && v != v);
+      rk += w > v || (w != w && v == v) || (same && t < j);
+    }
     rank[j] = rk;
   }
 }
@@ -598,13 +982,9 @@ __global__ void svd_gather_kernel(int p, int q, const double* M, const double* V
 // accurate Jacobi SVD algorithm", SIAM J. Matrix Anal. Appl. 29, 2008).
 // Plain one-sided Jacobi on the truncation blocks of the sweeps, whose
 // singular values fall over fifteen decades, needs 25-35 sweeps; on the
-// transposed triangular factor of a QR of the column-sorted matrix it needs
-// 6-8.  So for M (p x q, p >= q):
-//   M P = Q R   (columns sorted by decreasing norm, blocked Householder QR:
-//                one-CTA panels of QRP_NB columns, trailing update by FP64
-//                GEMMs over the whole GPU with the compact WY form)
-//   R^T = Ux S J^T   (one-sided Jacobi on the q x q matrix R^T)
-//   M = (Q J) S (P Ux)^T.
+// transposed triangular factor of a QR of the column-sorted matrix 7-10, on
+// that of a second QR 4-7 (svd_tall_qr below).  The factors are applied in
+// compact WY form, panels of QRP_NB columns, by FP64 GEMMs.
 // ---------------------------------------------------------------------------
 constexpr int QRP_NB = 32;
 constexpr int QRP_NT = 1024;
@@ -791,6 +1171,68 @@ __global__ void __launch_bounds__(QRC_NT) qr_panel_coop_kernel(int m, int w, dou
   }
 }
 
+// The triangular factors T of all panels of a factored matrix F (rows x q,
+// leading dimension rows): panel k holds columns QRP_NB k.., its T is w x w at
+// Tf + k QRP_NB^2 (leading dimension QRP_NB).  A cluster of QRT_CL CTAs per
+// panel shares the rows of its Gram matrix Y^T Y, added in rank order; rank 0
+// runs the recurrence T[0:i, i] = -tau_i T[0:i, 0:i] (Y^T Y)[0:i, i].
+constexpr int QRT_CL = 8, QRT_NT = 256, QRT_ROWS = 32;
+__global__ void __launch_bounds__(QRT_NT) qr_t_kernel(int rows, int q, const double* __restrict__ F,
+                                                      const double* __restrict__ tau, double* __restrict__ Tf) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ double Y[QRP_NB][QRT_ROWS + 1];
+  __shared__ double gram[QRP_NB][QRP_NB + 1];     // [j][i]
+  __shared__ double zt[QRP_NB];
+  const int tid = threadIdx.x, i = tid & 31, jw = tid >> 5;
+  const int k = blockIdx.x, j0 = k * QRP_NB, w = min(QRP_NB, q - j0), m = rows - j0;
+  const double* A = F + j0 + (i64)rows * j0;
+  double acc[QRP_NB / 8];
+#pragma unroll
+  for (int t = 0; t < QRP_NB / 8; ++t) acc[t] = 0.0;
+  for (int r0 = blockIdx.y * QRT_ROWS; r0 < m; r0 += gridDim.y * QRT_ROWS) {
+    for (int e = tid; e < QRP_NB * QRT_ROWS; e += QRT_NT) {
+      const int r = r0 + (e & (QRT_ROWS - 1)), c = e / QRT_ROWS;
+      Y[c][e & (QRT_ROWS - 1)] = (r < m && c < w) ? (r > c ? A[r + (i64)rows * c] : (r == c ? 1.0 : 0.0)) : 0.0;
+    }
+    __syncthreads();
+    for (int r = 0; r < QRT_ROWS; ++r) {
+      const double yi = Y[i][r];
+#pragma unroll
+      for (int t = 0; t < QRP_NB / 8; ++t) acc[t] = fma(yi, Y[jw + 8 * t][r], acc[t]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int t = 0; t < QRP_NB / 8; ++t) gram[jw + 8 * t][i] = acc[t];
+  cl.sync();
+  if (cl.block_rank() == 0) {
+    double v[QRP_NB / 8];
+#pragma unroll
+    for (int t = 0; t < QRP_NB / 8; ++t) {
+      v[t] = 0.0;
+      for (unsigned b = 0; b < cl.num_blocks(); ++b) v[t] += cl.map_shared_rank(&gram[jw + 8 * t][i], b)[0];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < QRP_NB / 8; ++t) gram[jw + 8 * t][i] = v[t];
+    double* T = Tf + (size_t)k * QRP_NB * QRP_NB;
+    for (int e = tid; e < QRP_NB * QRP_NB; e += QRT_NT) T[e] = 0.0;
+    __syncthreads();
+    for (int c = 0; c < w; ++c) {
+      if (tid < c) zt[tid] = -tau[j0 + c] * gram[c][tid];
+      __syncthreads();
+      if (tid < c) {
+        double u = 0.0;
+        for (int l = tid; l < c; ++l) u = fma(T[tid + QRP_NB * l], zt[l], u);
+        T[tid + QRP_NB * c] = u;
+      }
+      if (tid == 0) T[c + QRP_NB * c] = tau[j0 + c];
+      __syncthreads();
+    }
+  }
+  cl.sync();   // no CTA leaves while rank 0 still reads its sums
+}
+
 // Y (m x w) with the unit diagonal and zeros above it, from a factored panel
 __global__ void qr_make_y_kernel(int m, int w, const double* __restrict__ A, i64 lda,
                                  double* __restrict__ Y) {
@@ -834,9 +1276,9 @@ static size_t svd_qr_work(size_t p, size_t q) {
   const size_t npan = (q + QRP_NB - 1) / QRP_NB;
   const size_t coop = QRP_NB * QRC_GMAX + QRP_NB * QRC_GMAX * QRP_NB + QRC_GMAX * QRP_NB * QRP_NB;
   // first QR (A, X, Ux, Vtx, Tf, Yp, G1, G2, tau, perm, coop partials), then
-  // the second QR's R2^T, Q2 V2, T factors and tau
+  // the second QR's R2^T, Q2 V2, T factors and tau; the factorisation's work
   return p * q + 3 * q * q + npan * QRP_NB * QRP_NB + p * QRP_NB + 2 * QRP_NB * q + 2 * q + 256 +
-         coop + 64 + 2 * q * q + npan * QRP_NB * QRP_NB + q + 64;
+         coop + 64 + 2 * q * q + npan * QRP_NB * QRP_NB + q + 128 + qr_work_elems(p, q);
 }
 
 size_t svd_scratch(int p, int q) {
@@ -855,19 +1297,14 @@ static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double*
                      double* tmp, cudaStream_t s, double* qrwork = nullptr);
 
 // The QR-preconditioned path (q >= SVD_QR_MIN_Q):
-//   M P = Q1 R1        columns sorted by norm, blocked Householder QR
-//   R1^T = Q2 R2       for q >= SVD_QR2_MIN_Q a second QR, of R1^T
+//   M P = Q1 R1        columns sorted by norm, Householder QR
+//   R1^T = Q2 R2       a second QR, of R1^T
 //   R2^T = U2 S V2^T   one-sided Jacobi on R2^T (rotations accumulated in V2)
-// so M = (Q1 U2) S (P Q2 V2)^T; without the second QR (Q2 = I, R2 = R1)
-// the Jacobi runs on R1^T itself and M = (Q1 V2') S (P U2')^T with the roles
-// of the factors exchanged.  The second QR leaves R2^T closer to orthogonal
-// columns: on graded blocks (singular values 1 to 1e-13) the sweeps drop
-// from 9-10 to about 6; measured on GB300 that pays from q ~ 200 (2048 x 512:
-// 59.2 -> 53.8 ms) but not at q = 128 (320 x 128: 7.6 -> 7.3 ms, and the
-// d=20 solve, whose blocks are mostly narrower, slower by its ~30 extra
-// launches per SVD).
-constexpr int SVD_QR2_MIN_Q = 192;
-
+// so M = (Q1 U2) S (P Q2 V2)^T.  The second QR leaves R2^T closer to orthogonal
+// columns: on graded blocks (singular values 1 to 1e-13) the sweeps drop from
+// 7-10 to 4-7, which measured faster at every width from 16 on (GB300, one ->
+// two QR: 32 x 16 491 -> 468 us, 160 x 64 2.09 -> 1.97 ms, 320 x 128 4.67 ->
+// 4.05 ms, 2048 x 512 35 -> 30.6 ms).
 static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, double* Vt,
                         double* V, double* nrm, int* rank, int* counters, int* status,
                         double* tmp, double* work, cudaStream_t s) {
@@ -889,6 +1326,7 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   double* W = X2 + (size_t)q * q;                       // q x q: Q2 V2
   double* Tf2 = W + (size_t)q * q;                      // NB x NB per panel (second QR)
   double* tau2 = Tf2 + (size_t)npan * QRP_NB * QRP_NB;  // q
+  double* qrw = tau2 + q + 64;                          // work of the factorisation
   auto gemm = [&](int M, int N, int K, const double* Am, i64 sAm, i64 sAk, const double* Bm,
                   i64 sBk, i64 sBn, double* C, i64 sCm, i64 sCn, double alpha, double beta) {
     GemmF64 g;
@@ -901,7 +1339,15 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   };
   // blocked Householder QR of F (rows x q, leading dimension rows) in place:
   // reflectors below the diagonal, R on and above it, panel T factors in Tk
+  // Over the whole GPU with the rows in shared memory (ttg_qr.cu), or, where
+  // they do not fit, panel by panel with GEMM updates
   auto qr_factor = [&](int rows, double* F, double* Tfac, double* tv) {
+    if (qr_rows_factor(rows, q, F, qrw, qr_work_elems(rows, q), s)) {
+      TTG_CUDA(cudaMemcpyAsync(tv, qrw, sizeof(double) * q, cudaMemcpyDeviceToDevice, s));
+      launch_clustered(qr_t_kernel, dim3(npan, QRT_CL), dim3(QRT_NT), dim3(1, QRT_CL, 1), 0, s, rows,
+                       q, (const double*)F, (const double*)tv, Tfac);
+      return;
+    }
     for (int k = 0; k < npan; ++k) {
       const int j0 = k * QRP_NB, w = std::min(QRP_NB, q - j0), m = rows - j0;
       double* Ap = F + j0 + (i64)rows * j0;
@@ -966,20 +1412,15 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   TTG_CHECK_LAUNCH();
   qr_factor(p, A, Tf, tau);                             // M P = Q1 R1
   (void)tmp;
-  const bool qr2 = q >= SVD_QR2_MIN_Q;
-  if (qr2) {
-    rt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, A, p, X);   // X = R1^T
-    TTG_CHECK_LAUNCH();
-    qr_factor(q, X, Tf2, tau2);                                // R1^T = Q2 R2
-    rt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, X, q, X2);  // X2 = R2^T
-  } else {
-    rt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, A, p, X2);  // X2 = R1^T
-  }
+  rt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, A, p, X);   // X = R1^T
+  TTG_CHECK_LAUNCH();
+  qr_factor(q, X, Tf2, tau2);                                // R1^T = Q2 R2
+  rt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, X, q, X2);  // X2 = R2^T
   TTG_CHECK_LAUNCH();
   // one-sided Jacobi on R2^T, FP64 sweeps over the grid from the identity
   // (FP32 pre-sweeps do not pay here: the preconditioned matrix converges in
   // a few FP64 sweeps, and FP32 cannot resolve its small columns)
-  svd_sweeps<double>(q, q, X2, V, counters, status, 0, sqrt((double)q) * DBL_EPSILON,
+  svd_sweeps(q, q, X2, V, counters, status, 0, sqrt((double)q) * DBL_EPSILON,
                      (double)q * DBL_EPSILON, SVD_MAX_SWEEPS, s);
   svd_finish_kernel<<<nb, 256, 0, s>>>(q, q, X2, V, nullptr, nullptr, nullptr, nrm, rank);
   TTG_CHECK_LAUNCH();
@@ -988,22 +1429,13 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   // Ux = U2 (sorted), sigma, Vtx = V2^T (sorted rows)
   svd_gather_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, q, X2, V, nrm, rank, Ux, sigma, Vtx);
   TTG_CHECK_LAUNCH();
-  if (qr2) {
-    // U = Q1 [U2; 0]; W = Q2 V2, Vt = (P W)^T
-    qr_c0n_kernel<<<gbl((i64)p * q), 256, 0, s>>>(p, q, Ux, U);
-    TTG_CHECK_LAUNCH();
-    qr_apply(p, A, Tf, U);
-    transpose_f64(q, q, Vtx, W, s);
-    qr_apply(q, X, Tf2, W);
-    qr_vt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, W, perm, Vt);
-  } else {
-    // R1 = V2 S U2^T: U = Q1 [V2; 0], Vt = (P U2)^T
-    transpose_f64(q, q, Vtx, W, s);
-    qr_c0n_kernel<<<gbl((i64)p * q), 256, 0, s>>>(p, q, W, U);
-    TTG_CHECK_LAUNCH();
-    qr_apply(p, A, Tf, U);
-    qr_vt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, Ux, perm, Vt);
-  }
+  // U = Q1 [U2; 0]; W = Q2 V2, Vt = (P W)^T
+  qr_c0n_kernel<<<gbl((i64)p * q), 256, 0, s>>>(p, q, Ux, U);
+  TTG_CHECK_LAUNCH();
+  qr_apply(p, A, Tf, U);
+  transpose_f64(q, q, Vtx, W, s);
+  qr_apply(q, X, Tf2, W);
+  qr_vt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, W, perm, Vt);
   TTG_CHECK_LAUNCH();
 }
 
@@ -1036,7 +1468,7 @@ static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double*
       float* V32 = (float*)Y;
       d2f_kernel<<<(int)std::min<i64>(4096, ((i64)p * q + 255) / 256), 256, 0, s>>>((i64)p * q, Mw, M32);
       TTG_CHECK_LAUNCH();
-      svd_sweeps<float>(p, q, M32, V32, counters, status, 0, sqrtf((float)p) * FLT_EPSILON,
+      svd_sweeps32(p, q, M32, V32, counters, status, sqrtf((float)p) * FLT_EPSILON,
                         (float)p * FLT_EPSILON, 30, s);
       f2d_kernel<<<(int)std::min<i64>(4096, ((i64)q * q + 255) / 256), 256, 0, s>>>((i64)q * q, V32, V);
       TTG_CHECK_LAUNCH();
@@ -1068,7 +1500,7 @@ static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double*
     TTG_CUDA(cudaMemcpyAsync(Mw, W, sizeof(double) * p * q, cudaMemcpyDeviceToDevice, s));
     init_v = 1;
   }
-  svd_sweeps<double>(p, q, Mw, V, counters, status, init_v, sqrt((double)p) * DBL_EPSILON,
+  svd_sweeps(p, q, Mw, V, counters, status, init_v, sqrt((double)p) * DBL_EPSILON,
                      (double)p * DBL_EPSILON, SVD_MAX_SWEEPS, s);
   int nb = std::max(1, std::min(1024, ceil_div((i64)q * 32, 256)));
   svd_finish_kernel<<<nb, 256, 0, s>>>(p, q, Mw, V, U, sigma, Vt, nrm, rank);

@@ -328,8 +328,9 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
   }
   __syncthreads();
 
-  // R: rows 0..r-1, zero below the diagonal
-  for (int c = warp; c < m; c += NT / 32)
+  // R: rows 0..r-1, zero below the diagonal (R null: factor only, A keeps the
+  // reflectors below R)
+  for (int c = R ? warp : m; c < m; c += NT / 32)
     for (int i = lane; i < nloc; i += 32) {
       const int gi = b + G * i;
       if (gi < r) R[gi + (i64)r * c] = fail ? O::nan() : (gi <= c ? A[(size_t)ld * c + i] : O::zero());
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
   __syncthreads();
 
   // Q in place: columns r-1..0; column j becomes H_j e_j, later columns H_j q_c
-  for (int j = r - 1; j >= 0 && !fail; --j) {
+  for (int j = R ? r - 1 : -1; j >= 0 && !fail; --j) {
     const T ta = tau[j];
     const int i0 = j > b ? (j - b + G - 1) / G : 0;
     T* aj = A + (size_t)ld * j;
@@ -414,13 +415,15 @@ template <class T> bool grid_ok(int n, int m, int G) {
 //    256 x   8 complex   190 | 75  120   123   144
 struct Pick { int G; bool grid; };
 template <class T>
-Pick pick(int n, int m, bool have_work) {
+Pick pick(int n, int m, bool form_q, bool have_work) {
   const double cx = sizeof(T) == 16 ? 4.0 : 1.0;
   const int r = std::min(n, m);
-  const double cols = (double)r * m - 0.5 * (double)r * r + 0.5 * (double)r * r;   // later columns, both passes
+  // later columns of all columns, in the factorisation and in forming Q
+  const double cols = (double)r * m - 0.5 * (double)r * r + (form_q ? 0.5 * (double)r * r : 0.0);
+  const double steps = (form_q ? 2.0 : 1.0) * r;
   auto est = [&](int G, bool grid) {
     const double rows = (n + G - 1) / G;
-    return 2.0 * cx * rows * cols / 1.9e3 + (grid ? 2.6 + 0.02 * G : (G == 1 ? 2.0 : 2.2)) * 2.0 * r;
+    return 2.0 * cx * rows * cols / 1.9e3 + (grid ? 2.6 + 0.02 * G : (G == 1 ? 2.0 : 2.2)) * steps;
   };
   Pick best{0, false};
   double bt = 1e300;
@@ -442,7 +445,7 @@ Pick pick(int n, int m, bool have_work) {
 template <class T>
 bool run(int n, int m, T* A, T* R, T* tau, size_t work, cudaStream_t s) {
   const bool have = work >= qr_work_elems(n, m);
-  Pick p = pick<T>(n, m, have);
+  Pick p = pick<T>(n, m, R != nullptr, have);
   if (p.G == 0) return false;
   const int r = std::min(n, m);
   const size_t smem = qr::smem_elems(n, m, p.G, p.grid) * sizeof(T);
@@ -484,6 +487,9 @@ bool run(int n, int m, T* A, T* R, T* tau, size_t work, cudaStream_t s) {
 
 bool qr_rows(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s) {
   return run<double>(n, m, A, R, tau, work, s);
+}
+bool qr_rows_factor(int n, int m, double* A, double* tau, size_t work, cudaStream_t s) {
+  return run<double>(n, m, A, (double*)nullptr, tau, work, s);
 }
 bool qr_rows(int n, int m, double2* A, double2* R, double2* tau, size_t work, cudaStream_t s) {
   return run<double2>(n, m, A, R, tau, work, s);
