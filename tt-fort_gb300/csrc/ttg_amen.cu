@@ -19,6 +19,7 @@
 // The enrichment TT z starts from the splitmix64/Box-Muller stream shared
 // with the oracle.
 #include "ttg_davidson.cuh"
+#include "ttg_words.cuh"
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -120,34 +121,148 @@ __global__ void lu_solve_kernel(int N, double* B, double* x, int* info) {
   }
 }
 
-// GMRES Hessenberg column j (h[0..j+1]): apply previous rotations, make a
-// new one, update g; res[0] = |g[j+1]|.  One thread.
-__global__ void givens_kernel(int j, double* h, double* cs, double* sn, double* g, double* R,
-                              int ldr, double* res) {
-  for (int i = 0; i < j; ++i) {
-    const double a = h[i], b = h[i + 1];
-    h[i] = cs[i] * a + sn[i] * b;
-    h[i + 1] = -sn[i] * a + cs[i] * b;
+// One Arnoldi step after the matvec, over a resident grid: w = V[:, j+1] is made
+// orthogonal to V[:, 0..j] by classical Gram-Schmidt applied twice and scaled to
+// norm 1; h[0..j] the coefficients, h[j+1] the norm.  CTA b holds its rows of w
+// in shared memory; V is read four times from L2.  The parts of the products
+// are exchanged as tagged words (CTA c % G adds those of column c in CTA order),
+// with them |w|^2 in the second pass: |w - V h2|^2 = |w|^2 - |h2|^2 as long as
+// the second pass takes off less than a tenth, else the norm is summed afresh.
+// Bound by its two exchanges (about 9 us) and 4 N (j + 1) FMAs; the nine
+// launches it replaces took about 65 us more a step (AMEn solve of the d = 4,
+// n = 24 grid, 3400 steps of up to 24 * 82 * 28 unknowns: 412 -> 187 ms).
+constexpr int AR_NT = 256, AR_G = 152, AR_SLOTS = 64, AR_CHUNK = 8192;
+constexpr size_t AR_WORDS = 2 * (size_t)(AR_G + 1) * AR_SLOTS + 8;   // 64-bit words of an exchange area
+__global__ void __launch_bounds__(AR_NT) arnoldi_kernel(i64 N, int j, int chunk, double* __restrict__ V,
+                                                        double* __restrict__ h,
+                                                        unsigned long long* part, unsigned int epoch) {
+  extern __shared__ double w[];                          // [chunk]
+  __shared__ double seg_s[8][AR_SLOTS];
+  __shared__ double tot_s[AR_SLOTS], h_s[AR_SLOTS];
+  __shared__ int fail;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, G = gridDim.x, b = blockIdx.x;
+  const i64 lo = (i64)b * chunk;
+  const int n = (int)max((i64)0, min((i64)chunk, N - lo));
+  unsigned long long* tot = part + (size_t)G * AR_SLOTS * 2;
+  unsigned int* flag = (unsigned int*)(part + 2 * (size_t)(AR_G + 1) * AR_SLOTS);
+  const double* Vb = V + lo;
+  double* wg = V + N * (j + 1) + lo;
+  if (tid == 0) fail = 0;
+  for (int i = tid; i < n; i += AR_NT) w[i] = wg[i];
+  __syncthreads();
+  // tot_s[c] = V_c . w for c < nc, then w . w when ww
+  auto products = [&](int nc, bool ww) {
+    const int C = nc + (ww ? 1 : 0), nseg = C >= 8 ? 1 : 8 / C;
+    for (int t = warp; t < C * nseg; t += AR_NT / 32) {
+      const int c = t % C, sg = t / C, i1 = (int)((i64)n * (sg + 1) / nseg);
+      const double* v = Vb + N * c;
+      double a0 = 0.0, a1 = 0.0;
+      int i = (int)((i64)n * sg / nseg) + lane;
+      if (c < nc) {
+        for (; i + 96 < i1; i += 128) {
+          const double x0 = v[i], x1 = v[i + 32], x2 = v[i + 64], x3 = v[i + 96];
+          a0 = fma(x0, w[i], a0);
+          a1 = fma(x1, w[i + 32], a1);
+          a0 = fma(x2, w[i + 64], a0);
+          a1 = fma(x3, w[i + 96], a1);
+        }
+        for (; i < i1; i += 32) a0 = fma(v[i], w[i], a0);
+      } else {
+        for (; i < i1; i += 32) a0 = fma(w[i], w[i], a0);
+      }
+      a0 += a1;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) a0 += __shfl_xor_sync(0xffffffffu, a0, o);
+      if (lane == 0) seg_s[sg][c] = a0;
+    }
+    __syncthreads();
+    if (tid < C) {
+      double t = 0.0;
+      for (int sg = 0; sg < nseg; ++sg) t += seg_s[sg][tid];
+      if (G == 1) tot_s[tid] = t;
+      else words::put(part + ((size_t)b * AR_SLOTS + tid) * 2, t, epoch);
+    }
+    if (G > 1) {
+      for (int c = b + warp * G; c < C; c += G * (AR_NT / 32)) {
+        constexpr int QL = (AR_G + 31) / 32;
+        unsigned long long x[QL][2];
+#pragma unroll
+        for (int k = 0; k < QL; ++k)
+          if (lane + 32 * k < G) words::load<double>(part + ((size_t)(lane + 32 * k) * AR_SLOTS + c) * 2, x[k]);
+        double t = 0.0;
+#pragma unroll
+        for (int k = 0; k < QL; ++k) {
+          double v;
+          if (lane + 32 * k < G) {
+            if (words::take<double>(part + ((size_t)(lane + 32 * k) * AR_SLOTS + c) * 2, x[k], v, epoch, flag)) t += v;
+            else fail = 1;
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (lane == 0) words::put(tot + (size_t)c * 2, t, epoch);
+      }
+      if (tid < C) {
+        unsigned long long x[2];
+        double v = 0.0;
+        words::load<double>(tot + (size_t)tid * 2, x);
+        if (!words::take<double>(tot + (size_t)tid * 2, x, v, epoch, flag)) fail = 1;
+        tot_s[tid] = v;
+      }
+    }
+    ++epoch;
+    __syncthreads();
+  };
+  // w -= V[:, 0..j] tot_s
+  auto subtract = [&]() {
+    for (int i = tid; i < n; i += AR_NT) {
+      double a0 = w[i], a1 = 0.0;
+      int c = 0;
+      for (; c + 8 <= j + 1; c += 8) {
+        double x[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) x[u] = Vb[N * (c + u) + i];
+#pragma unroll
+        for (int u = 0; u < 8; u += 2) {
+          a0 = fma(-x[u], tot_s[c + u], a0);
+          a1 = fma(-x[u + 1], tot_s[c + u + 1], a1);
+        }
+      }
+      for (; c <= j; ++c) a0 = fma(-Vb[N * c + i], tot_s[c], a0);
+      w[i] = a0 + a1;
+    }
+    __syncthreads();
+  };
+  products(j + 1, false);
+  if (tid <= j) h_s[tid] = tot_s[tid];
+  subtract();
+  products(j + 1, true);
+  double h2 = 0.0;
+  if (warp == 0) {
+    for (int c = lane; c <= j; c += 32) h2 = fma(tot_s[c], tot_s[c], h2);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) h2 += __shfl_xor_sync(0xffffffffu, h2, o);
+    if (lane == 0) {
+      const double ww = tot_s[j + 1];
+      h_s[AR_SLOTS - 1] = h2 <= 0.1 * ww ? ww - h2 : -1.0;   // NaN: summed afresh
+    }
   }
-  const double a = h[j], b = h[j + 1];
-  const double den = hypot(a, b);
-  const double c = den > 0 ? a / den : 1.0, s = den > 0 ? b / den : 0.0;
-  cs[j] = c;
-  sn[j] = s;
-  h[j] = den;
-  h[j + 1] = 0.0;
-  g[j + 1] = -s * g[j];
-  g[j] = c * g[j];
-  for (int i = 0; i <= j; ++i) R[i + ldr * j] = h[i];
-  res[0] = fabs(g[j + 1]);
-}
-
-// y = R^{-1} g (upper triangular k x k); one thread
-__global__ void trsv_kernel(int k, const double* R, int ldr, const double* g, double* y) {
-  for (int i = k - 1; i >= 0; --i) {
-    double v = g[i];
-    for (int j = i + 1; j < k; ++j) v -= R[i + ldr * j] * y[j];
-    y[i] = v / R[i + ldr * i];
+  if (tid <= j) h_s[tid] += tot_s[tid];
+  subtract();
+  double n2 = h_s[AR_SLOTS - 1];                             // the same value in every CTA
+  if (!(n2 >= 0.0)) {
+    products(0, true);
+    n2 = tot_s[0];
+  }
+  if (tid == 0) seg_s[0][0] = sqrt(n2);
+  __syncthreads();
+  const double nrm = fail ? __longlong_as_double(0x7ff8000000000000ll) : seg_s[0][0];
+  const double sc = 1.0 / nrm;
+  for (int i = tid; i < n; i += AR_NT) wg[i] = w[i] * sc;
+  if (b == 0) {
+    if (tid <= j) h[tid] = h_s[tid];
+    if (tid == j + 1) h[tid] = nrm;
   }
 }
 
@@ -220,10 +335,11 @@ struct Arena {
 inline size_t al8(size_t count) { return (count * sizeof(double) + 255) & ~size_t(255); }
 
 // device buffers of one GMRES: V (N x (nr+1)), w (N), gm (4096 doubles:
-// Hessenberg columns, rotations, rhs, Ritz coefficients, R), red (64), h
-// (pinned host, >= 4 doubles)
+// Hessenberg columns, Ritz coefficients), red (64), h (pinned host, >= 1024
+// doubles), words (AR_WORDS 64-bit words: the Arnoldi steps' exchanges)
 struct GmresBufs {
   double *V, *w, *gm, *red, *h;
+  unsigned long long* words;
 };
 
 // GMRES(nr) x iters for L x = b (x0 = 0) with Arnoldi by classical
@@ -231,23 +347,68 @@ struct GmresBufs {
 // Householder GMRES of the reference minimises the same residual over the
 // same Krylov space, ttlocsolve.f90:509-682, tt_linalg.f90:651-845).
 // Returns whether the residual reached tol (false: stopped after iters
-// restarts, which the reference tolerates).
+// restarts, which the reference tolerates).  The Hessenberg columns come to the
+// host four steps at a time, which applies their Givens rotations and solves
+// for the coefficients (serial work on at most 61 numbers: a CUDA thread took
+// 10 us a column and 50 us a solve for it).
 template <class MV>
 bool gmres_cgs2(const MV& mv, i64 N, const double* b, double* x, double tol, int nr, int iters,
                 const GmresBufs& G, cudaStream_t s) {
-  double* H = G.gm;                    // Hessenberg column (first pass)
-  double* H2 = G.gm + 64;              // second Gram-Schmidt pass
-  double* cs = G.gm + 128;
-  double* sn = G.gm + 192;
-  double* g = G.gm + 256;
-  double* y = G.gm + 320;
-  double* hres = G.gm + 384;
-  double* Rm = G.gm + 448;             // (nr+1) x nr, nr <= 60
-  const int ldr = nr + 1;
+  double* H = G.gm;                    // four Hessenberg columns of AR_SLOTS
+  double* y = G.gm + 4 * AR_SLOTS;
   double* V = G.V;
   double* red = G.red;
-  double* h = G.h;
+  double* h = G.h;                     // pinned: scalars, then Hessenberg columns, then y
+  double* hH = h + 16;
+  double* hy = hH + 4 * AR_SLOTS;
+  std::vector<double> R((size_t)(nr + 1) * nr), cs(nr), sn(nr), g(nr + 1);
   auto sync = [&]() { TTG_CUDA(cudaStreamSynchronize(s)); };
+  static const int coop = [] {
+    int dev = 0, nsm = 0, per = 0;
+    if (cudaFuncSetAttribute(arnoldi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             AR_CHUNK * (int)sizeof(double)) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, arnoldi_kernel, AR_NT,
+                                                      AR_CHUNK * sizeof(double)) != cudaSuccess)
+      return 0;
+    return nsm * per;
+  }();
+  // CTAs: at least 128 rows each, at most one per SM and AR_CHUNK rows (larger
+  // problems take the separate products)
+  const int ctas = (int)std::max<i64>(1, std::min<i64>(std::min(AR_G, coop), (N + 127) / 128));
+  int chunk = (int)std::min<i64>((N + ctas - 1) / ctas, AR_CHUNK + 1);
+  const bool fused = coop > 0 && chunk <= AR_CHUNK;
+  unsigned int epoch = 1;
+  if (fused) TTG_CUDA(cudaMemsetAsync(G.words, 0, AR_WORDS * sizeof(unsigned long long), s));
+  auto arnoldi = [&](int j, double* hcol) {
+    double* wv = V + N * (j + 1);
+    if (fused) {
+      i64 NN = N;
+      int jj = j;
+      double *vv = V, *hh = hcol;
+      unsigned long long* ww = G.words;
+      void* args[] = {&NN, &jj, &chunk, &vv, &hh, &ww, &epoch};
+      TTG_CUDA(cudaLaunchCooperativeKernel((const void*)arnoldi_kernel, dim3(ctas), dim3(AR_NT), args,
+                                           (size_t)chunk * sizeof(double), s));
+      ++g_launches;
+      epoch += 3;
+      return;
+    }
+    double* h2 = G.gm + 5 * AR_SLOTS;
+    gemm_tn_small(j + 1, 1, N, V, N, wv, N, hcol, j + 2, 1.0, 0.0, s);
+    gemm_nn_small(N, 1, j + 1, V, N, hcol, j + 2, wv, N, -1.0, 1.0, s);
+    gemm_tn_small(j + 1, 1, N, V, N, wv, N, h2, j + 2, 1.0, 0.0, s);
+    gemm_nn_small(N, 1, j + 1, V, N, h2, j + 2, wv, N, -1.0, 1.0, s);
+    axpy_kernel<<<1, 64, 0, s>>>(j + 1, 1.0, h2, hcol);
+    TTG_CHECK_LAUNCH();
+    sqnorm_cols(N, wv, N, 1, red, s);
+    sqrt_kernel<<<1, 32, 0, s>>>(1, red);
+    TTG_CHECK_LAUNCH();
+    TTG_CUDA(cudaMemcpyAsync(hcol + j + 1, red, sizeof(double), cudaMemcpyDeviceToDevice, s));
+    scal_kernel<<<eb(N), 256, 0, s>>>(N, red, 1, wv);
+    TTG_CHECK_LAUNCH();
+  };
   TTG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * N, s));
   double nrmb = -1.0, curres = 1.0;
   for (int it = 0; it < iters; ++it) {
@@ -266,50 +427,52 @@ bool gmres_cgs2(const MV& mv, i64 N, const double* b, double* x, double tol, int
     TTG_CUDA(cudaMemcpyAsync(red + 8, h + 1, sizeof(double), cudaMemcpyHostToDevice, s));
     scal_kernel<<<eb(N), 256, 0, s>>>(N, red + 8, 0, V);
     TTG_CHECK_LAUNCH();
-    TTG_CUDA(cudaMemsetAsync(g, 0, sizeof(double) * 64, s));
-    h[2] = beta;
-    TTG_CUDA(cudaMemcpyAsync(g, h + 2, sizeof(double), cudaMemcpyHostToDevice, s));
+    std::fill(g.begin(), g.end(), 0.0);
+    g[0] = beta;
     int jdone = 0;
     for (int j = 0; j < nr; ++j) {
-      double* vj = V + N * j;
-      double* wv = V + N * (j + 1);
-      mv(vj, wv, 1);
-      // CGS2 against V[:, 0..j]
-      gemm_tn_small(j + 1, 1, N, V, N, wv, N, H, j + 2, 1.0, 0.0, s);
-      gemm_nn_small(N, 1, j + 1, V, N, H, j + 2, wv, N, -1.0, 1.0, s);
-      gemm_tn_small(j + 1, 1, N, V, N, wv, N, H2, j + 2, 1.0, 0.0, s);
-      gemm_nn_small(N, 1, j + 1, V, N, H2, j + 2, wv, N, -1.0, 1.0, s);
-      axpy_kernel<<<1, 64, 0, s>>>(j + 1, 1.0, H2, H);
-      TTG_CHECK_LAUNCH();
-      sqnorm_cols(N, wv, N, 1, red, s);
-      sqrt_kernel<<<1, 32, 0, s>>>(1, red);
-      TTG_CHECK_LAUNCH();
-      TTG_CUDA(cudaMemcpyAsync(H + j + 1, red, sizeof(double), cudaMemcpyDeviceToDevice, s));
-      scal_kernel<<<eb(N), 256, 0, s>>>(N, red, 1, wv);
-      TTG_CHECK_LAUNCH();
-      givens_kernel<<<1, 1, 0, s>>>(j, H, cs, sn, g, Rm, ldr, hres + j);
-      TTG_CHECK_LAUNCH();
+      mv(V + N * j, V + N * (j + 1), 1);
+      arnoldi(j, H + AR_SLOTS * (j & 3));
       jdone = j + 1;
-      // the residual estimates are read back every 4th step (and at the
+      // the Hessenberg columns are read back every 4th step (and at the
       // last): a host synchronisation per step would bound the solve by
       // latency.  The first step below tol ends the cycle exactly as a
       // per-step test would: the Givens-reduced R and g of steps 0..j are
       // final after step j, so the extra steps only cost their matvecs.
       if (jdone % 4 == 0 || jdone == nr) {
         const int j0 = ((jdone - 1) / 4) * 4;
-        TTG_CUDA(cudaMemcpyAsync(h, hres + j0, sizeof(double) * (jdone - j0),
+        TTG_CUDA(cudaMemcpyAsync(hH, H, sizeof(double) * AR_SLOTS * (jdone - j0),
                                  cudaMemcpyDeviceToHost, s));
         sync();
         bool conv = false;
-        for (int q = 0; q < jdone - j0; ++q) {
-          curres = h[q] / nrmb;
-          if (curres < tol) { jdone = j0 + q + 1; conv = true; break; }
+        for (int q = j0; q < jdone && !conv; ++q) {
+          // previous rotations, a new one, g
+          double* c = hH + AR_SLOTS * (q - j0);
+          for (int i = 0; i < q; ++i) {
+            const double a = c[i], e = c[i + 1];
+            c[i] = cs[i] * a + sn[i] * e;
+            c[i + 1] = -sn[i] * a + cs[i] * e;
+          }
+          const double a = c[q], e = c[q + 1], den = std::hypot(a, e);
+          cs[q] = den > 0 ? a / den : 1.0;
+          sn[q] = den > 0 ? e / den : 0.0;
+          c[q] = den;
+          g[q + 1] = -sn[q] * g[q];
+          g[q] = cs[q] * g[q];
+          for (int i = 0; i <= q; ++i) R[i + (size_t)(nr + 1) * q] = c[i];
+          curres = std::fabs(g[q + 1]) / nrmb;
+          if (curres < tol) { jdone = q + 1; conv = true; }
         }
         if (conv) break;
       }
     }
-    trsv_kernel<<<1, 1, 0, s>>>(jdone, Rm, ldr, g, y);
-    TTG_CHECK_LAUNCH();
+    for (int i = jdone - 1; i >= 0; --i) {
+      double v = g[i];
+      for (int k = i + 1; k < jdone; ++k) v -= R[i + (size_t)(nr + 1) * k] * hy[k];
+      hy[i] = v / R[i + (size_t)(nr + 1) * i];
+    }
+    // hy is rewritten only after a later synchronisation
+    TTG_CUDA(cudaMemcpyAsync(y, hy, sizeof(double) * jdone, cudaMemcpyHostToDevice, s));
     gemm_nn_small(N, 1, jdone, V, N, y, jdone, x, N, 1.0, 1.0, s);
     if (curres < tol) return true;
   }
@@ -363,6 +526,7 @@ class AmenSolver {
   std::vector<double*> A_;
   std::vector<double*> pxax_, pxy_, pzax_, pzy_;
   size_t tau_n_ = 0;   // elements of tau_
+  unsigned long long* words_ = nullptr;   // exchanges of the Arnoldi steps
   double *tmpA_, *tmpB_, *tmpC_, *R_, *tau_, *rhs_, *resid_, *sol_, *xnew_, *scr_, *svU_, *svS_,
       *svVt_, *svScr_, *cand_, *candY_, *red_, *V_, *w_, *gm_, *dense_;
   double* h_ = nullptr;   // pinned
@@ -476,7 +640,7 @@ void AmenSolver::gmres(const LocalDims& L, int k, const double* b, double* x, do
   const double* p1 = pxax_[k];
   const double* p2 = pxax_[k + 1];
   auto mv = [&](const double* in, double* out, int nv) { local_mv(L, p1, p2, k, in, out, nv); };
-  if (!gmres_cgs2(mv, N, b, x, tol, nr, P_.local_iters, GmresBufs{V_, w_, gm_, red_, h_}, s_))
+  if (!gmres_cgs2(mv, N, b, x, tol, nr, P_.local_iters, GmresBufs{V_, w_, gm_, red_, h_, words_}, s_))
     note_capped(ctx_, "dtt_amen_solve");
 }
 
@@ -494,7 +658,7 @@ void AmenSolver::gmres_split(const LocalDims& L, int k, const double* b, double*
   split_matvec_factory(L, pxax_[k], A_[k], pxax_[k + 1], kBatch, split_mem_, split_bytes_, s_,
                        &mvlow);
   auto mvs = [&](const double* in, double* out, int nv) { mvlow(in, out, nv); split_mv_ += nv; };
-  const GmresBufs G{V_, w_, gm_, red_, h_};
+  const GmresBufs G{V_, w_, gm_, red_, h_, words_};
   const double nb = norm2(b, N);
   TTG_CUDA(cudaMemsetAsync(x, 0, sizeof(double) * N, s_));
   TTG_CUDA(cudaMemcpyAsync(ir_r_, b, sizeof(double) * N, cudaMemcpyDeviceToDevice, s_));
@@ -636,7 +800,7 @@ void AmenSolver::run(AmenOut& out) {
   }
   total += 2 * al8(cmax) + al8(tcap) + al8(Nmax) * 5 + al8(cmax) + al8(tau_n_) + scr + 256;
   total += svds + 256 + 3 * al8(cmax) + al8(8192);
-  total += 2 * al8(Nmax * kBatch) + al8(Nmax * (nr + 1)) + al8(Nmax) + al8(4096) +
+  total += 2 * al8(Nmax * kBatch) + al8(Nmax * (nr + 1)) + al8(Nmax) + al8(4096) + al8(AR_WORDS) +
            al8((size_t)std::min<i64>(P_.max_full_size, 64) * 64) + (1 << 16);
   size_t splitb = 0;
   if (P_.method == TTG_METHOD_SPLIT) {
@@ -679,6 +843,7 @@ void AmenSolver::run(AmenOut& out) {
   V_ = mem_.take(Nmax * (nr + 1));
   red_ = mem_.take(64);
   gm_ = mem_.take(4096);
+  words_ = (unsigned long long*)mem_.take(AR_WORDS);
   dense_ = mem_.take(64 * 64);
   if (P_.method == TTG_METHOD_SPLIT) {
     split_mem_ = (void*)mem_.take(splitb / sizeof(double) + 128);
@@ -1048,6 +1213,7 @@ class AlsSolver {
   Arena mem_;
   std::vector<i64> n_, rx_, cap_;
   size_t tau_n_ = 0;   // elements of tau_
+  unsigned long long* words_ = nullptr;   // exchanges of the Arnoldi steps
   std::vector<double*> x_, A_, Y_, phiA_, phiy_;
   double *rhs_, *r0_, *sol_, *w_, *V_, *gm_, *red_, *kickY_, *kickB_, *tA_, *tB_, *tC_, *U_, *S_,
       *Vt_, *svScr_, *cand_, *candY_, *Um_, *Rm_, *Rq_, *tau_, *tmp_, *scr_, *du_, *dd_, *small_;
@@ -1214,7 +1380,8 @@ void AlsSolver::run(AmenOut& out) {
   size_t total = al8(at) + al8(yt);
   for (int k = 0; k < d; ++k) total += al8(cap_[k] * n_[k] * cap_[k + 1]);
   for (int k = 0; k <= d; ++k) total += al8(cap_[k] * cap_[k] * ra[k]) + al8(cap_[k] * ry[k]);
-  total += 4 * al8(Nmax) + al8(Nmax * (nr + 1)) + al8(4096) + al8(64) + al8(Cmax) + al8(KB) +
+  total += 4 * al8(Nmax) + al8(Nmax * (nr + 1)) + al8(4096) + al8(AR_WORDS) + al8(64) + al8(Cmax) +
+           al8(KB) +
            3 * al8(T) + al8(SVD) + al8(1024) + al8(SVD) + svs + 256 + 2 * al8(Nmax * kBatch) +
            al8(M2) + 2 * al8(M2) + al8(tau_n_) + al8(M2) + scr + 256 + al8(Mmax * 16) +
            al8(Mmax) + al8(1024) + al8(64) + (1 << 16);
@@ -1238,6 +1405,7 @@ void AlsSolver::run(AmenOut& out) {
   rhs_ = mem_.take(Nmax); r0_ = mem_.take(Nmax); sol_ = mem_.take(Nmax); w_ = mem_.take(Nmax);
   V_ = mem_.take(Nmax * (nr + 1));
   gm_ = mem_.take(4096);
+  words_ = (unsigned long long*)mem_.take(AR_WORDS);
   red_ = mem_.take(64);
   kickY_ = mem_.take(Cmax);
   kickB_ = mem_.take(KB);
@@ -1281,7 +1449,7 @@ void AlsSolver::run(AmenOut& out) {
     upd_left(i);
   }
 
-  const GmresBufs G{V_, w_, gm_, red_, h_};
+  const GmresBufs G{V_, w_, gm_, red_, h_, words_};
   double res_max = 0.0, last_res = 0.0, err_max = 0.0;
   int i = d - 1, dir = -1, swp = 1, kick = kick0;
   while (swp <= P_.nswp) {

@@ -16,44 +16,77 @@ static constexpr double RESTART_DROP = 1e-10;
 // ---------------------------------------------------------------------------
 constexpr int TS_MAXN = 16;
 
+// Sums of NV values over a warp, NV in {1, 2, 4, 8, 16}: while the values
+// outnumber the lanes that share them, each half of the lanes keeps half of the
+// values (a warp-wide FP64 addition holds its pipe 64 clocks; five per value
+// otherwise).  Lane l returns the sum of value (l * NV) >> 5.
+template <int NV>
+__device__ __forceinline__ double warp_sums(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int h = NV / 2; h > 0; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double give = up ? v[k] : v[k + h];
+      v[k] = (up ? v[k + h] : v[k]) + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
 // C (M x N, ldc) = alpha * A^T B + beta * C, A (K x M, lda), B (K x N, ldb),
-// N <= 16.  Grid (M, nk), one cluster of nk CTAs per column m of A: CTA
+// N <= NV <= 16.  Grid (M, nk), one cluster of nk CTAs per column m of A: CTA
 // (m, c) reduces k-chunk c against all N columns of B, then rank 0 adds the
 // nk partials in rank order (deterministic, no atomics, no pre-scaling pass).
-__global__ void tn_small_kernel(int M, int N, i64 K, const double* __restrict__ A, i64 lda,
-                                const double* __restrict__ B, i64 ldb, double* __restrict__ C,
-                                int ldc, double alpha, double beta, i64 kchunk) {
+// Bound by the latency of its loads: four k per step are requested together.
+template <int NV>
+__global__ void __launch_bounds__(256) tn_small_kernel(int M, int N, i64 K, const double* __restrict__ A,
+                                                       i64 lda, const double* __restrict__ B, i64 ldb,
+                                                       double* __restrict__ C, int ldc, double alpha,
+                                                       double beta, i64 kchunk) {
   namespace cgr = cooperative_groups;
   pdl_trigger();
   pdl_wait();
   const int m = blockIdx.x;
   const i64 k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
-  double acc[TS_MAXN];
+  double acc[NV];
 #pragma unroll
-  for (int n = 0; n < TS_MAXN; ++n) acc[n] = 0.0;
+  for (int n = 0; n < NV; ++n) acc[n] = 0.0;
   const double* a = A + lda * m;
-  for (i64 k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+  constexpr int UN = NV <= 4 ? 4 : 2;
+  i64 k = k0 + threadIdx.x;
+  for (; k + (UN - 1) * 256 < k1; k += UN * 256) {
+    double av[UN], bv[UN][NV];
+#pragma unroll
+    for (int u = 0; u < UN; ++u) {
+      av[u] = a[k + 256 * u];
+#pragma unroll
+      for (int n = 0; n < NV; ++n) bv[u][n] = n < N ? B[k + 256 * u + ldb * n] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < UN; ++u)
+#pragma unroll
+      for (int n = 0; n < NV; ++n)
+        if (n < N) acc[n] = fma(av[u], bv[u][n], acc[n]);
+  }
+  for (; k < k1; k += 256) {
     const double av = a[k];
 #pragma unroll
-    for (int n = 0; n < TS_MAXN; ++n)
+    for (int n = 0; n < NV; ++n)
       if (n < N) acc[n] = fma(av, B[k + ldb * n], acc[n]);
   }
-  __shared__ double red[TS_MAXN][8];
-  __shared__ double part[TS_MAXN];
+  __shared__ double red[NV][8];
+  __shared__ double part[NV];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int n = 0; n < TS_MAXN; ++n) {
-    if (n >= N) break;
-    double v = acc[n];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[n][wid] = v;
-  }
+  const double t = warp_sums<NV>(acc);
+  if ((lane & (32 / NV - 1)) == 0) red[lane * NV >> 5][wid] = t;
   __syncthreads();
   if (threadIdx.x < N) {
-    double v = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) v += red[threadIdx.x][w];
-    part[threadIdx.x] = v;
+    const double* r = red[threadIdx.x];
+    part[threadIdx.x] = ((r[0] + r[1]) + (r[2] + r[3])) + ((r[4] + r[5]) + (r[6] + r[7]));
   }
   cgr::cluster_group cl = cgr::this_cluster();
   cl.sync();
@@ -76,12 +109,21 @@ void gemm_tn_small(int M, int N, i64 K, const double* A, i64 lda, const double* 
   i64 nk = std::max<i64>(1, std::min<i64>((304 + M - 1) / M, (K + 255) / 256));
   nk = std::min<i64>(nk, kMaxCluster);
   i64 kchunk = std::max<i64>(1, (K + nk - 1) / nk);
-  launch_ex(tn_small_kernel, dim3(M, (unsigned)nk), dim3(256), dim3(1, (unsigned)nk, 1), true, 0, s,
-            M, N, K, A, lda, B, ldb, C, ldc, alpha, beta, kchunk);
+  auto go = [&](auto kern) {
+    launch_ex(kern, dim3(M, (unsigned)nk), dim3(256), dim3(1, (unsigned)nk, 1), true, 0, s, M, N, K, A,
+              lda, B, ldb, C, ldc, alpha, beta, kchunk);
+  };
+  if (N == 1) go(tn_small_kernel<1>);
+  else if (N == 2) go(tn_small_kernel<2>);
+  else if (N <= 4) go(tn_small_kernel<4>);
+  else if (N <= 8) go(tn_small_kernel<8>);
+  else go(tn_small_kernel<16>);
 }
 
 // C (R x N, ldc) = alpha * A (R x K, lda) * B (K x N, ldb) + beta * C, with
-// K <= 128 and N <= 16: one thread per row, B in shared memory.
+// K <= 128 and N <= 16: one thread per row, B in shared memory.  Bound by the
+// latency of its loads: eight columns of A are requested together (one by one,
+// the K = 40 products of a GMRES cycle took 24 us).
 __global__ void nn_small_kernel(i64 R, int N, int K, const double* __restrict__ A, i64 lda,
                                 const double* __restrict__ B, int ldb, double* __restrict__ C,
                                 i64 ldc, double alpha, double beta) {
@@ -94,11 +136,18 @@ __global__ void nn_small_kernel(i64 R, int N, int K, const double* __restrict__ 
     double acc[TS_MAXN];
 #pragma unroll
     for (int n = 0; n < TS_MAXN; ++n) acc[n] = 0.0;
-    for (int k = 0; k < K; ++k) {
-      const double av = A[r + lda * k];
+    constexpr int UN = 8;
+    for (int k = 0; k < K; k += UN) {
+      double av[UN];
 #pragma unroll
-      for (int n = 0; n < TS_MAXN; ++n)
-        if (n < N) acc[n] = fma(av, Bs[k + K * n], acc[n]);
+      for (int u = 0; u < UN; ++u) av[u] = k + u < K ? A[r + lda * (k + u)] : 0.0;
+#pragma unroll
+      for (int u = 0; u < UN; ++u) {
+        if (k + u >= K) break;
+#pragma unroll
+        for (int n = 0; n < TS_MAXN; ++n)
+          if (n < N) acc[n] = fma(av[u], Bs[k + u + K * n], acc[n]);
+      }
     }
 #pragma unroll
     for (int n = 0; n < TS_MAXN; ++n) {
@@ -113,8 +162,9 @@ void gemm_nn_small(i64 R, int N, int K, const double* A, i64 lda, const double* 
                    double* C, i64 ldc, double alpha, double beta, cudaStream_t s) {
   if (R <= 0 || N <= 0) return;
   TTG_REQUIRE(N <= TS_MAXN && K <= 128, "gemm_nn_small: N > 16 or K > 128");
-  int blocks = (int)std::min<i64>(2048, (R + 127) / 128);
-  launch_pdl(nn_small_kernel, dim3(blocks), dim3(128), 0, s, R, N, K, A, lda, B, ldb, C, ldc, alpha,
+  const int nt = R < 128 * 152 ? 64 : 128;   // few rows: half the block, twice the SMs
+  int blocks = (int)std::min<i64>(2048, (R + nt - 1) / nt);
+  launch_pdl(nn_small_kernel, dim3(blocks), dim3(nt), 0, s, R, N, K, A, lda, B, ldb, C, ldc, alpha,
              beta);
 }
 

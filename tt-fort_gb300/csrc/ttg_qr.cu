@@ -15,16 +15,14 @@
 //   cluster form  G <= 8 CTAs of one cluster exchange through distributed
 //                 shared memory, one cluster barrier per column;
 //   grid form     up to one CTA per SM (cooperative launch): parts go to
-//                 global memory, CTA j % G adds those of column j in CTA order
-//                 and hands the sum to all.  Each 32-bit half of a value
-//                 travels in one 64-bit word with the number of its exchange,
-//                 so a reader knows from the word itself that it is there and
-//                 no barrier or fence is needed (a step of the 5248 x 86 block
-//                 took 7.8 us with two grid barriers, 7.0 so).
-//                 Waits are bounded; a CTA whose wait ran out fills its rows
+//                 global memory as tagged words (ttg_words.cuh), CTA j % G adds
+//                 those of column j in CTA order and hands the sum to all (a
+//                 step of the 5248 x 86 block took 7.8 us with two grid
+//                 barriers, 7.0 so).  A CTA whose wait ran out fills its rows
 //                 with NaN.
 // Both add the parts in a fixed order, so results are bit-reproducible.
 #include "ttg_common.cuh"
+#include "ttg_words.cuh"
 #include <algorithm>
 
 namespace ttg {
@@ -105,7 +103,6 @@ template <> struct C<double2> {
 
 constexpr int NT = 256;
 constexpr int GMAX = 152;            // CTAs of the grid form
-constexpr long long SPIN_LIMIT = 1ll << 24;
 
 // elements of T in shared memory: rows, reflector, next column, sums and row of
 // the current column, tau, and (cluster form) this CTA's parts and row, twice
@@ -127,7 +124,7 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.x, r = min(n, m);
-  constexpr int W = (int)(sizeof(T) / 4);               // exchange words of a value
+  constexpr int W = words::count<T>;
   const int chunk = (n + G - 1) / G, ld = chunk | 1;
   const int nloc = b < n ? (n - b + G - 1) / G : 0;     // rows b, b + G, ...
   T* A = reinterpret_cast<T*>(dyn);
@@ -149,48 +146,19 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
     for (int i = lane; i < nloc; i += 32) A[(size_t)ld * c + i] = Ag[(i64)n * c + b + (i64)G * i];
   __syncthreads();
 
-  // grid form: words of exchange number `epoch` (from 1; the buffers start at 0)
-  auto put_words = [&](unsigned long long* w, T v) {
-    const unsigned int* h = reinterpret_cast<const unsigned int*>(&v);
-    const unsigned long long tag = (unsigned long long)epoch << 32;
-#pragma unroll
-    for (int k = 0; k < W; k += 2)
-      asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(w + k), "l"(tag | h[k]),
-                   "l"(tag | h[k + 1])
-                   : "memory");
-  };
-  auto load_words = [&](const unsigned long long* w, unsigned long long (&x)[W]) {
-#pragma unroll
-    for (int k = 0; k < W; k += 2)
-      asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x[k]), "=l"(x[k + 1]) : "l"(w + k) : "memory");
-  };
-  // x holds a first load of w: the value once its words carry this exchange's
-  // number; false (nothing in v) once the wait ran out here or in another CTA
-  auto take_words = [&](const unsigned long long* w, unsigned long long (&x)[W], T& v) {
-    unsigned int* h = reinterpret_cast<unsigned int*>(&v);
-    for (long long spin = 0; spin < SPIN_LIMIT; ++spin) {
-      bool all = true;
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        h[k] = (unsigned int)x[k];
-        all = all && (unsigned int)(x[k] >> 32) == epoch;
-      }
-      if (all) return true;
-      if ((spin & 255) == 255 && *(volatile unsigned int*)bar != 0u) break;
-      load_words(w, x);
-    }
-    atomicExch(bar, 1u);
+  auto got = [&](const unsigned long long* w, unsigned long long (&x)[W], T& v) {
+    if (words::take<T>(w, x, v, epoch, bar)) return true;
     s_fail = 1;
     return false;
   };
   // the parts that publish() left for columns [j0, j1) and (with_row) the row
   // beside them: sums to S, row to row
   auto publish = [&](int j, T s) {
-    if (GRID) put_words(part + ((size_t)b * m + j) * W, s);
+    if (GRID) words::put(part + ((size_t)b * m + j) * W, s, epoch);
     else mine[(size_t)par * m + j] = s;
   };
   auto publish_row = [&](int j, T v) {
-    if (GRID) put_words(rowg + ((size_t)par * m + j) * W, v);
+    if (GRID) words::put(rowg + ((size_t)par * m + j) * W, v, epoch);
     else mine[(size_t)(2 + par) * m + j] = v;
   };
   // for the factorisation (with_row) warp 0 goes straight on to the reflector
@@ -205,25 +173,25 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
         unsigned long long x[QL][W];
 #pragma unroll
         for (int k = 0; k < QL; ++k)
-          if (lane + 32 * k < G) load_words(part + ((size_t)(lane + 32 * k) * m + j) * W, x[k]);
+          if (lane + 32 * k < G) words::load<T>(part + ((size_t)(lane + 32 * k) * m + j) * W, x[k]);
         T t = O::zero();
 #pragma unroll
         for (int k = 0; k < QL; ++k) {
           T v;
-          if (lane + 32 * k < G && take_words(part + ((size_t)(lane + 32 * k) * m + j) * W, x[k], v))
+          if (lane + 32 * k < G && got(part + ((size_t)(lane + 32 * k) * m + j) * W, x[k], v))
             t = O::add(t, v);
         }
         __syncwarp();
         for (int o = 16; o > 0; o >>= 1) t = O::add(t, O::shfl(t, o));
-        if (lane == 0) put_words(tot + (size_t)j * W, t);
+        if (lane == 0) words::put(tot + (size_t)j * W, t, epoch);
       }
       for (int j = j0 + tid; j < j1; j += NT) {
         T v;
         unsigned long long x[W], y[W];
-        load_words(tot + (size_t)j * W, x);
-        if (with_row) load_words(rowg + ((size_t)par * m + j) * W, y);
-        if (take_words(tot + (size_t)j * W, x, v)) S[j] = v;
-        if (with_row && take_words(rowg + ((size_t)par * m + j) * W, y, v)) row[j] = v;
+        words::load<T>(tot + (size_t)j * W, x);
+        if (with_row) words::load<T>(rowg + ((size_t)par * m + j) * W, y);
+        if (got(tot + (size_t)j * W, x, v)) S[j] = v;
+        if (with_row && got(rowg + ((size_t)par * m + j) * W, y, v)) row[j] = v;
       }
     } else {
       cgr::cluster_group cl = cgr::this_cluster();
