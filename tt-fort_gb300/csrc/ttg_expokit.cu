@@ -137,10 +137,20 @@ __global__ void ne_sign_kernel(i64 total, const double2* X, double2* S) {
   }
 }
 
-// h(i) = max_j |X(i,j)|; top-t rows by (h desc, index asc); out: ind[0..t),
-// red[0] = h of the top row, red[1] = h(ibest).  One CTA of TOPK_NT threads.
+// h(i) = max_j |X(i,j)|, over the whole GPU: a modulus is some thirty FP64
+// operations, and one SM has two per clock (n = 2048, t = 4: 20 of the 32 us
+// that the selection below took with them)
+__global__ void ne_rowmax_kernel(i64 n, int t, const double2* __restrict__ X, double* __restrict__ h) {
+  for (i64 i = blockIdx.x * (i64)blockDim.x + threadIdx.x; i < n; i += (i64)gridDim.x * blockDim.x) {
+    double m = 0.0;
+    for (int j = 0; j < t; ++j) m = fmax(m, cabsd(X[i + n * j]));
+    h[i] = m;
+  }
+}
+// top-t rows by (h desc, index asc); out: ind[0..t), red[0] = h of the top row,
+// red[1] = h(ibest).  One CTA of TOPK_NT threads.
 constexpr int TOPK_NT = 256;
-__global__ void __launch_bounds__(TOPK_NT) ne_topk_kernel(i64 n, int t, const double2* X, int ibest,
+__global__ void __launch_bounds__(TOPK_NT) ne_topk_kernel(i64 n, int t, const double* hrow, int ibest,
                                                           int* ind, double* red_out) {
   __shared__ double cv[TOPK_NT * 4];
   __shared__ long long ci[TOPK_NT * 4];
@@ -152,8 +162,7 @@ __global__ void __launch_bounds__(TOPK_NT) ne_topk_kernel(i64 n, int t, const do
   long long li[4];
   for (int q = 0; q < 4; ++q) { lv[q] = -1.0; li[q] = -1; }
   for (i64 i = tid; i < n; i += blockDim.x) {
-    double h = 0.0;
-    for (int j = 0; j < t; ++j) h = fmax(h, cabsd(X[i + n * j]));
+    const double h = hrow[i];
     if (i == ibest) red_out[1] = h;
     // insert (h, i) into the local sorted list (desc h, asc index)
     for (int q = 0; q < t; ++q) {
@@ -259,7 +268,10 @@ double znormest_dev(ExpWork& w, i64 n, int t0, const ZMatvecFn& mv, const ZMatve
     } else {
       std::swap(w.X, w.Y);
     }
-    ne_topk_kernel<<<1, TOPK_NT, 0, s>>>(n, t, w.X, ibest, w.ired, w.red);
+    double* hrow = (double*)w.tmp;
+    ne_rowmax_kernel<<<(int)std::min<i64>(1024, (n + 31) / 32), 32, 0, s>>>(n, t, w.X, hrow);
+    TTG_CHECK_LAUNCH();
+    ne_topk_kernel<<<1, TOPK_NT, 0, s>>>(n, t, hrow, ibest, w.ired, w.red);
     TTG_CHECK_LAUNCH();
     TTG_CUDA(cudaMemcpyAsync(h, w.red, sizeof(double) * 2, cudaMemcpyDeviceToHost, s));
     TTG_CUDA(cudaMemcpyAsync(h + 8, w.ired, sizeof(int) * t, cudaMemcpyDeviceToHost, s));
@@ -294,74 +306,108 @@ __global__ void znrm2_kernel(i64 n, const double2* x, double* out) {
   if (threadIdx.x == 0) out[0] = sqrt(acc);
 }
 
-// Modified Gram-Schmidt of column j+1 of V against columns 0..j (one CTA).
+// Modified Gram-Schmidt of column j+1 of V against columns 0..j: one cluster of
+// CTAs, each thread holding E entries of the new column in registers and
+// requesting the next column of V while the sums of this one are formed.
 // flag[0] = mbrkdwn (0 while no breakdown): once set, later steps do nothing.
-__global__ void mgs_kernel(i64 n, int j, int mh, double2* V, double2* H, int* flag,
-                           double break_tol) {
-  __shared__ double red[33];
+// Bound by its chain of j + 2 sums (5 additions in a warp, 3 over the warps, a
+// cluster barrier, 3 over the CTAs: about 1.4 us each); measured per step on
+// GB300 at n = 2048 (n = 64): 33 (15) us with a grid barrier per sum (one warp
+// on global memory), 14 (8) us so.
+constexpr int MGC_NT = 256;
+template <int E>
+__global__ void __launch_bounds__(MGC_NT) mgs_cluster_kernel(i64 n, int j, int mh, double2* V, double2* H,
+                                                             int* flag, double break_tol) {
+  cg::cluster_group cl = cg::this_cluster();
+  __shared__ double2 wsum_s[MGC_NT / 32];
+  __shared__ double2 mine[2];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  const int C = gridDim.x, b = blockIdx.x;
+  // a breakdown is flagged after the last cluster barrier of an earlier launch
   if (flag[0] != 0) return;
   double2* p = V + n * (j + 1);
-  for (int i = 0; i <= j; ++i) {
-    const double2* vi = V + n * i;
-    double ar = 0.0, ai = 0.0;
-    for (i64 k = threadIdx.x; k < n; k += blockDim.x) {
-      // conj(vi) * p
-      ar += vi[k].x * p[k].x + vi[k].y * p[k].y;
-      ai += vi[k].x * p[k].y - vi[k].y * p[k].x;
-    }
-    ar = bsum(ar, red);
-    ai = bsum(ai, red);
-    const double2 hij = make_double2(ar, ai);
-    for (i64 k = threadIdx.x; k < n; k += blockDim.x) p[k] = csub(p[k], cmul(hij, vi[k]));
-    if (threadIdx.x == 0) H[i + (i64)mh * j] = hij;
+  const i64 i0 = (i64)b * blockDim.x + tid, step = (i64)C * blockDim.x;
+  double2 x[E], v[E], nx[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const i64 i = i0 + e * step;
+    x[e] = i < n ? p[i] : make_double2(0.0, 0.0);
+    v[e] = i < n ? V[i] : make_double2(0.0, 0.0);
+  }
+  int par = 0;
+  // sum of (a, c) over all threads of the cluster, the same in every thread
+  auto total = [&](double a, double c) {
+    // lanes below 16 carry a, the others c
+    double t = (lane & 16 ? c : a) + __shfl_xor_sync(0xffffffffu, lane & 16 ? a : c, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 15) == 0) reinterpret_cast<double*>(&wsum_s[warp])[lane >> 4] = t;
     __syncthreads();
-  }
-  double acc = 0.0;
-  for (i64 k = threadIdx.x; k < n; k += blockDim.x) acc += cabs2(p[k]);
-  const double nrm = sqrt(bsum(acc, red));
-  if (nrm <= break_tol) {
-    if (threadIdx.x == 0) flag[0] = j + 1;
-    return;
-  }
-  if (threadIdx.x == 0) H[(j + 1) + (i64)mh * j] = make_double2(nrm, 0.0);
-  const double inv = 1.0 / nrm;
-  for (i64 k = threadIdx.x; k < n; k += blockDim.x) p[k] = cscale(p[k], inv);
-}
-
-// The same step in one warp, for small vectors (S-step problems): warp
-// shuffles only, no block barriers.
-__global__ void mgs_warp_kernel(i64 n, int j, int mh, double2* V, double2* H, int* flag,
-                                double break_tol) {
-  if (flag[0] != 0) return;
-  double2* p = V + n * (j + 1);
-  const int lane = threadIdx.x;
-  for (int i = 0; i <= j; ++i) {
-    const double2* vi = V + n * i;
-    double ar = 0.0, ai = 0.0;
-    for (i64 k = lane; k < n; k += 32) {
-      const double2 a = vi[k], c = p[k];
-      ar += a.x * c.x + a.y * c.y;
-      ai += a.x * c.y - a.y * c.x;
+    if (warp == 0) {
+      // lane: component lane >> 4, warp lane & 15
+      double u = (lane & 15) < nw ? reinterpret_cast<double*>(&wsum_s[lane & 15])[lane >> 4] : 0.0;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+      if ((lane & 15) == 0) reinterpret_cast<double*>(&mine[par])[lane >> 4] = u;
     }
-    const double2 hij = make_double2(wsum(ar), wsum(ai));
-    for (i64 k = lane; k < n; k += 32) p[k] = csub(p[k], cmul(hij, vi[k]));
-    if (lane == 0) H[i + (i64)mh * j] = hij;
-    __syncwarp();
+    if (C == 1) {
+      __syncthreads();
+      const double2 r = mine[par];
+      par ^= 1;
+      return r;
+    }
+    cl.sync();
+    // lane: component lane >> 4, CTA lane & 7
+    double u = (lane & 7) < C ? reinterpret_cast<double*>(cl.map_shared_rank(&mine[par], lane & 7))[lane >> 4] : 0.0;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) u += __shfl_xor_sync(0xffffffffu, u, o);
+    par ^= 1;
+    return make_double2(__shfl_sync(0xffffffffu, u, 0), __shfl_sync(0xffffffffu, u, 16));
+  };
+  for (int i = 0; i <= j; ++i) {
+    double ar = 0.0, ai = 0.0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const i64 k = i0 + e * step;
+      nx[e] = (i < j && k < n) ? V[n * (i + 1) + k] : make_double2(0.0, 0.0);
+      ar = fma(v[e].x, x[e].x, ar);     // conj(v) x
+      ar = fma(v[e].y, x[e].y, ar);
+      ai = fma(v[e].x, x[e].y, ai);
+      ai = fma(-v[e].y, x[e].x, ai);
+    }
+    const double2 h = total(ar, ai);
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      x[e].x = fma(-h.x, v[e].x, x[e].x);
+      x[e].x = fma(h.y, v[e].y, x[e].x);
+      x[e].y = fma(-h.x, v[e].y, x[e].y);
+      x[e].y = fma(-h.y, v[e].x, x[e].y);
+      v[e] = nx[e];
+    }
+    if (b == 0 && tid == 0) H[i + (i64)mh * j] = h;
   }
   double acc = 0.0;
-  for (i64 k = lane; k < n; k += 32) acc += cabs2(p[k]);
-  const double nrm = sqrt(wsum(acc));
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc = fma(x[e].x, x[e].x, fma(x[e].y, x[e].y, acc));
+  const double nrm = sqrt(total(acc, 0.0).x);
+  if (C > 1) cl.sync();                 // no CTA leaves, or flags, while another still reads
   if (nrm <= break_tol) {
-    if (lane == 0) flag[0] = j + 1;
+    if (b == 0 && tid == 0) flag[0] = j + 1;
+    // the reference leaves the orthogonalised column
+#pragma unroll
+    for (int e = 0; e < E; ++e)
+      if (i0 + e * step < n) p[i0 + e * step] = x[e];
     return;
   }
-  if (lane == 0) H[(j + 1) + (i64)mh * j] = make_double2(nrm, 0.0);
+  if (b == 0 && tid == 0) H[(j + 1) + (i64)mh * j] = make_double2(nrm, 0.0);
   const double inv = 1.0 / nrm;
-  for (i64 k = lane; k < n; k += 32) p[k] = cscale(p[k], inv);
+#pragma unroll
+  for (int e = 0; e < E; ++e)
+    if (i0 + e * step < n) p[i0 + e * step] = cscale(x[e], inv);
 }
 
-// The same modified Gram-Schmidt step spread over the CTAs of a cooperative
-// grid: FP64 runs at two FMAs per clock per SM on GB300, so one CTA would
+// The same step for columns beyond a cluster's registers, spread over the CTAs
+// of a cooperative grid: FP64 runs at two FMAs per clock per SM on GB300, so one CTA would
 // leave the step FP64-bound on a single SM.  Each CTA owns a contiguous slice
 // of the vector; per column the slices' partial dot products go to their own
 // slots of part (round r uses part[r * gridDim.x ...]), and after a grid
@@ -434,17 +480,20 @@ static void mgs_step(ExpWork& w, i64 n, int j, int mh, double break_tol, cudaStr
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, mgs_coop_kernel, MGS_NT, 0);
     return std::max(1, std::min(64, per * sms));
   }();
+  if (n <= 4 * kMaxCluster * MGC_NT) {
+    // one entry a thread while the cluster lasts; 64 threads for the smallest
+    const int nt = n <= 64 ? 64 : (n <= 128 ? 128 : MGC_NT);
+    const int C = (int)std::min<i64>(kMaxCluster, (n + nt - 1) / nt);
+    const i64 e = (n + (i64)C * nt - 1) / ((i64)C * nt);
+    auto go = [&](auto kern) {
+      launch_ex(kern, dim3(C), dim3(nt), dim3(C, 1, 1), false, 0, s, n, j, mh, w.V, w.H, w.ired, break_tol);
+    };
+    if (e <= 1) go(mgs_cluster_kernel<1>);
+    else if (e <= 2) go(mgs_cluster_kernel<2>);
+    else go(mgs_cluster_kernel<4>);
+    return;
+  }
   const int G = (int)std::max<i64>(1, std::min<i64>(G_MAX, (n + 2 * MGS_NT - 1) / (2 * MGS_NT)));
-  if (n <= 1024) {
-    mgs_warp_kernel<<<1, 32, 0, s>>>(n, j, mh, w.V, w.H, w.ired, break_tol);
-    TTG_CHECK_LAUNCH();
-    return;
-  }
-  if (G == 1) {
-    mgs_kernel<<<1, 1024, 0, s>>>(n, j, mh, w.V, w.H, w.ired, break_tol);
-    TTG_CHECK_LAUNCH();
-    return;
-  }
   double2* part = w.part;
   void* args[] = {&n, &j, &mh, &w.V, &w.H, &w.ired, &break_tol, &part};
   TTG_CUDA(cudaLaunchCooperativeKernel((const void*)mgs_coop_kernel, dim3(G), dim3(MGS_NT), args, 0, s));
