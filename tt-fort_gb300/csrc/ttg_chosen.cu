@@ -102,7 +102,7 @@ __global__ void col_dots_kernel(i64 N, const double* __restrict__ U, const doubl
 static void col_dots(i64 N, int t, const double* U, const double* V, double* out, double* part,
                      unsigned int* count, cudaStream_t s) {
   TTG_REQUIRE(t <= CG_MAXT, "col_dots: too many columns");
-  int bx = (int)std::max<i64>(1, std::min<i64>(CG_MAXBX, (N + 2047) / 2048));
+  int bx = (int)std::max<i64>(1, std::min<i64>(CG_MAXBX, (N + 511) / 512));
   launch_pdl(col_dots_kernel, dim3(bx, t), dim3(256), 0, s, N, U, V, out, part, count);
 }
 
@@ -125,6 +125,7 @@ __global__ void shift_kernel(i64 N, int t, const double* __restrict__ theta,
 // projection of the CG step fused with its p^T q (deterministic grid sum:
 // part t x gridDim.x, one counter)
 constexpr int PD_MAXT = 16;
+template <int NV>
 __global__ void __launch_bounds__(128) proj_dot_kernel(i64 N, int t, int nb,
                                                        const double* __restrict__ X,
                                                        const double* __restrict__ C,
@@ -134,41 +135,40 @@ __global__ void __launch_bounds__(128) proj_dot_kernel(i64 N, int t, int nb,
                                                        double* __restrict__ part,
                                                        unsigned int* __restrict__ count) {
   __shared__ double Cs[PD_MAXT * PD_MAXT];
-  __shared__ double red[4][PD_MAXT];
+  __shared__ double red[4][NV];
   pdl_trigger();
   pdl_wait();
   for (int e = threadIdx.x; e < nb * t; e += blockDim.x) Cs[e] = C[e];
   __syncthreads();
-  double acc[PD_MAXT];
+  double acc[NV];
 #pragma unroll
-  for (int j = 0; j < PD_MAXT; ++j) acc[j] = 0.0;
+  for (int j = 0; j < NV; ++j) acc[j] = 0.0;
   for (i64 r = blockIdx.x * (i64)blockDim.x + threadIdx.x; r < N; r += (i64)gridDim.x * blockDim.x) {
-    double xr[PD_MAXT];
+    double xr[NV], qr[NV], pr[NV];
 #pragma unroll
-    for (int k = 0; k < PD_MAXT; ++k) xr[k] = k < nb ? X[r + N * k] : 0.0;
+    for (int k = 0; k < NV; ++k) xr[k] = k < nb ? X[r + N * k] : 0.0;
 #pragma unroll
-    for (int j = 0; j < PD_MAXT; ++j) {
+    for (int j = 0; j < NV; ++j) {
+      qr[j] = j < t ? q[r + N * j] : 0.0;
+      pr[j] = j < t ? p[r + N * j] : 0.0;
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
       if (j >= t) break;
-      double v = q[r + N * j];
+      double v = qr[j];
 #pragma unroll
-      for (int k = 0; k < PD_MAXT; ++k)
+      for (int k = 0; k < NV; ++k)
         if (k < nb) v = fma(-xr[k], Cs[k + nb * j], v);
       q[r + N * j] = v;
-      acc[j] = fma(p[r + N * j], v, acc[j]);
+      acc[j] = fma(pr[j], v, acc[j]);
     }
   }
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int j = 0; j < PD_MAXT; ++j) {
-    if (j >= t) break;
-    double v = acc[j];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if (lane == 0) red[w][j] = v;
-  }
+  const double s = warp_sums<NV>(acc);
+  if ((lane & (32 / NV - 1)) == 0) red[w][lane * NV >> 5] = s;
   __syncthreads();
   if (threadIdx.x < t) {
-    const double v = red[0][threadIdx.x] + red[1][threadIdx.x] + red[2][threadIdx.x] + red[3][threadIdx.x];
+    const double v = (red[0][threadIdx.x] + red[1][threadIdx.x]) + (red[2][threadIdx.x] + red[3][threadIdx.x]);
     part[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = v;
     __threadfence();
   }
@@ -326,7 +326,9 @@ struct JdCg {
     double* rr0 = sc + 3 * 64;
     const double tol2 = rel_tol * rel_tol;
     const size_t bytes_t = sizeof(double) * N * t;
-    int bx = (int)std::max<i64>(1, std::min<i64>(CG_MAXBX, (N + 2047) / 2048));
+    // two rows a thread: a column's blocks cover the SMs (eight left 112 of them
+    // idle at N = 16384, t = 5: 10 us)
+    int bx = (int)std::max<i64>(1, std::min<i64>(CG_MAXBX, (N + 511) / 512));
     int eb = (int)std::min<i64>(4096, (N * t + 255) / 256);
     // x = 0, r = -rhs (already orthogonal to X), p = r
     TTG_CUDA(cudaMemsetAsync(x, 0, bytes_t, s));
@@ -346,8 +348,10 @@ struct JdCg {
         // q = P q with pq = p^T q in the same pass
         double* c = sc + 6 * 64;
         gemm_tn_small(nb, t, N, X, N, q, N, c, nb, 1.0, 0.0, s);
-        launch_pdl(proj_dot_kernel, dim3(pb), dim3(128), 0, s, N, t, nb, X, (const double*)c,
-                   (const double*)p, q, pq, part_pd, cnt + 2 * CG_MAXT);
+        const int nv = std::max(t, nb);
+        launch_pdl(nv <= 4 ? proj_dot_kernel<4> : (nv <= 8 ? proj_dot_kernel<8> : proj_dot_kernel<16>),
+                   dim3(pb), dim3(128), 0, s, N, t, nb, X, (const double*)c, (const double*)p, q, pq,
+                   part_pd, cnt + 2 * CG_MAXT);
       } else {
         project(q, t, X, nb);                         // q = P q
         col_dots(N, t, p, q, pq, part_cd, cnt, s);

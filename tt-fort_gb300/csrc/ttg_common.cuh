@@ -89,6 +89,27 @@ __device__ __forceinline__ double cluster_sum(double v) {
   return out;
 }
 
+// Sums of NV values over a warp, NV in {1, 2, 4, 8, 16}: while the values
+// outnumber the lanes that share them, each half of the lanes keeps half of the
+// values (a warp-wide FP64 addition holds its pipe 64 clocks; five per value
+// otherwise).  Lane l returns the sum of value (l * NV) >> 5.
+template <int NV>
+__device__ __forceinline__ double warp_sums(double (&v)[NV]) {
+  const int lane = threadIdx.x & 31;
+  int o = 16;
+#pragma unroll
+  for (int h = NV / 2; h > 0; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double give = up ? v[k] : v[k + h];
+      v[k] = (up ? v[k + h] : v[k]) + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
 // -------------------------------------------------------------------------
 // Programmatic dependent launch.  A kernel launched with launch_pdl may start
 // while the kernel before it in the stream is still running: its CTAs run

@@ -16,27 +16,6 @@ static constexpr double RESTART_DROP = 1e-10;
 // ---------------------------------------------------------------------------
 constexpr int TS_MAXN = 16;
 
-// Sums of NV values over a warp, NV in {1, 2, 4, 8, 16}: while the values
-// outnumber the lanes that share them, each half of the lanes keeps half of the
-// values (a warp-wide FP64 addition holds its pipe 64 clocks; five per value
-// otherwise).  Lane l returns the sum of value (l * NV) >> 5.
-template <int NV>
-__device__ __forceinline__ double warp_sums(double (&v)[NV]) {
-  const int lane = threadIdx.x & 31;
-  int o = 16;
-#pragma unroll
-  for (int h = NV / 2; h > 0; h >>= 1, o >>= 1) {
-    const bool up = lane & o;
-#pragma unroll
-    for (int k = 0; k < h; ++k) {
-      const double give = up ? v[k] : v[k + h];
-      v[k] = (up ? v[k + h] : v[k]) + __shfl_xor_sync(0xffffffffu, give, o);
-    }
-  }
-  for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-  return v[0];
-}
-
 // C (M x N, ldc) = alpha * A^T B + beta * C, A (K x M, lda), B (K x N, ldb),
 // N <= NV <= 16.  Grid (M, nk), one cluster of nk CTAs per column m of A: CTA
 // (m, c) reduces k-chunk c against all N columns of B, then rank 0 adds the

@@ -140,6 +140,64 @@ __device__ __forceinline__ void rr_pair(int K, int r, int i, int& a, int& b) {
   else { a = (r + i) % (K - 1); b = (r - i + K - 1) % (K - 1); }
 }
 
+// The rotation that makes two columns with squared norms A, B and product G
+// orthogonal, as three shears: with p = tan(theta / 2) and s = sin(theta) =
+// 2 p / (1 + p^2),
+//   x <- x - p y,  y <- y + s x,  x <- x - p y
+// is x <- c x - s y, y <- s x + c y: three FMAs per element in place of two
+// products and two FMAs.  p comes from FP32 arithmetic on the leading bits (an
+// angle off by FP32 rounding leaves ~1e-7 of G for the next sweep); s is formed
+// from that p in FP64, so the rotation is orthogonal to FP64 precision whatever
+// p is: 1/(1 + p^2) by one third-order step from the FP32 quotient.  Exponents
+// are moved as integers, so no FP32 range is passed, and FP32 values become
+// FP64 ones by their bits.  A dependent FP64 operation takes about 100 clocks
+// here, and this is the serial part of every round: six of them, against about
+// forty with FP64 quotients, square roots and tests.
+__device__ __forceinline__ float lead24(double v) {   // mantissa of v in [1, 2), truncated
+  return __uint_as_float(0x3f800000u | (((unsigned)__double2hiint(v) & 0xfffffu) << 3) |
+                         ((unsigned)__double2loint(v) >> 29));
+}
+__device__ __forceinline__ int exp_bits(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
+__device__ __forceinline__ double widen(float f, int e, unsigned sign) {   // f 2^e, f > 0 normal
+  const unsigned b = __float_as_uint(f);
+  const int he = (int)(b >> 23) + 896 + e;
+  return __hiloint2double((int)(((unsigned)he << 20) | ((b & 0x7fffffu) >> 3) | sign), (int)(b << 29));
+}
+__device__ __forceinline__ void jacobi_shears(double A, double Bv, double G, double& p, double& s) {
+  const double d = Bv - A;
+  const int k = exp_bits(d) - exp_bits(G) - 1;        // zeta = d / (2 G) = +-(fd / fg) 2^k
+  const float fd = lead24(d), fg = lead24(G);
+  const unsigned sg = ((unsigned)__double2hiint(d) ^ (unsigned)__double2hiint(G)) & 0x80000000u;
+  float pf = 0.41421356f;                             // |p| = pf 2^pe; here tan(pi / 8)
+  int pe = 0;
+  if (k > 30) {
+    pf = __fdividef(fg, fd);                          // 1 / (4 zeta)
+    pe = -k - 2;
+  } else if (d != 0.0 && k >= -60) {
+    const float z = __fdividef(fd, fg) * __uint_as_float((unsigned)(127 + k) << 23);
+    const float t = __fdividef(1.f, z + sqrtf(fmaf(z, z, 1.f)));
+    pf = __fdividef(t, 1.f + sqrtf(fmaf(t, t, 1.f)));
+  }
+  if (pe < -850) {                                    // no FP64 value of the columns moves
+    p = s = 0.0;
+    return;
+  }
+  p = widen(pf, pe, sg);
+  const double u = fma(p, p, 1.0);
+  const double z0 = widen(__fdividef(1.f, pe < 0 ? 1.f : fmaf(pf, pf, 1.f)), 0, 0u);
+  const double e = fma(-u, z0, 1.0);
+  const double w = fma(z0, fma(e, e, e), z0);         // 1 / (1 + p^2) in [0.85, 1]
+  s = p * __hiloint2double(__double2hiint(w) + (1 << 20), __double2loint(w));
+}
+// G^2 > tol2 A B on the leading 24 bits; false for G = 0 and anything not finite
+__device__ __forceinline__ bool above(double A, double Bv, double G, float tol2) {
+  const int ea = exp_bits(A), eb = exp_bits(Bv), eg = exp_bits(G);
+  const int k = 2 * eg - ea - eb;
+  if (eg == 0 || max(ea, max(eb, eg)) == 0x7ff || k < -124) return false;
+  const float fg = lead24(G);
+  return k > 60 || fg * fg * __uint_as_float((unsigned)(127 + k) << 23) > tol2 * (lead24(A) * lead24(Bv));
+}
+
 // ---------------------------------------------------------------------------
 // symmetric eigensolver: cyclic Jacobi in one CTA
 // ---------------------------------------------------------------------------
@@ -226,13 +284,17 @@ __global__ void __launch_bounds__(JAC_NT) syev_jacobi_kernel(int k, double* Ag, 
         rr_pair(K, r, pi, p, q);
         double c = 1.0, s = 0.0;
         if (p < k && q < k) {
-          double app = A[p + (i64)la * p], aqq = A[q + (i64)la * q], apq = A[p + (i64)la * q];
-          if (apq != 0.0 && fabs(apq) > 1e-18 * sqrt(fro2) &&
-              fabs(apq) > DBL_EPSILON * 0.5 * sqrt(fabs(app) * fabs(aqq))) {
-            double theta = (aqq - app) / (2.0 * apq);
-            double t = (theta >= 0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
-            c = 1.0 / sqrt(t * t + 1.0);
-            s = t * c;
+          const double app = A[p + (i64)la * p], aqq = A[q + (i64)la * q], apq = A[p + (i64)la * q];
+          // |apq| > 1e-18 ||A||_F and > eps/2 sqrt(|app aqq|), in squares.  The
+          // angle's tangent from FP32 as in the one-sided sweeps: what is left of
+          // apq (1e-7 of it) goes with the next sweep, and the serial part of a
+          // round is eight dependent FP64 operations, not some forty (k = 10:
+          // 89 -> 56 us a solve)
+          if (above(fro2, 1.0, apq, 1e-36f) &&
+              above(app, aqq, apq, (float)(0.25 * DBL_EPSILON * DBL_EPSILON))) {
+            double h;
+            jacobi_shears(app, aqq, apq, h, s);
+            c = fma(-h, s, 1.0);
             atomicAdd(&rot_count, 1);
           }
         }
@@ -332,64 +394,6 @@ __device__ __forceinline__ T warp_sum_t(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// The rotation that makes two columns with squared norms A, B and product G
-// orthogonal, as three shears: with p = tan(theta / 2) and s = sin(theta) =
-// 2 p / (1 + p^2),
-//   x <- x - p y,  y <- y + s x,  x <- x - p y
-// is x <- c x - s y, y <- s x + c y: three FMAs per element in place of two
-// products and two FMAs.  p comes from FP32 arithmetic on the leading bits (an
-// angle off by FP32 rounding leaves ~1e-7 of G for the next sweep); s is formed
-// from that p in FP64, so the rotation is orthogonal to FP64 precision whatever
-// p is: 1/(1 + p^2) by one third-order step from the FP32 quotient.  Exponents
-// are moved as integers, so no FP32 range is passed, and FP32 values become
-// FP64 ones by their bits.  A dependent FP64 operation takes about 100 clocks
-// here, and this is the serial part of every round: six of them, against about
-// forty with FP64 quotients, square roots and tests.
-__device__ __forceinline__ float lead24(double v) {   // mantissa of v in [1, 2), truncated
-  return __uint_as_float(0x3f800000u | (((unsigned)__double2hiint(v) & 0xfffffu) << 3) |
-                         ((unsigned)__double2loint(v) >> 29));
-}
-__device__ __forceinline__ int exp_bits(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
-__device__ __forceinline__ double widen(float f, int e, unsigned sign) {   // f 2^e, f > 0 normal
-  const unsigned b = __float_as_uint(f);
-  const int he = (int)(b >> 23) + 896 + e;
-  return __hiloint2double((int)(((unsigned)he << 20) | ((b & 0x7fffffu) >> 3) | sign), (int)(b << 29));
-}
-__device__ __forceinline__ void jacobi_shears(double A, double Bv, double G, double& p, double& s) {
-  const double d = Bv - A;
-  const int k = exp_bits(d) - exp_bits(G) - 1;        // zeta = d / (2 G) = +-(fd / fg) 2^k
-  const float fd = lead24(d), fg = lead24(G);
-  const unsigned sg = ((unsigned)__double2hiint(d) ^ (unsigned)__double2hiint(G)) & 0x80000000u;
-  float pf = 0.41421356f;                             // |p| = pf 2^pe; here tan(pi / 8)
-  int pe = 0;
-  if (k > 30) {
-    pf = __fdividef(fg, fd);                          // 1 / (4 zeta)
-    pe = -k - 2;
-  } else if (d != 0.0 && k >= -60) {
-    const float z = __fdividef(fd, fg) * __uint_as_float((unsigned)(127 + k) << 23);
-    const float t = __fdividef(1.f, z + sqrtf(fmaf(z, z, 1.f)));
-    pf = __fdividef(t, 1.f + sqrtf(fmaf(t, t, 1.f)));
-  }
-  if (pe < -850) {                                    // no FP64 value of the columns moves
-    p = s = 0.0;
-    return;
-  }
-  p = widen(pf, pe, sg);
-  const double u = fma(p, p, 1.0);
-  const double z0 = widen(__fdividef(1.f, pe < 0 ? 1.f : fmaf(pf, pf, 1.f)), 0, 0u);
-  const double e = fma(-u, z0, 1.0);
-  const double w = fma(z0, fma(e, e, e), z0);         // 1 / (1 + p^2) in [0.85, 1]
-  s = p * __hiloint2double(__double2hiint(w) + (1 << 20), __double2loint(w));
-}
-// G^2 > tol2 A B on the leading 24 bits; false for G = 0 and anything not finite
-__device__ __forceinline__ bool above(double A, double Bv, double G, float tol2) {
-  const int ea = exp_bits(A), eb = exp_bits(Bv), eg = exp_bits(G);
-  const int k = 2 * eg - ea - eb;
-  if (eg == 0 || max(ea, max(eb, eg)) == 0x7ff || k < -124) return false;
-  const float fg = lead24(G);
-  return k > 60 || fg * fg * __uint_as_float((unsigned)(127 + k) << 23) > tol2 * (lead24(A) * lead24(Bv));
 }
 
 // lanes 0-7 return the warp's sum of a, 8-15 that of b, 16-31 that of g: values
