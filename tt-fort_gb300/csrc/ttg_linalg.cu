@@ -1179,14 +1179,15 @@ __global__ void __launch_bounds__(QRC_NT) qr_panel_coop_kernel(int m, int w, dou
 // leading dimension rows): panel k holds columns QRP_NB k.., its T is w x w at
 // Tf + k QRP_NB^2 (leading dimension QRP_NB).  A cluster of QRT_CL CTAs per
 // panel shares the rows of its Gram matrix Y^T Y, added in rank order; rank 0
-// runs the recurrence T[0:i, i] = -tau_i T[0:i, 0:i] (Y^T Y)[0:i, i].
+// joins blocks of columns two by two (column by column, 32 dependent products,
+// took 49 us, so 29).
 constexpr int QRT_CL = 8, QRT_NT = 256, QRT_ROWS = 32;
 __global__ void __launch_bounds__(QRT_NT) qr_t_kernel(int rows, int q, const double* __restrict__ F,
                                                       const double* __restrict__ tau, double* __restrict__ Tf) {
   cg::cluster_group cl = cg::this_cluster();
   __shared__ double Y[QRP_NB][QRT_ROWS + 1];
   __shared__ double gram[QRP_NB][QRP_NB + 1];     // [j][i]
-  __shared__ double zt[QRP_NB];
+  __shared__ double T_s[QRP_NB][QRP_NB + 1], W_s[QRP_NB][QRP_NB + 1];   // [column][row]
   const int tid = threadIdx.x, i = tid & 31, jw = tid >> 5;
   const int k = blockIdx.x, j0 = k * QRP_NB, w = min(QRP_NB, q - j0), m = rows - j0;
   const double* A = F + j0 + (i64)rows * j0;
@@ -1219,20 +1220,32 @@ __global__ void __launch_bounds__(QRT_NT) qr_t_kernel(int rows, int q, const dou
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < QRP_NB / 8; ++t) gram[jw + 8 * t][i] = v[t];
-    double* T = Tf + (size_t)k * QRP_NB * QRP_NB;
-    for (int e = tid; e < QRP_NB * QRP_NB; e += QRT_NT) T[e] = 0.0;
+    // T of two neighbouring blocks of columns from their own T1, T2:
+    // T12 = -T1 (Y1^T Y2) T2, from single columns (T = tau) up to the panel
+    for (int e = tid; e < QRP_NB * QRP_NB; e += QRT_NT) {
+      const int r = e % QRP_NB, c = e / QRP_NB;
+      T_s[c][r] = (r == c && c < w) ? tau[j0 + c] : 0.0;
+    }
     __syncthreads();
-    for (int c = 0; c < w; ++c) {
-      if (tid < c) zt[tid] = -tau[j0 + c] * gram[c][tid];
-      __syncthreads();
-      if (tid < c) {
-        double u = 0.0;
-        for (int l = tid; l < c; ++l) u = fma(T[tid + QRP_NB * l], zt[l], u);
-        T[tid + QRP_NB * c] = u;
+    for (int h = 1; h < QRP_NB; h *= 2) {
+      // entry (r, c) of the upper right block of pair g; 16 h of them in all
+      for (int e = tid; e < QRP_NB / 2 * h; e += QRT_NT) {
+        const int g = e / (h * h), r = g * 2 * h + e % h, c = g * 2 * h + h + (e / h) % h;
+        double u = 0.0;                           // (Y1^T Y2) T2
+        for (int l = g * 2 * h + h; l <= c; ++l) u = fma(gram[l][r], T_s[c][l], u);
+        W_s[c][r] = u;
       }
-      if (tid == 0) T[c + QRP_NB * c] = tau[j0 + c];
+      __syncthreads();
+      for (int e = tid; e < QRP_NB / 2 * h; e += QRT_NT) {
+        const int g = e / (h * h), r = g * 2 * h + e % h, c = g * 2 * h + h + (e / h) % h;
+        double u = 0.0;
+        for (int l = r; l < g * 2 * h + h; ++l) u = fma(T_s[l][r], W_s[c][l], u);
+        T_s[c][r] = -u;
+      }
       __syncthreads();
     }
+    double* T = Tf + (size_t)k * QRP_NB * QRP_NB;
+    for (int e = tid; e < QRP_NB * QRP_NB; e += QRT_NT) T[e] = T_s[e / QRP_NB][e % QRP_NB];
   }
   cl.sync();   // no CTA leaves while rank 0 still reads its sums
 }
