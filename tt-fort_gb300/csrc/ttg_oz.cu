@@ -72,6 +72,7 @@ struct Side {                   // one operand, element (r, k) = src[map(r) + k 
   int rtiles;
   unsigned char* planes;        // [rtile][K step][plane][R x 16 bf16, core matrices]
   int* expo;                    // per split row
+  int vec;                      // real with sk == 1 and 16-byte aligned rows
   int cplx;                     // 0 real, 1: rows (re, im) x K (re, im), 2: K (re, im) only
   int conj;
 };
@@ -146,6 +147,13 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
           v[2 * q] = z.x;
           v[2 * q + 1] = S.conj ? -z.y : z.y;
         }
+      }
+    } else if (S.vec && g * 8 + 8 <= K) {
+#pragma unroll
+      for (int q = 0; q < 8; q += 2) {
+        const double2 z = *reinterpret_cast<const double2*>(p + g * 8 + q);
+        v[q] = z.x;
+        v[q + 1] = z.y;
       }
     } else {
 #pragma unroll
@@ -604,8 +612,11 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   const int nz0 = z_split(s);
   const int kper = (int)((s.kt + nz0 - 1) / nz0), nz = (int)((s.kt + kper - 1) / kper);
   longlong2* part = nz > 1 ? (longlong2*)take(sizeof(longlong2) * nz * ra * rb) : nullptr;
-  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, g.cplx ? 1 : 0, g.conjA};
-  const Side b{g.B, g.bn, g.bk, g.N, BN, (int)s.nt, Bd, eb, g.cplx ? 2 : 0, g.conjB};
+  auto vec = [&](const double* src, const OzMap& m, i64 sk) {
+    return !g.cplx && sk == 1 && ((uintptr_t)src & 15) == 0 && (m.s1 & 1) == 0 && (m.s2 & 1) == 0;
+  };
+  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? 1 : 0, g.conjA};
+  const Side b{g.B, g.bn, g.bk, g.N, BN, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? 2 : 0, g.conjB};
   const int nA = (int)(ra / (g.cplx ? 2 : 1) / SROWS), nB = (int)(rb / SROWS);
   // few rows and a long K: K over a cluster (246 + 82 rows, K = 4928: 50 -> 17 us)
   int ky = 1;
