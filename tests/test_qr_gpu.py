@@ -84,3 +84,24 @@ def test_qr_is_reproducible(torch_cuda, ctx):
     for _ in range(3):
         b = run(torch_cuda, ctx, A)
         assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+
+
+@pytest.mark.parametrize("n,m", [(700, 7), (700, 8), (700, 9), (40, 15), (40, 17), (900, 33),
+                                 (300, 129), (1500, 140), (2500, 40), (100, 150), (1344, 30)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_qr_panels(torch_cuda, ctx, n, m, cplx):
+    """Q is formed a panel of 8 reflectors at a time: columns below, at and above
+    a multiple of it, in the cluster and the grid form; columns above the grid
+    form's limit of directly added parts.  Tolerance as above."""
+    test_qr_sizes(torch_cuda, ctx, n, m, cplx)
+
+
+@pytest.mark.parametrize("n", [64, 2000])
+def test_qr_nan_leaves_earlier_columns(torch_cuda, ctx, n):
+    """Column c of Q is the product of reflectors 0..c with e_c: a NaN in
+    column 11, the middle of a panel, does not reach the columns before it."""
+    A = np.random.default_rng(n).standard_normal((n, 20))
+    A[n // 2, 11] = np.nan
+    Q, R = run(torch_cuda, ctx, A)
+    assert np.isfinite(Q[:, :11]).all() and np.isfinite(R[:, :11]).all()
+    assert np.isnan(Q[:, 11:]).all()

@@ -417,7 +417,7 @@ void svd_jacobi(int p, int q, const double* M, double* U, double* sigma, double*
 // Householder QR with LAPACK's convention: A (n x m) -> Q (n x min), R (min x m).
 // tau: work elements, at least min(n, m); with qr_work_elems(n, m) of them large
 // blocks run over the whole GPU (ttg_qr.cu)
-size_t qr_work_elems(i64 n, i64 m);
+size_t qr_work_elems(i64 n, i64 m, bool form_q = true);
 void qr_householder(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s);
 void qr_householder_z(int n, int m, double2* A, double2* R, double2* tau, size_t work,
                       cudaStream_t s);

@@ -1295,7 +1295,7 @@ static size_t svd_qr_work(size_t p, size_t q) {
   // first QR (A, X, Ux, Vtx, Tf, Yp, G1, G2, tau, perm, coop partials), then
   // the second QR's R2^T, Q2 V2, T factors and tau; the factorisation's work
   return p * q + 3 * q * q + npan * QRP_NB * QRP_NB + p * QRP_NB + 2 * QRP_NB * q + 2 * q + 256 +
-         coop + 64 + 2 * q * q + npan * QRP_NB * QRP_NB + q + 128 + qr_work_elems(p, q);
+         coop + 64 + 2 * q * q + npan * QRP_NB * QRP_NB + q + 128 + qr_work_elems(p, q, false);
 }
 
 size_t svd_scratch(int p, int q) {
@@ -1359,7 +1359,7 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   // Over the whole GPU with the rows in shared memory (ttg_qr.cu), or, where
   // they do not fit, panel by panel with GEMM updates
   auto qr_factor = [&](int rows, double* F, double* Tfac, double* tv) {
-    if (qr_rows_factor(rows, q, F, qrw, qr_work_elems(rows, q), s)) {
+    if (qr_rows_factor(rows, q, F, qrw, qr_work_elems(rows, q, false), s)) {
       TTG_CUDA(cudaMemcpyAsync(tv, qrw, sizeof(double) * q, cudaMemcpyDeviceToDevice, s));
       launch_clustered(qr_t_kernel, dim3(npan, QRT_CL), dim3(QRT_NT), dim3(1, QRT_CL, 1), 0, s, rows,
                        q, (const double*)F, (const double*)tv, Tfac);
