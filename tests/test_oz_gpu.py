@@ -189,3 +189,27 @@ def test_interface_updates(torch_cuda, ctx, r1, m, r2, ry1, n, ry2):
     for got, ref in ((L, ops.phi_left(r1, m, r2, ry1, n, ry2, ra1, ra2, q1, A, x, y)),
                      (R, ops.phi_right(r1, m, r2, ry1, n, ry2, ra1, ra2, q2, A, x, y))):
         assert np.linalg.norm(got.cpu().numpy() - ref) <= 1e-14 * np.linalg.norm(ref)
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (256, 120, 256), (256, 120, 400), (250, 120, 512), (256, 120, 560), (200, 128, 700),
+    (256, 120, 1000), (1000, 128, 700),
+])
+def test_k_split_over_clusters(torch_cuda, ctx, M, N, K):
+    """K in 4, 5, 8 and 7 chunks of one cluster (no summing kernel), in two and
+    three clusters of four (one chunk of the last is empty), with ragged
+    columns shared out: bounds as above, flagged rows among them."""
+    rng = np.random.default_rng(M + N + K)
+    X, P2 = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    X[5, K // 2], X[M - 1, 0] = np.nan, np.inf
+    P2[K - 1, N - 1] = np.inf
+    got, launches = plain_product(torch_cuda, ctx, X, P2)
+    assert launches > 3, "the split product was not taken"
+    with np.errstate(all="ignore"):
+        ref = X @ P2
+    assert np.array_equal(np.isfinite(got), np.isfinite(ref))
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    rows, cols = np.isfinite(X).all(1), np.isfinite(P2).all(0)
+    A, B = X[rows], P2[:, cols]
+    err = abs(got[rows][:, cols] - A @ B)
+    assert (err <= oz_bound(A, B) + (K + 4) * U * (abs(A) @ abs(B))).all()

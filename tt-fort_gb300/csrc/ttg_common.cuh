@@ -254,6 +254,7 @@ struct GemmF64 {
                     // partial tiles added in a fixed order (deterministic)
 };
 void gemm_f64(const GemmF64& g, cudaStream_t s);
+double gemm_fp64_us(int M, int N, int K, int nbatch, bool cplx);   // ttg_gemm.cu's own estimate
 
 // standard normals from the splitmix64/Box-Muller stream shared with the oracle
 void sm_normals(unsigned long long seed, i64 count, double* out);

@@ -272,13 +272,14 @@ void launch_tile(const Args<T>& a, int nbatch, cudaStream_t s) {
 //   two steps of the complex time stepper (d=16, n=32, r=8)   213 -> 124 ms
 struct TilePick {
   int tile, splitk, kchunk;
+  double clocks;
 };
 template <class T>
 TilePick pick_tile(int M, int N, int K, int nbatch, int want_split) {
   constexpr int kSMs = 152;
   constexpr double kStep = 700.0, kSplit = 2500.0;
   constexpr double per_fma = sizeof(T) == 16 ? 2.0 : 0.5;   // clocks
-  TilePick best{32, 1, ceil_div(K, BK) * BK};
+  TilePick best{32, 1, ceil_div(K, BK) * BK, 0.0};
   double best_t = 1e300;
   for (int tile : {32, 16}) {
     const int wm = tile == 32 ? 8 : 4, wn = tile == 32 ? 16 : 8;
@@ -299,7 +300,7 @@ TilePick pick_tile(int M, int N, int K, int nbatch, int want_split) {
                        (real > 1 ? kSplit : 0.0);
       if (t < 0.98 * best_t) {
         best_t = t;
-        best = {tile, real, chunk};
+        best = {tile, real, chunk, t};
       }
     }
   }
@@ -362,6 +363,12 @@ void launch(Args<T> a, int nbatch, cudaStream_t s) {
 }
 
 }  // namespace
+
+// the model's time (us) of a product on these kernels, launch included
+double gemm_fp64_us(int M, int N, int K, int nbatch, bool cplx) {
+  const TilePick p = cplx ? pick_tile<double2>(M, N, K, nbatch, 1) : pick_tile<double>(M, N, K, nbatch, 1);
+  return p.clocks / 1900.0 + 3.0;
+}
 
 void gemm_f64(const GemmF64& g, cudaStream_t s) {
   Args<double> a{g.M, g.N, g.K, g.A, g.sAm, g.sAk, g.B, g.sBk, g.sBn, g.C, g.sCm, g.sCn,

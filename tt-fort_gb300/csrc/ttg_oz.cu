@@ -28,10 +28,10 @@
 // FMA chain, so infinities, NaN and extreme ranges give what they give there.
 //
 // Measured on GB300, FP64 kernels -> split products: chain product r=256, block
-// of 8: 4560 -> 243 us (22.6 TFLOP/s of FP64 accuracy; its two products run at
-// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 40.3
-// us; grid interface updates r = 82, 77, n = 64: 1908 -> 170 us; complex
-// operator and adjoint r=48, n=32, block of 4: 6968 -> 408 us.  What bounds the
+// of 8: 4560 -> 241 us (22.7 TFLOP/s of FP64 accuracy; its two products run at
+// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 38.4
+// us; grid interface updates r = 82, 77, n = 64: 1908 -> 167 us; complex
+// operator and adjoint r=48, n=32, block of 4: 6968 -> 403 us.  What bounds the
 // product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
 // measured against 900 of MMA), for small ones its fixed ~10 us (pipeline
 // fill, one drain, rounding); oz_us below holds both.
@@ -81,10 +81,11 @@ struct Args {
   const unsigned char *Ad, *Bd;
   const int *ea, *eb;
   int M, N, K;                  // product rows and columns; logical K (for the FP64 chain)
-  int kt, kper, mtiles, ntiles, nz;
+  int kt, kper, mtiles, ntiles;
+  int nz, cs;                   // K splits of a tile; cs > 1: added over clusters of cs CTAs
   double* C;
   OzMap cm, cn;
-  longlong2* part;              // nz > 1: partial sums [z][n][row]
+  longlong2* part;              // nz > cs: the clusters' sums [z / cs][n][row]
   const double *A, *B;          // original operands (flagged rows)
   OzMap am, bn;
   i64 ak, bk;
@@ -318,6 +319,7 @@ __device__ __noinline__ void slow_fix(const Args& g, i64 crow, int row, int n, i
   else if (ea == SLOW || g.eb[n] == SLOW) g.C[crow + c_col(g, n)] = fma_chain(g, row, n);
 }
 
+constexpr int kMaxSplit = kMaxCluster;            // CTAs of a cluster that share a tile
 constexpr float kCarry = 3221225472.f;   // 1.5 2^31: FP32 spacing 256
 // an integer |x| < 2^22 held in FP32, without the conversion unit
 __device__ __forceinline__ int small_int(float x) {
@@ -340,7 +342,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
   volatile int* fail = &fail_s;
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int per_z = g.mtiles * g.ntiles, total = per_z * g.nz;
+  const int total = g.mtiles * g.ntiles * g.nz;
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(smem_u32(&full_bar[s]), 1);
@@ -367,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
       int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const int rz = t % per_z, mt = rz % g.mtiles, nt = rz / g.mtiles, z = t / per_z;
+        const int z = t % g.nz, rz = t / g.nz, mt = rz % g.mtiles, nt = rz / g.mtiles;
         const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
         for (int k = k0; k < k1; ++k, ++it) {
           const int s = it % STAGES;
@@ -398,7 +400,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
       int it = 0, use = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < total && ok; t += gridDim.x) {
-        const int z = t / per_z, k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
+        const int z = t % g.nz, k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
         for (int kc = k0; kc < k1 && ok; kc += KCHUNK, ++use) {
           if (use > 0 && !mbar_wait_f(smem_u32(&acc_empty), (uint32_t)((use - 1) & 1), fail)) {
             ok = false;
@@ -442,7 +444,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     int use = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
-      const int rz = t % per_z, mt = rz % g.mtiles, nt = rz / g.mtiles, z = t / per_z;
+      const int z = t % g.nz, rz = t / g.nz, mt = rz % g.mtiles, nt = rz / g.mtiles;
       const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
       long long hi[16];                              // sum = hi 2^32 + lo, in 2^-48
       uint32_t lo[16];
@@ -489,13 +491,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         }
       }
       const int row = mt * BM + q * 32 + lane, n0 = nt * BN + cb;
-      if (g.nz > 1) {
-        longlong2* o = g.part + ((size_t)z * g.ntiles * BN + n0) * ((size_t)g.mtiles * BM) + row;
+      if (g.cs > 1) {
+        // the CTA's only tile: every copy has landed and every MMA has read it,
+        // so the ring holds the sums for the cluster (after a failure fail_s counts)
+        longlong2* o = reinterpret_cast<longlong2*>(base) + cb * BM + q * 32 + lane;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
-          // a failed CTA's partials carry a mark the finishing kernel turns into NaN
-          o[(size_t)c * g.mtiles * BM] = ok ? make_longlong2(hi[c], (long long)lo[c]) : make_longlong2(LLONG_MIN, 0);
-        }
+        for (int c = 0; c < 16; ++c) o[c * BM] = make_longlong2(hi[c], (long long)lo[c]);
       } else {
         // lane c holds column c's exponent and offset
         const int nl = n0 + (lane & 15);
@@ -520,13 +521,54 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     }
   }
   pdl_trigger();
+  if (g.cs > 1) {
+    // one tile per CTA; CTA `rank` adds its share of the columns over the
+    // cluster (exact integers) and rounds, or leaves the cluster's sum
+    namespace cgr = cooperative_groups;
+    cgr::cluster_group cl = cgr::this_cluster();
+    cl.sync();
+    const int z = (int)blockIdx.x % g.nz, rz = (int)blockIdx.x / g.nz;
+    const int mt = rz % g.mtiles, nt = rz / g.mtiles, rank = (int)cl.block_rank();
+    const int share = (BN + g.cs - 1) / g.cs;
+    bool bad = false;
+    for (int p = 0; p < g.cs; ++p) bad = bad || *cl.map_shared_rank(&fail_s, p) != 0;
+    const int row = mt * BM + (tid & (BM - 1));
+    const longlong2* mine = reinterpret_cast<const longlong2*>(base) + (tid & (BM - 1));
+    const bool live = tid < 4 * BM && row < g.M;
+    const int ea = live ? g.ea[row] : 0;
+    const i64 cr = live ? c_row(g, row) : 0;
+    for (int c = rank * share + (tid >> 7); c < min(BN, (rank + 1) * share); c += 4) {
+      const int n = nt * BN + c;
+      if (!live || n >= g.N) break;
+      longlong2 v[kMaxSplit];
+#pragma unroll
+      for (int p = 0; p < kMaxSplit; ++p)
+        v[p] = p < g.cs ? *cl.map_shared_rank(mine + c * BM, p) : make_longlong2(0, 0);
+      long long hi = v[0].x, lo = v[0].y;
+#pragma unroll
+      for (int p = 1; p < kMaxSplit; ++p) {
+        hi += v[p].x;
+        lo += v[p].y;
+      }
+      if (g.nz > g.cs) {
+        // a failed cluster's sums carry a mark the finishing kernel turns into NaN
+        g.part[((size_t)(z / g.cs) * g.ntiles * BN + n) * ((size_t)g.mtiles * BM) + row] =
+            bad ? make_longlong2(LLONG_MIN, 0) : make_longlong2(hi, lo);
+      } else {
+        const int eb = g.eb[n];
+        if (bad || ea == SLOW || eb == SLOW) slow_fix(g, cr, row, n, ea, bad);
+        else g.C[cr + c_col(g, n)] = to_double(hi, lo, ea + eb - 62);
+      }
+    }
+    cl.sync();   // no CTA leaves while another reads its sums
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (warp == 1) tmem_dealloc(taddr, 512);
 }
 
-// adds the K-split partials (exact integers) and rounds
+// adds the clusters' sums (exact integers) and rounds
 __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
   pdl_wait();
   pdl_trigger();
@@ -537,7 +579,7 @@ __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
     if (row >= g.M) continue;
     long long hi = 0, lo = 0;
     bool bad = false;
-    for (int z = 0; z < g.nz; ++z) {
+    for (int z = 0; z < g.nz / g.cs; ++z) {
       const longlong2 v = g.part[((size_t)z * Np + n) * Mp + row];
       bad = bad || v.x == LLONG_MIN;
       hi += v.x;
@@ -563,11 +605,26 @@ static Shape shape(i64 M, i64 N, i64 K, bool cplx) {
   s.kt = (s.K + 15) / 16;
   return s;
 }
-// K split: only where the tiles leave SMs idle; at least 8 K steps per chunk
-static int z_split(const Shape& s) {
+// K split: only where the tiles leave SMs idle; at least KMIN K steps per chunk
+// (a last chunk may be empty).  Up to eight chunks are one cluster where the
+// GPU holds all of them (it holds 14 clusters of eight of these CTAs, 36 of
+// four), more are clusters of four whose sums a second kernel adds.  Measured,
+// at least 8 steps and a second kernel for every split -> this: r=64 chain
+// product 40.1 -> 38.3 us, time stepper (d=16, n=32, r=8) 92.1 -> 88.4 ms,
+// operator and adjoint r=48 407 -> 403 us, K = 5248 in 36 chunks unchanged
+// (clusters of eight there: 167 -> 171 us; at least 2 steps: 88.4 -> 92 ms).
+constexpr int KMIN = 4;
+struct Split { int nz, cs, kper; };
+static Split z_split(const Shape& s) {
   const i64 tiles = s.mt * s.nt;
-  if (tiles * 2 > SMS) return 1;
-  return (int)std::max<i64>(1, std::min<i64>(SMS / tiles, s.kt / 8));
+  i64 nz = tiles * 2 > SMS ? 1 : std::max<i64>(1, std::min<i64>(144 / tiles, s.kt / KMIN)), cs = nz;
+  if (nz > 4 && (s.kt / KMIN > kMaxSplit || tiles * nz > 112)) {
+    nz -= nz % 4;
+    cs = 4;
+  }
+  const i64 kper = (s.kt + nz - 1) / nz;
+  if (cs == nz) cs = nz = (s.kt + kper - 1) / kper;
+  return {(int)nz, (int)cs, (int)kper};
 }
 static inline size_t al(size_t b) { return (b + 255) & ~size_t(255); }
 
@@ -575,12 +632,13 @@ static inline size_t al(size_t b) { return (b + 255) & ~size_t(255); }
 
 double oz_us(i64 M, i64 N, i64 K, bool cplx) {
   const oz::Shape s = oz::shape(M, N, K, cplx);
-  const int nz = oz::z_split(s);
+  const oz::Split z = oz::z_split(s);
+  const int nz = z.nz;
   const double waves = (double)((s.mt * s.nt * nz + oz::SMS - 1) / oz::SMS);
   const double ks = (double)((s.kt + nz - 1) / nz);
   const double mma = waves * (ks * 950.0 + (ks / oz::KCHUNK + 1) * 2500.0 + 3000.0) / 1900.0;
   const double split = ((double)s.M + s.N) * s.K * 22.0 / 4.0e6;
-  return mma + split + 12.0 + (nz > 1 ? 4.0 : 0.0);
+  return mma + split + 12.0 + (nz > z.cs ? 5.0 : (nz > 1 ? 1.5 : 0.0));
 }
 
 size_t oz_bytes(i64 M, i64 N, i64 K, bool cplx) {
@@ -609,9 +667,9 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   unsigned char* Bd = (unsigned char*)take(14 * 16 * (size_t)s.kt * rb);
   int* ea = (int*)take(4 * ra);
   int* eb = (int*)take(4 * rb);
-  const int nz0 = z_split(s);
-  const int kper = (int)((s.kt + nz0 - 1) / nz0), nz = (int)((s.kt + kper - 1) / kper);
-  longlong2* part = nz > 1 ? (longlong2*)take(sizeof(longlong2) * nz * ra * rb) : nullptr;
+  const Split z = z_split(s);
+  const int nz = z.nz, groups = nz / z.cs;
+  longlong2* part = groups > 1 ? (longlong2*)take(sizeof(longlong2) * groups * ra * rb) : nullptr;
   auto vec = [&](const double* src, const OzMap& m, i64 sk) {
     return !g.cplx && sk == 1 && ((uintptr_t)src & 15) == 0 && (m.s1 & 1) == 0 && (m.s2 & 1) == 0;
   };
@@ -626,7 +684,7 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   Args x{};
   x.Ad = Ad; x.Bd = Bd; x.ea = ea; x.eb = eb;
   x.M = (int)s.M; x.N = (int)s.N; x.K = g.K;
-  x.kt = (int)s.kt; x.kper = kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.nz = nz;
+  x.kt = (int)s.kt; x.kper = z.kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.nz = nz; x.cs = z.cs;
   x.C = g.C; x.cm = g.cm; x.cn = g.cn; x.part = part;
   x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
   x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
@@ -634,8 +692,8 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
       cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
   TTG_CUDA(attr_rc);
   const int grid = (int)std::min<i64>(SMS, s.mt * s.nt * nz);
-  launch_pdl(gemm_kernel, dim3(grid), dim3(THREADS), SMEM, st, x);
-  if (nz > 1) {
+  launch_ex(gemm_kernel, dim3(grid), dim3(THREADS), dim3(z.cs > 1 ? z.cs : 0, 1, 1), true, SMEM, st, x);
+  if (groups > 1) {
     const int fb = (int)std::min<i64>(1024, ((i64)ra * s.N + 255) / 256);
     launch_pdl(finish_kernel, dim3(fb), dim3(256), 0, st, x);
   }
@@ -668,8 +726,7 @@ static bool oz_try_impl(const G& g, bool cplx, bool conjA, bool conjB, bool plai
   if (M >= (1ll << 29) || N >= (1ll << 29)) return false;
   const i64 Mo = swap ? N : M, No = swap ? M : N;
   if (!oz_fits(Mo, No, g.K, cplx)) return false;
-  const double fp64 = (cplx ? 8.0 : 2.0) * (double)M * (double)N * g.K / 1.0e6 + 4.0;   // us
-  if (oz_us(Mo, No, g.K, cplx) >= fp64) return false;
+  if (oz_us(Mo, No, g.K, cplx) >= gemm_fp64_us(g.M, g.N, g.K, (int)nb, cplx)) return false;
   OzGemm o;
   o.M = (int)Mo; o.N = (int)No; o.K = g.K; o.cplx = cplx;
   o.A = (const double*)(swap ? g.B : g.A); o.am = swap ? bn : am; o.ak = swap ? g.sBk : g.sAk;
