@@ -82,3 +82,23 @@ def test_reproducible(torch_cuda, ctx):
     for _ in range(3):
         b = svd(torch_cuda, ctx, M)
         assert all(np.array_equal(x, y) for x, y in zip(a, b))
+
+
+@pytest.mark.parametrize("q", [12, 63, 128, 200])
+@pytest.mark.parametrize("kind", ["random", "clusters", "nearly equal", "orthogonal"])
+def test_last_sweep_left_out(torch_cuda, ctx, q, kind):
+    """The sweeps end without a look at the result where the last rotations were
+    small enough: no pair of columns may be left above the level at which a
+    sweep would have counted it, q 2^-52, whatever the spectrum (equal values
+    turn by large angles at tiny cosines); the SVD's bounds as above."""
+    rng = np.random.default_rng(q + len(kind))
+    p = 2 * q
+    U0, V0 = np.linalg.qr(rng.standard_normal((p, q)))[0], np.linalg.qr(rng.standard_normal((q, q)))[0]
+    s0 = {"random": rng.random(q) + 0.01, "clusters": np.repeat(rng.random(q // 3 + 1) + 0.1, 3)[:q],
+          "nearly equal": 1 + 1e-10 * rng.standard_normal(q), "orthogonal": np.ones(q)}[kind]
+    M = (U0 * s0) @ V0.T
+    U, s, Vt = svd(torch_cuda, ctx, M)
+    # plus the rounding of U's own dot products
+    assert abs(U.T @ U - np.eye(q)).max() <= q * 2.0 ** -52 + 2 * p * 2.0 ** -53
+    assert abs(s - np.sort(s0)[::-1]).max() <= 1e-14 * p
+    assert np.linalg.norm((U * s) @ Vt - M) <= 1e-13 * p
