@@ -15,6 +15,7 @@
 //                 convention (beta = -sign(alpha)*||x||), so Q and R match the
 //                 reference's up to rounding.
 #include "ttg_common.cuh"
+#include "ttg_words.cuh"
 #include <cooperative_groups.h>
 #include <cfloat>
 #include <cstdlib>
@@ -592,14 +593,19 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_sweep64_kernel(int p, int q, d
 // once a sweep also {a0 a1, b0 b1}.  Half the barriers and half the traffic of
 // the kernel above; the two pairs of a step share one reduction (nine
 // additions for four norms and two products) and one lane each forms their
-// rotations.  Warps 4-7 turn V by the round before, as above.  All sweeps of a
+// rotations.  Warps 4-7 turn V by the round before, as above.  WORDS: instead of
+// the barriers between rounds each CTA hands its columns (of M, and a round later
+// of V) on in place as tagged words (ttg_words.cuh), and the CTA that takes a
+// column next waits for its words alone: one trip through L2 in place of the
+// columns' stores, the barrier's two trips and the loads.  All sweeps of a
 // 320 x 128 (2048 x 512) block: 5.6 (30) ms before, 3.75 (19.7) with the pair
-// kernel above, 2.2 (17.2) ms so.
-template <int R>
+// kernel above, 2.2 (17.2) ms so, with barriers.
+template <int R, bool WORDS>
 __global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, double* M, double* V,
                                                                int* counters, int* status, int init_v,
                                                                float tol2, float tol2_count,
-                                                               int max_sweeps) {
+                                                               int max_sweeps,
+                                                               unsigned long long* wm) {
   __shared__ double red[4][8];
   __shared__ double rot[2][3][2][2];               // [round parity][step][pair][p, s]
   __shared__ int act[2][3];                        // either pair turns
@@ -607,11 +613,15 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, dou
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool on_m = tid < SVD_MG;
   const int KB = ((q + 1) / 2 + 1) & ~1;           // blocks, even
-  if (!init_v)
+  constexpr int W = words::count<double>;
+  unsigned long long* wv = wm + (size_t)p * q * W;
+  unsigned int* flag = (unsigned int*)(counters + 3);
+  if (!WORDS && !init_v)
     for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)q * q; e += (i64)gridDim.x * blockDim.x)
       V[e] = (e % q == e / q) ? 1.0 : 0.0;
-  bool ok = bar.sync();
+  bool ok = WORDS || bar.sync();
   int par = 0, last_r = -1, sweep = 0;
+  unsigned int round = 0;                          // rounds done: the number its words carry
   Largest seen;
   // columns of step st (0: a0 a1 | b0 b1, 1: a0 b0 | a1 b1, 2: a0 b1 | a1 b0) as
   // positions in (a0, b0, a1, b1)
@@ -637,22 +647,39 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, dou
     rr_pair(KB, r, blockIdx.x, a, b);
     col[0] = 2 * a; col[1] = 2 * b; col[2] = 2 * a + 1; col[3] = 2 * b + 1;
   };
-  auto turn_v = [&]() {
+  // V by the rotations of round `done` (the words of the round before carry its
+  // number); to V itself after the last round
+  auto turn_v = [&](unsigned int done, bool last) {
     if (last_r < 0) return;
     const int o = par ^ 1;
-    if (!(act[o][0] | act[o][1] | act[o][2])) return;
+    if (!WORDS && !(act[o][0] | act[o][1] | act[o][2])) return;
     int col[4];
     columns(last_r, col);
     for (int i = tid - SVD_MG; i < q; i += SVD_MG) {
       double x[4];
+      unsigned long long w[4][W];
+      if (WORDS && done > 0) {
 #pragma unroll
-      for (int c = 0; c < 4; ++c) x[c] = col[c] < q ? V[(i64)q * col[c] + i] : 0.0;
+        for (int c = 0; c < 4; ++c)
+          if (col[c] < q) words::load<double>(wv + ((size_t)q * col[c] + i) * W, w[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        x[c] = 0.0;
+        if (col[c] >= q) continue;
+        if (!WORDS) x[c] = V[(i64)q * col[c] + i];
+        else if (done == 0) x[c] = init_v ? V[(i64)q * col[c] + i] : (col[c] == i ? 1.0 : 0.0);
+        else words::take<double>(wv + ((size_t)q * col[c] + i) * W, w[c], x[c], done, flag);
+      }
 #pragma unroll
       for (int st = 0; st < 3; ++st)
         if (act[o][st]) turn4(x, st, rot[o][st]);
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (col[c] < q) V[(i64)q * col[c] + i] = x[c];
+      for (int c = 0; c < 4; ++c) {
+        if (col[c] >= q) continue;
+        if (!WORDS || last) V[(i64)q * col[c] + i] = x[c];
+        else words::put(wv + ((size_t)q * col[c] + i) * W, x[c], done + 1);
+      }
     }
   };
   for (sweep = 0; sweep < max_sweeps && ok; ++sweep) {
@@ -662,13 +689,31 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, dou
         int col[4];
         columns(r, col);
         double x[R][4];
+        constexpr int RC = R < 4 ? R : 4;          // rows whose words are requested together
 #pragma unroll
-        for (int k = 0; k < R; ++k)
+        for (int k0 = 0; k0 < R; k0 += RC) {
+          unsigned long long w[RC][4][W];
+          if (WORDS && round > 0) {
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int i = tid + SVD_MG * k;
-            x[k][c] = (i < p && col[c] < q) ? M[(i64)p * col[c] + i] : 0.0;
+            for (int k = 0; k < RC; ++k)
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const int i = tid + SVD_MG * (k0 + k);
+                if (i < p && col[c] < q) words::load<double>(wm + ((size_t)p * col[c] + i) * W, w[k][c]);
+              }
           }
+#pragma unroll
+          for (int k = 0; k < RC; ++k)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const int i = tid + SVD_MG * (k0 + k);
+              double& v = x[k0 + k][c];
+              v = 0.0;
+              if (i >= p || col[c] >= q) continue;
+              if (!WORDS || round == 0) v = M[(i64)p * col[c] + i];
+              else words::take<double>(wm + ((size_t)p * col[c] + i) * W, w[k][c], v, round, flag);
+            }
+        }
         bool any = false;
 #pragma unroll
         for (int st = 0; st < 3; ++st) {
@@ -733,23 +778,26 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, dou
             for (int k = 0; k < R; ++k) turn4(x[k], st, rt);
           }
         }
-        if (any) {
 #pragma unroll
-          for (int k = 0; k < R; ++k)
+        for (int k = 0; k < R; ++k)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const int i = tid + SVD_MG * k;
-              if (i < p && col[c] < q) M[(i64)p * col[c] + i] = x[k][c];
-            }
-        }
+          for (int c = 0; c < 4; ++c) {
+            const int i = tid + SVD_MG * k;
+            if (i >= p || col[c] >= q) continue;
+            if (WORDS) words::put(wm + ((size_t)p * col[c] + i) * W, x[k][c], round + 1);
+            else if (any) M[(i64)p * col[c] + i] = x[k][c];
+          }
         if (r == KB - 2) seen.give(top);
       } else {
-        turn_v();
+        if (round > 0) turn_v(round - 1, false);
       }
-      ok = bar.sync();
+      if (WORDS) __syncthreads();
+      else ok = bar.sync();
       last_r = r;
       par ^= 1;
+      ++round;
     }
+    if (WORDS) ok = bar.sync();
     const int done = *((volatile int*)cnt) == 0 || sweep_settled(top, q, tol2);
     ok = bar.sync() && ok;
     if (blockIdx.x == 0 && tid == 0) {
@@ -759,10 +807,27 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_block_kernel(int p, int q, dou
     ok = bar.sync() && ok;
     if (done) break;
   }
-  if (!on_m) turn_v();
-  if (!ok)   // a wait ran out: nothing here may be taken for a result
-    for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)p * q; e += (i64)gridDim.x * blockDim.x)
-      M[e] = __longlong_as_double(0x7ff8000000000000ll);
+  // (WORDS: the last round's columns are this CTA's own)
+  if (!on_m) {
+    turn_v(round - 1, true);
+  } else if (!WORDS) {
+    if (!ok)   // a wait ran out: nothing here may be taken for a result
+      for (i64 e = blockIdx.x * (i64)SVD_MG + tid; e < (i64)p * q; e += (i64)gridDim.x * SVD_MG)
+        M[e] = __longlong_as_double(0x7ff8000000000000ll);
+  } else {
+    int col[4];
+    columns(last_r, col);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      for (int i = tid; i < p && col[c] < q; i += SVD_MG) {
+        unsigned long long w[W];
+        double v = 0.0;
+        words::load<double>(wm + ((size_t)p * col[c] + i) * W, w);
+        words::take<double>(wm + ((size_t)p * col[c] + i) * W, w, v, round, flag);
+        const bool good = ok && *(volatile unsigned int*)flag == 0u;
+        M[(i64)p * col[c] + i] = good ? v : __longlong_as_double(0x7ff8000000000000ll);
+      }
+  }
   if (blockIdx.x == 0 && tid == 0 && status) *status = sweep;
 }
 
@@ -863,11 +928,12 @@ static int coop_blocks(const void* k, int nt) {
 }
 
 static void svd_sweeps(int p, int q, double* M, double* V, int* counters, int* status, int init_v,
-                       double tol, double tol_count, int max_sweeps, cudaStream_t s) {
+                       double tol, double tol_count, int max_sweeps, double* work, cudaStream_t s) {
   float tol2 = (float)(tol * tol), tol2_count = (float)(tol_count * tol_count);
   // rotations of even and odd sweeps, barrier, its failure, cosines, sines
   TTG_CUDA(cudaMemsetAsync(counters, 0, 8 * sizeof(int), s));
-  void* args[] = {&p, &q, &M, &V, &counters, &status, &init_v, &tol2, &tol2_count, &max_sweeps};
+  unsigned long long* wm = (unsigned long long*)(((uintptr_t)work + 15) & ~(uintptr_t)15);
+  void* args[] = {&p, &q, &M, &V, &counters, &status, &init_v, &tol2, &tol2_count, &max_sweeps, &wm};
   auto launch = [&](const void* k, int blocks) {
     TTG_CUDA(cudaLaunchCooperativeKernel(k, dim3(blocks), dim3(2 * SVD_MG), args, 0, s));
     ++g_launches;
@@ -876,12 +942,18 @@ static void svd_sweeps(int p, int q, double* M, double* V, int* counters, int* s
   // columns to a CTA (a resident grid of q / 4 CTAs always fits)
   const int kb = ((q + 1) / 2 + 1) & ~1;
   if (p <= 8 * SVD_MG && q >= 4) {
-    static const int max_block = coop_blocks((const void*)svd_block_kernel<8>, 2 * SVD_MG);
+    static const int max_block = coop_blocks((const void*)svd_block_kernel<8, false>, 2 * SVD_MG);
     if (kb / 2 <= max_block) {
-      if (p <= SVD_MG) launch((const void*)svd_block_kernel<1>, kb / 2);
-      else if (p <= 2 * SVD_MG) launch((const void*)svd_block_kernel<2>, kb / 2);
-      else if (p <= 4 * SVD_MG) launch((const void*)svd_block_kernel<4>, kb / 2);
-      else launch((const void*)svd_block_kernel<8>, kb / 2);
+      // Columns handed on as words up to 128 rows: 128 x 64 1864 -> 1717 us, 64 x
+      // 24 690 -> 661, 320 x 128 (a 128 x 128 triangle) 4352 -> 4078; with
+      // more rows a thread the words cost what the barrier did (256 x 160 6201 ->
+      // 6049, 256 x 256 9997 -> 10218) or more (512 x 300 15.8 -> 16.9 ms).
+      if (p <= SVD_MG) {
+        TTG_CUDA(cudaMemsetAsync(wm, 0, 16 * (size_t)(p + q) * q, s));
+        launch((const void*)svd_block_kernel<1, true>, kb / 2);
+      } else if (p <= 2 * SVD_MG) launch((const void*)svd_block_kernel<2, false>, kb / 2);
+      else if (p <= 4 * SVD_MG) launch((const void*)svd_block_kernel<4, false>, kb / 2);
+      else launch((const void*)svd_block_kernel<8, false>, kb / 2);
       return;
     }
   }
@@ -1348,11 +1420,13 @@ static size_t svd_qr_work(size_t p, size_t q) {
 
 size_t svd_scratch(int p, int q) {
   // working copy of M (max(p,q) x min(p,q)), V (min^2), norms, ranks, counters, Ut,
-  // for the FP32 pre-sweeps two min^2 and one max x min temporaries, and the
-  // workspace of the QR-preconditioned path
+  // for the FP32 pre-sweeps two min^2 and one max x min temporaries, the
+  // workspace of the QR-preconditioned path, and the columns that the block
+  // sweeps hand on as tagged words (two doubles per value)
   size_t pp = std::max(p, q), qq = std::min(p, q);
   return (pp * qq + qq * qq + 2 * qq + 64) * sizeof(double) + pp * qq * sizeof(double) +
-         (2 * qq * qq + pp * qq) * sizeof(double) + svd_qr_work(pp, qq) * sizeof(double);
+         (2 * qq * qq + pp * qq) * sizeof(double) + svd_qr_work(pp, qq) * sizeof(double) +
+         (4 * (size_t)SVD_MG * std::min(qq, (size_t)SVD_MG) + 2) * sizeof(double);
 }
 
 static inline int gbl(i64 n) { return (int)std::max<i64>(1, std::min<i64>(4096, (n + 255) / 256)); }
@@ -1486,7 +1560,7 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   // (FP32 pre-sweeps do not pay here: the preconditioned matrix converges in
   // a few FP64 sweeps, and FP32 cannot resolve its small columns)
   svd_sweeps(q, q, X2, V, counters, status, 0, sqrt((double)q) * DBL_EPSILON,
-                     (double)q * DBL_EPSILON, SVD_MAX_SWEEPS, s);
+                     (double)q * DBL_EPSILON, SVD_MAX_SWEEPS, work + svd_qr_work(p, q), s);
   svd_finish_kernel<<<nb, 256, 0, s>>>(q, q, X2, V, nullptr, nullptr, nullptr, nrm, rank);
   TTG_CHECK_LAUNCH();
   svd_rank_kernel<<<ceil_div(q, 256), 256, 0, s>>>(q, nrm, rank);
@@ -1566,7 +1640,7 @@ static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double*
     init_v = 1;
   }
   svd_sweeps(p, q, Mw, V, counters, status, init_v, sqrt((double)p) * DBL_EPSILON,
-                     (double)p * DBL_EPSILON, SVD_MAX_SWEEPS, s);
+                     (double)p * DBL_EPSILON, SVD_MAX_SWEEPS, qrwork + svd_qr_work(p, q), s);
   int nb = std::max(1, std::min(1024, ceil_div((i64)q * 32, 256)));
   svd_finish_kernel<<<nb, 256, 0, s>>>(p, q, Mw, V, U, sigma, Vt, nrm, rank);
   TTG_CHECK_LAUNCH();
