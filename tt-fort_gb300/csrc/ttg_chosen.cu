@@ -18,6 +18,7 @@
 // The FP64 matvecs of phase B are the judge: the returned eigenpairs meet the
 // same FP64 residual test as the plain method.
 #include "ttg_davidson.cuh"
+#include "ttg_words.cuh"
 #include <algorithm>
 #include <cstdlib>
 
@@ -223,6 +224,257 @@ __global__ void cg_dir_kernel(i64 N, int t, const double* __restrict__ rr,
   }
 }
 
+// A whole CG step after its operator product, in one resident grid:
+//   q = A~ p - theta p;  C = X^T q;  pq = p^T q;  q -= X C;
+//   x, r, |r|^2 as in cg_update_kernel;  p = r + beta p
+// for up to CT_NV columns and Ritz vectors.  A thread keeps its RPT rows of p
+// and q in registers; the three sums are exchanged as tagged words
+// (ttg_words.cuh): C and pq through one CTA per value, |r|^2 read by every CTA
+// from all.  The five kernels it stands for (shift, X^T q, proj_dot, cg_update,
+// cg_dir) took 3 to 8 us each, mostly launch, ramp and the last block's sum;
+// this one takes 12 (N up to 2560, five columns).  Local problems with blocks of
+// five, solved to 1e-9: N = 8192 11.6 -> 10.2 ms, 19200 14.0 -> 11.7, 76800 26.2
+// -> 20.4; block eigenproblem d = 12: 136.4 -> 119.7 ms.
+// Every wait is bounded; a CTA whose wait ran out leaves NaN in its rows.
+constexpr int CT_NT = 128, CT_NV = 8, CT_GMAX = 152;
+constexpr int CT_NC = CT_NV * (CT_NV + 1);          // C and pq
+constexpr size_t kTailWords = 2 * (size_t)(CT_GMAX * (CT_NC + CT_NV) + CT_NC) + 2;
+template <int RPT, int CS>
+__global__ void __launch_bounds__(CT_NT) cg_tail_kernel(i64 N, int t, int nb,
+                                                        const double* __restrict__ X,
+                                                        const double* __restrict__ theta, double tol2,
+                                                        const double* __restrict__ rr0,
+                                                        const double* __restrict__ rr,
+                                                        double* __restrict__ rr_new,
+                                                        double* __restrict__ x, double* __restrict__ r,
+                                                        double* __restrict__ p,
+                                                        const double* __restrict__ q,
+                                                        unsigned long long* __restrict__ words,
+                                                        unsigned int epoch) {
+  constexpr int NV = CT_NV, NC = CT_NC, NW = CT_NT / 32, W = words::count<double>;
+  constexpr int QC = (CT_GMAX + 31) / 32, LS = CT_NT / NV, QS = (CT_GMAX + LS - 1) / LS;
+  __shared__ double red[NW][NC], Cs[NC], tot[NV], coef[NV];
+  __shared__ bool on_s[NV];
+  __shared__ int s_fail;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, b = blockIdx.x, G = gridDim.x;
+  unsigned long long* partC = words;
+  unsigned long long* totC = partC + (size_t)CT_GMAX * NC * W;
+  unsigned long long* partS = totC + (size_t)NC * W;              // [CT_GMAX][NV]
+  unsigned int* flag = (unsigned int*)(partS + (size_t)CT_GMAX * NV * W);
+  if (tid == 0) s_fail = 0;
+  auto got = [&](const unsigned long long* w, unsigned long long (&y)[W], double& v) {
+    if (words::take<double>(w, y, v, epoch, flag)) return true;
+    s_fail = 1;
+    return false;
+  };
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  // warp w holds rows of group w / CS and columns w % CS, w % CS + CS, ...
+  constexpr int NJ = NV / CS, NR = NW / CS;
+  const int rg = warp / CS, j0 = warp % CS;
+  double pv[RPT][NJ], qv[RPT][NJ], rv[RPT][NJ], xk[RPT][NV];
+  i64 row[RPT];
+  bool in[RPT];
+#pragma unroll
+  for (int k = 0; k < RPT; ++k) {
+    row[k] = (((i64)k * G + b) * NR + rg) * 32 + lane;
+    in[k] = row[k] < N;
+#pragma unroll
+    for (int v = 0; v < NV; ++v) xk[k][v] = in[k] && v < nb ? X[row[k] + N * v] : 0.0;
+#pragma unroll
+    for (int c = 0; c < NJ; ++c) {
+      const int j = j0 + CS * c;
+      const bool there = in[k] && j < t;
+      pv[k][c] = there ? p[row[k] + N * j] : 0.0;
+      qv[k][c] = there ? q[row[k] + N * j] : 0.0;
+      rv[k][c] = there ? r[row[k] + N * j] : 0.0;
+    }
+#pragma unroll
+    for (int c = 0; c < NJ; ++c)
+      if (j0 + CS * c < t) qv[k][c] -= theta[j0 + CS * c] * pv[k][c];
+  }
+  // sums of a warp's NJ columns over its rows, to red[rg][first + j]
+  auto column_sums = [&](double (&a)[NJ], int first) {
+    const double sum = warp_sums<NJ>(a);
+    if ((lane & (32 / NJ - 1)) == 0) red[rg][first + j0 + CS * (lane * NJ >> 5)] = sum;
+  };
+  // C = X^T q, and pq = p^T q: p has no part along X, so taking X C out of q
+  // first (as proj_dot does) changes p^T q by less than its rounding
+  double a[NJ];
+#pragma unroll
+  for (int c = 0; c < NJ; ++c) {
+    a[c] = 0.0;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) a[c] = fma(pv[k][c], qv[k][c], a[c]);
+  }
+  column_sums(a, NV * NV);
+#pragma unroll
+  for (int c = 0; c < NJ; ++c) {
+    if (j0 + CS * c >= t) break;
+    double y[NV];
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+      y[v] = 0.0;
+      if (v < nb) {
+#pragma unroll
+        for (int k = 0; k < RPT; ++k) y[v] = fma(xk[k][v], qv[k][c], y[v]);
+      }
+    }
+    const double sum = warp_sums<NV>(y);
+    if ((lane & (32 / NV - 1)) == 0) red[rg][NV * (j0 + CS * c) + (lane * NV >> 5)] = sum;
+  }
+  __syncthreads();
+  auto valid = [&](int v) { return v < NV * NV ? v % NV < nb && v / NV < t : v - NV * NV < t; };
+  const bool mine = tid < NC && valid(tid);
+  if (mine) {
+    double v = red[0][tid];
+#pragma unroll
+    for (int w = 1; w < NR; ++w) v += red[w][tid];
+    words::put(partC + ((size_t)b * NC + tid) * W, v, epoch);
+  }
+  for (int v = b + G * warp; v < NC; v += G * NW) {
+    if (!valid(v)) continue;
+    unsigned long long y[QC][W];
+#pragma unroll
+    for (int k = 0; k < QC; ++k)
+      if (lane + 32 * k < G) words::load<double>(partC + ((size_t)(lane + 32 * k) * NC + v) * W, y[k]);
+    double sum = 0.0;
+#pragma unroll
+    for (int k = 0; k < QC; ++k) {
+      double z;
+      if (lane + 32 * k < G && got(partC + ((size_t)(lane + 32 * k) * NC + v) * W, y[k], z)) sum += z;
+    }
+    __syncwarp();
+    sum = warp_sum_d(sum);
+    if (lane == 0) words::put(totC + (size_t)v * W, sum, epoch);
+  }
+  if (mine) {
+    unsigned long long y[W];
+    double v = 0.0;
+    words::load<double>(totC + (size_t)tid * W, y);
+    got(totC + (size_t)tid * W, y, v);
+    Cs[tid] = v;
+  }
+  __syncthreads();
+  // alpha (zero for a frozen column, whose x and r stay)
+  bool active = false;
+  if (tid < t) {
+    const double pq = Cs[NV * NV + tid];
+    active = pq > 0.0 && rr[tid] > tol2 * rr0[tid];
+    coef[tid] = active ? rr[tid] / pq : 0.0;
+    on_s[tid] = active;
+  }
+  // q -= X C
+#pragma unroll
+  for (int c = 0; c < NJ; ++c) {
+    const int j = j0 + CS * c;
+    if (j >= t) continue;
+#pragma unroll
+    for (int k = 0; k < RPT; ++k)
+#pragma unroll
+      for (int e = 0; e < NV; ++e)
+        if (e < nb) qv[k][c] = fma(-xk[k][e], Cs[e + NV * j], qv[k][c]);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int c = 0; c < NJ; ++c) {
+    const int j = j0 + CS * c;
+    a[c] = 0.0;
+    if (j >= t) continue;
+    const double al = coef[j];
+    const bool on = on_s[j];
+#pragma unroll
+    for (int k = 0; k < RPT; ++k) {
+      if (!in[k]) continue;
+      const i64 e = row[k] + N * j;
+      if (on) {
+        x[e] = fma(al, pv[k][c], x[e]);
+        rv[k][c] = fma(-al, qv[k][c], rv[k][c]);
+        r[e] = rv[k][c];
+      }
+      a[c] = fma(rv[k][c], rv[k][c], a[c]);
+    }
+  }
+  // |r|^2, added in the same order in every CTA
+  {
+    column_sums(a, 0);
+    __syncthreads();
+    unsigned long long* ps = partS;
+    if (tid < t) {
+      double v = red[0][tid];
+#pragma unroll
+      for (int w = 1; w < NR; ++w) v += red[w][tid];
+      words::put(ps + ((size_t)b * NV + tid) * W, v, epoch);
+    }
+    const int j = tid % NV, l = tid / NV;
+    unsigned long long y[QS][W];
+#pragma unroll
+    for (int k = 0; k < QS; ++k)
+      if (j < t && l + LS * k < G) words::load<double>(ps + ((size_t)(l + LS * k) * NV + j) * W, y[k]);
+    double g = 0.0;
+#pragma unroll
+    for (int k = 0; k < QS; ++k) {
+      double z;
+      if (j < t && l + LS * k < G && got(ps + ((size_t)(l + LS * k) * NV + j) * W, y[k], z)) g += z;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int o = NV; o < 32; o <<= 1) g += __shfl_xor_sync(0xffffffffu, g, o);
+    __syncthreads();
+    if (lane < NV) red[warp][lane] = g;
+    __syncthreads();
+    if (tid < NV) {
+      double v = red[0][tid];
+#pragma unroll
+      for (int w = 1; w < NW; ++w) v += red[w][tid];
+      tot[tid] = v;
+    }
+  }
+  if (tid < t) {
+    const double g = tot[tid];
+    coef[tid] = (active && rr[tid] > 0.0) ? g / rr[tid] : 0.0;
+    if (b == 0) rr_new[tid] = s_fail ? nan : g;
+  }
+  __syncthreads();
+  const bool fail = s_fail != 0;
+#pragma unroll
+  for (int c = 0; c < NJ; ++c) {
+    const int j = j0 + CS * c;
+    if (j >= t) continue;
+    const double be = coef[j];
+#pragma unroll
+    for (int k = 0; k < RPT; ++k)
+      if (in[k]) {
+        const i64 e = row[k] + N * j;
+        p[e] = fail ? nan : rv[k][c] + be * pv[k][c];
+        if (fail) x[e] = nan;
+      }
+  }
+}
+// The form for N rows (null: the five kernels) and its grid.  A warp's FP64
+// instructions hold its partition of the SM for 64 clocks each whatever the
+// rows, some 200 of them at five columns, so while SMs are idle the columns are
+// split over the warps: 32 rows a CTA (128 rows there: 20 us in place of 12), then
+// 64, then 128, then more a thread.
+static const void* cg_tail_form(i64 N, int t, int nb, int& grid) {
+  constexpr i64 full = (i64)CT_GMAX * CT_NT;
+  if (t > CT_NV || nb > CT_NV || N > 4 * full) return nullptr;
+  static const int held = [] {
+    int dev = 0, nsm = 0, per = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, cg_tail_kernel<4, 1>, CT_NT, 0) != cudaSuccess)
+      return 0;
+    return nsm * per;
+  }();
+  const int rows = N <= full / 4 ? 32 : (N <= full / 2 ? 64 : CT_NT);
+  grid = (int)std::min<i64>(CT_GMAX, (N + rows - 1) / rows);
+  if (held < grid) return nullptr;
+  if (rows == 32) return (const void*)cg_tail_kernel<1, 4>;
+  if (rows == 64) return (const void*)cg_tail_kernel<1, 2>;
+  return N <= full ? (const void*)cg_tail_kernel<1, 1>
+                   : (N <= 2 * full ? (const void*)cg_tail_kernel<2, 1> : (const void*)cg_tail_kernel<4, 1>);
+}
+
 void gemm_tn_small(int M, int N, i64 K, const double* A, i64 lda, const double* B, i64 ldb,
                    double* C, int ldc, double alpha, double beta, cudaStream_t s);
 void gemm_nn_small(i64 R, int N, int K, const double* A, i64 lda, const double* B, int ldb,
@@ -237,11 +489,12 @@ struct JdCg {
   cudaStream_t s;
   double *x, *r, *p, *q, *sc;   // N x Bmax each; sc: scalars
   double *part_cd, *part_cu, *part_pd;   // partial sums of the grid reductions
+  unsigned long long* words;             // cg_tail_kernel's exchanges
   unsigned int* cnt;                     // their ticket counters (zero between uses)
 
   static constexpr size_t kParts = 2 * (size_t)CG_MAXT * CG_MAXBX + (size_t)CG_MAXT * CG_MAXPB;
   static size_t bytes(i64 N, int Bmax) {
-    return (4 * (size_t)N * Bmax + 16 * 64 + kParts + 64) * sizeof(double) + 4096;
+    return (4 * (size_t)N * Bmax + 16 * 64 + kParts + 64 + kTailWords + 2) * sizeof(double) + 4096;
   }
 
   void bind(void* mem) {
@@ -253,6 +506,7 @@ struct JdCg {
     part_pd = part_cu + (size_t)CG_MAXT * CG_MAXBX;
     cnt = (unsigned int*)(part_pd + (size_t)CG_MAXT * CG_MAXPB);   // 3 x 16 counters
     TTG_CUDA(cudaMemsetAsync(cnt, 0, 64 * sizeof(double), s));
+    words = (unsigned long long*)(((uintptr_t)(cnt + 128) + 15) & ~(uintptr_t)15);
   }
 
   // project out X (N x nb): v -= X (X^T v)
@@ -262,10 +516,10 @@ struct JdCg {
     gemm_nn_small(N, t, nb, X, N, c, nb, v, N, -1.0, 1.0, s);
   }
 
-  // The fixed-length CG solve issues ~12 launches per step and has no host
+  // The fixed-length CG solve issues 4 to 12 launches per step and has no host
   // synchronisation, so after its first call for a given (block, shift,
   // Ritz-vector) set of buffers and widths it is captured once into a CUDA
-  // graph and replayed: one launch per correction solve instead of ~150.
+  // graph and replayed: one launch per correction solve instead of 50 to 150.
   bool use_graph = true;
   struct Cached {
     double* T;
@@ -340,8 +594,21 @@ struct JdCg {
     TTG_CUDA(cudaMemcpyAsync(rr0, rr, sizeof(double) * t, cudaMemcpyDeviceToDevice, s));
     const bool fused = t <= PD_MAXT && nb <= PD_MAXT;
     int pb = (int)std::max<i64>(1, std::min<i64>(CG_MAXPB, (N + 127) / 128));
+    int tail_grid = 0;
+    const void* tail = cg_tail_form(N, t, nb, tail_grid);
+    if (tail) TTG_CUDA(cudaMemsetAsync(words, 0, kTailWords * 8, s));
     for (int it = 0; it < iters; ++it) {
       low(p, q, t);                                   // q = A~ p
+      if (tail) {
+        i64 n = N;
+        double tl = tol2;
+        unsigned int epoch = (unsigned)it + 1;
+        void* args[] = {&n, &t, &nb, &X, &theta, &tl, &rr0, &rr, &rr_new, &x, &r, &p, &q, &words, &epoch};
+        TTG_CUDA(cudaLaunchCooperativeKernel(tail, dim3(tail_grid), dim3(CT_NT), args, 0, s));
+        ++g_launches;
+        std::swap(rr, rr_new);
+        continue;
+      }
       launch_pdl(shift_kernel, dim3(eb), dim3(256), 0, s, N, t, theta, (const double*)p, q, pq,
                  rr_new);                               // q -= theta p
       if (fused) {
