@@ -239,9 +239,10 @@ __device__ __forceinline__ bool sweep_settled(const int* top, int q, float tol2)
 // ---------------------------------------------------------------------------
 // symmetric eigensolver: cyclic Jacobi in one CTA
 // ---------------------------------------------------------------------------
-constexpr int JAC_NT = 1024;
+constexpr int JAC_SMALL = 32;   // up to this order: 256 threads
 constexpr int JAC_MAX_SWEEPS = 40;
 
+template <int JAC_NT>
 __global__ void __launch_bounds__(JAC_NT) syev_jacobi_kernel(int k, double* Ag, int lda,
                                                              double* w, double* Vg, int ldv,
                                                              int* status, int smem_mode,
@@ -410,14 +411,21 @@ void syev_jacobi(int k, double* A, int lda, double* w, double* V, int ldv, int* 
   int mode = smem <= 200 * 1024 ? 1 : 0;
   if (mode) {
     // thread-safe one-time set-up (C++ static initialisation)
-    static const cudaError_t attr_rc = cudaFuncSetAttribute(
-        syev_jacobi_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    static const cudaError_t attr_rc = [] {
+      const cudaError_t r = cudaFuncSetAttribute(syev_jacobi_kernel<256>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+      return r != cudaSuccess ? r
+                              : cudaFuncSetAttribute(syev_jacobi_kernel<1024>,
+                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+    }();
     TTG_CUDA(attr_rc);
   } else {
     smem = 0;
   }
-  syev_jacobi_kernel<<<1, JAC_NT, smem, s>>>(k, A, lda, w, V, ldv, status, mode,
-                                             warm ? P0 : nullptr, warm ? kp : 0, ldp);
+  // a round has four barriers: eight warps are enough for small matrices (k = 10
+  // to 20: 78 -> 70 us)
+  (k <= JAC_SMALL ? syev_jacobi_kernel<256> : syev_jacobi_kernel<1024>)<<<1, k <= JAC_SMALL ? 256 : 1024, smem, s>>>(
+      k, A, lda, w, V, ldv, status, mode, warm ? P0 : nullptr, warm ? kp : 0, ldp);
   TTG_CHECK_LAUNCH();
 }
 
