@@ -209,3 +209,21 @@ def test_programmatic_dependent_launch_changes_no_result(torch_cuda):
         assert out.returncode == 0, out.stderr[-2000:]
         res[mode] = json.loads(out.stdout.strip().splitlines()[-1])
     assert res["0"] == res["1"]
+
+
+@pytest.mark.parametrize("persistent", ["1", "0"])
+def test_split_gemm_narrow_tile_vs_oracle(torch_cuda, persistent):
+    """32-column tiles (small products), in the persistent kernel and in the one
+    with a tile per CTA."""
+    import json
+    import os
+    import subprocess
+    import sys
+    from conftest import ROOT
+    env = dict(os.environ, TTG_SPLIT_BN="32", TTG_GEMM_WS=persistent,
+               PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tt-fort_gb300")]))
+    out = subprocess.run([sys.executable, "-c", _FUSED_CHILD, json.dumps(WIDE_SHAPES)],
+                         capture_output=True, text=True, env=env, timeout=600)
+    assert out.returncode == 0, out.stderr[-2000:]
+    errs = json.loads(out.stdout.strip().splitlines()[-1])
+    assert max(errs) < TOL_SPLIT, errs

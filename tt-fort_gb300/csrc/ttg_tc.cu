@@ -386,7 +386,7 @@ __global__ void __launch_bounds__(WS_THREADS, 1)
                          i64 rpv, i64 vstride, i64 rstride, i64 cstride, int* __restrict__ err,
                          int kchunk, i64 zstride, const EpiT2 ep) {
   static_assert(NPROD == 1 || NPROD == 3, "one or three bf16 products");
-  static_assert(BN == 64 || BN == 128 || BN == 256, "tile width");
+  static_assert(BN == 32 || BN == 64 || BN == 128 || BN == 256, "tile width");
   constexpr int STAGES = ws_stages<BN, NPROD>();
   constexpr uint32_t A_BYTES = TM * TK * 2;
   constexpr uint32_t B_BYTES = BN * TK * 2;
@@ -1275,11 +1275,14 @@ constexpr size_t smem_for(int bn) {
 // number of waves (CTAs over SMs x resident CTAs) times the per-tile cost
 // (K loop of MMAs and bulk copies plus the epilogue), so small products pick
 // narrow tiles that spread over more SMs and large ones pick wide tiles.
+// 32 columns halve the epilogue of a small product, whose FP64 conversions hold
+// each SM partition (r = 64 chain, block of 5: 13.6 us with 64, 12.3 with 32, the
+// same bits; d = 12 block eigenproblem 114.8 -> 113.9 ms).
 static int pick_bn(int M, int N, int K) {
   const int mt = ceil_div(M, TM), kt = ceil_div(K, TK), nsm = num_sms();
   int best = 64;
   double best_cost = 1e300;
-  for (int bn : {256, 128, 64}) {
+  for (int bn : {256, 128, 64, 32}) {
     const int per_sm = use_ws() ? 1 : (int)std::max<size_t>(1, 228 * 1024 / (smem_for(bn) + 1024));
     const long long ctas = (long long)mt * ceil_div(N, bn);
     const long long waves = (ctas + (long long)nsm * per_sm - 1) / ((long long)nsm * per_sm);
@@ -1357,7 +1360,8 @@ static void gemm_launch(const Tiled& A, const Tiled& B, int M, int N, OutT* out,
   TTG_REQUIRE(A.R == TM, "split gemm: A tiles must have 128 rows");
   if (B.R == 256) gemm_launch_bn<256>(A, B, M, N, out, rpv, vstride, rstride, cstride, err, s);
   else if (B.R == 128) gemm_launch_bn<128>(A, B, M, N, out, rpv, vstride, rstride, cstride, err, s);
-  else gemm_launch_bn<64>(A, B, M, N, out, rpv, vstride, rstride, cstride, err, s);
+  else if (B.R == 64) gemm_launch_bn<64>(A, B, M, N, out, rpv, vstride, rstride, cstride, err, s);
+  else gemm_launch_bn<32>(A, B, M, N, out, rpv, vstride, rstride, cstride, err, s);
 }
 
 // product whose epilogue writes the split T2 operand (EPI = 1)
@@ -1373,8 +1377,11 @@ static void gemm_launch_t2(const Tiled& A, const Tiled& B, int M, int N, const E
   else if (B.R == 128)
     ws_launch<128, float, 3, 1>(A.hi, A.lo, B.hi, B.lo, M, N, A.ktiles, A.rtiles, B.rtiles, 1, none,
                                 1ll << 40, 0, 1, 0, err, 0, 0, s, ep);
-  else
+  else if (B.R == 64)
     ws_launch<64, float, 3, 1>(A.hi, A.lo, B.hi, B.lo, M, N, A.ktiles, A.rtiles, B.rtiles, 1, none,
+                               1ll << 40, 0, 1, 0, err, 0, 0, s, ep);
+  else
+    ws_launch<32, float, 3, 1>(A.hi, A.lo, B.hi, B.lo, M, N, A.ktiles, A.rtiles, B.rtiles, 1, none,
                                1ll << 40, 0, 1, 0, err, 0, 0, s, ep);
 }
 
@@ -1543,11 +1550,11 @@ static int tuned_bn(int M, int N, int K, bool out_double, cudaStream_t s) {
     const char* v = std::getenv("TTG_AUTOTUNE");
     return !(v && v[0] == '0');
   }();
-  // TTG_SPLIT_BN=64|128|256 fixes the tile width of every split product
+  // TTG_SPLIT_BN=32|64|128|256 fixes the tile width of every split product
   static const int forced = [] {
     const char* v = std::getenv("TTG_SPLIT_BN");
     const int b = v ? std::atoi(v) : 0;
-    return (b == 64 || b == 128 || b == 256) ? b : 0;
+    return (b == 32 || b == 64 || b == 128 || b == 256) ? b : 0;
   }();
   if (forced) return forced;
   const int model = pick_bn(M, N, K);
@@ -1578,7 +1585,7 @@ static int tuned_bn(int M, int N, int K, bool out_double, cudaStream_t s) {
   int* err = (int*)(mem + abytes + bbytes + obytes);
   int best = model;
   float best_ms = 1e30f;
-  for (int bn : {64, 128, 256}) {
+  for (int bn : {32, 64, 128, 256}) {
     const float ms = out_double ? time_bn<double>(bn, A, bbuf, M, N, K, (double*)out, err, s)
                                 : time_bn<float>(bn, A, bbuf, M, N, K, (float*)out, err, s);
     if (ms < best_ms * 0.97f || (bn == model && ms < best_ms * 1.03f)) { best_ms = ms; best = bn; }
@@ -1888,7 +1895,7 @@ void split_op_prepare(SplitOp* op, const LocalDims& L, int nvec_max, const doubl
 static void core_apply(SplitOp* op, int nvec, cudaStream_t s) {
   const LocalDims& L = op->L;
   const tc::Tiled& T2 = op->T2;
-  const int lgR3 = T2.R == 256 ? 8 : (T2.R == 128 ? 7 : 6);
+  const int lgR3 = T2.R == 256 ? 8 : (T2.R == 128 ? 7 : (T2.R == 64 ? 6 : 5));
   const int ja = (int)(L.m * L.ra2), na = (int)(L.n * L.ra1);
   if (op->coef_kind > 0) {
     const bool wide = L.rx1 % 8 == 0 && (L.rx1 / 8) * L.ry2 * nvec >= 32768;
@@ -1998,7 +2005,7 @@ void split_op_apply(SplitOp* op, const double* x, double* y, int nvec, cudaStrea
     tc::EpiT2 ep;
     ep.rx1 = (int)L.rx1;
     ep.nry2 = (int)(L.n * L.ry2);
-    ep.lgR3 = T2b.R == 256 ? 8 : (T2b.R == 128 ? 7 : 6);
+    ep.lgR3 = T2b.R == 256 ? 8 : (T2b.R == 128 ? 7 : (T2b.R == 64 ? 6 : 5));
     ep.ktiles3 = T2b.ktiles;
     ep.hi = T2b.hi;
     ep.lo = T2b.lo;
