@@ -213,3 +213,17 @@ def test_k_split_over_clusters(torch_cuda, ctx, M, N, K):
     A, B = X[rows], P2[:, cols]
     err = abs(got[rows][:, cols] - A @ B)
     assert (err <= oz_bound(A, B) + (K + 4) * U * (abs(A) @ abs(B))).all()
+
+
+@pytest.mark.parametrize("M,N,K", [
+    (640, 320, 128), (129, 33, 640), (1000, 31, 300), (2000, 97, 256), (2432, 130, 200), (2433, 127, 200),
+])
+def test_narrow_tiles(torch_cuda, ctx, M, N, K):
+    """32 columns a tile where 64 leave more than half of the SMs idle, at the
+    edges of a tile and on both sides of the rule (76 tiles of 128 x 64)."""
+    rng = np.random.default_rng(M + N + K)
+    X, P2 = rng.standard_normal((M, K)), rng.standard_normal((K, N))
+    got, launches = plain_product(torch_cuda, ctx, X, P2)
+    assert launches > 3, "the split product was not taken"
+    err = abs(got - X @ P2)
+    assert (err <= oz_bound(X, P2) + (K + 4) * U * (abs(X) @ abs(P2))).all()

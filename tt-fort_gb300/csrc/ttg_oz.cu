@@ -29,15 +29,15 @@
 //
 // Measured on GB300, FP64 kernels -> split products: chain product r=256, block
 // of 8: 4560 -> 241 us (22.7 TFLOP/s of FP64 accuracy; its two products run at
-// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 38.4
-// us; grid interface updates r = 82, 77, n = 64: 1908 -> 167 us; complex
+// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 32.8
+// us; grid interface updates r = 82, 77, n = 64: 1908 -> 160 us; complex
 // operator and adjoint r=48, n=32, block of 4: 6968 -> 403 us.  What bounds the
 // product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
 // measured against 900 of MMA), for small ones its fixed ~10 us (pipeline
 // fill, one drain, rounding); oz_us below holds both.
 //
-// Tensor memory: a 128 x 64 tile with its seven groups side by side (448 of
-// the 512 columns).  The digit planes of B sit stacked along N, so the MMA of
+// Tensor memory: a 128 x 64 tile (128 x 32 for small products) with its seven
+// groups side by side (448 of the 512 columns).  The digit planes of B sit stacked along N, so the MMA of
 // A's plane p with B's planes 0..6-p writes groups p..6 in one instruction
 // (two where N > 256): ten instructions per 16-wide K step, and A's planes are
 // read from shared memory once per step.
@@ -52,13 +52,14 @@ namespace oz {
 using namespace tc;
 
 constexpr int P = 7;            // digit planes
-constexpr int BM = 128, BN = 64;
+constexpr int BM = 128;         // rows of A's tiles; B's: 64, or 32 for small products
 constexpr int KCHUNK = 16;      // 16-wide K steps between drains (256 K)
 constexpr int STAGES = 5;
-constexpr uint32_t A_PLANE = BM * 32, B_PLANE = BN * 32;   // bytes of a plane in one K step
-constexpr uint32_t A_BYTES = P * A_PLANE, B_BYTES = P * B_PLANE;
-constexpr uint32_t STAGE = A_BYTES + B_BYTES;              // 43,008
-constexpr size_t SMEM = (size_t)STAGES * STAGE + 1024;
+constexpr uint32_t A_PLANE = BM * 32;                      // bytes of a plane in one K step
+constexpr uint32_t A_BYTES = P * A_PLANE;
+__host__ __device__ constexpr uint32_t b_bytes(int bn) { return P * bn * 32; }
+__host__ __device__ constexpr uint32_t stage_bytes(int bn) { return A_BYTES + b_bytes(bn); }   // 43,008 for 64
+constexpr size_t smem_bytes(int bn) { return (size_t)STAGES * stage_bytes(bn) + 1024; }
 constexpr int EPI_WARPS = 16;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
 constexpr int SLOW = 1 << 20;   // exponent of a flagged row
@@ -81,7 +82,7 @@ struct Args {
   const unsigned char *Ad, *Bd;
   const int *ea, *eb;
   int M, N, K;                  // product rows and columns; logical K (for the FP64 chain)
-  int kt, kper, mtiles, ntiles;
+  int kt, kper, mtiles, ntiles, btile;
   int nz, cs;                   // K splits of a tile; cs > 1: added over clusters of cs CTAs
   double* C;
   OzMap cm, cn;
@@ -333,7 +334,12 @@ __device__ __forceinline__ int small_int(float x) {
 // and keeps their two 64-bit sums in registers over the tile's drains.  Every
 // wait is bounded; a CTA whose wait ran out fills the outputs it has not
 // finished with NaN.  The outputs are scaled by 2^(ea + eb - 14): hi 2^-16 + lo 2^-48.
+template <int BN>
 __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
+  constexpr uint32_t B_BYTES = b_bytes(BN), STAGE = stage_bytes(BN);
+  constexpr uint32_t TMEM = BN == 64 ? 512 : 256;   // columns: 7 BN, a power of two
+  constexpr int CB = BN / 4;                        // columns of a draining warp
+  static_assert(P * BN <= (int)TMEM && CB % 4 == 0, "tile width");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
   __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     fence_mbar_init();
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&tmem_slot), 512);
+    tmem_alloc(smem_u32(&tmem_slot), TMEM);
     tmem_relinquish();
   }
   tc_fence_before();
@@ -439,17 +445,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     }
     __syncwarp();
   } else {
-    const int q = warp & 3, cb = ((warp - 2) >> 2) * 16;
+    const int q = warp & 3, cb = ((warp - 2) >> 2) * CB;
     const uint32_t tb = taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
     int use = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
       const int z = t % g.nz, rz = t / g.nz, mt = rz % g.mtiles, nt = rz / g.mtiles;
       const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
-      long long hi[16];                              // sum = hi 2^32 + lo, in 2^-48
-      uint32_t lo[16];
+      long long hi[CB];                              // sum = hi 2^32 + lo, in 2^-48
+      uint32_t lo[CB];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) { hi[c] = 0; lo[c] = 0u; }
+      for (int c = 0; c < CB; ++c) { hi[c] = 0; lo[c] = 0u; }
       for (int kc = k0; kc < k1 && ok; kc += KCHUNK, ++use) {
         ok = __all_sync(0xffffffffu, mbar_wait_f(smem_u32(&acc_full), (uint32_t)(use & 1), fail));
         if (!ok) {
@@ -458,12 +464,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         }
         tc_fence_after();
 #pragma unroll
-        for (int c0 = 0; c0 < 16; c0 += 4) {
+        for (int c0 = 0; c0 < CB; c0 += 4) {
           uint32_t v[P][4];
 #pragma unroll
           for (int p = 0; p < P; ++p) tmem_ld4(tb + (uint32_t)(p * BN + c0), v[p]);
           tmem_ld_wait();
-          if (c0 == 12) {
+          if (c0 == CB - 4) {
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&acc_empty));
@@ -496,17 +502,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         // so the ring holds the sums for the cluster (after a failure fail_s counts)
         longlong2* o = reinterpret_cast<longlong2*>(base) + cb * BM + q * 32 + lane;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) o[c * BM] = make_longlong2(hi[c], (long long)lo[c]);
+        for (int c = 0; c < CB; ++c) o[c * BM] = make_longlong2(hi[c], (long long)lo[c]);
       } else {
         // lane c holds column c's exponent and offset
-        const int nl = n0 + (lane & 15);
+        const int nl = n0 + (lane & (CB - 1));
         const int my_eb = nl < g.N ? g.eb[nl] : 0;
         const i64 my_col = nl < g.N ? c_col(g, nl) : 0;
         const int ea = row < g.M ? g.ea[row] : 0;
         const i64 cr = row < g.M ? c_row(g, row) : 0;
         bool slow = ea == SLOW || !ok;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < CB; ++c) {
           const int eb = __shfl_sync(0xffffffffu, my_eb, c);
           const i64 col = __shfl_sync(0xffffffffu, my_col, c);
           slow = slow || eb == SLOW;
@@ -515,7 +521,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         }
         if (slow && row < g.M) {
 #pragma unroll 1
-          for (int n = n0; n < min(n0 + 16, g.N); ++n) slow_fix(g, cr, row, n, ea, !ok);
+          for (int n = n0; n < min(n0 + CB, g.N); ++n) slow_fix(g, cr, row, n, ea, !ok);
         }
       }
     }
@@ -565,14 +571,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (warp == 1) tmem_dealloc(taddr, 512);
+  if (warp == 1) tmem_dealloc(taddr, TMEM);
 }
 
 // adds the clusters' sums (exact integers) and rounds
 __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
   pdl_wait();
   pdl_trigger();
-  const size_t Mp = (size_t)g.mtiles * BM, Np = (size_t)g.ntiles * BN;
+  const size_t Mp = (size_t)g.mtiles * BM, Np = (size_t)g.ntiles * g.btile;
   const i64 total = (i64)Mp * g.N;
   for (i64 e = blockIdx.x * (i64)blockDim.x + threadIdx.x; e < total; e += (i64)gridDim.x * blockDim.x) {
     const int row = (int)(e % (i64)Mp), n = (int)(e / (i64)Mp);
@@ -597,11 +603,20 @@ constexpr int SMS = 152;
 struct Shape {
   i64 M, N, K;                  // split rows, columns, K
   i64 mt, nt, kt;
+  int bn;
 };
+// 64 columns of B a tile, or 32 where those leave more than half of the SMs
+// idle: half the drain and the rounding per CTA (r=64 chain product 38.5 -> 32.8
+// us, grid interface updates 166 -> 160, time stepper 87.0 -> 85.1 ms, AMEn solve
+// 170 -> 167 ms)
 static Shape shape(i64 M, i64 N, i64 K, bool cplx) {
-  Shape s{cplx ? 2 * M : M, N, cplx ? 2 * K : K, 0, 0, 0};
+  Shape s{cplx ? 2 * M : M, N, cplx ? 2 * K : K, 0, 0, 0, 64};
   s.mt = (s.M + BM - 1) / BM;
-  s.nt = (s.N + BN - 1) / BN;
+  s.nt = (s.N + 63) / 64;
+  if (s.mt * s.nt * 2 <= SMS) {
+    s.bn = 32;
+    s.nt = (s.N + 31) / 32;
+  }
   s.kt = (s.K + 15) / 16;
   return s;
 }
@@ -636,7 +651,9 @@ double oz_us(i64 M, i64 N, i64 K, bool cplx) {
   const int nz = z.nz;
   const double waves = (double)((s.mt * s.nt * nz + oz::SMS - 1) / oz::SMS);
   const double ks = (double)((s.kt + nz - 1) / nz);
-  const double mma = waves * (ks * 950.0 + (ks / oz::KCHUNK + 1) * 2500.0 + 3000.0) / 1900.0;
+  const bool wide = s.bn == 64;
+  const double mma = waves * (ks * (wide ? 950.0 : 800.0) + (ks / oz::KCHUNK + 1) * (wide ? 2500.0 : 1300.0) +
+                              (wide ? 3000.0 : 2000.0)) / 1900.0;
   const double split = ((double)s.M + s.N) * s.K * 22.0 / 4.0e6;
   return mma + split + 12.0 + (nz > z.cs ? 5.0 : (nz > 1 ? 1.5 : 0.0));
 }
@@ -647,7 +664,7 @@ size_t oz_bytes(i64 M, i64 N, i64 K, bool cplx) {
   // rows of both operands padded to the larger tile: either may become A
   const double rows = 128.0 * (double)((s.M + 127) / 128 + (s.N * (cplx ? 2 : 1) + 127) / 128);
   const double need = 14.0 * 16.0 * (double)s.kt * rows + 4.0 * rows +
-                      (double)oz::SMS * oz::BM * oz::BN * 16.0 + 4096.0;
+                      (double)oz::SMS * oz::BM * 64 * 16.0 + 4096.0;
   return need > (double)kOzMaxBytes ? kOzMaxBytes : (size_t)need;
 }
 
@@ -659,10 +676,10 @@ bool oz_fits(i64 M, i64 N, i64 K, bool cplx) {
 void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   using namespace oz;
   const Shape s = shape(g.M, g.N, g.K, g.cplx);
-  TTG_REQUIRE(s.M < (1ll << 31) - BM && s.N < (1ll << 31) - BN && s.K < (1ll << 30), "oz: size");
+  TTG_REQUIRE(s.M < (1ll << 31) - BM && s.N < (1ll << 31) - 64 && s.K < (1ll << 30), "oz: size");
   char* p = (char*)ws;
   auto take = [&](size_t b) { char* r = p; p += al(b); return r; };
-  const size_t ra = (size_t)s.mt * BM, rb = (size_t)s.nt * BN;
+  const size_t ra = (size_t)s.mt * BM, rb = (size_t)s.nt * s.bn;
   unsigned char* Ad = (unsigned char*)take(14 * 16 * (size_t)s.kt * ra);
   unsigned char* Bd = (unsigned char*)take(14 * 16 * (size_t)s.kt * rb);
   int* ea = (int*)take(4 * ra);
@@ -674,7 +691,7 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
     return !g.cplx && sk == 1 && ((uintptr_t)src & 15) == 0 && (m.s1 & 1) == 0 && (m.s2 & 1) == 0;
   };
   const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? 1 : 0, g.conjA};
-  const Side b{g.B, g.bn, g.bk, g.N, BN, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? 2 : 0, g.conjB};
+  const Side b{g.B, g.bn, g.bk, g.N, s.bn, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? 2 : 0, g.conjB};
   const int nA = (int)(ra / (g.cplx ? 2 : 1) / SROWS), nB = (int)(rb / SROWS);
   // few rows and a long K: K over a cluster (246 + 82 rows, K = 4928: 50 -> 17 us)
   int ky = 1;
@@ -684,15 +701,21 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   Args x{};
   x.Ad = Ad; x.Bd = Bd; x.ea = ea; x.eb = eb;
   x.M = (int)s.M; x.N = (int)s.N; x.K = g.K;
-  x.kt = (int)s.kt; x.kper = z.kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.nz = nz; x.cs = z.cs;
+  x.kt = (int)s.kt; x.kper = z.kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.btile = s.bn; x.nz = nz; x.cs = z.cs;
   x.C = g.C; x.cm = g.cm; x.cn = g.cn; x.part = part;
   x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
   x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
-  static const cudaError_t attr_rc =
-      cudaFuncSetAttribute(gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+  static const cudaError_t attr_rc = [] {
+    const cudaError_t r = cudaFuncSetAttribute(gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)smem_bytes(64));
+    return r != cudaSuccess ? r
+                            : cudaFuncSetAttribute(gemm_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   (int)smem_bytes(32));
+  }();
   TTG_CUDA(attr_rc);
   const int grid = (int)std::min<i64>(SMS, s.mt * s.nt * nz);
-  launch_ex(gemm_kernel, dim3(grid), dim3(THREADS), dim3(z.cs > 1 ? z.cs : 0, 1, 1), true, SMEM, st, x);
+  launch_ex(s.bn == 64 ? gemm_kernel<64> : gemm_kernel<32>, dim3(grid), dim3(THREADS),
+            dim3(z.cs > 1 ? z.cs : 0, 1, 1), true, smem_bytes(s.bn), st, x);
   if (groups > 1) {
     const int fb = (int)std::min<i64>(1024, ((i64)ra * s.N + 255) / 256);
     launch_pdl(finish_kernel, dim3(fb), dim3(256), 0, st, x);
