@@ -156,7 +156,7 @@ template <class T> inline size_t grid_words(int n, int m, int clusters, int nb) 
 template <class T, bool GRID>
 __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict__ Ag,
                                                      T* __restrict__ R, T* __restrict__ taug, int G,
-                                                     int lgt, int nb, unsigned long long* part,
+                                                     int CL, int lgt, int nb, unsigned long long* part,
                                                      unsigned int* bar) {
   using O = C<T>;
   namespace cgr = cooperative_groups;
@@ -166,7 +166,6 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int b = blockIdx.x, r = min(n, m);
   cgr::cluster_group cl = cgr::this_cluster();
-  const int CL = GRID ? (int)cl.num_blocks() : G;
   constexpr int W = words::count<T>;
   const int chunk = (n + G - 1) / G, ld = chunk | 1;
   const int nloc = b < n ? (n - b + G - 1) / G : 0;     // rows b, b + G, ...
@@ -186,6 +185,14 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
   unsigned int epoch = 1;
   bool fail = false;
   if (tid < 2) s_fail[tid] = 0;
+  // A grid that did not come as clusters of CL (a profiler that starts a
+  // cooperative launch by itself can lose them) must not go on: the layout of
+  // the words and the shared-memory ranks follow CL
+  if ((int)cl.num_blocks() != CL || (int)gridDim.x != G) {
+    for (int c = warp; c < m; c += NT / 32)
+      for (int i = lane; i < nloc; i += 32) Ag[(i64)n * c + b + (i64)G * i] = O::nan();
+    return;
+  }
 
   for (int c = warp; c < m; c += NT / 32)
     for (int i = lane; i < nloc; i += 32) A[(size_t)ld * c + i] = Ag[(i64)n * c + b + (i64)G * i];
@@ -608,7 +615,7 @@ Pick pick(int n, int m, bool form_q, size_t work) {
     const int G = CL * nc;
     const bool grid = nc > 1;
     if (G > 1 && n < 2 * G) return;
-    if (grid && nc > max_clusters<T>(CL)) return;
+    if (grid && (nc > max_clusters<T>(CL) || G > qr::GMAX)) return;
     // the widest panel that fits
     int nb = form_q ? qr::NB : 0;
     auto fits = [&] {
@@ -656,7 +663,7 @@ bool run(int n, int m, T* A, T* R, T* tau, size_t work, cudaStream_t s) {
     cfg.stream = s;
     cfg.attrs = at;
     cfg.numAttrs = 2;
-    TTG_CUDA(cudaLaunchKernelEx(&cfg, qr::qr_rows_kernel<T, true>, n, m, A, R, tau, G, lgt, nb, part, bar));
+    TTG_CUDA(cudaLaunchKernelEx(&cfg, qr::qr_rows_kernel<T, true>, n, m, A, R, tau, G, p.CL, lgt, nb, part, bar));
     ++g_launches;
     return true;
   }
@@ -664,7 +671,7 @@ bool run(int n, int m, T* A, T* R, T* tau, size_t work, cudaStream_t s) {
       qr::qr_rows_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax);
   TTG_CUDA(rc);
   launch_ex(qr::qr_rows_kernel<T, false>, dim3(p.G), dim3(qr::NT), dim3(p.G, 1, 1), false, smem, s, n,
-            m, A, R, tau, G, lgt, nb, (unsigned long long*)nullptr, (unsigned int*)nullptr);
+            m, A, R, tau, G, G, lgt, nb, (unsigned long long*)nullptr, (unsigned int*)nullptr);
   return true;
 }
 }  // namespace
