@@ -227,3 +227,44 @@ def test_narrow_tiles(torch_cuda, ctx, M, N, K):
     assert launches > 3, "the split product was not taken"
     err = abs(got - X @ P2)
     assert (err <= oz_bound(X, P2) + (K + 4) * U * (abs(X) @ abs(P2))).all()
+
+
+@pytest.mark.parametrize("r1,n,r2,ra,nvec", [(40, 24, 17, 6, 3), (17, 30, 40, 5, 2), (24, 16, 24, 2, 1)])
+def test_complex_doubled_side(torch_cuda, ctx, r1, n, r2, ra, nvec):
+    """Complex products double the rows of the smaller operand: stages with
+    either side the smaller, odd columns, an infinite and a NaN element (their
+    rows and columns take the FP64 chain), against numpy by einsum to 4 K u of
+    the absolute values per stage."""
+    import ttgpu
+    rng = np.random.default_rng(r1 + n)
+
+    def z(*s):
+        return rng.standard_normal(s) + 1j * rng.standard_normal(s)
+    p1, A, p2 = z(r1, r1, ra), z(ra, n, n, ra), z(r2, ra, r2)   # [c,b,a] [a,i,j,e] [b,e,c]
+    x = z(r1, n, r2, nvec)
+    t = [_t(torch_cuda, np.ravel(v, order="F")) for v in (p1, A, p2, x)]
+    y = torch_cuda.zeros(r1 * n * r2 * nvec, dtype=torch_cuda.complex128, device="cuda")
+    ttgpu.zbfun3(r1, n, r2, r1, n, r2, ra, ra, *t, y, nvec)
+    ctx.synchronize()
+    got = y.cpu().numpy().reshape(r1, n, r2, nvec, order="F")
+
+    def product(P1, C, P2, X):
+        T = np.einsum("xjbv,bec->xjecv", X, P2, optimize=True)
+        T = np.einsum("aije,xjecv->xaicv", C, T, optimize=True)
+        return np.einsum("cxa,xaidv->cidv", P1, T, optimize=True)
+    ref = product(p1, A, p2, x)
+    size = product(abs(p1), abs(A), abs(p2), abs(x))
+    K = r2 + n * ra + r1 * ra
+    # the split stages' bound is relative to row and column maxima: each factor's
+    # largest element over its mean square is below 8 at these sizes
+    assert (abs(got - ref) <= 8 * 4 * K * U * size.max()).all()
+    x[1, 2, 3, 0] = np.inf
+    x[0, 1, 2, nvec - 1] = np.nan
+    t[3] = _t(torch_cuda, np.ravel(x, order="F"))
+    ttgpu.zbfun3(r1, n, r2, r1, n, r2, ra, ra, *t, y, nvec)
+    ctx.synchronize()
+    bad = y.cpu().numpy().reshape(r1, n, r2, nvec, order="F")
+    # every output of those vectors sees the element; the others stay finite
+    assert not np.isfinite(bad[..., 0]).any() and not np.isfinite(bad[..., nvec - 1]).any()
+    if nvec > 2:
+        assert np.isfinite(bad[..., 1]).all()

@@ -31,7 +31,7 @@
 // of 8: 4560 -> 241 us (22.7 TFLOP/s of FP64 accuracy; its two products run at
 // 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 32.8
 // us; grid interface updates r = 82, 77, n = 64: 1908 -> 160 us; complex
-// operator and adjoint r=48, n=32, block of 4: 6968 -> 403 us.  What bounds the
+// operator and adjoint r=48, n=32, block of 4: 6968 -> 351 us.  What bounds the
 // product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
 // measured against 900 of MMA), for small ones its fixed ~10 us (pipeline
 // fill, one drain, rounding); oz_us below holds both.
@@ -90,7 +90,7 @@ struct Args {
   const double *A, *B;          // original operands (flagged rows)
   OzMap am, bn;
   i64 ak, bk;
-  int cplx, conjA, conjB;
+  int cplx, conjA, conjB;       // complex: product rows (PAIR: columns) are (re, im)
 };
 
 // 32-bit division: a 64-bit one per stored element took a third of the product
@@ -278,6 +278,7 @@ __device__ __forceinline__ double to_double(long long hi, long long lo, int sc) 
 }
 
 // The FP64 FMA chain of one output (flagged rows): what gemm_kernel forms
+template <bool PAIR>
 __device__ __noinline__ double fma_chain(const Args& g, int row, int n) {
   if (!g.cplx) {
     const double* a = g.A + at(g.am, row);
@@ -286,8 +287,8 @@ __device__ __noinline__ double fma_chain(const Args& g, int row, int n) {
     for (int k = 0; k < g.K; ++k) c = fma(a[(i64)k * g.ak], b[(i64)k * g.bk], c);
     return c;
   }
-  const double2* a = reinterpret_cast<const double2*>(g.A) + at(g.am, row >> 1);
-  const double2* b = reinterpret_cast<const double2*>(g.B) + at(g.bn, n);
+  const double2* a = reinterpret_cast<const double2*>(g.A) + at(g.am, PAIR ? row : row >> 1);
+  const double2* b = reinterpret_cast<const double2*>(g.B) + at(g.bn, PAIR ? n >> 1 : n);
   double cx = 0.0, cy = 0.0;
   for (int k = 0; k < g.K; ++k) {
     double2 x = a[(i64)k * g.ak], y = b[(i64)k * g.bk];
@@ -298,10 +299,12 @@ __device__ __noinline__ double fma_chain(const Args& g, int row, int n) {
     cy = fma(x.x, y.y, cy);
     cy = fma(x.y, y.x, cy);
   }
-  return (row & 1) ? cy : cx;
+  return ((PAIR ? n : row) & 1) ? cy : cx;
 }
 
+template <bool PAIR>
 __device__ __forceinline__ i64 c_row(const Args& g, int row) {
+  if (PAIR) return 2 * at(g.cm, row);
   return g.cplx ? 2 * at(g.cm, row >> 1) + (row & 1) : at(g.cm, row);
 }
 
@@ -311,13 +314,16 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&r)[4]) {
                : "r"(taddr));
 }
 
+template <bool PAIR>
 __device__ __forceinline__ i64 c_col(const Args& g, int n) {
+  if (PAIR) return 2 * at(g.cn, n >> 1) + (n & 1);
   return at(g.cn, n) * (g.cplx ? 2 : 1);
 }
 // an output whose row or column is flagged, or whose sums are not there
+template <bool PAIR>
 __device__ __noinline__ void slow_fix(const Args& g, i64 crow, int row, int n, int ea, bool bad) {
-  if (bad) g.C[crow + c_col(g, n)] = __longlong_as_double(0x7ff8000000000000ll);
-  else if (ea == SLOW || g.eb[n] == SLOW) g.C[crow + c_col(g, n)] = fma_chain(g, row, n);
+  if (bad) g.C[crow + c_col<PAIR>(g, n)] = __longlong_as_double(0x7ff8000000000000ll);
+  else if (ea == SLOW || g.eb[n] == SLOW) g.C[crow + c_col<PAIR>(g, n)] = fma_chain<PAIR>(g, row, n);
 }
 
 constexpr int kMaxSplit = kMaxCluster;            // CTAs of a cluster that share a tile
@@ -334,7 +340,7 @@ __device__ __forceinline__ int small_int(float x) {
 // and keeps their two 64-bit sums in registers over the tile's drains.  Every
 // wait is bounded; a CTA whose wait ran out fills the outputs it has not
 // finished with NaN.  The outputs are scaled by 2^(ea + eb - 14): hi 2^-16 + lo 2^-48.
-template <int BN>
+template <int BN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
   constexpr uint32_t B_BYTES = b_bytes(BN), STAGE = stage_bytes(BN);
   constexpr uint32_t TMEM = BN == 64 ? 512 : 256;   // columns: 7 BN, a power of two
@@ -507,21 +513,35 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         // lane c holds column c's exponent and offset
         const int nl = n0 + (lane & (CB - 1));
         const int my_eb = nl < g.N ? g.eb[nl] : 0;
-        const i64 my_col = nl < g.N ? c_col(g, nl) : 0;
+        const i64 my_col = nl < g.N ? c_col<PAIR>(g, nl) : 0;
         const int ea = row < g.M ? g.ea[row] : 0;
-        const i64 cr = row < g.M ? c_row(g, row) : 0;
+        const i64 cr = row < g.M ? c_row<PAIR>(g, row) : 0;
         bool slow = ea == SLOW || !ok;
+        if constexpr (PAIR) {
+          // columns (re, im) of one output: stored as a pair (N is even)
 #pragma unroll
-        for (int c = 0; c < CB; ++c) {
-          const int eb = __shfl_sync(0xffffffffu, my_eb, c);
-          const i64 col = __shfl_sync(0xffffffffu, my_col, c);
-          slow = slow || eb == SLOW;
-          if (row < g.M && n0 + c < g.N)
-            g.C[cr + col] = to_double(hi[c], (long long)lo[c], ea + eb - 62);
+          for (int c = 0; c < CB; c += 2) {
+            const int eb = __shfl_sync(0xffffffffu, my_eb, c);
+            const i64 col = __shfl_sync(0xffffffffu, my_col, c);
+            slow = slow || eb == SLOW;
+            if (row < g.M && n0 + c < g.N)
+              *reinterpret_cast<double2*>(g.C + cr + col) =
+                  make_double2(to_double(hi[c], (long long)lo[c], ea + eb - 62),
+                               to_double(hi[c + 1], (long long)lo[c + 1], ea + eb - 62));
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < CB; ++c) {
+            const int eb = __shfl_sync(0xffffffffu, my_eb, c);
+            const i64 col = __shfl_sync(0xffffffffu, my_col, c);
+            slow = slow || eb == SLOW;
+            if (row < g.M && n0 + c < g.N)
+              g.C[cr + col] = to_double(hi[c], (long long)lo[c], ea + eb - 62);
+          }
         }
         if (slow && row < g.M) {
 #pragma unroll 1
-          for (int n = n0; n < min(n0 + CB, g.N); ++n) slow_fix(g, cr, row, n, ea, !ok);
+          for (int n = n0; n < min(n0 + CB, g.N); ++n) slow_fix<PAIR>(g, cr, row, n, ea, !ok);
         }
       }
     }
@@ -542,7 +562,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     const longlong2* mine = reinterpret_cast<const longlong2*>(base) + (tid & (BM - 1));
     const bool live = tid < 4 * BM && row < g.M;
     const int ea = live ? g.ea[row] : 0;
-    const i64 cr = live ? c_row(g, row) : 0;
+    const i64 cr = live ? c_row<PAIR>(g, row) : 0;
     for (int c = rank * share + (tid >> 7); c < min(BN, (rank + 1) * share); c += 4) {
       const int n = nt * BN + c;
       if (!live || n >= g.N) break;
@@ -562,8 +582,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
             bad ? make_longlong2(LLONG_MIN, 0) : make_longlong2(hi, lo);
       } else {
         const int eb = g.eb[n];
-        if (bad || ea == SLOW || eb == SLOW) slow_fix(g, cr, row, n, ea, bad);
-        else g.C[cr + c_col(g, n)] = to_double(hi, lo, ea + eb - 62);
+        if (bad || ea == SLOW || eb == SLOW) slow_fix<PAIR>(g, cr, row, n, ea, bad);
+        else g.C[cr + c_col<PAIR>(g, n)] = to_double(hi, lo, ea + eb - 62);
       }
     }
     cl.sync();   // no CTA leaves while another reads its sums
@@ -575,6 +595,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
 }
 
 // adds the clusters' sums (exact integers) and rounds
+template <bool PAIR>
 __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
   pdl_wait();
   pdl_trigger();
@@ -591,10 +612,10 @@ __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
       hi += v.x;
       lo += v.y;
     }
-    const i64 cr = c_row(g, row);
+    const i64 cr = c_row<PAIR>(g, row);
     const int ea = g.ea[row], eb = g.eb[n];
-    if (bad || ea == SLOW || eb == SLOW) slow_fix(g, cr, row, n, ea, bad);
-    else g.C[cr + c_col(g, n)] = to_double(hi, lo, ea + eb - 62);
+    if (bad || ea == SLOW || eb == SLOW) slow_fix<PAIR>(g, cr, row, n, ea, bad);
+    else g.C[cr + c_col<PAIR>(g, n)] = to_double(hi, lo, ea + eb - 62);
   }
 }
 
@@ -604,13 +625,14 @@ struct Shape {
   i64 M, N, K;                  // split rows, columns, K
   i64 mt, nt, kt;
   int bn;
+  bool dup_b;                   // complex: B's columns doubled, not A's rows
 };
 // 64 columns of B a tile, or 32 where those leave more than half of the SMs
 // idle: half the drain and the rounding per CTA (r=64 chain product 38.5 -> 32.8
 // us, grid interface updates 166 -> 160, time stepper 87.0 -> 85.1 ms, AMEn solve
 // 170 -> 167 ms)
-static Shape shape(i64 M, i64 N, i64 K, bool cplx) {
-  Shape s{cplx ? 2 * M : M, N, cplx ? 2 * K : K, 0, 0, 0, 64};
+static Shape shape_of(i64 M, i64 N, i64 K, bool cplx, bool dup_b) {
+  Shape s{cplx && !dup_b ? 2 * M : M, cplx && dup_b ? 2 * N : N, cplx ? 2 * K : K, 0, 0, 0, 64, dup_b};
   s.mt = (s.M + BM - 1) / BM;
   s.nt = (s.N + 63) / 64;
   if (s.mt * s.nt * 2 <= SMS) {
@@ -620,13 +642,25 @@ static Shape shape(i64 M, i64 N, i64 K, bool cplx) {
   s.kt = (s.K + 15) / 16;
   return s;
 }
+// A complex product is a real one with the rows of one operand doubled to (re,
+// -im) and (im, re): the smaller operand, whose digits are then written twice,
+// unless the tiles get more padding by it (complex
+// operator and adjoint r=48, n=32, block of 4: 403 -> 351 us, the digits of its
+// intermediates 38 -> 20 us)
+static Shape shape(i64 M, i64 N, i64 K, bool cplx) {
+  const Shape a = shape_of(M, N, K, cplx, false);
+  if (!cplx || N >= M) return a;
+  const Shape b = shape_of(M, N, K, true, true);
+  const double area_a = (double)a.mt * a.nt * a.bn, area_b = (double)b.mt * b.nt * b.bn;
+  return area_b <= 1.05 * area_a ? b : a;
+}
 // K split: only where the tiles leave SMs idle; at least KMIN K steps per chunk
 // (a last chunk may be empty).  Up to eight chunks are one cluster where the
 // GPU holds all of them (it holds 14 clusters of eight of these CTAs, 36 of
 // four), more are clusters of four whose sums a second kernel adds.  Measured,
 // at least 8 steps and a second kernel for every split -> this: r=64 chain
 // product 40.1 -> 38.3 us, time stepper (d=16, n=32, r=8) 92.1 -> 88.4 ms,
-// operator and adjoint r=48 407 -> 403 us, K = 5248 in 36 chunks unchanged
+// operator and adjoint r=48 407 -> 403 us (351 since), K = 5248 in 36 chunks unchanged
 // (clusters of eight there: 167 -> 171 us; at least 2 steps: 88.4 -> 92 ms).
 constexpr int KMIN = 4;
 struct Split { int nz, cs, kper; };
@@ -660,10 +694,11 @@ double oz_us(i64 M, i64 N, i64 K, bool cplx) {
 
 size_t oz_bytes(i64 M, i64 N, i64 K, bool cplx) {
   if ((cplx ? 4.0 : 1.0) * (double)M * (double)N * (double)K < kOzMinMNK) return 0;
-  const oz::Shape s = oz::shape(M, N, K, cplx);
-  // rows of both operands padded to the larger tile: either may become A
-  const double rows = 128.0 * (double)((s.M + 127) / 128 + (s.N * (cplx ? 2 : 1) + 127) / 128);
-  const double need = 14.0 * 16.0 * (double)s.kt * rows + 4.0 * rows +
+  // rows of both operands padded to the larger tile, doubled if complex: either
+  // may become A and either may be the doubled one
+  const i64 f = cplx ? 2 : 1, kt = (f * K + 15) / 16;
+  const double rows = 128.0 * (double)((f * M + 127) / 128 + (f * N + 127) / 128);
+  const double need = 14.0 * 16.0 * (double)kt * rows + 4.0 * rows +
                       (double)oz::SMS * oz::BM * 64 * 16.0 + 4096.0;
   return need > (double)kOzMaxBytes ? kOzMaxBytes : (size_t)need;
 }
@@ -690,9 +725,9 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   auto vec = [&](const double* src, const OzMap& m, i64 sk) {
     return !g.cplx && sk == 1 && ((uintptr_t)src & 15) == 0 && (m.s1 & 1) == 0 && (m.s2 & 1) == 0;
   };
-  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? 1 : 0, g.conjA};
-  const Side b{g.B, g.bn, g.bk, g.N, s.bn, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? 2 : 0, g.conjB};
-  const int nA = (int)(ra / (g.cplx ? 2 : 1) / SROWS), nB = (int)(rb / SROWS);
+  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? (s.dup_b ? 2 : 1) : 0, g.conjA};
+  const Side b{g.B, g.bn, g.bk, g.N, s.bn, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? (s.dup_b ? 1 : 2) : 0, g.conjB};
+  const int nA = (int)(ra / (a.cplx == 1 ? 2 : 1) / SROWS), nB = (int)(rb / (b.cplx == 1 ? 2 : 1) / SROWS);
   // few rows and a long K: K over a cluster (246 + 82 rows, K = 4928: 50 -> 17 us)
   int ky = 1;
   while (ky < kMaxCluster && (nA + nB) * ky < 2 * SMS && 2 * s.kt > 32 * ky) ky *= 2;
@@ -706,19 +741,26 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
   x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
   static const cudaError_t attr_rc = [] {
-    const cudaError_t r = cudaFuncSetAttribute(gemm_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem_bytes(64));
-    return r != cudaSuccess ? r
-                            : cudaFuncSetAttribute(gemm_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)smem_bytes(32));
+    cudaError_t r = cudaSuccess;
+    auto set = [&](auto* k, int bn) {
+      if (r == cudaSuccess)
+        r = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(bn));
+    };
+    set(gemm_kernel<64, false>, 64);
+    set(gemm_kernel<64, true>, 64);
+    set(gemm_kernel<32, false>, 32);
+    set(gemm_kernel<32, true>, 32);
+    return r;
   }();
   TTG_CUDA(attr_rc);
   const int grid = (int)std::min<i64>(SMS, s.mt * s.nt * nz);
-  launch_ex(s.bn == 64 ? gemm_kernel<64> : gemm_kernel<32>, dim3(grid), dim3(THREADS),
+  auto kern = s.bn == 64 ? (s.dup_b ? gemm_kernel<64, true> : gemm_kernel<64, false>)
+                         : (s.dup_b ? gemm_kernel<32, true> : gemm_kernel<32, false>);
+  launch_ex(kern, dim3(grid), dim3(THREADS),
             dim3(z.cs > 1 ? z.cs : 0, 1, 1), true, smem_bytes(s.bn), st, x);
   if (groups > 1) {
     const int fb = (int)std::min<i64>(1024, ((i64)ra * s.N + 255) / 256);
-    launch_pdl(finish_kernel, dim3(fb), dim3(256), 0, st, x);
+    launch_pdl(s.dup_b ? finish_kernel<true> : finish_kernel<false>, dim3(fb), dim3(256), 0, st, x);
   }
 }
 
