@@ -266,10 +266,11 @@ void launch_tile(const Args<T>& a, int nbatch, cudaStream_t s) {
 // Measured on GB300 before (128 x 16, 16 x 128, 32 x 32 and 64 x 64 tiles
 // picked by N <= 16, M <= 16 and the tile count) and after:
 //   r=16 chain product, block of 4 (M, N, K of 10..80)       65.6 -> 9.2 us
+//   two steps of the complex time stepper (d=16, n=32, r=8)   213 -> 124 ms
+// and of products that the exact-split kernels have taken since
 //   r=64 chain product, block of 5                          104.4 -> 76.6 us
 //   grid interface updates, r = 82, 77, n = 64               2745 -> 1908 us
 //   complex operator and adjoint, r = 48, n = 32, block of 4 9284 -> 6968 us
-//   two steps of the complex time stepper (d=16, n=32, r=8)   213 -> 124 ms
 struct TilePick {
   int tile, splitk, kchunk;
   double clocks;

@@ -15,7 +15,7 @@
 // are enough to apply them one after the other (w_k = tau_k (v_k^H q - sum_{l>k}
 // v_k^H v_l w_l), q -= sum_k v_k w_k).  One reflector per exchange took as
 // long as the factorisation: 1240 us in all for 5248 x 86, 407 for 844 x 41,
-// 329 for 128 x 64; now 830, 246, 282, three quarters of it the factorisation.
+// 329 for 128 x 64; now 840, 246, 282, three quarters of it the factorisation.
 //
 //   cluster form  G <= 8 CTAs of one cluster exchange through distributed
 //                 shared memory, one cluster barrier per column (2.2k clocks,
