@@ -15,7 +15,7 @@
 // are enough to apply them one after the other (w_k = tau_k (v_k^H q - sum_{l>k}
 // v_k^H v_l w_l), q -= sum_k v_k w_k).  One reflector per exchange took as
 // long as the factorisation: 1240 us in all for 5248 x 86, 407 for 844 x 41,
-// 329 for 128 x 64; now 840, 246, 282, three quarters of it the factorisation.
+// 329 for 128 x 64; now 835, 246, 272, three quarters of it the factorisation.
 //
 //   cluster form  G <= 8 CTAs of one cluster exchange through distributed
 //                 shared memory, one cluster barrier per column (2.2k clocks,
@@ -303,10 +303,14 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
         if (with_row) row[j] = cl.map_shared_rank(mine_row, owner)[(size_t)par * m + j];
       }
     }
-    if (GRID && with_row && warp == 1) {
-      // the two quotients on two partitions of the SM (the barrier above was for all)
+    if (with_row && warp == NT / 32 - 1) {
+      // the quotients on two partitions of the SM (in the cluster form this warp,
+      // seldom with a column of its own, adds column j0 once more: 128 x 64 284 ->
+      // 272 us)
       T be, ta, sc;
-      O::reflect(row[j0], O::sq(Sx[j0]), be, ta, sc);
+      if (GRID) O::reflect(row[j0], O::sq(Sx[j0]), be, ta, sc);
+      else O::reflect(cl.map_shared_rank(mine_row, owner)[(size_t)par * m + j0],
+                      O::sq(cluster_sum(j0 + (size_t)par * m)), be, ta, sc);
       if (lane == 0) s_sc = sc;
     }
     if (with_row && warp == 0) {
@@ -316,7 +320,6 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
       if (lane == 0) {
         s_beta = be;
         s_tau = ta;
-        if (!GRID) s_sc = sc;
         tau[j0] = ta;
       }
     }
@@ -566,7 +569,7 @@ constexpr size_t kSmemMax = 220 * 1024;
 // 3.0, nc clusters 4.2 + 0.12 nc).  Measured on GB300 over G (us; one CTA of
 // the former kernel, then G = 8, 32, 64, 112; clusters of 4 took 875 us at
 // G = 128 for the 5248 x 86 block, 2280 for 512 x 256):
-//    128 x  64     895 |  282   288   334     -
+//    128 x  64     895 |  272   288   334     -
 //    320 x 128    4400 |  890   671   746   824
 //    512 x 256   22407 | 3392  1856  1732  1846
 //   1968 x  82    8776 | 2011   753   620   619
