@@ -24,8 +24,9 @@
 // (tests/test_oz_gpu.py).
 //
 // A row whose elements are not all finite, or whose largest element lies
-// outside 2^(+-400), is flagged and its outputs are formed by the plain FP64
-// FMA chain, so infinities, NaN and extreme ranges give what they give there.
+// outside 2^(+-400), is flagged, and the tiles that it meets are formed by the
+// plain FP64 FMA chain, so infinities, NaN and extreme ranges give what they
+// give there.
 //
 // Measured on GB300, FP64 kernels -> split products: chain product r=256, block
 // of 8: 4560 -> 241 us (22.7 TFLOP/s of FP64 accuracy; its two products run at
@@ -45,6 +46,7 @@
 #include "ttg_tcgen05.cuh"
 #include <algorithm>
 #include <climits>
+#include <type_traits>
 
 namespace ttg {
 namespace oz {
@@ -277,31 +279,6 @@ __device__ __forceinline__ double to_double(long long hi, long long lo, int sc) 
   return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
-// The FP64 FMA chain of one output (flagged rows): what gemm_kernel forms
-template <bool PAIR>
-__device__ __noinline__ double fma_chain(const Args& g, int row, int n) {
-  if (!g.cplx) {
-    const double* a = g.A + at(g.am, row);
-    const double* b = g.B + at(g.bn, n);
-    double c = 0.0;
-    for (int k = 0; k < g.K; ++k) c = fma(a[(i64)k * g.ak], b[(i64)k * g.bk], c);
-    return c;
-  }
-  const double2* a = reinterpret_cast<const double2*>(g.A) + at(g.am, PAIR ? row : row >> 1);
-  const double2* b = reinterpret_cast<const double2*>(g.B) + at(g.bn, PAIR ? n >> 1 : n);
-  double cx = 0.0, cy = 0.0;
-  for (int k = 0; k < g.K; ++k) {
-    double2 x = a[(i64)k * g.ak], y = b[(i64)k * g.bk];
-    if (g.conjA) x.y = -x.y;
-    if (g.conjB) y.y = -y.y;
-    cx = fma(x.x, y.x, cx);
-    cx = fma(-x.y, y.y, cx);
-    cy = fma(x.x, y.y, cy);
-    cy = fma(x.y, y.x, cy);
-  }
-  return ((PAIR ? n : row) & 1) ? cy : cx;
-}
-
 template <bool PAIR>
 __device__ __forceinline__ i64 c_row(const Args& g, int row) {
   if (PAIR) return 2 * at(g.cm, row);
@@ -319,11 +296,150 @@ __device__ __forceinline__ i64 c_col(const Args& g, int n) {
   if (PAIR) return 2 * at(g.cn, n >> 1) + (n & 1);
   return at(g.cn, n) * (g.cplx ? 2 : 1);
 }
-// an output whose row or column is flagged, or whose sums are not there
-template <bool PAIR>
-__device__ __noinline__ void slow_fix(const Args& g, i64 crow, int row, int n, int ea, bool bad) {
-  if (bad) g.C[crow + c_col<PAIR>(g, n)] = __longlong_as_double(0x7ff8000000000000ll);
-  else if (ea == SLOW || g.eb[n] == SLOW) g.C[crow + c_col<PAIR>(g, n)] = fma_chain<PAIR>(g, row, n);
+
+// whether any draining thread says so (all of them call it)
+__device__ __forceinline__ bool epi_or(bool v) {
+  uint32_t r;
+  asm volatile(
+      "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n barrier.cta.red.or.pred p, 1, %2, q;\n"
+      " selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(r)
+      : "r"((uint32_t)v), "n"(32 * EPI_WARPS)
+      : "memory");
+  return r != 0;
+}
+
+// FP64 FMA chains of a unit, 32 rows x BN / 4 columns (a sixteenth of a tile),
+// over logical K [kbeg, kend): the 16 draining warps take every 16th k, a lane
+// rows ly + 4 i and columns lx + 8 j, and the warps' sums are added in order from
+// red.  To C, or (over clusters) to o, the sums' place in shared memory.  Bound
+// by the FP64 pipe, as gemm_kernel of ttg_gemm.cu is: a load serves two to eight
+// FMAs of 64 clocks each.  Units this small, and K over the warps, because a
+// product of 80 tiles would leave half of the SMs idle if each kept its own
+// (phi_left, r = 256, n = 2, an infinity in Phi: 1124 us so, 720 in units).  One
+// thread per flagged output took 1472 us there and 2436 us at r = 82, n = 64 (now
+// 1162); the FP64 kernels take 777 and 1426.
+template <int BN, bool PAIR, bool CPLX>
+__device__ __noinline__ void fp64_unit(const Args& g, int rt, int ct, int kbeg, int kend, bool fail,
+                                       double* red, longlong2* o) {
+  constexpr int NI = 8, NJ = BN / 32, E = 32 * NI * NJ;
+  using T = typename std::conditional<CPLX, double2, double>::type;
+  const int e = threadIdx.x - 64, warp = e >> 5, lane = e & 31, ly = lane >> 3, lx = lane & 7;
+  const int r0 = rt * 32, c0 = ct * (BN / 4);
+  if (r0 >= g.M || c0 >= g.N) return;
+  const T *a[NI], *b[NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i) {
+    const int r = min(r0 + ly + 4 * i, g.M - 1);
+    a[i] = reinterpret_cast<const T*>(g.A) + at(g.am, CPLX && !PAIR ? r >> 1 : r) + (i64)(kbeg + warp) * g.ak;
+  }
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    const int n = min(c0 + lx + 8 * j, g.N - 1);
+    b[j] = reinterpret_cast<const T*>(g.B) + at(g.bn, CPLX && PAIR ? n >> 1 : n) + (i64)(kbeg + warp) * g.bk;
+  }
+  double acc[NI][NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) acc[i][j] = 0.0;
+  const bool im = ((PAIR ? lx : ly) & 1) != 0;       // the imaginary part's row or column
+  T x[NI], y[NJ];
+  auto load = [&] {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      x[i] = *a[i];
+      a[i] += EPI_WARPS * g.ak;
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      y[j] = *b[j];
+      b[j] += EPI_WARPS * g.bk;
+    }
+  };
+  constexpr bool AHEAD = !CPLX;                      // (complex: four times the FMAs per load)
+  if (AHEAD && kbeg + warp < kend) load();
+  for (int k = kbeg + warp; k < kend; k += EPI_WARPS) {
+    if (!AHEAD) load();
+    T u[NI], v[NJ];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) u[i] = x[i];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) v[j] = y[j];
+    if (AHEAD && k + EPI_WARPS < kend) load();
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        if constexpr (CPLX) {
+          const double ui = g.conjA ? -u[i].y : u[i].y, vi = g.conjB ? -v[j].y : v[j].y;
+          acc[i][j] = fma(u[i].x, im ? vi : v[j].x, acc[i][j]);
+          acc[i][j] = fma(ui, im ? v[j].x : -vi, acc[i][j]);
+        } else {
+          acc[i][j] = fma(u[i], v[j], acc[i][j]);
+        }
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) red[warp * E + (i * NJ + j) * 32 + lane] = acc[i][j];
+  epi_or(false);
+  if (e < E) {
+    double v = red[e];
+    for (int w = 1; w < EPI_WARPS; ++w) v += red[w * E + e];
+    if (fail) v = __longlong_as_double(0x7ff8000000000000ll);
+    const int r = r0 + ly + 4 * ((e >> 5) / NJ), n = c0 + lx + 8 * ((e >> 5) % NJ);
+    if (o) o[(n & (BN - 1)) * BM + (r & (BM - 1))] = make_longlong2(__double_as_longlong(v), 0);
+    else if (r < g.M && n < g.N) g.C[c_row<PAIR>(g, r) + c_col<PAIR>(g, n)] = v;
+  }
+}
+
+// whether draining thread e sees a flagged row or column of tile (mt, nt)
+template <int BN>
+__device__ __forceinline__ bool flagged(const Args& g, int mt, int nt, int e) {
+  const int r = mt * BM + e, n = nt * BN + e;
+  return (e < BM && r < g.M && g.ea[r] == SLOW) || (e < BN && n < g.N && g.eb[n] == SLOW);
+}
+// A CTA's units, should their tiles be left to fp64_unit: without a K split an
+// even share of all, else its own tile's for its K.  units_flagged: whether a
+// draining thread sees a flag in them; run_units: forms those that have one.
+struct Units { int u0, u1; };
+__device__ __forceinline__ Units my_units(const Args& g) {
+  const i64 n = (i64)g.mtiles * g.ntiles * 16;
+  return {(int)(n * blockIdx.x / gridDim.x), (int)(n * (blockIdx.x + 1) / gridDim.x)};
+}
+template <int BN>
+__device__ __noinline__ bool units_flagged(const Args& g) {
+  const Units w = my_units(g);
+  bool any = false;
+  for (int v = w.u0 / 16; v * 16 < w.u1; ++v)
+    any = any || flagged<BN>(g, v % g.mtiles, v / g.mtiles, threadIdx.x - 64);
+  return any;
+}
+template <int BN, bool PAIR>
+__device__ __noinline__ void run_units(const Args& g, unsigned char* base, bool fail) {
+  const bool split = g.cs > 1;
+  const int z = split ? (int)blockIdx.x % g.nz : 0, own = (int)blockIdx.x / g.nz;
+  const int per = g.cplx ? 8 : 16, k0 = z * g.kper * per, k1 = min(g.K, k0 + g.kper * per);
+  longlong2* o = split ? reinterpret_cast<longlong2*>(base) : nullptr;
+  constexpr int E = EPI_WARPS * 8 * BN;
+  // the warps' sums of a unit: two areas in turn, so that one barrier a unit is enough
+  double* red = reinterpret_cast<double*>(base + (split ? sizeof(longlong2) * BM * BN : 0));
+  static_assert(sizeof(longlong2) * BM * BN + sizeof(double) * E <= STAGES * stage_bytes(BN) &&
+                    2 * sizeof(double) * E <= STAGES * stage_bytes(BN),
+                "the ring holds them");
+  const Units w = split ? Units{16 * own, 16 * own + 16} : my_units(g);
+  bool tile_flag = false;
+  for (int u = w.u0; u < w.u1; ++u) {
+    const int mt = u / 16 % g.mtiles, nt = u / 16 / g.mtiles;
+    if (u == w.u0 || u % 16 == 0) tile_flag = epi_or(flagged<BN>(g, mt, nt, threadIdx.x - 64));
+    if (!tile_flag) continue;
+    const int rt = mt * 4 + (u & 3), ct = nt * 4 + (u >> 2 & 3);
+    if (g.cplx) fp64_unit<BN, PAIR, true>(g, rt, ct, k0, k1, fail, red + (split ? 0 : (u & 1) * E), o);
+    else if constexpr (!PAIR) fp64_unit<BN, false, false>(g, rt, ct, k0, k1, fail, red + (split ? 0 : (u & 1) * E), o);
+    if (split) epi_or(false);                        // beside the cluster's sums there is one area
+  }
 }
 
 constexpr int kMaxSplit = kMaxCluster;            // CTAs of a cluster that share a tile
@@ -340,8 +456,10 @@ __device__ __forceinline__ int small_int(float x) {
 // and keeps their two 64-bit sums in registers over the tile's drains.  Every
 // wait is bounded; a CTA whose wait ran out fills the outputs it has not
 // finished with NaN.  The outputs are scaled by 2^(ea + eb - 14): hi 2^-16 + lo 2^-48.
+// Tiles with a flagged row or column are left to fp64_unit, after the others and
+// dealt out over all CTAs.
 template <int BN, bool PAIR>
-__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
+__global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ Args g) {
   constexpr uint32_t B_BYTES = b_bytes(BN), STAGE = stage_bytes(BN);
   constexpr uint32_t TMEM = BN == 64 ? 512 : 256;   // columns: 7 BN, a power of two
   constexpr int CB = BN / 4;                        // columns of a draining warp
@@ -350,7 +468,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
   __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int fail_s;
+  __shared__ int fail_s, fix_s;                     // a wait ran out; there are units for fp64_unit
   volatile int* fail = &fail_s;
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -363,7 +481,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     mbar_init(smem_u32(&acc_full), 1);
     mbar_init(smem_u32(&acc_empty), EPI_WARPS);
     mbar_init(smem_u32(&done_bar), 1);
-    fail_s = 0;
+    fail_s = fix_s = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -455,9 +573,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
     const uint32_t tb = taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
     int use = 0;
     bool ok = true;
+    if (g.cs == 1 && units_flagged<BN>(g)) fix_s = 1;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
       const int z = t % g.nz, rz = t / g.nz, mt = rz % g.mtiles, nt = rz / g.mtiles;
       const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
+      const bool fix = epi_or(flagged<BN>(g, mt, nt, tid - 64));
+      if (fix && g.cs > 1) fix_s = 1;
       long long hi[CB];                              // sum = hi 2^32 + lo, in 2^-48
       uint32_t lo[CB];
 #pragma unroll
@@ -503,6 +624,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         }
       }
       const int row = mt * BM + q * 32 + lane, n0 = nt * BN + cb;
+      if (fix) continue;
       if (g.cs > 1) {
         // the CTA's only tile: every copy has landed and every MMA has read it,
         // so the ring holds the sums for the cluster (after a failure fail_s counts)
@@ -516,14 +638,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
         const i64 my_col = nl < g.N ? c_col<PAIR>(g, nl) : 0;
         const int ea = row < g.M ? g.ea[row] : 0;
         const i64 cr = row < g.M ? c_row<PAIR>(g, row) : 0;
-        bool slow = ea == SLOW || !ok;
         if constexpr (PAIR) {
           // columns (re, im) of one output: stored as a pair (N is even)
 #pragma unroll
           for (int c = 0; c < CB; c += 2) {
             const int eb = __shfl_sync(0xffffffffu, my_eb, c);
             const i64 col = __shfl_sync(0xffffffffu, my_col, c);
-            slow = slow || eb == SLOW;
             if (row < g.M && n0 + c < g.N)
               *reinterpret_cast<double2*>(g.C + cr + col) =
                   make_double2(to_double(hi[c], (long long)lo[c], ea + eb - 62),
@@ -534,27 +654,31 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
           for (int c = 0; c < CB; ++c) {
             const int eb = __shfl_sync(0xffffffffu, my_eb, c);
             const i64 col = __shfl_sync(0xffffffffu, my_col, c);
-            slow = slow || eb == SLOW;
             if (row < g.M && n0 + c < g.N)
               g.C[cr + col] = to_double(hi[c], (long long)lo[c], ea + eb - 62);
           }
         }
-        if (slow && row < g.M) {
+        if (!ok && row < g.M) {
 #pragma unroll 1
-          for (int n = n0; n < min(n0 + CB, g.N); ++n) slow_fix<PAIR>(g, cr, row, n, ea, !ok);
+          for (int n = n0; n < min(n0 + CB, g.N); ++n)
+            g.C[cr + c_col<PAIR>(g, n)] = __longlong_as_double(0x7ff8000000000000ll);
         }
       }
     }
   }
   pdl_trigger();
+  __syncthreads();                                   // fix_s; the ring is free
+  const bool fix = fix_s != 0, failed = fail_s != 0;
+  if (fix && warp >= 2) run_units<BN, PAIR>(g, base, failed);
   if (g.cs > 1) {
     // one tile per CTA; CTA `rank` adds its share of the columns over the
-    // cluster (exact integers) and rounds, or leaves the cluster's sum
+    // cluster (exact integers, or the FP64 chains') and rounds, or leaves the
+    // cluster's sum
     namespace cgr = cooperative_groups;
     cgr::cluster_group cl = cgr::this_cluster();
-    cl.sync();
     const int z = (int)blockIdx.x % g.nz, rz = (int)blockIdx.x / g.nz;
     const int mt = rz % g.mtiles, nt = rz / g.mtiles, rank = (int)cl.block_rank();
+    cl.sync();
     const int share = (BN + g.cs - 1) / g.cs;
     bool bad = false;
     for (int p = 0; p < g.cs; ++p) bad = bad || *cl.map_shared_rank(&fail_s, p) != 0;
@@ -571,20 +695,27 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const Args g) {
       for (int p = 0; p < kMaxSplit; ++p)
         v[p] = p < g.cs ? *cl.map_shared_rank(mine + c * BM, p) : make_longlong2(0, 0);
       long long hi = v[0].x, lo = v[0].y;
+      if (fix || bad) {
+        double sum = __longlong_as_double(hi);
 #pragma unroll
-      for (int p = 1; p < kMaxSplit; ++p) {
-        hi += v[p].x;
-        lo += v[p].y;
-      }
-      if (g.nz > g.cs) {
-        // a failed cluster's sums carry a mark the finishing kernel turns into NaN
-        g.part[((size_t)(z / g.cs) * g.ntiles * BN + n) * ((size_t)g.mtiles * BM) + row] =
-            bad ? make_longlong2(LLONG_MIN, 0) : make_longlong2(hi, lo);
+        for (int p = 1; p < kMaxSplit; ++p)
+          if (p < g.cs) sum += __longlong_as_double(v[p].x);
+        if (bad) sum = __longlong_as_double(0x7ff8000000000000ll);
+        hi = __double_as_longlong(sum);
+        lo = LLONG_MIN;                              // marks an FP64 value
       } else {
-        const int eb = g.eb[n];
-        if (bad || ea == SLOW || eb == SLOW) slow_fix<PAIR>(g, cr, row, n, ea, bad);
-        else g.C[cr + c_col<PAIR>(g, n)] = to_double(hi, lo, ea + eb - 62);
+#pragma unroll
+        for (int p = 1; p < kMaxSplit; ++p) {
+          hi += v[p].x;
+          lo += v[p].y;
+        }
       }
+      if (g.nz > g.cs)
+        g.part[((size_t)(z / g.cs) * g.ntiles * BN + n) * ((size_t)g.mtiles * BM) + row] =
+            make_longlong2(hi, lo);
+      else
+        g.C[cr + c_col<PAIR>(g, n)] =
+            lo == LLONG_MIN ? __longlong_as_double(hi) : to_double(hi, lo, ea + g.eb[n] - 62);
     }
     cl.sync();   // no CTA leaves while another reads its sums
   }
@@ -604,18 +735,23 @@ __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
   for (i64 e = blockIdx.x * (i64)blockDim.x + threadIdx.x; e < total; e += (i64)gridDim.x * blockDim.x) {
     const int row = (int)(e % (i64)Mp), n = (int)(e / (i64)Mp);
     if (row >= g.M) continue;
+    // FP64 values (marked) where the tile was left to the FMA chains, and then
+    // in every cluster; beside a failed cluster's NaN the integers do not count
     long long hi = 0, lo = 0;
-    bool bad = false;
+    double sum = 0.0;
+    bool chain = false;
     for (int z = 0; z < g.nz / g.cs; ++z) {
       const longlong2 v = g.part[((size_t)z * Np + n) * Mp + row];
-      bad = bad || v.x == LLONG_MIN;
-      hi += v.x;
-      lo += v.y;
+      if (v.y == LLONG_MIN) {
+        chain = true;
+        sum += __longlong_as_double(v.x);
+      } else {
+        hi += v.x;
+        lo += v.y;
+      }
     }
-    const i64 cr = c_row<PAIR>(g, row);
-    const int ea = g.ea[row], eb = g.eb[n];
-    if (bad || ea == SLOW || eb == SLOW) slow_fix<PAIR>(g, cr, row, n, ea, bad);
-    else g.C[cr + c_col<PAIR>(g, n)] = to_double(hi, lo, ea + eb - 62);
+    g.C[c_row<PAIR>(g, row) + c_col<PAIR>(g, n)] =
+        chain ? sum : to_double(hi, lo, g.ea[row] + g.eb[n] - 62);
   }
 }
 
@@ -753,7 +889,8 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
     return r;
   }();
   TTG_CUDA(attr_rc);
-  const int grid = (int)std::min<i64>(SMS, s.mt * s.nt * nz);
+  // (without a K split every SM gets a CTA: units for fp64_unit are dealt out to all)
+  const int grid = z.cs > 1 ? (int)(s.mt * s.nt * nz) : SMS;
   auto kern = s.bn == 64 ? (s.dup_b ? gemm_kernel<64, true> : gemm_kernel<64, false>)
                          : (s.dup_b ? gemm_kernel<32, true> : gemm_kernel<32, false>);
   launch_ex(kern, dim3(grid), dim3(THREADS),
