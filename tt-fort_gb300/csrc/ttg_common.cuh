@@ -301,16 +301,46 @@ struct OzGemm {
   const double* B = nullptr; OzMap bn{1, 0, 0}; i64 bk = 0;
   double* C = nullptr;       OzMap cm{1, 0, 0}, cn{1, 0, 0};
   bool cplx = false, conjA = false, conjB = false;
+  // row r of A (B) belongs to group r / gd % gn: the outputs of a pair of groups
+  // get the accuracy of their own largest
+  int gdA = 1, gnA = 1, gdB = 1, gnB = 1;
+  // scales along K by an interface's operator rank blocks: k is of block k / kd %
+  // kr, whose elements lie at phi[(o kr + block) inner + i]; A's elements are
+  // divided by the block's power of two and B's multiplied (norm = 1), or the
+  // reverse (-1).  kr = 0: none
+  const double* phi = nullptr;
+  i64 inner = 0, outer = 0;
+  int kd = 1, kr = 0, norm = 0;
+  void* stat = nullptr;        // oz_stat_bytes of them
 };
+// What a strided product is in a chain of them: the operator rank on one side's
+// rows (side 1: A, 2: B; runs of `run` rows of one block, or 0: block by block
+// interleaved), the scales along K as above, the vectors joined by its batch
+struct OzHint {
+  int side = 0, groups = 1, run = 0;
+  const double* phi = nullptr;
+  i64 inner = 0, outer = 0;
+  int kd = 1, kr = 0, norm = 0;
+  int nvec = 1;
+};
+constexpr int kOzProducts = 3;                   // products of a call
+constexpr int kOzMaxGroups = 256;               // of a side; more: FP64
+constexpr int kOzMaxVec = 64;                    // more vectors: one group
+constexpr int kOzMaxTable = 4096;                // more operator rank blocks: no scales
 constexpr double kOzMinMNK = 2.0e6;              // below: never split
 constexpr size_t kOzMaxBytes = (size_t)4 << 30;  // workspace limit: larger products stay FP64
 size_t oz_bytes(i64 M, i64 N, i64 K, bool cplx); // workspace, non-decreasing in every size
 bool oz_fits(i64 M, i64 N, i64 K, bool cplx);    // within both limits
 double oz_us(i64 M, i64 N, i64 K, bool cplx);    // estimated time
-void oz_gemm(const OzGemm& g, void* ws, cudaStream_t s);
-// runs g as a split product when it has the form for it and that is faster
-bool oz_try(const GemmF64& g, void* ws, cudaStream_t s);
-bool oz_try(const GemmZ& g, void* ws, cudaStream_t s);
+// of OzGemm::stat (rows: M + N, groups: gnA + gnB)
+size_t oz_stat_bytes(i64 rows, i64 K, i64 groups, i64 kr);
+// whether g has the form for a split product and that is faster
+bool oz_plan(const GemmF64& g, const OzHint& h, OzGemm* out);
+bool oz_plan(const GemmZ& g, const OzHint& h, OzGemm* out);
+// The products of a call need stat set.  oz_gemm forms the scales of `later` ones
+// on its way (their phi is there by then), oz_prepare those of the first.
+void oz_prepare(const OzGemm* const* g, int n, cudaStream_t s);
+void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, cudaStream_t s);
 
 // ---------------------------------------------------------------------------
 // Local operator kernels (ttg_local.cu)

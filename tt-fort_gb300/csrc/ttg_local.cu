@@ -29,6 +29,17 @@ static i64 q_size(const LocalDims& L, int nvec) {
   if (L.n * L.m > 4 || oz_bytes(L.rx1 * nvec, L.n * L.ry2 * L.ra1, L.m * L.rx2, false) == 0) return 0;
   return L.n * L.ry2 * L.ra1 * L.m * L.rx2;
 }
+// group maxima and tables of a call's split products, whichever they are
+static size_t stat_bytes(const LocalDims& L, int nvec) {
+  const i64 K = std::max({L.rx2, L.m * L.ra2, L.rx1 * L.ra1, L.m * L.rx2, L.ry1, L.ra1 * L.n,
+                          L.ra2 * L.ry2, L.n * L.ry2, L.rx1 * L.m});
+  const i64 r = std::max(L.ra1, L.ra2);
+  const i64 rows = std::max({L.rx1 * L.m * nvec + L.ra2 * L.ry2, L.rx1 * L.ry2 * nvec + L.ra1 * L.n,
+                             L.rx1 * L.ry2 * nvec + L.ra2 * L.m, L.ry1 + L.n * L.ry2 * nvec,
+                             L.rx1 * nvec + L.n * L.ry2 * L.ra1, L.rx1 * L.ra1 + L.n * L.ry2 * nvec,
+                             L.rx1 * L.m * nvec + L.rx2, L.ry2 * L.ra2 + L.rx2, L.rx1 * L.ra1 + L.ry1});
+  return kOzProducts * oz_stat_bytes(rows, K, r + std::min(nvec, kOzMaxVec), r);
+}
 static size_t bfun3_oz_bytes(const LocalDims& L, int nvec, bool cplx) {
   size_t b = std::max({oz_bytes(L.rx1 * L.m * nvec, L.ra2 * L.ry2, L.rx2, cplx),
                        oz_bytes(L.rx1 * L.ry2 * nvec, L.ra1 * L.n, L.m * L.ra2, cplx),
@@ -39,7 +50,7 @@ static size_t bfun3_oz_bytes(const LocalDims& L, int nvec, bool cplx) {
     b = std::max({b, oz_bytes(L.rx1 * L.ra1, L.n * L.ry2 * nvec, L.ry1, true),
                   oz_bytes(L.rx1 * L.ry2 * nvec, L.m * L.ra2, L.ra1 * L.n, true),
                   oz_bytes(L.rx1 * L.m * nvec, L.rx2, L.ra2 * L.ry2, true)});
-  return b;
+  return b > 0 ? b + stat_bytes(L, nvec) : 0;
 }
 static size_t bfun3_t_bytes(const LocalDims& L, int nvec) {
   return al256((size_t)(std::max(L.t1size() * nvec, q_size(L, nvec)) + L.t2size() * nvec) * sizeof(double));
@@ -60,11 +71,11 @@ static size_t phi_t_bytes(const LocalDims& L, size_t elem) {
   return al256((size_t)(a + b) * elem);
 }
 static size_t phi_oz_bytes(const LocalDims& L, bool cplx) {
-  return std::max({bfun3_oz_bytes(L, 1, cplx),
-                   oz_bytes(L.rx1 * L.ra1, L.n * L.ry2, L.ry1, cplx),
-                   oz_bytes(L.rx1 * L.ry2, L.m * L.ra2, L.ra1 * L.n, cplx),
-                   oz_bytes(L.ry2 * L.ra2, L.rx2, L.rx1 * L.m, cplx),
-                   oz_bytes(L.rx1 * L.ra1, L.ry1, L.n * L.ry2, cplx)});
+  const size_t b = std::max({oz_bytes(L.rx1 * L.ra1, L.n * L.ry2, L.ry1, cplx),
+                             oz_bytes(L.rx1 * L.ry2, L.m * L.ra2, L.ra1 * L.n, cplx),
+                             oz_bytes(L.ry2 * L.ra2, L.rx2, L.rx1 * L.m, cplx),
+                             oz_bytes(L.rx1 * L.ra1, L.ry1, L.n * L.ry2, cplx)});
+  return std::max(bfun3_oz_bytes(L, 1, cplx), b > 0 ? b + stat_bytes(L, 1) : 0);
 }
 size_t phi_f64_scratch(const LocalDims& L) {
   return phi_t_bytes(L, sizeof(double)) + phi_oz_bytes(L, false);
@@ -73,17 +84,56 @@ size_t phi_z_scratch(const LocalDims& L) {
   return phi_t_bytes(L, sizeof(double2)) + phi_oz_bytes(L, true);
 }
 
-// one product: on the tensor cores where that is faster (ws: their workspace,
-// null for the FP64 kernels only)
-static void product(const GemmF64& g, void* ws, cudaStream_t s) {
-  if (!oz_try(g, ws, s)) gemm_f64(g, s);
+static void fp64_product(const GemmF64& g, cudaStream_t s) { gemm_f64(g, s); }
+static void fp64_product(const GemmZ& g, cudaStream_t s) { gemm_z(g, s); }
+
+// The products g[0..n) of a call, each on the tensor cores where that is faster
+// (ws: their workspace, null for the FP64 kernels only).  Interfaces mix blocks of
+// different scale along an operator rank (1 and 1/h^2 for a Laplacian), and the
+// two factors of a product whose K runs over it mix them the opposite way, so the
+// hints name that rank where it is in K (the split products divide it out of both
+// factors) and where it is in the rows (each block's outputs have an accuracy of
+// their own).
+template <class G>
+static void run_products(const G* g, const OzHint* h, int n, void* ws, cudaStream_t s) {
+  OzGemm o[kOzProducts];
+  const OzGemm* split[kOzProducts];
+  bool on[kOzProducts];
+  int ns = 0;
+  char* p = (char*)ws;
+  for (int i = 0; i < n; ++i) {
+    on[i] = ws && oz_plan(g[i], h[i], &o[i]);
+    if (!on[i]) continue;
+    o[i].stat = p;
+    p += oz_stat_bytes((i64)o[i].M + o[i].N, o[i].K, o[i].gnA + o[i].gnB, o[i].kr);
+    split[ns++] = &o[i];
+  }
+  // the first split product forms the others' scales
+  if (ns > 0 && split[0]->kr > 0) oz_prepare(split, 1, s);
+  for (int i = 0; i < n; ++i) {
+    const bool first = on[i] && &o[i] == split[0];
+    if (on[i]) oz_gemm(o[i], p, split + 1, first ? ns - 1 : 0, s);
+    else fp64_product(g[i], s);
+  }
 }
-static void product(const GemmZ& g, void* ws, cudaStream_t s) {
-  if (!oz_try(g, ws, s)) gemm_z(g, s);
+// K of a product over (inner part, operator rank) or (operator rank, inner part):
+// scales by Phi1's blocks (Phi1[c1, b1, a1]) or Phi2's (Phi2[b2, a2, c2])
+template <class T>
+static void scale_by_phi1(OzHint& h, const LocalDims& L, const T* phi1, int norm, i64 kd) {
+  h.phi = (const double*)phi1; h.inner = L.ry1 * L.rx1; h.outer = 1;
+  h.kr = (int)L.ra1; h.kd = (int)kd; h.norm = norm;
+}
+template <class T>
+static void scale_by_phi2(OzHint& h, const LocalDims& L, const T* phi2, int norm, i64 kd) {
+  h.phi = (const double*)phi2; h.inner = L.rx2; h.outer = L.ry2;
+  h.kr = (int)L.ra2; h.kd = (int)kd; h.norm = norm;
+}
+static void rows_of(OzHint& h, int side, i64 groups, i64 run) {
+  h.side = side; h.groups = (int)groups; h.run = (int)run;
 }
 
 template <class G, class T>
-static void stage1(G& g, const LocalDims& L, const T* x, const T* phi2, T* T1, int nvec) {
+static void stage1(G& g, OzHint& h, const LocalDims& L, const T* x, const T* phi2, T* T1, int nvec) {
   // T1 (rx1*m x ra2*ry2) = x (rx1*m x rx2) * phi2 (rx2 x ra2*ry2)
   g.M = (int)(L.rx1 * L.m); g.N = (int)(L.ra2 * L.ry2); g.K = (int)L.rx2;
   g.A = x;    g.sAm = 1; g.sAk = L.rx1 * L.m;
@@ -91,10 +141,12 @@ static void stage1(G& g, const LocalDims& L, const T* x, const T* phi2, T* T1, i
   g.C = T1;   g.sCm = 1; g.sCn = L.rx1 * L.m;
   g.nb1 = 1; g.nb2 = nvec;
   g.bA2 = L.xsize(); g.bB2 = 0; g.bC2 = L.t1size();
+  h.nvec = nvec;
+  rows_of(h, 2, L.ra2, 0);
 }
 
 template <class G, class T>
-static void stage2(G& g, const LocalDims& L, const T* A, const T* T1, T* T2, int nvec) {
+static void stage2(G& g, OzHint& h, const LocalDims& L, const T* A, const T* T1, const T* phi2, T* T2, int nvec) {
   // per (c2, vec): T2[b1,(a1,i)] = sum_(j,a2) A[(a1,i),(j,a2)] T1[b1,(j,a2)]
   g.M = (int)(L.ra1 * L.n); g.N = (int)L.rx1; g.K = (int)(L.m * L.ra2);
   g.A = A;  g.sAm = 1; g.sAk = L.ra1 * L.n;
@@ -104,10 +156,13 @@ static void stage2(G& g, const LocalDims& L, const T* A, const T* T1, T* T2, int
   g.bA1 = 0; g.bA2 = 0;
   g.bB1 = L.rx1 * L.m * L.ra2; g.bB2 = L.t1size();
   g.bC1 = L.rx1 * L.ra1 * L.n; g.bC2 = L.t2size();
+  h.nvec = nvec;
+  rows_of(h, 1, L.ra1, 0);
+  scale_by_phi2(h, L, phi2, -1, L.m);
 }
 
 template <class G, class T>
-static void stage3(G& g, const LocalDims& L, const T* phi1, const T* T2, T* y, int nvec) {
+static void stage3(G& g, OzHint& h, const LocalDims& L, const T* phi1, const T* T2, T* y, int nvec) {
   // y (ry1 x n*ry2) = phi1 (ry1 x rx1*ra1) * T2 (rx1*ra1 x n*ry2)
   g.M = (int)L.ry1; g.N = (int)(L.n * L.ry2); g.K = (int)(L.rx1 * L.ra1);
   g.A = phi1; g.sAm = 1; g.sAk = L.ry1;
@@ -115,6 +170,8 @@ static void stage3(G& g, const LocalDims& L, const T* phi1, const T* T2, T* y, i
   g.C = y;    g.sCm = 1; g.sCn = L.ry1;
   g.nb1 = 1; g.nb2 = nvec;
   g.bA2 = 0; g.bB2 = L.t2size(); g.bC2 = L.ysize();
+  h.nvec = nvec;
+  scale_by_phi1(h, L, phi1, 1, L.rx1);
 }
 
 // Q[kq + KQ (i + n (c2 + ry2 a1))] = sum_a2 A(a1,i,j,a2) Phi2(b2,a2,c2), kq = j + m b2.
@@ -154,8 +211,9 @@ __global__ void __launch_bounds__(128) q_kernel(int m, int rx2, int n, int ry2, 
 // beside 46 us for each of the two large products).  Contracting the core into
 // Phi2 first costs K_Q times ra2 FMAs per row instead (11 us there) and makes
 // the first product n times larger.
-static bool bfun3_q(const LocalDims& L, const double* A, const double* phi2, const double* x,
-                    double* Q, double* T2, int nvec, void* ws, cudaStream_t s) {
+static bool bfun3_q(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
+                    const double* x, double* Q, double* T2, double* y, int nvec, void* ws,
+                    cudaStream_t s) {
   const i64 M = L.rx1 * nvec, N = L.n * L.ry2 * L.ra1, K = L.m * L.rx2;
   if (q_size(L, nvec) == 0 || !oz_fits(M, N, K, false)) return false;
   const double core = 2.0 * (double)(L.ra1 * L.n) * (double)(L.m * L.ra2) * (double)(L.ry2 * L.rx1) * nvec / 1.0e6;
@@ -165,15 +223,34 @@ static bool bfun3_q(const LocalDims& L, const double* A, const double* phi2, con
   const double build = 2.0 * (double)N * (double)K * (double)L.ra2 / 1.0e6 + 4.0;
   if (build + oz_us(M, N, K, false) >= general) return false;
   if (L.ra1 >= 65536 || L.n * L.m * L.ra2 > 4096) return false;   // grid and shared memory
-  launch_pdl(q_kernel, dim3((unsigned)L.ry2, (unsigned)L.ra1), dim3(128),
-             sizeof(double) * L.n * L.m * L.ra2, s, (int)L.m, (int)L.rx2, (int)L.n, (int)L.ry2,
-             (int)L.ra1, (int)L.ra2, A, phi2, Q);
   OzGemm g;   // T2[b1,a1,i,c2,v] = sum_kq X_v[b1,kq] Q[(i,c2,a1),kq]
   g.M = (int)M; g.N = (int)N; g.K = (int)K;
   g.A = x; g.am = {(int)L.rx1, 1, L.xsize()}; g.ak = L.rx1;
   g.B = Q; g.bn = {(int)N, K, 0}; g.bk = 1;
   g.C = T2; g.cm = {(int)L.rx1, 1, L.t2size()}; g.cn = {(int)(L.n * L.ry2), L.rx1 * L.ra1, L.rx1};
-  oz_gemm(g, ws, s);
+  g.gdB = (int)(L.n * L.ry2); g.gnB = (int)L.ra1;
+  if (nvec > 1 && nvec <= kOzMaxVec && L.rx1 >= 8) { g.gdA = (int)L.rx1; g.gnA = nvec; }
+  else g.gdA = g.M;
+  if ((L.ra1 > 1 && g.gdB < 8) || L.ra1 > kOzMaxGroups) return false;
+  GemmF64 g3;
+  OzHint h3;
+  stage3(g3, h3, L, phi1, T2, y, nvec);
+  OzGemm o3;
+  const bool on = oz_plan(g3, h3, &o3);
+  const OzGemm* later = &o3;
+  char* p = (char*)ws;
+  g.stat = p;
+  p += oz_stat_bytes((i64)g.M + g.N, g.K, g.gnA + g.gnB, 0);
+  if (on) {
+    o3.stat = p;
+    p += oz_stat_bytes((i64)o3.M + o3.N, o3.K, o3.gnA + o3.gnB, o3.kr);
+  }
+  launch_pdl(q_kernel, dim3((unsigned)L.ry2, (unsigned)L.ra1), dim3(128),
+             sizeof(double) * L.n * L.m * L.ra2, s, (int)L.m, (int)L.rx2, (int)L.n, (int)L.ry2,
+             (int)L.ra1, (int)L.ra2, A, phi2, Q);
+  oz_gemm(g, p, &later, on ? 1 : 0, s);
+  if (on) oz_gemm(o3, p, nullptr, 0, s);
+  else gemm_f64(g3, s);
   return true;
 }
 
@@ -183,21 +260,25 @@ void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const do
   double* T1 = scratch;
   double* T2 = scratch + t1;
   void* ws = split ? (char*)scratch + bfun3_t_bytes(L, nvec) : nullptr;
-  if (!ws || !bfun3_q(L, A, phi2, x, T1, T2, nvec, ws, s)) {
-    { GemmF64 g; stage1(g, L, x, phi2, T1, nvec); product(g, ws, s); }
-    { GemmF64 g; stage2(g, L, A, T1, T2, nvec); product(g, ws, s); }
-  }
-  { GemmF64 g; stage3(g, L, phi1, T2, y, nvec); product(g, ws, s); }
+  if (ws && bfun3_q(L, phi1, A, phi2, x, T1, T2, y, nvec, ws, s)) return;
+  GemmF64 g[3];
+  OzHint h[3];
+  stage1(g[0], h[0], L, x, phi2, T1, nvec);
+  stage2(g[1], h[1], L, A, T1, phi2, T2, nvec);
+  stage3(g[2], h[2], L, phi1, T2, y, nvec);
+  run_products(g, h, 3, ws, s);
 }
 
 void bfun3_z(const LocalDims& L, const double2* phi1, const double2* A, const double2* phi2,
              const double2* x, double2* y, int nvec, double2* scratch, cudaStream_t s) {
   double2* T1 = scratch;
   double2* T2 = scratch + L.t1size() * nvec;
-  void* ws = (char*)scratch + bfun3_z_t_bytes(L, nvec);
-  { GemmZ g; stage1(g, L, x, phi2, T1, nvec); product(g, ws, s); }
-  { GemmZ g; stage2(g, L, A, T1, T2, nvec); product(g, ws, s); }
-  { GemmZ g; stage3(g, L, phi1, T2, y, nvec); product(g, ws, s); }
+  GemmZ g[3];
+  OzHint h[3];
+  stage1(g[0], h[0], L, x, phi2, T1, nvec);
+  stage2(g[1], h[1], L, A, T1, phi2, T2, nvec);
+  stage3(g[2], h[2], L, phi1, T2, y, nvec);
+  run_products(g, h, 3, (char*)scratch + bfun3_z_t_bytes(L, nvec), s);
 }
 
 // Adjoint product (zbfun3_transp, ttals.f90:85-108): x has the y layout
@@ -209,18 +290,19 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
   const i64 p2 = L.rx1 * L.m * L.ra2 * L.ry2;     // R2[b1,j,a2,c2]
   double2* R1 = scratch;
   double2* R2 = scratch + p1 * nvec;
-  void* ws = (char*)scratch + bfun3_z_t_bytes(L, nvec);
+  GemmZ gs[3];
+  OzHint h[3];
   {
-    GemmZ g;   // R1[(b1,a1),(i,c2)] = sum_c1 conj(phi1[c1,(b1,a1)]) x[c1,(i,c2)]
+    GemmZ& g = gs[0];   // R1[(b1,a1),(i,c2)] = sum_c1 conj(phi1[c1,(b1,a1)]) x[c1,(i,c2)]
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)(L.n * L.ry2); g.K = (int)L.ry1;
     g.A = phi1; g.sAm = L.ry1; g.sAk = 1; g.conjA = true;
     g.B = x; g.sBk = 1; g.sBn = L.ry1;
     g.C = R1; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
     g.nb2 = nvec; g.bB2 = L.ysize(); g.bC2 = p1;
-    product(g, ws, s);
+    rows_of(h[0], 1, L.ra1, L.rx1);
   }
   {
-    GemmZ g;   // per (c2, vec): R2[b1,(j,a2)] = sum_p conj(A[p,(j,a2)]) R1[b1,p]
+    GemmZ& g = gs[1];   // per (c2, vec): R2[b1,(j,a2)] = sum_p conj(A[p,(j,a2)]) R1[b1,p]
     g.M = (int)(L.m * L.ra2); g.N = (int)L.rx1; g.K = (int)(L.ra1 * L.n);
     g.A = A; g.sAm = L.ra1 * L.n; g.sAk = 1; g.conjA = true;
     g.B = R1; g.sBk = L.rx1; g.sBn = 1;
@@ -228,17 +310,20 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
     g.nb1 = (int)L.ry2; g.nb2 = nvec;
     g.bB1 = L.rx1 * L.ra1 * L.n; g.bB2 = p1;
     g.bC1 = L.rx1 * L.m * L.ra2; g.bC2 = p2;
-    product(g, ws, s);
+    rows_of(h[1], 1, L.ra2, L.m);
+    scale_by_phi1(h[1], L, phi1, -1, 1);
   }
   {
-    GemmZ g;   // y[(b1,j), b2] = sum_(a2,c2) R2[(b1,j),(a2,c2)] conj(phi2[b2,(a2,c2)])
+    GemmZ& g = gs[2];   // y[(b1,j), b2] = sum_(a2,c2) R2[(b1,j),(a2,c2)] conj(phi2[b2,(a2,c2)])
     g.M = (int)(L.rx1 * L.m); g.N = (int)L.rx2; g.K = (int)(L.ra2 * L.ry2);
     g.A = R2; g.sAm = 1; g.sAk = L.rx1 * L.m;
     g.B = phi2; g.sBk = L.rx2; g.sBn = 1; g.conjB = true;
     g.C = y; g.sCm = 1; g.sCn = L.rx1 * L.m;
     g.nb2 = nvec; g.bA2 = p2; g.bC2 = L.xsize();
-    product(g, ws, s);
+    scale_by_phi2(h[2], L, phi2, -1, 1);
   }
+  for (OzHint& k : h) k.nvec = nvec;
+  run_products(gs, h, 3, (char*)scratch + bfun3_z_t_bytes(L, nvec), s);
 }
 
 template <class G, class T>
@@ -246,19 +331,21 @@ static void phi_right_impl(const LocalDims& L, const T* phi2_old, const T* A, co
                            const T* y, T* phi2_new, T* scratch, bool conj_y, cudaStream_t s) {
   T* T1 = scratch;
   T* T2 = scratch + L.t1size();
-  void* ws = (char*)scratch + phi_t_bytes(L, sizeof(T));
-  { G g; stage1(g, L, x, phi2_old, T1, 1); product(g, ws, s); }
-  { G g; stage2(g, L, A, T1, T2, 1); product(g, ws, s); }
+  G gs[3];
+  OzHint h[3];
+  stage1(gs[0], h[0], L, x, phi2_old, T1, 1);
+  stage2(gs[1], h[1], L, A, T1, phi2_old, T2, 1);
   {
     // phi2_new (rx1*ra1 x ry1) = T2 (rx1*ra1 x n*ry2) * y^T (n*ry2 x ry1)
-    G g;
+    G& g = gs[2];
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)L.ry1; g.K = (int)(L.n * L.ry2);
     g.A = T2; g.sAm = 1; g.sAk = L.rx1 * L.ra1;
     g.B = y; g.sBk = L.ry1; g.sBn = 1;
     g.C = phi2_new; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
     if constexpr (sizeof(T) == 16) g.conjB = conj_y;
-    product(g, ws, s);
+    rows_of(h[2], 1, L.ra1, L.rx1);
   }
+  run_products(gs, h, 3, (char*)scratch + phi_t_bytes(L, sizeof(T)), s);
 }
 
 template <class G, class T>
@@ -267,34 +354,37 @@ static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, con
   const i64 psz = L.rx1 * L.ra1 * L.n * L.ry2;   // P[b1,a1,i,c2]
   T* P = scratch;
   T* Q = scratch + psz;                           // Q[b1,j,a2,c2]
-  void* ws = (char*)scratch + phi_t_bytes(L, sizeof(T));
+  G gs[3];
+  OzHint h[3];
   {
-    G g;   // P[(b1,a1),(i,c2)] = sum_c1 phi1_old[c1,(b1,a1)] y[c1,(i,c2)]
+    G& g = gs[0];   // P[(b1,a1),(i,c2)] = sum_c1 phi1_old[c1,(b1,a1)] y[c1,(i,c2)]
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)(L.n * L.ry2); g.K = (int)L.ry1;
     g.A = phi1_old; g.sAm = L.ry1; g.sAk = 1;
     g.B = y; g.sBk = 1; g.sBn = L.ry1;
     g.C = P; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
     if constexpr (sizeof(T) == 16) g.conjB = conj_y;
-    product(g, ws, s);
+    rows_of(h[0], 1, L.ra1, L.rx1);
   }
   {
-    G g;   // per c2: Q[b1,(j,a2)] = sum_(a1,i) A[(a1,i),(j,a2)] P[b1,(a1,i)]
+    G& g = gs[1];   // per c2: Q[b1,(j,a2)] = sum_(a1,i) A[(a1,i),(j,a2)] P[b1,(a1,i)]
     g.M = (int)(L.m * L.ra2); g.N = (int)L.rx1; g.K = (int)(L.ra1 * L.n);
     g.A = A; g.sAm = L.ra1 * L.n; g.sAk = 1;
     g.B = P; g.sBk = L.rx1; g.sBn = 1;
     g.C = Q; g.sCm = L.rx1; g.sCn = 1;
     g.nb1 = (int)L.ry2; g.bB1 = L.rx1 * L.ra1 * L.n; g.bC1 = L.rx1 * L.m * L.ra2;
-    product(g, ws, s);
+    rows_of(h[1], 1, L.ra2, L.m);
+    scale_by_phi1(h[1], L, phi1_old, -1, 1);
   }
   {
-    G g;   // per a2: phi1_new[c2, b2] = sum_(b1,j) Q[(b1,j), a2, c2] x[(b1,j), b2]
+    G& g = gs[2];   // per a2: phi1_new[c2, b2] = sum_(b1,j) Q[(b1,j), a2, c2] x[(b1,j), b2]
     g.M = (int)L.ry2; g.N = (int)L.rx2; g.K = (int)(L.rx1 * L.m);
     g.A = Q; g.sAm = L.rx1 * L.m * L.ra2; g.sAk = 1;
     g.B = x; g.sBk = 1; g.sBn = L.rx1 * L.m;
     g.C = phi1_new; g.sCm = 1; g.sCn = L.ry2;
     g.nb1 = (int)L.ra2; g.bA1 = L.rx1 * L.m; g.bC1 = L.ry2 * L.rx2;
-    product(g, ws, s);
+    rows_of(h[2], 1, L.ra2, L.ry2);
   }
+  run_products(gs, h, 3, (char*)scratch + phi_t_bytes(L, sizeof(T)), s);
 }
 
 void phi_right_f64(const LocalDims& L, const double* phi2_old, const double* A,

@@ -19,21 +19,34 @@
 // -128, and a rounding there lies at 2^-24 2^-32.  After 256 K the groups are
 // drained into two 64-bit integers per element (no FP64 arithmetic), which
 // sum exactly in any order, and the end result is rounded once.  The error
-// left is that of I (2^-55 of a row's largest element) and of the dropped
-// products: measured against 64-bit values below that of the FP64 FMA chain
-// (tests/test_oz_gpu.py).
+// left is that of I and of the dropped products: below 2^-51 K max_k |a_mk| max_k
+// |b_kn|, while the FP64 FMA chain's bound is 2^-53 K sum_k |a_mk| |b_kn|.  With
+// elements of one size the first is the smaller in practice (normal data, relative
+// error in the norm 2.0 to 3.6e-16 against 2.8 to 9.2e-16).  A row that spans
+// scales would lose its small elements' bits, and the operators' parts do differ in
+// scale along the operator rank (1 and 1/h^2 in a Laplacian), the opposite way in
+// the two factors of a product whose K runs over it: with elements 1 and nu, error
+// nu 2e-17.  So
+//   - the elements of A and B are scaled along K by powers of two (exact) from the
+//     largest element of each operator rank block of an interface (OzGemm::phi),
+//   - it is checked that for every group of rows of A and of columns of B (an
+//     operator rank block of the result, a vector of a block) some k holds elements
+//     of both whose product is within 2^5 of the groups' largest: then the error in
+//     that part of the result is below 2^-46 K times the largest sum_k |a| |b| in it
+//     (measured 2 to 3e-16 in the norm at nu = 1 to 1e12), and
+//   - products that fail it (3% of a time stepper's, 2 to 9% of a linear solver's;
+//     none with Gaussian interfaces) are formed by FP64 FMA chains.
 //
 // A row whose elements are not all finite, or whose largest element lies
-// outside 2^(+-400), is flagged, and the tiles that it meets are formed by the
-// plain FP64 FMA chain, so infinities, NaN and extreme ranges give what they
-// give there.
+// outside 2^(+-400), is flagged, and its product is formed by plain FP64 FMA
+// chains, so infinities, NaN and extreme ranges give what they give there.
 //
 // Measured on GB300, FP64 kernels -> split products: chain product r=256, block
-// of 8: 4560 -> 241 us (22.7 TFLOP/s of FP64 accuracy; its two products run at
-// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 32.8
-// us; grid interface updates r = 82, 77, n = 64: 1908 -> 160 us; complex
-// operator and adjoint r=48, n=32, block of 4: 6968 -> 351 us.  What bounds the
-// product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
+// of 8: 4560 -> 248 us (22 TFLOP/s of FP64 accuracy; its two products run at
+// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 38.2
+// us; grid interface updates r = 82, 77, n = 64: 1908 -> 180 us; complex
+// operator and adjoint r=48, n=32, block of 4: 6968 -> 383 us (without scales and
+// check 241, 32.8, 160 and 351).  What bounds the product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
 // measured against 900 of MMA), for small ones its fixed ~10 us (pipeline
 // fill, one drain, rounding); oz_us below holds both.
 //
@@ -64,9 +77,23 @@ __host__ __device__ constexpr uint32_t stage_bytes(int bn) { return A_BYTES + b_
 constexpr size_t smem_bytes(int bn) { return (size_t)STAGES * stage_bytes(bn) + 1024; }
 constexpr int EPI_WARPS = 16;
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
-constexpr int SLOW = 1 << 20;   // exponent of a flagged row
 constexpr int EMAX = 400;       // largest |exponent| of the fast path
 
+// Largest elements of an operand's row groups (group r / gd of row r, gn gd = rows)
+// as scaled exponents + EBIAS, 0 for zeros only, and where they are: per block of
+// eight rows, its first group's rows and the next one's, over all of K; and along K
+// for up to SLOTS blocks of a group, spread over it (rows of the first group).
+constexpr int SROWS = 8, SLOTS = 16, EBIAS = 8192, FLAGGED = 1 << 30;
+struct Groups {
+  int rows, gd, gn;
+  int stride;                   // every how manyth block that starts in a group has a slot
+  int4* bm;                     // [block]: largest, its k, of the next group; FLAGGED
+  short* part;                  // [group][slot][K]
+  __host__ __device__ int first_block(int group) const { return (group * gd + SROWS - 1) / SROWS; }
+  __device__ int slots(int group) const {
+    return (first_block(group + 1) - first_block(group) + stride - 1) / stride;
+  }
+};
 struct Side {                   // one operand, element (r, k) = src[map(r) + k * sk]
   const double* src;
   OzMap map;
@@ -78,6 +105,9 @@ struct Side {                   // one operand, element (r, k) = src[map(r) + k 
   int vec;                      // real with sk == 1 and 16-byte aligned rows
   int cplx;                     // 0 real, 1: rows (re, im) x K (re, im), 2: K (re, im) only
   int conj;
+  const short* tab;             // scales along K (null: none) by block k / kd % kr
+  int kd, kr, sgn;
+  Groups gr;
 };
 
 struct Args {
@@ -89,9 +119,10 @@ struct Args {
   double* C;
   OzMap cm, cn;
   longlong2* part;              // nz > cs: the clusters' sums [z / cs][n][row]
-  const double *A, *B;          // original operands (flagged rows)
+  const double *A, *B;          // original operands (FP64 chains)
   OzMap am, bn;
   i64 ak, bk;
+  Groups ga, gb;
   int cplx, conjA, conjB;       // complex: product rows (PAIR: columns) are (re, im)
 };
 
@@ -114,18 +145,71 @@ __device__ __forceinline__ uint32_t top_pair(int ta, int tb) {
   return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
+// The largest exponents of an interface's operator rank blocks, in TPARTS parts
+// each: element i of block a, outer index o, lies at (o kr + a) inner + i.
+constexpr int TPARTS = 8, TNONE = -32768, TSPAN = 300, NTABLES = kOzProducts - 1;
+struct Table { const double* phi; short* tab; i64 inner, outer; int kr; };
+struct Tables { Table t[NTABLES]; };
+// block b of 256 threads, kr TPARTS of them per table
+__device__ __forceinline__ void table_block(const Tables& ts, int b) {
+  __shared__ int best_s;
+  static_assert(NTABLES == 2, "two tables");
+  const bool second = b >= ts.t[0].kr * TPARTS;
+  if (second) b -= ts.t[0].kr * TPARTS;
+  const Table t = second ? ts.t[1] : ts.t[0];
+  const int a = b / TPARTS, part = b % TPARTS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) best_s = TNONE;
+  __syncthreads();
+  // 8 warps per part: over the outer index, or over the elements of the only one
+  const i64 w = part * 8 + warp, nw = TPARTS * 8;
+  int best = TNONE;
+  auto see = [&](double v) {
+    const int e = (__double2hiint(v) >> 20) & 0x7ff;
+    if (((__double2hiint(v) << 1) | __double2loint(v)) != 0 && e != 0x7ff) best = max(best, max(e, 1) - 1022);
+  };
+  if (t.outer == 1) {
+    const double* x = t.phi + t.inner * a;
+#pragma unroll 4
+    for (i64 i = w * 32 + lane; i < t.inner; i += nw * 32) see(x[i]);
+  } else {
+    for (i64 o = w; o < t.outer; o += nw) {
+      const double* x = t.phi + t.inner * (o * t.kr + a);
+#pragma unroll 4
+      for (i64 i = lane; i < t.inner; i += 32) see(x[i]);
+    }
+  }
+  best = __reduce_max_sync(0xffffffffu, best);
+  if (lane == 0) atomicMax(&best_s, best);
+  __syncthreads();
+  if (threadIdx.x == 0) t.tab[a * TPARTS + part] = (short)best_s;
+}
+__global__ void __launch_bounds__(256) tables_kernel(Tables t) {
+  pdl_wait();
+  pdl_trigger();
+  table_block(t, blockIdx.x);
+}
+
 // Splits two operands in one launch (blocks [0, nblkA) take A).  A cluster of
 // gridDim.y blocks takes 8 rows and all of K, its blocks every gridDim.y-th
 // run of 256: a first pass finds the rows' largest exponents (joined over the
 // cluster), a second writes the digits, each thread one 16-byte core-matrix
-// row (8 K) per plane.  Bound by its 8 bytes read and 14 written per element
-// (integer digits, no FP64 arithmetic).
-constexpr int SROWS = 8;
-__global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA, int K, int kt) {
+// row (8 K) per plane, and notes the largest exponents of the row groups.  Blocks
+// past B's form the tables that the call's later products need.  Bound by its 8
+// bytes read and 14 written per element (integer digits, no FP64 arithmetic).
+// One copy of the code for both operands, and one of the stores: at these sizes its
+// fetching counts (with a copy for each operand the kernel took 4 us more).
+__global__ void __launch_bounds__(256, 3) split_kernel(const __grid_constant__ Side a, const __grid_constant__ Side b,
+                                                       int nblkA, int nblk, const __grid_constant__ Tables tabs,
+                                                       int K, int kt) {
   namespace cgr = cooperative_groups;
   cgr::cluster_group cl = cgr::this_cluster();
-  __shared__ unsigned int key_s[SROWS];
+  __shared__ int key_s[SROWS], scaled_s;
+  extern __shared__ __align__(16) short tab_s[];
   pdl_wait();
+  if ((int)blockIdx.x >= nblk) {
+    if (blockIdx.y == 0) table_block(tabs, blockIdx.x - nblk);
+    return;
+  }
   const bool isA = (int)blockIdx.x < nblkA;
   const Side& S = isA ? a : b;
   const int blk = isA ? blockIdx.x : blockIdx.x - nblkA;
@@ -135,8 +219,6 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
   const bool real = r < S.rows;
   const double* p = S.src + (real ? at(S.map, r) * (S.cplx ? 2 : 1) : 0);
   const int groups = 2 * kt;
-  if (threadIdx.x < SROWS) key_s[threadIdx.x] = 0u;
-  __syncthreads();
   double v[8];
   auto load = [&](int g) {
 #pragma unroll
@@ -167,13 +249,83 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
       }
     }
   };
-  unsigned int key = 0u;
-  for (int g = kg0; g < groups; g += kgs) {
-    load(g);
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      key = max(key, ((unsigned)__double2hiint(v[q]) & 0x7fffffffu) | (__double2loint(v[q]) != 0 ? 1u : 0u));
+  // exponents of the scales of group g's eight + EBIAS, two to a word
+  constexpr int NONFINITE = 1 << 20;
+  uint32_t sc[4] = {EBIAS * 0x10001u, EBIAS * 0x10001u, EBIAS * 0x10001u, EBIAS * 0x10001u};
+  auto scales = [&](int g) {
+    if (S.cplx) {
+      const uint2 t = *reinterpret_cast<const uint2*>(tab_s + 4 * g);
+      sc[0] = __byte_perm(t.x, 0u, 0x1010);
+      sc[1] = __byte_perm(t.x, 0u, 0x3232);
+      sc[2] = __byte_perm(t.y, 0u, 0x1010);
+      sc[3] = __byte_perm(t.y, 0u, 0x3232);
+    } else {
+      const uint4 t = *reinterpret_cast<const uint4*>(tab_s + 8 * g);
+      sc[0] = t.x;
+      sc[1] = t.y;
+      sc[2] = t.z;
+      sc[3] = t.w;
+    }
+  };
+  auto scale = [&](int q) { return (int)(q & 1 ? sc[q >> 1] >> 16 : sc[q >> 1] & 0xffffu); };
+  // (zeros count as 2^-1022 and less here, which no unflagged row's largest is near:
+  // scales stay within 2^(+-300).  Integers only: an FP64 comparison holds the pipe
+  // for 64 clocks)
+  auto expo_of = [&](int q) { return (__double2hiint(v[q]) >> 20) & 0x7ff; };
+  load(kg0);                                         // (beyond K: zeros)
+  // while these are on their way: the block's place among the row groups, the scales
+  const int group = blk * SROWS / S.gr.gd, in_group = blk - S.gr.first_block(group);
+  const bool first = r / S.gr.gd == group, has_slot = blk * SROWS < S.rows && in_group % S.gr.stride == 0;
+  short* part = has_slot ? S.gr.part + (size_t)(group * SLOTS + in_group / S.gr.stride) * ((K + 7) & ~7) : nullptr;
+  if (threadIdx.x < SROWS) key_s[threadIdx.x] = 0;
+  // the operator rank blocks' scales, behind the places of each k's
+  const int per = S.cplx ? 4 : 8;
+  short* of_block = tab_s + groups * per;
+  if (S.tab && threadIdx.x < 32) {
+    int ref = TNONE, most = 0;
+    for (int c = threadIdx.x; c < S.kr; c += 32) {
+      const uint4 t = *reinterpret_cast<const uint4*>(S.tab + c * TPARTS);
+      const uint32_t m = __vmaxs2(__vmaxs2(t.x, t.y), __vmaxs2(t.z, t.w));
+      of_block[c] = (short)max((int)(short)(m & 0xffffu), (int)m >> 16);
+      ref = max(ref, (int)of_block[c]);
+    }
+    ref = __reduce_max_sync(0xffffffffu, ref);
+    // blocks within a factor of two of the largest stay as they are
+    for (int c = threadIdx.x; c < S.kr; c += 32) {
+      const int d = of_block[c] == TNONE ? 0 : max(of_block[c] - ref, -TSPAN);
+      of_block[c] = (short)(EBIAS + (d >= -1 ? 0 : S.sgn * d));
+      most = max(most, -d);
+    }
+    if (threadIdx.x == 0) scaled_s = 0;
+    __syncwarp();
+    if (most > 1) scaled_s = 1;
   }
+  __syncthreads();
+  const bool scaled = S.tab && scaled_s != 0;
+  if (scaled) {
+    for (int k = threadIdx.x; k < groups * per; k += blockDim.x) tab_s[k] = of_block[k / S.kd % S.kr];
+    __syncthreads();
+  }
+  int key = 0, key_g = kg0, top_e = 0;               // the row's largest here, in which group
+  unsigned int nonzero = 0u;
+  for (int g = kg0; g < groups; g += kgs) {
+    if (g != kg0) load(g);
+    if (scaled) scales(g);
+    int here = 0;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int x = expo_of(q);
+      here = max(here, x + scale(q));
+      top_e = max(top_e, x);
+      nonzero |= ((unsigned)__double2hiint(v[q]) & 0x7fffffffu) | (unsigned)__double2loint(v[q]);
+    }
+    if (here > key) {
+      key = here;
+      key_g = g;
+    }
+  }
+  key = nonzero == 0u ? 0 : (top_e == 0x7ff ? NONFINITE : key);
+  const int own = key;
   atomicMax(&key_s[row], key);
   if (gridDim.y > 1) {
     cl.sync();
@@ -183,12 +335,11 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
     __syncthreads();
     key = key_s[row];
   }
-  const int em = (int)(key >> 20);
-  const int e = em - 1022;
-  const bool slow = em == 0 ? key != 0u : (em == 0x7ff || e > EMAX || e < -EMAX);
-  const bool zero = em == 0 || slow;
+  const int e = key - EBIAS - 1022;
+  const bool flag = key == NONFINITE || (key != 0 && (e > EMAX || e < -EMAX));
+  const bool zero = key == 0 || flag;
   if (kg0 == 0) {
-    const int ex = slow ? SLOW : (zero ? 0 : e);
+    const int ex = zero ? 0 : e;
     if (S.cplx == 1) {
       S.expo[2 * r] = ex;
       S.expo[2 * r + 1] = ex;
@@ -196,8 +347,48 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
       S.expo[r] = ex;
     }
   }
-  for (int g = kg0; g < groups; g += kgs) {
-    if (groups > kgs) load(g);                       // one group per thread: still in registers
+  // the row groups' largest of this block (of one of them that has it, its k)
+  const int mine = real && !zero ? key : 0;
+  int* at = nullptr;
+  if (blk * SROWS < S.rows) {
+    const unsigned rows8 = 0xffu << (threadIdx.x & 24);
+    const int m0 = __reduce_max_sync(rows8, first ? mine : 0), m1 = __reduce_max_sync(rows8, first ? 0 : mine);
+    const bool bad = __any_sync(rows8, flag);
+    int* bm = reinterpret_cast<int*>(S.gr.bm + blk);
+    if (kg0 == 0 && row < 2) bm[2 * row] = row ? m1 : (bad ? FLAGGED : m0);
+    at = mine && own == key && key == (first ? m0 : m1) ? bm + (first ? 1 : 3) : nullptr;
+  }
+  for (int g = kg0; (g & ~3) < groups; g += kgs) {
+    if (groups > kgs) {                              // one group per thread: still in registers
+      load(g);
+      if (scaled) scales(g);
+    }
+    if (at && g == key_g) {
+      int k = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (expo_of(q) + scale(q) == key) k = q;
+      *at = S.cplx ? g * 4 + k / 2 : g * 8 + k;
+    }
+    if (part) {
+      // largest scaled exponents of these k over the rows, 16 bits each, by
+      // halving: lane `row` is left with k = row of the eight
+      uint32_t x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint32_t h = __byte_perm((unsigned)__double2hiint(v[2 * q]), (unsigned)__double2hiint(v[2 * q + 1]), 0x7632);
+        x[q] = mine && first ? (h >> 4 & 0x07ff07ffu) + sc[q] : 0u;
+        if (S.cplx) x[q] = __vmaxu2(x[q], __byte_perm(x[q], x[q], 0x1032));
+      }
+      uint32_t a0 = row & 4 ? x[2] : x[0], a1 = row & 4 ? x[3] : x[1];
+      a0 = __vmaxu2(a0, __shfl_xor_sync(0xffffffffu, row & 4 ? x[0] : x[2], 4));
+      a1 = __vmaxu2(a1, __shfl_xor_sync(0xffffffffu, row & 4 ? x[1] : x[3], 4));
+      uint32_t b0 = __vmaxu2(row & 2 ? a1 : a0, __shfl_xor_sync(0xffffffffu, row & 2 ? a0 : a1, 2));
+      b0 = __vmaxu2(b0, __shfl_xor_sync(0xffffffffu, b0, 1));
+      const int k = S.cplx ? g * 4 + row / 2 : g * 8 + row;
+      if (k < K && !(S.cplx && (row & 1))) part[k] = (short)(row & 1 ? b0 >> 16 : b0 & 0xffffu);
+    }
+    if (g >= groups) continue;
     int top[8];
     uint32_t jl[8], jh[8];                           // bytes of I + sum 128 256^i
 #pragma unroll
@@ -206,7 +397,7 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
       const int eq = (int)((hi >> 20) & 0x7ff);
       long long m = (long long)(((unsigned long long)(hi & 0xfffffu) << 32) | lo);
       if (eq) m |= 1ll << 52;
-      const int sh = em - (eq ? eq : 1) - 2;         // I = m 2^-sh
+      const int sh = key - (max(eq, 1) + scale(q)) - 2;   // I = m 2^-sh
       long long I = 0;
       if (!zero) I = sh <= 0 ? m << -sh : (sh < 55 ? (m + (1ll << (sh - 1))) >> sh : 0);
       if (hi >> 31) I = -I;
@@ -215,33 +406,35 @@ __global__ void __launch_bounds__(256, 3) split_kernel(Side a, Side b, int nblkA
       jh[q] = (uint32_t)((unsigned long long)J >> 32);
       top[q] = (int)(J >> 48);
     }
-    auto emit = [&](int rr, int neg_odd, bool swap) {
-      // pairs (0,1) (2,3) (4,5) (6,7); neg_odd: the second of a pair negated
-      // (I -> -I digit by digit is again balanced: digits in [-128, 128])
+    // pairs (0,1) (2,3) (4,5) (6,7).  A doubled complex operand: the real part's row
+    // (re, -im), then the imaginary part's (im, re); the second of a pair negated (I
+    // -> -I digit by digit is again balanced: digits in [-128, 128])
+    auto word = [&](int pl, int h) {
+      if (pl == 0) return top_pair(top[2 * h], top[2 * h + 1]);
+      if (pl < 3) return digit_pair(jh[2 * h], jh[2 * h + 1], pl == 1 ? 0x7651u : 0x7650u);
+      return digit_pair(jl[2 * h], jl[2 * h + 1], 0x7650u + (6 - pl));
+    };
+    auto place = [&](int rr) {
       const int rt = rr / S.R, ri = rr % S.R;
-      unsigned char* o = S.planes + ((size_t)rt * kt + (g >> 1)) * ((size_t)P * S.R * 32) +
-                         (size_t)((ri >> 3) * 256 + (g & 1) * 128 + (ri & 7) * 16);
+      return S.planes + ((size_t)rt * kt + (g >> 1)) * ((size_t)P * S.R * 32) +
+             (size_t)((ri >> 3) * 256 + (g & 1) * 128 + (ri & 7) * 16);
+    };
+    if (S.cplx != 1) {
+      unsigned char* o = place(r);
+#pragma unroll
+      for (int pl = 0; pl < P; ++pl)
+        *reinterpret_cast<uint4*>(o + (size_t)pl * S.R * 32) = make_uint4(word(pl, 0), word(pl, 1), word(pl, 2), word(pl, 3));
+    } else {
+      unsigned char* o = place(2 * r);               // 2 r + 1 lies 16 bytes on
+      auto minus = [](uint32_t x) { return (x & 0x7fff0000u) ? x ^ 0x80000000u : x; };
+      auto swap = [](uint32_t x) { return __byte_perm(x, x, 0x1032); };
 #pragma unroll
       for (int pl = 0; pl < P; ++pl) {
-        uint32_t w[4];
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          uint32_t x;
-          if (pl == 0) x = top_pair(top[2 * h], top[2 * h + 1]);
-          else if (pl < 3) x = digit_pair(jh[2 * h], jh[2 * h + 1], pl == 1 ? 0x7651u : 0x7650u);
-          else x = digit_pair(jl[2 * h], jl[2 * h + 1], 0x7650u + (6 - pl));
-          if (swap) x = __byte_perm(x, x, 0x1032);
-          if (neg_odd) x = (x & 0x7fff0000u) ? x ^ 0x80000000u : x;
-          w[h] = x;
-        }
-        *reinterpret_cast<uint4*>(o + (size_t)pl * S.R * 32) = make_uint4(w[0], w[1], w[2], w[3]);
+        const uint32_t w0 = word(pl, 0), w1 = word(pl, 1), w2 = word(pl, 2), w3 = word(pl, 3);
+        uint4* d = reinterpret_cast<uint4*>(o + (size_t)pl * S.R * 32);
+        d[0] = make_uint4(minus(w0), minus(w1), minus(w2), minus(w3));
+        d[1] = make_uint4(swap(w0), swap(w1), swap(w2), swap(w3));
       }
-    };
-    if (S.cplx == 1) {
-      emit(2 * r, 1, false);      // (re, -im): the real part's row
-      emit(2 * r + 1, 0, true);   // (im, re): the imaginary part's row
-    } else {
-      emit(r, 0, false);
     }
   }
   pdl_trigger();
@@ -326,7 +519,6 @@ __device__ __noinline__ void fp64_unit(const Args& g, int rt, int ct, int kbeg, 
   using T = typename std::conditional<CPLX, double2, double>::type;
   const int e = threadIdx.x - 64, warp = e >> 5, lane = e & 31, ly = lane >> 3, lx = lane & 7;
   const int r0 = rt * 32, c0 = ct * (BN / 4);
-  if (r0 >= g.M || c0 >= g.N) return;
   const T *a[NI], *b[NJ];
 #pragma unroll
   for (int i = 0; i < NI; ++i) {
@@ -395,28 +587,94 @@ __device__ __noinline__ void fp64_unit(const Args& g, int rt, int ct, int kbeg, 
   }
 }
 
-// whether draining thread e sees a flagged row or column of tile (mt, nt)
-template <int BN>
-__device__ __forceinline__ bool flagged(const Args& g, int mt, int nt, int e) {
-  const int r = mt * BM + e, n = nt * BN + e;
-  return (e < BM && r < g.M && g.ea[r] == SLOW) || (e < BN && n < g.N && g.eb[n] == SLOW);
+// Whether a product is one for the FP64 chains: a row is flagged, or the large
+// elements of the operands do not meet.  For every group of A's rows and of B's
+// columns, 2^APART times some k's product of largest elements must reach the product
+// of the groups' largest (either 0: nothing to reach).  Looked for where one of
+// them has its largest, then everywhere.  Draining threads.
+constexpr int APART = 3;
+constexpr int PAIRS = 128;                        // pairs of groups looked at together
+constexpr int WHERE = 18;                         // bits of a largest element's k (beyond: not looked for there)
+struct Check {                                    // shared memory, zero at first
+  unsigned int mx[2 * kOzMaxGroups];              // A's groups, then B's: largest, its k
+  int seen[2][PAIRS];                             // the other side's largest there
+};
+__device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
+  constexpr int NE = 32 * EPI_WARPS, KMASK = (1 << WHERE) - 1;
+  const int e = threadIdx.x - 64, na = g.ga.gn, np = na * g.gb.gn, Kp = (g.K + 7) & ~7;
+  bool bad = false;
+#pragma unroll 1
+  for (int side = 0; side < 2; ++side) {
+    const Groups& s = side ? g.gb : g.ga;
+    unsigned int* m = sh.mx + (side ? na : 0);
+    const int n = (s.rows + SROWS - 1) / SROWS;
+    for (int b = e; b - (e & 31) < n; b += NE) {
+      const int4 v = b < n ? s.bm[b] : make_int4(0, 0, 0, 0);
+      bad = bad || v.x == FLAGGED;
+      const int group = s.gn == 1 ? 0 : min(b, n - 1) * SROWS / s.gd;
+      const unsigned x = v.x > 0 ? (unsigned)(v.x & 0x3fff) << WHERE | min(v.y, KMASK) : 0u;
+      int same;
+      __match_all_sync(0xffffffffu, group, &same);
+      if (same) {                                    // 32 atomics on one word are as many turns
+        const unsigned y = __reduce_max_sync(0xffffffffu, x);
+        if ((e & 31) == 0) atomicMax(&m[group], y);
+      } else {
+        atomicMax(&m[group], x);
+      }
+      if (v.z > 0) atomicMax(&m[group + 1], (unsigned)v.z << WHERE | min(v.w, KMASK));
+    }
+  }
+  if (epi_or(bad)) return true;
+  bool open = false;
+  for (int p0 = 0; p0 < np; p0 += PAIRS) {
+    const int n = min(PAIRS, np - p0);
+    // B's largest at A's k, and A's at B's: a load per pair, side and slot
+#pragma unroll 1
+    for (int t = e; t < n * 2 * SLOTS; t += NE) {
+      const int q = t % SLOTS, side = t / SLOTS & 1, p = p0 + t / (2 * SLOTS), pb = p / na, pa = p - pb * na;
+      const Groups& s = side ? g.ga : g.gb;
+      const int gi = side ? pa : pb, k = min((int)sh.mx[side ? na + pb : pa] & KMASK, g.K - 1);
+      int v = 0;
+      if (q * s.stride < s.first_block(gi + 1) - s.first_block(gi)) v = s.part[(size_t)(gi * SLOTS + q) * Kp + k];
+      v = __reduce_max_sync(0xffffu << (threadIdx.x & 16), v);
+      if (q == 0) sh.seen[side][p - p0] = v;
+    }
+    epi_or(false);
+    if (e < n) {
+      const unsigned a = sh.mx[(p0 + e) % na], b = sh.mx[na + (p0 + e) / na];
+      const int ma = a >> WHERE, mb = b >> WHERE;
+      const bool at_a = (int)(a & KMASK) < KMASK && sh.seen[0][e] >= mb - APART;
+      const bool at_b = (int)(b & KMASK) < KMASK && sh.seen[1][e] >= ma - APART;
+      open = open || (ma > 0 && mb > 0 && !at_a && !at_b);
+    }
+    open = epi_or(open);
+  }
+  if (!open) return false;
+#pragma unroll 1
+  for (int p = 0; p < np; ++p) {
+    const int a = sh.mx[p % na] >> WHERE, b = sh.mx[na + p / na] >> WHERE, need = a + b - APART;
+    if (a == 0 || b == 0) continue;
+    const int sa = g.ga.slots(p % na), sb = g.gb.slots(p / na);
+    const short* pa = g.ga.part + (size_t)(p % na) * SLOTS * Kp;
+    const short* pb = g.gb.part + (size_t)(p / na) * SLOTS * Kp;
+    bool meet = false;
+    for (int k0 = 0; k0 < g.K && !meet; k0 += NE) {
+      const int k = k0 + e;
+      int x = 0, y = 0;
+#pragma unroll 4
+      for (int q = 0; q < SLOTS; ++q) {
+        if (k < g.K && q < sa) x = max(x, (int)pa[(size_t)q * Kp + k]);
+        if (k < g.K && q < sb) y = max(y, (int)pb[(size_t)q * Kp + k]);
+      }
+      meet = epi_or(x != 0 && y != 0 && x + y >= need);
+    }
+    if (!meet) return true;
+  }
+  return false;
 }
-// A CTA's units, should their tiles be left to fp64_unit: without a K split an
-// even share of all, else its own tile's for its K.  units_flagged: whether a
-// draining thread sees a flag in them; run_units: forms those that have one.
-struct Units { int u0, u1; };
-__device__ __forceinline__ Units my_units(const Args& g) {
-  const i64 n = (i64)g.mtiles * g.ntiles * 16;
-  return {(int)(n * blockIdx.x / gridDim.x), (int)(n * (blockIdx.x + 1) / gridDim.x)};
-}
-template <int BN>
-__device__ __noinline__ bool units_flagged(const Args& g) {
-  const Units w = my_units(g);
-  bool any = false;
-  for (int v = w.u0 / 16; v * 16 < w.u1; ++v)
-    any = any || flagged<BN>(g, v % g.mtiles, v / g.mtiles, threadIdx.x - 64);
-  return any;
-}
+
+// A CTA's units of a product for the chains: without a K split an even share of
+// all, else its own tile's for its K.
 template <int BN, bool PAIR>
 __device__ __noinline__ void run_units(const Args& g, unsigned char* base, bool fail) {
   const bool split = g.cs > 1;
@@ -429,16 +687,17 @@ __device__ __noinline__ void run_units(const Args& g, unsigned char* base, bool 
   static_assert(sizeof(longlong2) * BM * BN + sizeof(double) * E <= STAGES * stage_bytes(BN) &&
                     2 * sizeof(double) * E <= STAGES * stage_bytes(BN),
                 "the ring holds them");
-  const Units w = split ? Units{16 * own, 16 * own + 16} : my_units(g);
-  bool tile_flag = false;
-  for (int u = w.u0; u < w.u1; ++u) {
+  const i64 n = (i64)g.mtiles * g.ntiles * 16;
+  const int u0 = split ? 16 * own : (int)(n * blockIdx.x / gridDim.x);
+  const int u1 = split ? u0 + 16 : (int)(n * (blockIdx.x + 1) / gridDim.x);
+  for (int u = u0, area = 0; u < u1; ++u) {
     const int mt = u / 16 % g.mtiles, nt = u / 16 / g.mtiles;
-    if (u == w.u0 || u % 16 == 0) tile_flag = epi_or(flagged<BN>(g, mt, nt, threadIdx.x - 64));
-    if (!tile_flag) continue;
     const int rt = mt * 4 + (u & 3), ct = nt * 4 + (u >> 2 & 3);
-    if (g.cplx) fp64_unit<BN, PAIR, true>(g, rt, ct, k0, k1, fail, red + (split ? 0 : (u & 1) * E), o);
-    else if constexpr (!PAIR) fp64_unit<BN, false, false>(g, rt, ct, k0, k1, fail, red + (split ? 0 : (u & 1) * E), o);
+    if (rt * 32 >= g.M || ct * (BN / 4) >= g.N) continue;
+    if (g.cplx) fp64_unit<BN, PAIR, true>(g, rt, ct, k0, k1, fail, red + area * E, o);
+    else if constexpr (!PAIR) fp64_unit<BN, false, false>(g, rt, ct, k0, k1, fail, red + area * E, o);
     if (split) epi_or(false);                        // beside the cluster's sums there is one area
+    else area ^= 1;
   }
 }
 
@@ -456,8 +715,8 @@ __device__ __forceinline__ int small_int(float x) {
 // and keeps their two 64-bit sums in registers over the tile's drains.  Every
 // wait is bounded; a CTA whose wait ran out fills the outputs it has not
 // finished with NaN.  The outputs are scaled by 2^(ea + eb - 14): hi 2^-16 + lo 2^-48.
-// Tiles with a flagged row or column are left to fp64_unit, after the others and
-// dealt out over all CTAs.
+// While the first K steps run they look whether the product is one for the FP64
+// chains, which are then formed after it, dealt out over all CTAs.
 template <int BN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ Args g) {
   constexpr uint32_t B_BYTES = b_bytes(BN), STAGE = stage_bytes(BN);
@@ -468,7 +727,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
   __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int fail_s, fix_s;                     // a wait ran out; there are units for fp64_unit
+  __shared__ int fail_s, fix_s;                      // a wait ran out; the product is for the chains
+  __shared__ Check check_s;
   volatile int* fail = &fail_s;
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -484,6 +744,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
     fail_s = fix_s = 0;
     fence_mbar_init();
   }
+  for (int i = tid; i < (int)(sizeof(Check) / sizeof(int)); i += THREADS) reinterpret_cast<int*>(&check_s)[i] = 0;
   if (warp == 1) {
     tmem_alloc(smem_u32(&tmem_slot), TMEM);
     tmem_relinquish();
@@ -573,12 +834,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
     const uint32_t tb = taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
     int use = 0;
     bool ok = true;
-    if (g.cs == 1 && units_flagged<BN>(g)) fix_s = 1;
+    const bool chains = needs_chains(g, check_s);    // beside the first K steps
+    if (chains && tid == 64) fix_s = 1;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
       const int z = t % g.nz, rz = t / g.nz, mt = rz % g.mtiles, nt = rz / g.mtiles;
       const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
-      const bool fix = epi_or(flagged<BN>(g, mt, nt, tid - 64));
-      if (fix && g.cs > 1) fix_s = 1;
       long long hi[CB];                              // sum = hi 2^32 + lo, in 2^-48
       uint32_t lo[CB];
 #pragma unroll
@@ -624,7 +884,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
         }
       }
       const int row = mt * BM + q * 32 + lane, n0 = nt * BN + cb;
-      if (fix) continue;
+      if (chains) continue;
       if (g.cs > 1) {
         // the CTA's only tile: every copy has landed and every MMA has read it,
         // so the ring holds the sums for the cluster (after a failure fail_s counts)
@@ -844,7 +1104,35 @@ bool oz_fits(i64 M, i64 N, i64 K, bool cplx) {
   return b > 0 && b < kOzMaxBytes;
 }
 
-void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
+size_t oz_stat_bytes(i64 rows, i64 K, i64 groups, i64 kr) {
+  using namespace oz;
+  return al(sizeof(int4) * (size_t)(rows / SROWS + 2)) + al(sizeof(short) * SLOTS * (size_t)(K + 7) * groups) +
+         al(sizeof(short) * TPARTS * (size_t)kr);
+}
+static short* oz_tab(const OzGemm& g) {          // at the end of stat
+  const size_t b = oz_stat_bytes((i64)g.M + g.N, g.K, g.gnA + g.gnB, g.kr);
+  return (short*)((char*)g.stat + b - oz::al(sizeof(short) * oz::TPARTS * (size_t)g.kr));
+}
+static oz::Tables oz_tables(const OzGemm* const* later, int n, int* blocks) {
+  oz::Tables t{};
+  int m = 0;
+  *blocks = 0;
+  for (int i = 0; i < n; ++i)
+    if (later[i]->kr > 0) {
+      const OzGemm& g = *later[i];
+      t.t[m++] = {g.phi, oz_tab(g), (g.cplx ? 2 : 1) * g.inner, g.outer, g.kr};
+      *blocks += g.kr * oz::TPARTS;
+    }
+  return t;
+}
+
+// shared memory of the scales: of every k, then of the operator rank blocks
+constexpr size_t kScaleSmem = 200 * 1024;
+static size_t split_smem(const OzGemm& g) {
+  return sizeof(short) * ((size_t)(((g.cplx ? 2 * (i64)g.K : g.K) + 15) / 16 * (g.cplx ? 8 : 16)) + g.kr);
+}
+
+void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, cudaStream_t st) {
   using namespace oz;
   const Shape s = shape(g.M, g.N, g.K, g.cplx);
   TTG_REQUIRE(s.M < (1ll << 31) - BM && s.N < (1ll << 31) - 64 && s.K < (1ll << 30), "oz: size");
@@ -861,21 +1149,19 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
   auto vec = [&](const double* src, const OzMap& m, i64 sk) {
     return !g.cplx && sk == 1 && ((uintptr_t)src & 15) == 0 && (m.s1 & 1) == 0 && (m.s2 & 1) == 0;
   };
-  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? (s.dup_b ? 2 : 1) : 0, g.conjA};
-  const Side b{g.B, g.bn, g.bk, g.N, s.bn, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? (s.dup_b ? 1 : 2) : 0, g.conjB};
+  const short* tab = g.kr > 0 ? oz_tab(g) : nullptr;
+  int4* bm = (int4*)g.stat;
+  short* gpart = (short*)((char*)g.stat + al(sizeof(int4) * (size_t)(((i64)g.M + g.N) / SROWS + 2)));
+  auto stride = [](int gd) { return ((gd + SROWS - 1) / SROWS + 1 + SLOTS - 1) / SLOTS; };
+  const Groups gra{g.M, g.gdA, g.gnA, stride(g.gdA), bm, gpart};
+  const Groups grb{g.N, g.gdB, g.gnB, stride(g.gdB), bm + (g.M + SROWS - 1) / SROWS, gpart + (size_t)SLOTS * ((g.K + 7) & ~7) * g.gnA};
+  int tblocks = 0;
+  const Tables tables = oz_tables(later, nlater, &tblocks);
+  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? (s.dup_b ? 2 : 1) : 0, g.conjA,
+               tab, g.kd, g.kr, -g.norm, gra};
+  const Side b{g.B, g.bn, g.bk, g.N, s.bn, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? (s.dup_b ? 1 : 2) : 0, g.conjB,
+               tab, g.kd, g.kr, g.norm, grb};
   const int nA = (int)(ra / (a.cplx == 1 ? 2 : 1) / SROWS), nB = (int)(rb / (b.cplx == 1 ? 2 : 1) / SROWS);
-  // few rows and a long K: K over a cluster (246 + 82 rows, K = 4928: 50 -> 17 us)
-  int ky = 1;
-  while (ky < kMaxCluster && (nA + nB) * ky < 2 * SMS && 2 * s.kt > 32 * ky) ky *= 2;
-  launch_ex(split_kernel, dim3(nA + nB, ky), dim3(256), dim3(ky > 1 ? 1 : 0, ky, 1), true, 0, st, a, b,
-            nA, g.K, (int)s.kt);
-  Args x{};
-  x.Ad = Ad; x.Bd = Bd; x.ea = ea; x.eb = eb;
-  x.M = (int)s.M; x.N = (int)s.N; x.K = g.K;
-  x.kt = (int)s.kt; x.kper = z.kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.btile = s.bn; x.nz = nz; x.cs = z.cs;
-  x.C = g.C; x.cm = g.cm; x.cn = g.cn; x.part = part;
-  x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
-  x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
   static const cudaError_t attr_rc = [] {
     cudaError_t r = cudaSuccess;
     auto set = [&](auto* k, int bn) {
@@ -886,11 +1172,29 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
     set(gemm_kernel<64, true>, 64);
     set(gemm_kernel<32, false>, 32);
     set(gemm_kernel<32, true>, 32);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScaleSmem);
     return r;
   }();
   TTG_CUDA(attr_rc);
-  // (without a K split every SM gets a CTA: units for fp64_unit are dealt out to all)
-  const int grid = z.cs > 1 ? (int)(s.mt * s.nt * nz) : SMS;
+  // few rows and a long K: K over a cluster (246 + 82 rows, K = 4928: 50 -> 17 us)
+  int ky = 1;
+  while (ky < kMaxCluster && (nA + nB) * ky < 2 * SMS && 2 * s.kt > 32 * ky) ky *= 2;
+  launch_ex(split_kernel, dim3(nA + nB + tblocks, ky), dim3(256), dim3(ky > 1 ? 1 : 0, ky, 1), true,
+            g.kr > 0 ? split_smem(g) : 0, st, a, b, nA, nA + nB, tables, g.K, (int)s.kt);
+  Args x{};
+  x.Ad = Ad; x.Bd = Bd; x.ea = ea; x.eb = eb;
+  x.M = (int)s.M; x.N = (int)s.N; x.K = g.K;
+  x.kt = (int)s.kt; x.kper = z.kper; x.mtiles = (int)s.mt; x.ntiles = (int)s.nt; x.btile = s.bn; x.nz = nz; x.cs = z.cs;
+  x.C = g.C; x.cm = g.cm; x.cn = g.cn; x.part = part;
+  x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
+  x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
+  x.ga = gra; x.gb = grb;
+  // Without a K split every SM gets a CTA, for the chains' sake, unless K is so short
+  // that the CTAs without a tile would leave when the others let the next kernel in:
+  // its CTAs then crowd on the SMs that are free first (phi_left and phi_right, r =
+  // 37, n = 24: 68 us with the tiles' CTAs alone, 118 with all)
+  const int grid = z.cs > 1 ? (int)(s.mt * s.nt * nz) : (s.kt >= KCHUNK ? SMS : (int)std::min<i64>(SMS, s.mt * s.nt));
   auto kern = s.bn == 64 ? (s.dup_b ? gemm_kernel<64, true> : gemm_kernel<64, false>)
                          : (s.dup_b ? gemm_kernel<32, true> : gemm_kernel<32, false>);
   launch_ex(kern, dim3(grid), dim3(THREADS),
@@ -904,12 +1208,11 @@ void oz_gemm(const OzGemm& g, void* ws, cudaStream_t st) {
 // A strided batched product as one split product: a batch over which one
 // operand does not move joins the rows (or columns) of the other.  The side
 // that C stores contiguously becomes the MMA's M (a warp's TMEM lanes).
-// Returns false, with nothing launched, when the product does not have that
-// form, does not fit the workspace rule, or the FP64 kernel is the faster.
+// Returns false when the product does not have that form, does not fit the
+// workspace rule, or the FP64 kernel is the faster.
 template <class G>
-static bool oz_try_impl(const G& g, bool cplx, bool conjA, bool conjB, bool plain, void* ws,
-                        cudaStream_t s) {
-  if (!ws || !plain || g.M <= 0 || g.N <= 0 || g.K <= 0) return false;
+static bool oz_plan_impl(const G& g, const OzHint& h, bool cplx, bool conjA, bool conjB, bool plain, OzGemm* out) {
+  if (!plain || g.M <= 0 || g.N <= 0 || g.K <= 0) return false;
   i64 nb = (i64)g.nb1 * g.nb2, bA = g.bA1, bB = g.bB1, bC = g.bC1;
   if (g.nb1 == 1) {
     bA = g.bA2; bB = g.bB2; bC = g.bC2;
@@ -918,9 +1221,10 @@ static bool oz_try_impl(const G& g, bool cplx, bool conjA, bool conjB, bool plai
   }
   i64 M = g.M, N = g.N;
   OzMap am{g.M, g.sAm, 0}, cm{g.M, g.sCm, 0}, bn{g.N, g.sBn, 0}, cn{g.N, g.sCn, 0};
+  bool joinA = false, joinB = false;
   if (nb > 1) {
-    if (bB == 0) { am.s2 = bA; cm.s2 = bC; M *= nb; }
-    else if (bA == 0) { bn.s2 = bB; cn.s2 = bC; N *= nb; }
+    if (bB == 0) { am.s2 = bA; cm.s2 = bC; M *= nb; joinA = true; }
+    else if (bA == 0) { bn.s2 = bB; cn.s2 = bC; N *= nb; joinB = true; }
     else return false;
   }
   const bool swap = g.sCm != 1;
@@ -929,21 +1233,62 @@ static bool oz_try_impl(const G& g, bool cplx, bool conjA, bool conjB, bool plai
   const i64 Mo = swap ? N : M, No = swap ? M : N;
   if (!oz_fits(Mo, No, g.K, cplx)) return false;
   if (oz_us(Mo, No, g.K, cplx) >= gemm_fp64_us(g.M, g.N, g.K, (int)nb, cplx)) return false;
+  // groups: the operator rank blocks of one side, the vectors of the other
+  int gd[2] = {(int)M, (int)N}, gn[2] = {1, 1};
+  if (h.side != 0) {
+    const int t = h.side - 1;
+    const i64 rows = t == 0 ? M : N;
+    gn[t] = h.groups;
+    if (h.run > 0) {
+      TTG_REQUIRE(rows == (i64)h.run * h.groups, "oz: groups");
+      gd[t] = h.run;
+    } else {
+      // interleaved: rows taken block by block instead (not the side C stores
+      // contiguously, not a joined one)
+      TTG_REQUIRE(!(t == 0 ? joinA : joinB) && rows % h.groups == 0, "oz: groups");
+      OzMap& mo = t == 0 ? am : bn;
+      OzMap& mc = t == 0 ? cm : cn;
+      gd[t] = (int)(rows / h.groups);
+      mo = {gd[t], mo.s1 * h.groups, mo.s1};
+      mc = {gd[t], mc.s1 * h.groups, mc.s1};
+    }
+  }
+  const int vt = joinA ? 0 : 1;
+  const i64 per_vec = (vt == 0 ? M : N) / std::max(h.nvec, 1);
+  if (h.nvec > 1 && h.nvec <= kOzMaxVec && (joinA || joinB) && gn[vt] == 1 && per_vec >= 8) {
+    gn[vt] = h.nvec;
+    gd[vt] = (int)per_vec;
+  }
+  // a group's runs hold the start of a block of eight rows
+  if ((gn[0] > 1 && gd[0] < 8) || (gn[1] > 1 && gd[1] < 8) || gn[0] + gn[1] > 2 * kOzMaxGroups) return false;
+  const int a = swap ? 1 : 0, b = 1 - a;
   OzGemm o;
   o.M = (int)Mo; o.N = (int)No; o.K = g.K; o.cplx = cplx;
   o.A = (const double*)(swap ? g.B : g.A); o.am = swap ? bn : am; o.ak = swap ? g.sBk : g.sAk;
   o.B = (const double*)(swap ? g.A : g.B); o.bn = swap ? am : bn; o.bk = swap ? g.sAk : g.sBk;
   o.C = (double*)g.C; o.cm = swap ? cn : cm; o.cn = swap ? cm : cn;
   o.conjA = swap ? conjB : conjA; o.conjB = swap ? conjA : conjB;
-  oz_gemm(o, ws, s);
+  o.gdA = gd[a]; o.gnA = gn[a]; o.gdB = gd[b]; o.gnB = gn[b];
+  if (h.phi && h.kr <= kOzMaxTable) {
+    o.phi = h.phi; o.inner = h.inner; o.outer = h.outer; o.kr = h.kr; o.kd = h.kd;
+    o.norm = swap ? -h.norm : h.norm;
+    if (split_smem(o) > kScaleSmem) o.kr = 0;          // (K beyond 100 thousand)
+  }
+  *out = o;
   return true;
 }
-bool oz_try(const GemmF64& g, void* ws, cudaStream_t s) {
-  return oz_try_impl(g, false, false, false, g.alpha == 1.0 && g.beta == 0.0, ws, s);
+// tables that g itself needs (no earlier split product to form them)
+void oz_prepare(const OzGemm* const* g, int n, cudaStream_t s) {
+  int blocks = 0;
+  const oz::Tables t = oz_tables(g, n, &blocks);
+  if (blocks > 0) launch_pdl(oz::tables_kernel, dim3(blocks), dim3(256), 0, s, t);
 }
-bool oz_try(const GemmZ& g, void* ws, cudaStream_t s) {
+bool oz_plan(const GemmF64& g, const OzHint& h, OzGemm* out) {
+  return oz_plan_impl(g, h, false, false, false, g.alpha == 1.0 && g.beta == 0.0, out);
+}
+bool oz_plan(const GemmZ& g, const OzHint& h, OzGemm* out) {
   const bool plain = g.alpha.x == 1.0 && g.alpha.y == 0.0 && g.beta.x == 0.0 && g.beta.y == 0.0;
-  return oz_try_impl(g, true, g.conjA, g.conjB, plain, ws, s);
+  return oz_plan_impl(g, h, true, g.conjA, g.conjB, plain, out);
 }
 
 }  // namespace ttg
