@@ -67,6 +67,17 @@ using namespace ttg;
   }                                                       \
   return TTG_OK;
 
+// Scratch of a call in the context's workspace: `bound` bytes where it holds that
+// many already, else the `exact` need (a bound holds room for products that are too
+// large to be split, up to 4 GiB)
+template <class F>
+static void* call_scratch(ttg_ctx* c, size_t bound, F exact) {
+  c->ws.reset();
+  const size_t bytes = bound <= c->ws.cap ? bound : exact();
+  c->ws.reserve(bytes);
+  return c->ws.take(bytes);
+}
+
 extern "C" {
 
 int ttg_version(void) { return 10000; }
@@ -134,9 +145,8 @@ int ttg_dbfun3(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1, ttg
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1 && A && phi2 && x && y && nvec > 0, "null pointer or nvec <= 0");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  c->ws.reset();
-  c->ws.reserve(bfun3_f64_scratch(L, (int)nvec));
-  double* scr = c->ws.takeT<double>(bfun3_f64_scratch(L, (int)nvec) / sizeof(double));
+  double* scr = (double*)call_scratch(c, bfun3_f64_scratch(L, (int)nvec),
+                                      [&] { return bfun3_f64_call(L, (int)nvec, (int)nvec); });
   bfun3_f64(L, phi1, A, phi2, x, y, (int)nvec, scr, c->stream);
   TTG_API_END(c)
 }
@@ -148,10 +158,8 @@ int ttg_zbfun3(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1, ttg
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1 && A && phi2 && x && y && nvec > 0, "null pointer or nvec <= 0");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  size_t bytes = bfun3_z_scratch(L, (int)nvec);
-  c->ws.reset();
-  c->ws.reserve(bytes);
-  double2* scr = (double2*)c->ws.take(bytes);
+  double2* scr = (double2*)call_scratch(c, bfun3_z_scratch(L, (int)nvec),
+                                        [&] { return bfun3_z_call(L, (int)nvec, false); });
   bfun3_z(L, (const double2*)phi1, (const double2*)A, (const double2*)phi2, (const double2*)x,
           (double2*)y, (int)nvec, scr, c->stream);
   TTG_API_END(c)
@@ -165,10 +173,8 @@ int ttg_zbfun3_transp(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int r
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1 && A && phi2 && x && y && nvec > 0, "null pointer or nvec <= 0");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  size_t bytes = bfun3_z_scratch(L, (int)nvec);
-  c->ws.reset();
-  c->ws.reserve(bytes);
-  double2* scr = (double2*)c->ws.take(bytes);
+  double2* scr = (double2*)call_scratch(c, bfun3_z_scratch(L, (int)nvec),
+                                        [&] { return bfun3_z_call(L, (int)nvec, true); });
   bfun3_transp_z(L, (const double2*)phi1, (const double2*)A, (const double2*)phi2,
                  (const double2*)x, (double2*)y, (int)nvec, scr, c->stream);
   TTG_API_END(c)
@@ -181,9 +187,7 @@ int ttg_dphi_left(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1, 
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1_old && A && x && y && phi1_new, "null pointer");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  c->ws.reset();
-  c->ws.reserve(phi_f64_scratch(L));
-  double* scr = (double*)c->ws.take(phi_f64_scratch(L));
+  double* scr = (double*)call_scratch(c, phi_f64_scratch(L), [&] { return phi_f64_call(L, true); });
   phi_left_f64(L, phi1_old, A, x, y, phi1_new, scr, c->stream);
   TTG_API_END(c)
 }
@@ -195,9 +199,7 @@ int ttg_dphi_right(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1,
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi2_old && A && x && y && phi2_new, "null pointer");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  c->ws.reset();
-  c->ws.reserve(phi_f64_scratch(L));
-  double* scr = (double*)c->ws.take(phi_f64_scratch(L));
+  double* scr = (double*)call_scratch(c, phi_f64_scratch(L), [&] { return phi_f64_call(L, false); });
   phi_right_f64(L, phi2_old, A, x, y, phi2_new, scr, c->stream);
   TTG_API_END(c)
 }
@@ -209,9 +211,7 @@ int ttg_zphi_left(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1, 
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi1_old && A && x && y && phi1_new, "null pointer");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  c->ws.reset();
-  c->ws.reserve(phi_z_scratch(L));
-  double2* scr = (double2*)c->ws.take(phi_z_scratch(L));
+  double2* scr = (double2*)call_scratch(c, phi_z_scratch(L), [&] { return phi_z_call(L, true); });
   phi_left_z(L, (const double2*)phi1_old, (const double2*)A, (const double2*)x,
              (const double2*)y, (double2*)phi1_new, scr, c->stream);
   TTG_API_END(c)
@@ -224,9 +224,7 @@ int ttg_zphi_right(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx2, ttg_int ry1,
   check_dims(rx1, m, rx2, ry1, n, ry2, ra1, ra2);
   TTG_REQUIRE(phi2_old && A && x && y && phi2_new, "null pointer");
   LocalDims L{rx1, m, rx2, ry1, n, ry2, ra1, ra2};
-  c->ws.reset();
-  c->ws.reserve(phi_z_scratch(L));
-  double2* scr = (double2*)c->ws.take(phi_z_scratch(L));
+  double2* scr = (double2*)call_scratch(c, phi_z_scratch(L), [&] { return phi_z_call(L, false); });
   phi_right_z(L, (const double2*)phi2_old, (const double2*)A, (const double2*)x,
               (const double2*)y, (double2*)phi2_new, scr, c->stream);
   TTG_API_END(c)

@@ -364,6 +364,12 @@ void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const do
 size_t bfun3_f64_scratch(const LocalDims& L, int nvec);
 size_t bfun3_z_scratch(const LocalDims& L, int nvec);   // bfun3_z and bfun3_transp_z
 size_t phi_z_scratch(const LocalDims& L);
+// Bytes of one call of these sizes (bfun3_f64: of nvec_min to nvec vectors): no more
+// than the above, and less where a product stays on the FP64 kernels.
+size_t bfun3_f64_call(const LocalDims& L, int nvec_min, int nvec);
+size_t bfun3_z_call(const LocalDims& L, int nvec, bool transp);
+size_t phi_f64_call(const LocalDims& L, bool left);
+size_t phi_z_call(const LocalDims& L, bool left);
 
 void phi_left_f64(const LocalDims& L, const double* phi1_old, const double* A,
                   const double* x, const double* y, double* phi1_new, double* scratch,

@@ -672,12 +672,12 @@ extern "C" int ttg_local_eig(ttg_ctx* ctx, ttg_int r1, ttg_int n, ttg_int r2, tt
     const int maxb = (int)std::min<i64>(std::max<i64>(4 * B, 32), N);
     const bool jd = method != TTG_METHOD_PLAIN;
     const size_t split_bytes = method == TTG_METHOD_SPLIT ? split_matvec_bytes(L, (int)B) : 0;
-    size_t total = al(bfun3_f64_scratch(L, (int)B)) + al(Davidson::bytes(N, (int)B, maxb)) +
+    size_t total = al(bfun3_f64_call(L, 1, (int)B)) + al(Davidson::bytes(N, (int)B, maxb)) +
                    al(sizeof(double) * N * B) + al(split_bytes) + (1 << 16);
     if (jd) total += al(chosen_bytes(N, (int)B));
     DevBlock mem;
     mem.alloc(total);
-    double* bfs = (double*)mem.take<char>(bfun3_f64_scratch(L, (int)B));
+    double* bfs = (double*)mem.take<char>(bfun3_f64_call(L, 1, (int)B));
     void* dav_mem = mem.take<char>(Davidson::bytes(N, (int)B, maxb));
     double* X0 = mem.take<double>(N * B);
     void* split_mem = split_bytes ? (void*)mem.take<char>(split_bytes) : nullptr;

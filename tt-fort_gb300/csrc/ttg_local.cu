@@ -94,6 +94,20 @@ static void fp64_product(const GemmZ& g, cudaStream_t s) { gemm_z(g, s); }
 // hints name that rank where it is in K (the split products divide it out of both
 // factors) and where it is in the rows (each block's outputs have an accuracy of
 // their own).
+static size_t stat_of(const OzGemm& o) {
+  return oz_stat_bytes((i64)o.M + o.N, o.K, o.gnA + o.gnB, o.kr);
+}
+template <class G>
+static size_t products_bytes(const G* g, const OzHint* h, int n) {   // the workspace of just these
+  size_t stat = 0, planes = 0;
+  for (int i = 0; i < n; ++i) {
+    OzGemm o;
+    if (!oz_plan(g[i], h[i], &o)) continue;
+    stat += stat_of(o);
+    planes = std::max(planes, oz_bytes(o.M, o.N, o.K, o.cplx));
+  }
+  return stat + planes;
+}
 template <class G>
 static void run_products(const G* g, const OzHint* h, int n, void* ws, cudaStream_t s) {
   OzGemm o[kOzProducts];
@@ -105,7 +119,7 @@ static void run_products(const G* g, const OzHint* h, int n, void* ws, cudaStrea
     on[i] = ws && oz_plan(g[i], h[i], &o[i]);
     if (!on[i]) continue;
     o[i].stat = p;
-    p += oz_stat_bytes((i64)o[i].M + o[i].N, o[i].K, o[i].gnA + o[i].gnB, o[i].kr);
+    p += stat_of(o[i]);
     split[ns++] = &o[i];
   }
   // the first split product forms the others' scales
@@ -211,9 +225,14 @@ __global__ void __launch_bounds__(128) q_kernel(int m, int rx2, int n, int ry2, 
 // beside 46 us for each of the two large products).  Contracting the core into
 // Phi2 first costs K_Q times ra2 FMAs per row instead (11 us there) and makes
 // the first product n times larger.
-static bool bfun3_q(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
-                    const double* x, double* Q, double* T2, double* y, int nvec, void* ws,
-                    cudaStream_t s) {
+struct QRoute {
+  OzGemm g, o3;     // T2 = X Q, then the third product (on: as a split product)
+  GemmF64 g3;
+  bool on = false;
+  size_t stat() const { return stat_of(g) + (on ? stat_of(o3) : 0); }
+};
+static bool bfun3_q_plan(const LocalDims& L, const double* phi1, const double* x, double* Q,
+                         double* T2, double* y, int nvec, QRoute* q) {
   const i64 M = L.rx1 * nvec, N = L.n * L.ry2 * L.ra1, K = L.m * L.rx2;
   if (q_size(L, nvec) == 0 || !oz_fits(M, N, K, false)) return false;
   const double core = 2.0 * (double)(L.ra1 * L.n) * (double)(L.m * L.ra2) * (double)(L.ry2 * L.rx1) * nvec / 1.0e6;
@@ -223,7 +242,7 @@ static bool bfun3_q(const LocalDims& L, const double* phi1, const double* A, con
   const double build = 2.0 * (double)N * (double)K * (double)L.ra2 / 1.0e6 + 4.0;
   if (build + oz_us(M, N, K, false) >= general) return false;
   if (L.ra1 >= 65536 || L.n * L.m * L.ra2 > 4096) return false;   // grid and shared memory
-  OzGemm g;   // T2[b1,a1,i,c2,v] = sum_kq X_v[b1,kq] Q[(i,c2,a1),kq]
+  OzGemm& g = q->g;   // T2[b1,a1,i,c2,v] = sum_kq X_v[b1,kq] Q[(i,c2,a1),kq]
   g.M = (int)M; g.N = (int)N; g.K = (int)K;
   g.A = x; g.am = {(int)L.rx1, 1, L.xsize()}; g.ak = L.rx1;
   g.B = Q; g.bn = {(int)N, K, 0}; g.bk = 1;
@@ -232,26 +251,35 @@ static bool bfun3_q(const LocalDims& L, const double* phi1, const double* A, con
   if (nvec > 1 && nvec <= kOzMaxVec && L.rx1 >= 8) { g.gdA = (int)L.rx1; g.gnA = nvec; }
   else g.gdA = g.M;
   if ((L.ra1 > 1 && g.gdB < 8) || L.ra1 > kOzMaxGroups) return false;
-  GemmF64 g3;
   OzHint h3;
-  stage3(g3, h3, L, phi1, T2, y, nvec);
-  OzGemm o3;
-  const bool on = oz_plan(g3, h3, &o3);
-  const OzGemm* later = &o3;
-  char* p = (char*)ws;
-  g.stat = p;
-  p += oz_stat_bytes((i64)g.M + g.N, g.K, g.gnA + g.gnB, 0);
-  if (on) {
-    o3.stat = p;
-    p += oz_stat_bytes((i64)o3.M + o3.N, o3.K, o3.gnA + o3.gnB, o3.kr);
-  }
+  stage3(q->g3, h3, L, phi1, T2, y, nvec);
+  q->on = oz_plan(q->g3, h3, &q->o3);
+  return true;
+}
+static bool bfun3_q(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
+                    const double* x, double* Q, double* T2, double* y, int nvec, void* ws,
+                    cudaStream_t s) {
+  QRoute q;
+  if (!bfun3_q_plan(L, phi1, x, Q, T2, y, nvec, &q)) return false;
+  const OzGemm* later = &q.o3;
+  char* p = (char*)ws + q.stat();
+  q.g.stat = ws;
+  q.o3.stat = (char*)ws + stat_of(q.g);
   launch_pdl(q_kernel, dim3((unsigned)L.ry2, (unsigned)L.ra1), dim3(128),
              sizeof(double) * L.n * L.m * L.ra2, s, (int)L.m, (int)L.rx2, (int)L.n, (int)L.ry2,
              (int)L.ra1, (int)L.ra2, A, phi2, Q);
-  oz_gemm(g, p, &later, on ? 1 : 0, s);
-  if (on) oz_gemm(o3, p, nullptr, 0, s);
-  else gemm_f64(g3, s);
+  oz_gemm(q.g, p, &later, q.on ? 1 : 0, s);
+  if (q.on) oz_gemm(q.o3, p, nullptr, 0, s);
+  else gemm_f64(q.g3, s);
   return true;
+}
+
+template <class G, class T>
+static void bfun3_products(G* g, OzHint* h, const LocalDims& L, const T* phi1, const T* A, const T* phi2,
+                           const T* x, T* T1, T* T2, T* y, int nvec) {
+  stage1(g[0], h[0], L, x, phi2, T1, nvec);
+  stage2(g[1], h[1], L, A, T1, phi2, T2, nvec);
+  stage3(g[2], h[2], L, phi1, T2, y, nvec);
 }
 
 void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
@@ -263,9 +291,7 @@ void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const do
   if (ws && bfun3_q(L, phi1, A, phi2, x, T1, T2, y, nvec, ws, s)) return;
   GemmF64 g[3];
   OzHint h[3];
-  stage1(g[0], h[0], L, x, phi2, T1, nvec);
-  stage2(g[1], h[1], L, A, T1, phi2, T2, nvec);
-  stage3(g[2], h[2], L, phi1, T2, y, nvec);
+  bfun3_products(g, h, L, phi1, A, phi2, x, T1, T2, y, nvec);
   run_products(g, h, 3, ws, s);
 }
 
@@ -275,23 +301,17 @@ void bfun3_z(const LocalDims& L, const double2* phi1, const double2* A, const do
   double2* T2 = scratch + L.t1size() * nvec;
   GemmZ g[3];
   OzHint h[3];
-  stage1(g[0], h[0], L, x, phi2, T1, nvec);
-  stage2(g[1], h[1], L, A, T1, phi2, T2, nvec);
-  stage3(g[2], h[2], L, phi1, T2, y, nvec);
+  bfun3_products(g, h, L, phi1, A, phi2, x, T1, T2, y, nvec);
   run_products(g, h, 3, (char*)scratch + bfun3_z_t_bytes(L, nvec), s);
 }
 
 // Adjoint product (zbfun3_transp, ttals.f90:85-108): x has the y layout
 // (ry1, n, ry2), output y has the x layout (rx1, m, rx2); y = B^H x.
-void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
-                    const double2* phi2, const double2* x, double2* y, int nvec,
-                    double2* scratch, cudaStream_t s) {
+static void transp_products(GemmZ* gs, OzHint* h, const LocalDims& L, const double2* phi1,
+                            const double2* A, const double2* phi2, const double2* x, double2* R1,
+                            double2* R2, double2* y, int nvec) {
   const i64 p1 = L.rx1 * L.ra1 * L.n * L.ry2;     // R1[b1,a1,i,c2]
   const i64 p2 = L.rx1 * L.m * L.ra2 * L.ry2;     // R2[b1,j,a2,c2]
-  double2* R1 = scratch;
-  double2* R2 = scratch + p1 * nvec;
-  GemmZ gs[3];
-  OzHint h[3];
   {
     GemmZ& g = gs[0];   // R1[(b1,a1),(i,c2)] = sum_c1 conj(phi1[c1,(b1,a1)]) x[c1,(i,c2)]
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)(L.n * L.ry2); g.K = (int)L.ry1;
@@ -322,17 +342,22 @@ void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
     g.nb2 = nvec; g.bA2 = p2; g.bC2 = L.xsize();
     scale_by_phi2(h[2], L, phi2, -1, 1);
   }
-  for (OzHint& k : h) k.nvec = nvec;
-  run_products(gs, h, 3, (char*)scratch + bfun3_z_t_bytes(L, nvec), s);
+  for (int i = 0; i < 3; ++i) h[i].nvec = nvec;
+}
+void bfun3_transp_z(const LocalDims& L, const double2* phi1, const double2* A,
+                    const double2* phi2, const double2* x, double2* y, int nvec,
+                    double2* scratch, cudaStream_t s) {
+  GemmZ g[3];
+  OzHint h[3];
+  transp_products(g, h, L, phi1, A, phi2, x, scratch, scratch + L.rx1 * L.ra1 * L.n * L.ry2 * nvec, y, nvec);
+  run_products(g, h, 3, (char*)scratch + bfun3_z_t_bytes(L, nvec), s);
 }
 
 template <class G, class T>
-static void phi_right_impl(const LocalDims& L, const T* phi2_old, const T* A, const T* x,
-                           const T* y, T* phi2_new, T* scratch, bool conj_y, cudaStream_t s) {
+static void phi_right_products(G* gs, OzHint* h, const LocalDims& L, const T* phi2_old, const T* A, const T* x,
+                               const T* y, T* phi2_new, T* scratch) {
   T* T1 = scratch;
   T* T2 = scratch + L.t1size();
-  G gs[3];
-  OzHint h[3];
   stage1(gs[0], h[0], L, x, phi2_old, T1, 1);
   stage2(gs[1], h[1], L, A, T1, phi2_old, T2, 1);
   {
@@ -342,27 +367,24 @@ static void phi_right_impl(const LocalDims& L, const T* phi2_old, const T* A, co
     g.A = T2; g.sAm = 1; g.sAk = L.rx1 * L.ra1;
     g.B = y; g.sBk = L.ry1; g.sBn = 1;
     g.C = phi2_new; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
-    if constexpr (sizeof(T) == 16) g.conjB = conj_y;
+    if constexpr (sizeof(T) == 16) g.conjB = true;
     rows_of(h[2], 1, L.ra1, L.rx1);
   }
-  run_products(gs, h, 3, (char*)scratch + phi_t_bytes(L, sizeof(T)), s);
 }
 
 template <class G, class T>
-static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, const T* x,
-                          const T* y, T* phi1_new, T* scratch, bool conj_y, cudaStream_t s) {
+static void phi_left_products(G* gs, OzHint* h, const LocalDims& L, const T* phi1_old, const T* A, const T* x,
+                              const T* y, T* phi1_new, T* scratch) {
   const i64 psz = L.rx1 * L.ra1 * L.n * L.ry2;   // P[b1,a1,i,c2]
   T* P = scratch;
   T* Q = scratch + psz;                           // Q[b1,j,a2,c2]
-  G gs[3];
-  OzHint h[3];
   {
     G& g = gs[0];   // P[(b1,a1),(i,c2)] = sum_c1 phi1_old[c1,(b1,a1)] y[c1,(i,c2)]
     g.M = (int)(L.rx1 * L.ra1); g.N = (int)(L.n * L.ry2); g.K = (int)L.ry1;
     g.A = phi1_old; g.sAm = L.ry1; g.sAk = 1;
     g.B = y; g.sBk = 1; g.sBn = L.ry1;
     g.C = P; g.sCm = 1; g.sCn = L.rx1 * L.ra1;
-    if constexpr (sizeof(T) == 16) g.conjB = conj_y;
+    if constexpr (sizeof(T) == 16) g.conjB = true;
     rows_of(h[0], 1, L.ra1, L.rx1);
   }
   {
@@ -384,28 +406,75 @@ static void phi_left_impl(const LocalDims& L, const T* phi1_old, const T* A, con
     g.nb1 = (int)L.ra2; g.bA1 = L.rx1 * L.m; g.bC1 = L.ry2 * L.rx2;
     rows_of(h[2], 1, L.ra2, L.ry2);
   }
-  run_products(gs, h, 3, (char*)scratch + phi_t_bytes(L, sizeof(T)), s);
 }
+
+// an interface update (the complex ones conjugate y)
+template <class G, class T, class F>
+static void phi_update(F products, const LocalDims& L, const T* phi, const T* A, const T* x, const T* y,
+                       T* phi_new, T* scratch, cudaStream_t s) {
+  G g[3];
+  OzHint h[3];
+  products(g, h, L, phi, A, x, y, phi_new, scratch);
+  run_products(g, h, 3, (char*)scratch + phi_t_bytes(L, sizeof(T)), s);
+}
+
+// Scratch of one call of known sizes, in bytes: the split products that it takes
+// and no others (the functions above bound every call of a sweep, and so hold room
+// for products that are too large to be split, up to kOzMaxBytes).
+template <class T> static T* any_pointer() { return (T*)256; }   // the plans look at none
+size_t bfun3_f64_call(const LocalDims& L, int nvec_min, int nvec) {
+  size_t most = 0;
+  for (int nv = nvec_min; nv <= nvec; ++nv) {
+    double* p = any_pointer<double>();
+    QRoute q;
+    GemmF64 g[3];
+    OzHint h[3];
+    bfun3_products(g, h, L, p, p, p, p, p, p, p, nv);
+    size_t b = products_bytes(g, h, 3);
+    if (bfun3_q_plan(L, p, p, p, p, p, nv, &q))
+      b = q.stat() + std::max(oz_bytes(q.g.M, q.g.N, q.g.K, false), q.on ? oz_bytes(q.o3.M, q.o3.N, q.o3.K, false) : 0);
+    most = std::max(most, bfun3_t_bytes(L, nv) + b);
+  }
+  return most;
+}
+size_t bfun3_z_call(const LocalDims& L, int nvec, bool transp) {
+  double2* p = any_pointer<double2>();
+  GemmZ g[3];
+  OzHint h[3];
+  if (transp) transp_products(g, h, L, p, p, p, p, p, p, p, nvec);
+  else bfun3_products(g, h, L, p, p, p, p, p, p, p, nvec);
+  return bfun3_z_t_bytes(L, nvec) + products_bytes(g, h, 3);
+}
+template <class G, class T> static size_t phi_call(const LocalDims& L, bool left) {
+  T* p = any_pointer<T>();
+  G g[3];
+  OzHint h[3];
+  if (left) phi_left_products(g, h, L, p, p, p, p, p, p);
+  else phi_right_products(g, h, L, p, p, p, p, p, p);
+  return phi_t_bytes(L, sizeof(T)) + products_bytes(g, h, 3);
+}
+size_t phi_f64_call(const LocalDims& L, bool left) { return phi_call<GemmF64, double>(L, left); }
+size_t phi_z_call(const LocalDims& L, bool left) { return phi_call<GemmZ, double2>(L, left); }
 
 void phi_right_f64(const LocalDims& L, const double* phi2_old, const double* A,
                    const double* x, const double* y, double* phi2_new, double* scratch,
                    cudaStream_t s) {
-  phi_right_impl<GemmF64, double>(L, phi2_old, A, x, y, phi2_new, scratch, false, s);
+  phi_update<GemmF64>(phi_right_products<GemmF64, double>, L, phi2_old, A, x, y, phi2_new, scratch, s);
 }
 void phi_left_f64(const LocalDims& L, const double* phi1_old, const double* A,
                   const double* x, const double* y, double* phi1_new, double* scratch,
                   cudaStream_t s) {
-  phi_left_impl<GemmF64, double>(L, phi1_old, A, x, y, phi1_new, scratch, false, s);
+  phi_update<GemmF64>(phi_left_products<GemmF64, double>, L, phi1_old, A, x, y, phi1_new, scratch, s);
 }
 void phi_right_z(const LocalDims& L, const double2* phi2_old, const double2* A,
                  const double2* x, const double2* y, double2* phi2_new, double2* scratch,
                  cudaStream_t s) {
-  phi_right_impl<GemmZ, double2>(L, phi2_old, A, x, y, phi2_new, scratch, true, s);
+  phi_update<GemmZ>(phi_right_products<GemmZ, double2>, L, phi2_old, A, x, y, phi2_new, scratch, s);
 }
 void phi_left_z(const LocalDims& L, const double2* phi1_old, const double2* A,
                 const double2* x, const double2* y, double2* phi1_new, double2* scratch,
                 cudaStream_t s) {
-  phi_left_impl<GemmZ, double2>(L, phi1_old, A, x, y, phi1_new, scratch, true, s);
+  phi_update<GemmZ>(phi_left_products<GemmZ, double2>, L, phi1_old, A, x, y, phi1_new, scratch, s);
 }
 
 void phi2_left_f64(i64 rx1, i64 rx2, i64 ry1, i64 n, i64 ry2, const double* phi1_old,

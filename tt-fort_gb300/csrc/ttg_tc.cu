@@ -2135,7 +2135,7 @@ extern "C" int ttg_localop_create(ttg_ctx* c, ttg_int rx1, ttg_int m, ttg_int rx
     op->ctx = c; op->L = L; op->method = method; op->nvec_max = (int)nvec_max;
     op->phi1 = phi1; op->A = A; op->phi2 = phi2; op->mem = nullptr;
     size_t bytes = method == TTG_METHOD_SPLIT ? split_op_bytes(L, (int)nvec_max)
-                                              : bfun3_f64_scratch(L, (int)nvec_max);
+                                              : bfun3_f64_call(L, 1, (int)nvec_max);
     if (method == TTG_METHOD_SPLIT) TTG_REQUIRE(split_op_supported(L), "too large for split");
     TTG_CUDA(cudaMalloc(&op->mem, bytes));
     if (method == TTG_METHOD_SPLIT)
