@@ -270,7 +270,7 @@ int ttg_dqr(ttg_ctx* c, ttg_int n, ttg_int m, double* A, double* R) {
   TTG_REQUIRE(n > 0 && m > 0 && A && R, "bad arguments");
   TTG_REQUIRE(n < (1ll << 31) && m < (1ll << 31), "size too large");
   c->ws.reset();
-  const size_t work = qr_work_elems(n, m);
+  const size_t work = qr_call_elems(n, m, false);
   c->ws.reserve(sizeof(double) * work);
   double* tau = c->ws.takeT<double>(work);
   qr_householder((int)n, (int)m, A, R, tau, work, c->stream);
@@ -282,7 +282,7 @@ int ttg_zqr(ttg_ctx* c, ttg_int n, ttg_int m, double* A, double* R) {
   TTG_REQUIRE(n > 0 && m > 0 && A && R, "bad arguments");
   TTG_REQUIRE(n < (1ll << 31) && m < (1ll << 31), "size too large");
   c->ws.reset();
-  const size_t work = qr_work_elems(n, m);
+  const size_t work = qr_call_elems(n, m, true);
   c->ws.reserve(sizeof(double2) * work);
   double2* tau = c->ws.takeT<double2>(work);
   qr_householder_z((int)n, (int)m, (double2*)A, (double2*)R, tau, work, c->stream);

@@ -452,9 +452,11 @@ void syev_lowest_svd(int N, int k, double* H, double* w, double* V, double* scra
 void svd_jacobi(int p, int q, const double* M, double* U, double* sigma, double* Vt,
                 double* scratch, int* status, cudaStream_t s);
 // Householder QR with LAPACK's convention: A (n x m) -> Q (n x min), R (min x m).
-// tau: work elements, at least min(n, m); with qr_work_elems(n, m) of them large
-// blocks run over the whole GPU (ttg_qr.cu)
+// tau: work elements, at least min(n, m); with qr_work_elems(n, m) of them (for up to
+// m columns), or qr_call_elems(n, m) (for this block), large blocks run over the
+// whole GPU (ttg_qr.cu)
 size_t qr_work_elems(i64 n, i64 m, bool form_q = true);
+size_t qr_call_elems(i64 n, i64 m, bool cplx);
 void qr_householder(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s);
 void qr_householder_z(int n, int m, double2* A, double2* R, double2* tau, size_t work,
                       cudaStream_t s);

@@ -33,6 +33,7 @@
 #include "ttg_words.cuh"
 #include <algorithm>
 #include <array>
+#include <cstdint>
 
 namespace ttg {
 namespace qr {
@@ -554,12 +555,6 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
 
 }  // namespace qr
 
-// work of the grid form, in elements: tau, then two words' worth per value of
-// parts, sums and rows; the failure flag
-size_t qr_work_elems(i64 n, i64 m, bool form_q) {
-  return (size_t)std::min(n, m) + 32 + qr::grid_words<double>((int)n, (int)m, qr::NCMAX, form_q ? qr::NB : 0);
-}
-
 namespace {
 constexpr size_t kSmemMax = 220 * 1024;
 
@@ -678,6 +673,19 @@ bool run(int n, int m, T* A, T* R, T* tau, size_t work, cudaStream_t s) {
   return true;
 }
 }  // namespace
+
+// Work of the grid form, in elements: tau, then two words' worth per value of
+// parts, sums and rows; the failure flag.  For blocks of up to m columns (the rows
+// that a sweep's have are not known):
+size_t qr_work_elems(i64 n, i64 m, bool form_q) {
+  return (size_t)std::min(n, m) + 32 + qr::grid_words<double>((int)n, (int)m, qr::NCMAX, form_q ? qr::NB : 0);
+}
+// and for one block, with Q: of the form that it takes (8 rows of a million columns
+// take none of the grid's, whose words would be 1.3 GB)
+size_t qr_call_elems(i64 n, i64 m, bool cplx) {
+  const Pick p = cplx ? pick<double2>((int)n, (int)m, true, SIZE_MAX) : pick<double>((int)n, (int)m, true, SIZE_MAX);
+  return (size_t)std::min(n, m) + 32 + (p.grid ? qr::grid_words<double>((int)n, (int)m, p.G / p.CL, p.nb) : 0);
+}
 
 bool qr_rows(int n, int m, double* A, double* R, double* tau, size_t work, cudaStream_t s) {
   return run<double>(n, m, A, R, tau, work, s);
