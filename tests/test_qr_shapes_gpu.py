@@ -32,3 +32,38 @@ def test_no_words_for_a_wide_qr(torch_cuda, ctx, cplx):
     Q, R = a[:n * n].view(n, n).T, r.view(m, n).T
     err = torch_cuda.linalg.norm(Q @ R - a0.view(m, n).T) / torch_cuda.linalg.norm(a0)
     assert float(err) <= 10 * n * 2.0 ** -53
+
+
+def test_a_long_column_runs_over_the_gpu(torch_cuda, ctx):
+    """25600 x 1 holds the elements of 3200 x 8 and an eighth of its reflectors: it may
+    not take longer."""
+    import ttgpu
+    import time
+    best = {}
+    for n, m in ((25600, 1), (3200, 8)):
+        a0 = torch_cuda.randn(n * m, dtype=torch_cuda.float64, device="cuda")
+        a, r = a0.clone(), torch_cuda.zeros(m * m, dtype=torch_cuda.float64, device="cuda")
+        times = []
+        for _ in range(20):
+            a.copy_(a0)
+            torch_cuda.cuda.synchronize()
+            t0 = time.perf_counter()
+            ttgpu.dqr(n, m, a, r, ctx=ctx)
+            ctx.synchronize()
+            times.append(time.perf_counter() - t0)
+        best[m] = min(times)
+    assert best[1] <= 0.8 * best[8], best
+
+
+@pytest.mark.parametrize("n,m", [(25600, 1), (9001, 2), (7777, 3), (5000, 5), (4099, 7)])
+@pytest.mark.parametrize("cplx", [False, True])
+def test_thin_blocks(torch_cuda, ctx, n, m, cplx):
+    import ttgpu
+    dt = torch_cuda.complex128 if cplx else torch_cuda.float64
+    a0 = torch_cuda.randn(n * m, dtype=dt, device="cuda")
+    a, r = a0.clone(), torch_cuda.zeros(m * m, dtype=dt, device="cuda")
+    ttgpu.dqr(n, m, a, r, complex_=cplx, ctx=ctx)
+    ctx.synchronize()
+    A, Q, R = (t.view(m, -1).T.cpu().numpy() for t in (a0, a, r))
+    assert np.linalg.norm(Q @ R - A) <= 10 * m * 2.0 ** -53 * np.linalg.norm(A)
+    assert np.linalg.norm(Q.conj().T @ Q - np.eye(m)) <= 10 * m * 2.0 ** -53 * np.sqrt(m)

@@ -603,6 +603,7 @@ template <class T> int max_clusters(int CL) {
 
 template <class T>
 Pick pick(int n, int m, bool form_q, size_t work) {
+  using qr::NT;
   const double cx = sizeof(T) == 16 ? 4.0 : 1.0;
   const int r = std::min(n, m);
   // later columns of all columns, in the factorisation and in forming Q
@@ -624,7 +625,11 @@ Pick pick(int n, int m, bool form_q, size_t work) {
     if (!fits()) return;
     const double rows = (n + G - 1) / G;
     const double step = grid ? 4.2 + 0.12 * nc : (G == 1 ? 2.8 : 3.0);
-    const double t = 2.0 * cx * rows * cols / 3.2e3 + step * r + (nb ? (1.0 + 1.0 / nb) * step * r / nb : 0.0);
+    double t = 2.0 * cx * rows * cols / 3.2e3 + step * r + (nb ? (1.0 + 1.0 / nb) * step * r / nb : 0.0);
+    // fewer columns than warps: 32 threads a column in the factorisation, FT in
+    // forming Q, each a chain of dependent FMAs over its rows (25600 x 1 in one cluster
+    // 107 us, over the GPU 61; 12000 x 2 171 and 58)
+    if (m < NT / 32) t += rows * (0.004 * r + (nb ? 0.022 : 0.0)) * (sizeof(T) == 16 ? 2.0 : 1.0);
     if (t < bt) { bt = t; best = {G, CL, grid, nb}; }
   };
   for (int CL : {1, 2, 4, 8}) try_form(CL, 1);
