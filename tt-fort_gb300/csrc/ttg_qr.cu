@@ -27,7 +27,7 @@
 //                 part does.  One trip through L2 per column; handing all parts
 //                 to one CTA and its sum back took two (10.2k clocks of a step
 //                 of 5248 x 86, so 8.8k).  A cluster whose wait ran out fills
-//                 its rows with NaN.
+//                 its rows of Q and R with NaN, and tau.
 // Both add the parts in a fixed order, so results are bit-reproducible.
 #include "ttg_common.cuh"
 #include "ttg_words.cuh"
@@ -191,7 +191,13 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
   // the words and the shared-memory ranks follow CL
   if ((int)cl.num_blocks() != CL || (int)gridDim.x != G) {
     for (int c = warp; c < m; c += NT / 32)
-      for (int i = lane; i < nloc; i += 32) Ag[(i64)n * c + b + (i64)G * i] = O::nan();
+      for (int i = lane; i < nloc; i += 32) {
+        const int gi = b + G * i;
+        Ag[(i64)n * c + gi] = O::nan();
+        if (R && gi < r) R[gi + (i64)r * c] = O::nan();
+      }
+    if (b == 0)
+      for (int c = tid; c < r; c += NT) taug[c] = O::nan();
     return;
   }
 
@@ -437,7 +443,7 @@ __global__ void __launch_bounds__(NT) qr_rows_kernel(int n, int m, T* __restrict
       if (gi < r) R[gi + (i64)r * c] = fail ? O::nan() : (gi <= c ? A[(size_t)ld * c + i] : O::zero());
     }
   if (b == 0)
-    for (int c = tid; c < r; c += NT) taug[c] = tau[c];
+    for (int c = tid; c < r; c += NT) taug[c] = fail ? O::nan() : tau[c];
   __syncthreads();
 
   // Q in place, a panel of nb reflectors at a time from the last: column c of a
