@@ -194,8 +194,10 @@ __global__ void __launch_bounds__(AR_NT) arnoldi_kernel(i64 N, int j, int chunk,
         for (int k = 0; k < QL; ++k) {
           double v;
           if (lane + 32 * k < G) {
+            // (a part that did not come: NaN to every CTA, or the others would take the
+            // sum of the rest)
             if (words::take<double>(part + ((size_t)(lane + 32 * k) * AR_SLOTS + c) * 2, x[k], v, epoch, flag)) t += v;
-            else fail = 1;
+            else t = __longlong_as_double(0x7ff8000000000000ll);
           }
         }
         __syncwarp();

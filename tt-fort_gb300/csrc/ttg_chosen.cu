@@ -341,7 +341,9 @@ __global__ void __launch_bounds__(CT_NT) cg_tail_kernel(i64 N, int t, int nb,
 #pragma unroll
     for (int k = 0; k < QC; ++k) {
       double z;
-      if (lane + 32 * k < G && got(partC + ((size_t)(lane + 32 * k) * NC + v) * W, y[k], z)) sum += z;
+      // (a part that did not come: NaN to every CTA, or the others would take the sum of
+      // the rest)
+      if (lane + 32 * k < G) sum += got(partC + ((size_t)(lane + 32 * k) * NC + v) * W, y[k], z) ? z : nan;
     }
     __syncwarp();
     sum = warp_sum_d(sum);
