@@ -18,6 +18,7 @@
 #include "ttg_words.cuh"
 #include <cooperative_groups.h>
 #include <cfloat>
+#include <climits>
 #include <cstdlib>
 
 namespace cg = cooperative_groups;
@@ -468,7 +469,7 @@ __device__ __forceinline__ double warp_sum3(double a, double b, double g) {
 // products 720 (1840), sum and rotation 2340 (2690) -> 1770 (3060), columns
 // turned 890 (3030) -> 400 (1360), barrier 2790 (3940) -> 2790 (3320).
 constexpr int SVD_MG = 128;                       // threads on M; as many on V
-constexpr int SVD_LAG = 16;                       // pairs of a CTA in one round
+constexpr int SVD_LAG = 16;                       // pairs of a CTA whose V waits for the next round
 struct GridBar {                                  // arrivals count up; bounded wait
   unsigned int* c;
   unsigned int target;
@@ -501,6 +502,8 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_sweep64_kernel(int p, int q, d
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const bool on_m = tid < SVD_MG;
   const int K = (q + 1) & ~1, npairs = K / 2;
+  // more pairs a CTA than that: V is turned with M, by the same threads
+  const bool late = npairs <= (i64)gridDim.x * SVD_LAG;
   // V = I, unless the pre-sweeps already supplied the rotation
   if (!init_v)
     for (i64 e = blockIdx.x * (i64)blockDim.x + tid; e < (i64)q * q; e += (i64)gridDim.x * blockDim.x)
@@ -520,7 +523,7 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_sweep64_kernel(int p, int q, d
   };
   // V by the rotations of round last_r, held in slot par ^ 1
   auto turn_v = [&]() {
-    if (last_r < 0) return;
+    if (last_r < 0 || !late) return;
     for (int pi = blockIdx.x, k = 0; pi < npairs; pi += gridDim.x, ++k) {
       if (!act[par ^ 1][k]) continue;
       int a, b;
@@ -532,11 +535,11 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_sweep64_kernel(int p, int q, d
     int* cnt = counters + (sweep & 1), *top = counters + 4 + (sweep & 1);
     for (int r = 0; r < K - 1 && ok; ++r) {
       if (on_m) {
-        for (int pi = blockIdx.x, k = 0; pi < npairs; pi += gridDim.x, ++k) {
+        for (int pi = blockIdx.x, k = 0; pi < npairs; pi += gridDim.x, k += late) {
           int a, b;
           rr_pair(K, r, pi, a, b);
           if (a >= q || b >= q) {
-            if (tid == 0) act[par][k] = 0;
+            if (late && tid == 0) act[par][k] = 0;
             continue;
           }
           double* ca = M + (i64)p * a;
@@ -568,7 +571,11 @@ __global__ void __launch_bounds__(2 * SVD_MG) svd_sweep64_kernel(int p, int q, d
             }
           }
           asm volatile("bar.sync 1, %0;" ::"n"(SVD_MG) : "memory");
-          if (act[par][k]) turn(ca, cb, p, tid, rot[par][k][0], rot[par][k][1]);
+          if (act[par][k]) {
+            const double ps = rot[par][k][0], sn = rot[par][k][1];
+            turn(ca, cb, p, tid, ps, sn);
+            if (!late) turn(V + (i64)q * a, V + (i64)q * b, q, tid, ps, sn);
+          }
         }
         if (r == K - 2) seen.give(top);
       } else {
@@ -949,9 +956,16 @@ static void svd_sweeps(int p, int q, double* M, double* V, int* counters, int* s
   // two columns to a block where their rows fit registers and there are four
   // columns to a CTA (a resident grid of q / 4 CTAs always fits)
   const int kb = ((q + 1) / 2 + 1) & ~1;
+  // TTG_SVD_CTAS bounds the resident grid (the many pairs of a CTA of a block too
+  // wide for the GPU, on a small one)
+  static const int most = [] {
+    const char* v = std::getenv("TTG_SVD_CTAS");
+    const int n = v ? std::atoi(v) : 0;
+    return n > 0 ? n : INT_MAX;
+  }();
   if (p <= 8 * SVD_MG && q >= 4) {
     static const int max_block = coop_blocks((const void*)svd_block_kernel<8, false>, 2 * SVD_MG);
-    if (kb / 2 <= max_block) {
+    if (kb / 2 <= std::min(max_block, most)) {
       // Columns handed on as words up to 128 rows: 128 x 64 1864 -> 1717 us, 64 x
       // 24 690 -> 661, 320 x 128 (a 128 x 128 triangle) 4352 -> 4078; with
       // more rows a thread the words cost what the barrier did (256 x 160 6201 ->
@@ -966,9 +980,8 @@ static void svd_sweeps(int p, int q, double* M, double* V, int* counters, int* s
     }
   }
   static const int max_coop = coop_blocks((const void*)svd_sweep64_kernel, 2 * SVD_MG);
-  const int npairs = (q + 1) / 2, blocks = std::max(1, std::min(npairs, max_coop));
   TTG_REQUIRE(max_coop > 0, "svd: occupancy query failed");
-  TTG_REQUIRE(ceil_div(npairs, blocks) <= SVD_LAG, "svd: too many columns");
+  const int npairs = (q + 1) / 2, blocks = std::max(1, std::min(npairs, std::min(max_coop, most)));
   launch((const void*)svd_sweep64_kernel, blocks);
 }
 static void svd_sweeps32(int p, int q, float* M, float* V, int* counters, int* status, float tol,
