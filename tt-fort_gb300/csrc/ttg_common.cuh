@@ -324,7 +324,7 @@ struct OzHint {
   int nvec = 1;
 };
 constexpr int kOzProducts = 3;                   // products of a call
-constexpr int kOzMaxGroups = 256;               // of a side; more: FP64
+constexpr int kOzMaxGroups = 256;                // of a side; more: FP64
 constexpr int kOzMaxVec = 64;                    // more vectors: one group
 constexpr int kOzMaxTable = 4096;                // more operator rank blocks: no scales
 constexpr double kOzMinMNK = 2.0e6;              // below: never split
@@ -359,8 +359,9 @@ struct LocalDims {
 void bfun3_f64(const LocalDims& L, const double* phi1, const double* A, const double* phi2,
                const double* x, double* y, int nvec, double* scratch, cudaStream_t s,
                bool split = true);
-// Bytes; non-decreasing in every size, so a sweep may size for its largest
-// ranks and hand the same scratch to every smaller problem.
+// Bytes; non-decreasing in the ranks and vectors, so a sweep may size for its
+// largest ranks and hand the same scratch to every smaller problem of a site (not
+// in the modes: n m > 4 leaves out the spin chains' form).
 size_t bfun3_f64_scratch(const LocalDims& L, int nvec);
 size_t bfun3_z_scratch(const LocalDims& L, int nvec);   // bfun3_z and bfun3_transp_z
 size_t phi_z_scratch(const LocalDims& L);

@@ -21,7 +21,7 @@
 // row or column of a tile that is not part of C) and SMs without a tile.  So
 // the tiles are small (32 x 32, or 16 x 16 where those leave SMs idle), each
 // warp owns a block of its tile and skips it when it lies outside C, the K
-// loop stops at the K that is there (rounded up to 4), and launch_fp64 picks
+// loop stops at the K that is there (rounded up to 4), and pick_tile takes
 // the tile and the K split whose busiest SM has the least FP64 work.
 #include "ttg_common.cuh"
 

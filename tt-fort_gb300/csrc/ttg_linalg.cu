@@ -1454,7 +1454,7 @@ static inline int gbl(i64 n) { return (int)std::max<i64>(1, std::min<i64>(4096, 
 
 static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double* Vt,
                      double* V, double* nrm, int* rank, int* counters, int* status,
-                     double* tmp, cudaStream_t s, double* qrwork = nullptr);
+                     double* tmp, cudaStream_t s, double* qrwork);
 
 // The QR-preconditioned path (q >= SVD_QR_MIN_Q):
 //   M P = Q1 R1        columns sorted by norm, Householder QR
@@ -1467,7 +1467,7 @@ static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double*
 // 4.05 ms, 2048 x 512 35 -> 30.6 ms).
 static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, double* Vt,
                         double* V, double* nrm, int* rank, int* counters, int* status,
-                        double* tmp, double* work, cudaStream_t s) {
+                        double* work, cudaStream_t s) {
   const int npan = ceil_div(q, QRP_NB);
   double* A = work;                                     // p x q
   double* X = A + (size_t)p * q;                        // q x q: R1^T, then its QR
@@ -1513,9 +1513,8 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
       double* Ap = F + j0 + (i64)rows * j0;
       double* Tk = Tfac + (size_t)k * QRP_NB * QRP_NB;
       // panels of 1024+ rows on a grid of CTAs (rows split, two grid
-      // barriers per column); narrower ones in one CTA (grids from 256 rows,
-      // one CTA per 32 or 64 rows, measured no faster on GB300: 7.8 against
-      // 7.55 ms for the 320 x 128 truncation)
+      // barriers per column); shorter ones, the last of a square block, in one
+      // CTA (grids from 256 rows, one CTA per 32 or 64 rows, were no faster)
       if (m >= 1024) {
         static const int coop_max = [] {
           int dev = 0, nsm = 0, per = 0;
@@ -1571,7 +1570,6 @@ static void svd_tall_qr(int p, int q, double* Mw, double* U, double* sigma, doub
   permute_cols_kernel<<<gbl((i64)p * q), 256, 0, s>>>(p, q, Mw, perm, A);
   TTG_CHECK_LAUNCH();
   qr_factor(p, A, Tf, tau);                             // M P = Q1 R1
-  (void)tmp;
   rt_kernel<<<gbl((i64)q * q), 256, 0, s>>>(q, A, p, X);   // X = R1^T
   TTG_CHECK_LAUNCH();
   qr_factor(q, X, Tf2, tau2);                                // R1^T = Q2 R2
@@ -1605,8 +1603,8 @@ static void svd_tall(int p, int q, double* Mw, double* U, double* sigma, double*
                      double* V, double* nrm, int* rank, int* counters, int* status,
                      double* tmp, cudaStream_t s, double* qrwork) {
   // Mw (p x q, p >= q) is overwritten.  tmp: 2 q^2 + p q doubles.
-  if (qrwork && q >= SVD_QR_MIN_Q) {
-    svd_tall_qr(p, q, Mw, U, sigma, Vt, V, nrm, rank, counters, status, tmp, qrwork, s);
+  if (q >= SVD_QR_MIN_Q) {
+    svd_tall_qr(p, q, Mw, U, sigma, Vt, V, nrm, rank, counters, status, qrwork, s);
     return;
   }
   int init_v = 0;
@@ -1706,7 +1704,7 @@ void svd_jacobi(int p, int q, const double* M, double* U, double* sigma, double*
 // ---------------------------------------------------------------------------
 // Householder QR, LAPACK reflector convention (real and complex): ttg_qr.cu,
 // and here one CTA on global memory for the blocks that do not fit shared
-// memory there (above ~28 MB, or callers that bring no workspace for it)
+// memory there (above ~25 MB, or callers that bring no workspace for it)
 // ---------------------------------------------------------------------------
 template <class T> struct CT;
 template <> struct CT<double> {

@@ -51,10 +51,10 @@
 // fill, one drain, rounding); oz_us below holds both.
 //
 // Tensor memory: a 128 x 64 tile (128 x 32 for small products) with its seven
-// groups side by side (448 of the 512 columns).  The digit planes of B sit stacked along N, so the MMA of
-// A's plane p with B's planes 0..6-p writes groups p..6 in one instruction
-// (two where N > 256): ten instructions per 16-wide K step, and A's planes are
-// read from shared memory once per step.
+// groups side by side (448 of the 512 columns).  The digit planes of B sit
+// stacked along N, so the MMA of A's plane p with B's planes 0..6-p writes groups
+// p..6 in one instruction (two where N > 256): ten instructions per 16-wide K
+// step, and A's planes are read from shared memory once per step.
 #include "ttg_common.cuh"
 #include "ttg_tcgen05.cuh"
 #include <algorithm>
@@ -99,7 +99,6 @@ struct Side {                   // one operand, element (r, k) = src[map(r) + k 
   OzMap map;
   i64 sk;
   int rows, R;                  // logical rows; rows of a tile (BM or BN)
-  int rtiles;
   unsigned char* planes;        // [rtile][K step][plane][R x 16 bf16, core matrices]
   int* expo;                    // per split row
   int vec;                      // real with sk == 1 and 16-byte aligned rows
@@ -1157,9 +1156,9 @@ void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, 
   const Groups grb{g.N, g.gdB, g.gnB, stride(g.gdB), bm + (g.M + SROWS - 1) / SROWS, gpart + (size_t)SLOTS * ((g.K + 7) & ~7) * g.gnA};
   int tblocks = 0;
   const Tables tables = oz_tables(later, nlater, &tblocks);
-  const Side a{g.A, g.am, g.ak, g.M, BM, (int)s.mt, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? (s.dup_b ? 2 : 1) : 0, g.conjA,
+  const Side a{g.A, g.am, g.ak, g.M, BM, Ad, ea, vec(g.A, g.am, g.ak), g.cplx ? (s.dup_b ? 2 : 1) : 0, g.conjA,
                tab, g.kd, g.kr, -g.norm, gra};
-  const Side b{g.B, g.bn, g.bk, g.N, s.bn, (int)s.nt, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? (s.dup_b ? 1 : 2) : 0, g.conjB,
+  const Side b{g.B, g.bn, g.bk, g.N, s.bn, Bd, eb, vec(g.B, g.bn, g.bk), g.cplx ? (s.dup_b ? 1 : 2) : 0, g.conjB,
                tab, g.kd, g.kr, g.norm, grb};
   const int nA = (int)(ra / (a.cplx == 1 ? 2 : 1) / SROWS), nB = (int)(rb / (b.cplx == 1 ? 2 : 1) / SROWS);
   static const cudaError_t attr_rc = [] {

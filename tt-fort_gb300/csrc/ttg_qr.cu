@@ -50,7 +50,6 @@ template <> struct C<double> {
   static __device__ __forceinline__ double fma(double a, double b, double c) { return ::fma(a, b, c); }
   static __device__ __forceinline__ bool is_zero(double a) { return a == 0.0; }
   static __device__ __forceinline__ double shfl(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
-  static __device__ __forceinline__ double ldcg(const double* p) { return __ldcg(p); }
   // reflector of (alpha, ||x||^2): beta, tau, scale of x (0 0 for none)
   static __device__ __forceinline__ void reflect(double alpha, double x2, double& beta, double& tau,
                                                  double& sc) {
@@ -92,7 +91,6 @@ template <> struct C<double2> {
     v.y = __shfl_xor_sync(0xffffffffu, v.y, o);
     return v;
   }
-  static __device__ __forceinline__ double2 ldcg(const double2* p) { return __ldcg(p); }
   static __device__ __forceinline__ void reflect(double2 alpha, double x2, double2& beta, double2& tau,
                                                  double2& sc) {
     if (x2 == 0.0 && alpha.y == 0.0) {
