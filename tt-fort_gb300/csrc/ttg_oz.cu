@@ -42,10 +42,10 @@
 // chains, so infinities, NaN and extreme ranges give what they give there.
 //
 // Measured on GB300, FP64 kernels -> split products: chain product r=256, block
-// of 8: 4560 -> 248 us (22 TFLOP/s of FP64 accuracy; its two products run at
-// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 38.2
-// us; grid interface updates r = 82, 77, n = 64: 1908 -> 180 us; complex
-// operator and adjoint r=48, n=32, block of 4: 6968 -> 383 us (without scales and
+// of 8: 4560 -> 251 us (22 TFLOP/s of FP64 accuracy; its two products run at
+// 46 and 44 TFLOP/s, i.e. 1.3 PFLOP/s of BF16); r=64, block of 5: 76.6 -> 36.0
+// us; grid interface updates r = 82, 77, n = 64: 1908 -> 179 us; complex
+// operator and adjoint r=48, n=32, block of 4: 6968 -> 384 us (without scales and
 // check 241, 32.8, 160 and 351).  What bounds the product kernel is the operand traffic (43 KB a K step per SM, 1.4k clocks
 // measured against 900 of MMA), for small ones its fixed ~10 us (pipeline
 // fill, one drain, rounding); oz_us below holds both.
@@ -94,6 +94,7 @@ struct Groups {
     return (first_block(group + 1) - first_block(group) + stride - 1) / stride;
   }
 };
+enum { UNKNOWN = 0, FINE = 1, CHAINS = 2 };
 struct Side {                   // one operand, element (r, k) = src[map(r) + k * sk]
   const double* src;
   OzMap map;
@@ -122,6 +123,9 @@ struct Args {
   OzMap am, bn;
   i64 ak, bk;
   Groups ga, gb;
+  int* state;                   // of the check: UNKNOWN, FINE, CHAINS
+  int rows, cols;               // logical rows and columns
+  int look;                     // CTA 0 of the product kernel makes it
   int cplx, conjA, conjB;       // complex: product rows (PAIR: columns) are (re, im)
 };
 
@@ -199,7 +203,7 @@ __global__ void __launch_bounds__(256) tables_kernel(Tables t) {
 // fetching counts (with a copy for each operand the kernel took 4 us more).
 __global__ void __launch_bounds__(256, 3) split_kernel(const __grid_constant__ Side a, const __grid_constant__ Side b,
                                                        int nblkA, int nblk, const __grid_constant__ Tables tabs,
-                                                       int K, int kt) {
+                                                       int K, int kt, int* state) {
   namespace cgr = cooperative_groups;
   cgr::cluster_group cl = cgr::this_cluster();
   __shared__ int key_s[SROWS], scaled_s;
@@ -209,6 +213,7 @@ __global__ void __launch_bounds__(256, 3) split_kernel(const __grid_constant__ S
     if (blockIdx.y == 0) table_block(tabs, blockIdx.x - nblk);
     return;
   }
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *state = UNKNOWN;
   const bool isA = (int)blockIdx.x < nblkA;
   const Side& S = isA ? a : b;
   const int blk = isA ? blockIdx.x : blockIdx.x - nblkA;
@@ -489,8 +494,9 @@ __device__ __forceinline__ i64 c_col(const Args& g, int n) {
   return at(g.cn, n) * (g.cplx ? 2 : 1);
 }
 
-// whether any draining thread says so (all of them call it)
-__device__ __forceinline__ bool epi_or(bool v) {
+// whether any of 512 threads (the draining ones, or all of check_kernel) says so; all
+// of them call it
+__device__ __forceinline__ bool any_of_512(bool v) {
   uint32_t r;
   asm volatile(
       "{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n barrier.cta.red.or.pred p, 1, %2, q;\n"
@@ -501,96 +507,12 @@ __device__ __forceinline__ bool epi_or(bool v) {
   return r != 0;
 }
 
-// FP64 FMA chains of a unit, 32 rows x BN / 4 columns (a sixteenth of a tile),
-// over logical K [kbeg, kend): the 16 draining warps take every 16th k, a lane
-// rows ly + 4 i and columns lx + 8 j, and the warps' sums are added in order from
-// red.  To C, or (over clusters) to o, the sums' place in shared memory.  Bound
-// by the FP64 pipe, as gemm_kernel of ttg_gemm.cu is: a load serves two to eight
-// FMAs of 64 clocks each.  Units this small, and K over the warps, because a
-// product of 80 tiles would leave half of the SMs idle if each kept its own
-// (phi_left, r = 256, n = 2, an infinity in Phi: 1124 us so, 720 in units).  One
-// thread per flagged output took 1472 us there and 2436 us at r = 82, n = 64 (now
-// 1162); the FP64 kernels take 777 and 1426.
-template <int BN, bool PAIR, bool CPLX>
-__device__ __noinline__ void fp64_unit(const Args& g, int rt, int ct, int kbeg, int kend, bool fail,
-                                       double* red, longlong2* o) {
-  constexpr int NI = 8, NJ = BN / 32, E = 32 * NI * NJ;
-  using T = typename std::conditional<CPLX, double2, double>::type;
-  const int e = threadIdx.x - 64, warp = e >> 5, lane = e & 31, ly = lane >> 3, lx = lane & 7;
-  const int r0 = rt * 32, c0 = ct * (BN / 4);
-  const T *a[NI], *b[NJ];
-#pragma unroll
-  for (int i = 0; i < NI; ++i) {
-    const int r = min(r0 + ly + 4 * i, g.M - 1);
-    a[i] = reinterpret_cast<const T*>(g.A) + at(g.am, CPLX && !PAIR ? r >> 1 : r) + (i64)(kbeg + warp) * g.ak;
-  }
-#pragma unroll
-  for (int j = 0; j < NJ; ++j) {
-    const int n = min(c0 + lx + 8 * j, g.N - 1);
-    b[j] = reinterpret_cast<const T*>(g.B) + at(g.bn, CPLX && PAIR ? n >> 1 : n) + (i64)(kbeg + warp) * g.bk;
-  }
-  double acc[NI][NJ];
-#pragma unroll
-  for (int i = 0; i < NI; ++i)
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) acc[i][j] = 0.0;
-  const bool im = ((PAIR ? lx : ly) & 1) != 0;       // the imaginary part's row or column
-  T x[NI], y[NJ];
-  auto load = [&] {
-#pragma unroll
-    for (int i = 0; i < NI; ++i) {
-      x[i] = *a[i];
-      a[i] += EPI_WARPS * g.ak;
-    }
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) {
-      y[j] = *b[j];
-      b[j] += EPI_WARPS * g.bk;
-    }
-  };
-  constexpr bool AHEAD = !CPLX;                      // (complex: four times the FMAs per load)
-  if (AHEAD && kbeg + warp < kend) load();
-  for (int k = kbeg + warp; k < kend; k += EPI_WARPS) {
-    if (!AHEAD) load();
-    T u[NI], v[NJ];
-#pragma unroll
-    for (int i = 0; i < NI; ++i) u[i] = x[i];
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) v[j] = y[j];
-    if (AHEAD && k + EPI_WARPS < kend) load();
-#pragma unroll
-    for (int i = 0; i < NI; ++i)
-#pragma unroll
-      for (int j = 0; j < NJ; ++j) {
-        if constexpr (CPLX) {
-          const double ui = g.conjA ? -u[i].y : u[i].y, vi = g.conjB ? -v[j].y : v[j].y;
-          acc[i][j] = fma(u[i].x, im ? vi : v[j].x, acc[i][j]);
-          acc[i][j] = fma(ui, im ? v[j].x : -vi, acc[i][j]);
-        } else {
-          acc[i][j] = fma(u[i], v[j], acc[i][j]);
-        }
-      }
-  }
-#pragma unroll
-  for (int i = 0; i < NI; ++i)
-#pragma unroll
-    for (int j = 0; j < NJ; ++j) red[warp * E + (i * NJ + j) * 32 + lane] = acc[i][j];
-  epi_or(false);
-  if (e < E) {
-    double v = red[e];
-    for (int w = 1; w < EPI_WARPS; ++w) v += red[w * E + e];
-    if (fail) v = __longlong_as_double(0x7ff8000000000000ll);
-    const int r = r0 + ly + 4 * ((e >> 5) / NJ), n = c0 + lx + 8 * ((e >> 5) % NJ);
-    if (o) o[(n & (BN - 1)) * BM + (r & (BM - 1))] = make_longlong2(__double_as_longlong(v), 0);
-    else if (r < g.M && n < g.N) g.C[c_row<PAIR>(g, r) + c_col<PAIR>(g, n)] = v;
-  }
-}
-
 // Whether a product is one for the FP64 chains: a row is flagged, or the large
 // elements of the operands do not meet.  For every group of A's rows and of B's
 // columns, 2^APART times some k's product of largest elements must reach the product
 // of the groups' largest (either 0: nothing to reach).  Looked for where one of
-// them has its largest, then everywhere.  Draining threads.
+// them has its largest, then everywhere.  Thread e of 512; global memory is read past
+// L1 (check_kernel looks before it waits for the kernels in front of it).
 constexpr int APART = 3;
 constexpr int PAIRS = 128;                        // pairs of groups looked at together
 constexpr int WHERE = 18;                         // bits of a largest element's k (beyond: not looked for there)
@@ -598,9 +520,9 @@ struct Check {                                    // shared memory, zero at firs
   unsigned int mx[2 * kOzMaxGroups];              // A's groups, then B's: largest, its k
   int seen[2][PAIRS];                             // the other side's largest there
 };
-__device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
+__device__ __noinline__ bool needs_chains(const Args& g, Check& sh, int e) {
   constexpr int NE = 32 * EPI_WARPS, KMASK = (1 << WHERE) - 1;
-  const int e = threadIdx.x - 64, na = g.ga.gn, np = na * g.gb.gn, Kp = (g.K + 7) & ~7;
+  const int na = g.ga.gn, np = na * g.gb.gn, Kp = (g.K + 7) & ~7;
   bool bad = false;
 #pragma unroll 1
   for (int side = 0; side < 2; ++side) {
@@ -608,7 +530,7 @@ __device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
     unsigned int* m = sh.mx + (side ? na : 0);
     const int n = (s.rows + SROWS - 1) / SROWS;
     for (int b = e; b - (e & 31) < n; b += NE) {
-      const int4 v = b < n ? s.bm[b] : make_int4(0, 0, 0, 0);
+      const int4 v = b < n ? __ldcg(s.bm + b) : make_int4(0, 0, 0, 0);
       bad = bad || v.x == FLAGGED;
       const int group = s.gn == 1 ? 0 : min(b, n - 1) * SROWS / s.gd;
       const unsigned x = v.x > 0 ? (unsigned)(v.x & 0x3fff) << WHERE | min(v.y, KMASK) : 0u;
@@ -623,7 +545,7 @@ __device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
       if (v.z > 0) atomicMax(&m[group + 1], (unsigned)v.z << WHERE | min(v.w, KMASK));
     }
   }
-  if (epi_or(bad)) return true;
+  if (any_of_512(bad)) return true;
   bool open = false;
   for (int p0 = 0; p0 < np; p0 += PAIRS) {
     const int n = min(PAIRS, np - p0);
@@ -634,11 +556,11 @@ __device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
       const Groups& s = side ? g.ga : g.gb;
       const int gi = side ? pa : pb, k = min((int)sh.mx[side ? na + pb : pa] & KMASK, g.K - 1);
       int v = 0;
-      if (q * s.stride < s.first_block(gi + 1) - s.first_block(gi)) v = s.part[(size_t)(gi * SLOTS + q) * Kp + k];
-      v = __reduce_max_sync(0xffffu << (threadIdx.x & 16), v);
+      if (q * s.stride < s.first_block(gi + 1) - s.first_block(gi)) v = __ldcg(s.part + (size_t)(gi * SLOTS + q) * Kp + k);
+      v = __reduce_max_sync(0xffffu << (e & 16), v);
       if (q == 0) sh.seen[side][p - p0] = v;
     }
-    epi_or(false);
+    any_of_512(false);
     if (e < n) {
       const unsigned a = sh.mx[(p0 + e) % na], b = sh.mx[na + (p0 + e) / na];
       const int ma = a >> WHERE, mb = b >> WHERE;
@@ -646,7 +568,7 @@ __device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
       const bool at_b = (int)(b & KMASK) < KMASK && sh.seen[1][e] >= ma - APART;
       open = open || (ma > 0 && mb > 0 && !at_a && !at_b);
     }
-    open = epi_or(open);
+    open = any_of_512(open);
   }
   if (!open) return false;
 #pragma unroll 1
@@ -662,42 +584,14 @@ __device__ __noinline__ bool needs_chains(const Args& g, Check& sh) {
       int x = 0, y = 0;
 #pragma unroll 4
       for (int q = 0; q < SLOTS; ++q) {
-        if (k < g.K && q < sa) x = max(x, (int)pa[(size_t)q * Kp + k]);
-        if (k < g.K && q < sb) y = max(y, (int)pb[(size_t)q * Kp + k]);
+        if (k < g.K && q < sa) x = max(x, (int)__ldcg(pa + (size_t)q * Kp + k));
+        if (k < g.K && q < sb) y = max(y, (int)__ldcg(pb + (size_t)q * Kp + k));
       }
-      meet = epi_or(x != 0 && y != 0 && x + y >= need);
+      meet = any_of_512(x != 0 && y != 0 && x + y >= need);
     }
     if (!meet) return true;
   }
   return false;
-}
-
-// A CTA's units of a product for the chains: without a K split an even share of
-// all, else its own tile's for its K.
-template <int BN, bool PAIR>
-__device__ __noinline__ void run_units(const Args& g, unsigned char* base, bool fail) {
-  const bool split = g.cs > 1;
-  const int z = split ? (int)blockIdx.x % g.nz : 0, own = (int)blockIdx.x / g.nz;
-  const int per = g.cplx ? 8 : 16, k0 = z * g.kper * per, k1 = min(g.K, k0 + g.kper * per);
-  longlong2* o = split ? reinterpret_cast<longlong2*>(base) : nullptr;
-  constexpr int E = EPI_WARPS * 8 * BN;
-  // the warps' sums of a unit: two areas in turn, so that one barrier a unit is enough
-  double* red = reinterpret_cast<double*>(base + (split ? sizeof(longlong2) * BM * BN : 0));
-  static_assert(sizeof(longlong2) * BM * BN + sizeof(double) * E <= STAGES * stage_bytes(BN) &&
-                    2 * sizeof(double) * E <= STAGES * stage_bytes(BN),
-                "the ring holds them");
-  const i64 n = (i64)g.mtiles * g.ntiles * 16;
-  const int u0 = split ? 16 * own : (int)(n * blockIdx.x / gridDim.x);
-  const int u1 = split ? u0 + 16 : (int)(n * (blockIdx.x + 1) / gridDim.x);
-  for (int u = u0, area = 0; u < u1; ++u) {
-    const int mt = u / 16 % g.mtiles, nt = u / 16 / g.mtiles;
-    const int rt = mt * 4 + (u & 3), ct = nt * 4 + (u >> 2 & 3);
-    if (rt * 32 >= g.M || ct * (BN / 4) >= g.N) continue;
-    if (g.cplx) fp64_unit<BN, PAIR, true>(g, rt, ct, k0, k1, fail, red + area * E, o);
-    else if constexpr (!PAIR) fp64_unit<BN, false, false>(g, rt, ct, k0, k1, fail, red + area * E, o);
-    if (split) epi_or(false);                        // beside the cluster's sums there is one area
-    else area ^= 1;
-  }
 }
 
 constexpr int kMaxSplit = kMaxCluster;            // CTAs of a cluster that share a tile
@@ -714,8 +608,8 @@ __device__ __forceinline__ int small_int(float x) {
 // and keeps their two 64-bit sums in registers over the tile's drains.  Every
 // wait is bounded; a CTA whose wait ran out fills the outputs it has not
 // finished with NaN.  The outputs are scaled by 2^(ea + eb - 14): hi 2^-16 + lo 2^-48.
-// While the first K steps run they look whether the product is one for the FP64
-// chains, which are then formed after it, dealt out over all CTAs.
+// In CTA 0 they look first, while the first K steps run, whether the product is one
+// for the FP64 chains (g.look; check_kernel does otherwise).
 template <int BN, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant__ Args g) {
   constexpr uint32_t B_BYTES = b_bytes(BN), STAGE = stage_bytes(BN);
@@ -726,7 +620,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
   __shared__ __align__(8) uint64_t full_bar[STAGES], empty_bar[STAGES];
   __shared__ __align__(8) uint64_t acc_full, acc_empty, done_bar;
   __shared__ uint32_t tmem_slot;
-  __shared__ int fail_s, fix_s;                      // a wait ran out; the product is for the chains
+  __shared__ int fail_s;
   __shared__ Check check_s;
   volatile int* fail = &fail_s;
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -740,10 +634,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
     mbar_init(smem_u32(&acc_full), 1);
     mbar_init(smem_u32(&acc_empty), EPI_WARPS);
     mbar_init(smem_u32(&done_bar), 1);
-    fail_s = fix_s = 0;
+    fail_s = 0;
     fence_mbar_init();
   }
-  for (int i = tid; i < (int)(sizeof(Check) / sizeof(int)); i += THREADS) reinterpret_cast<int*>(&check_s)[i] = 0;
+  if (g.look && blockIdx.x == 0)
+    for (int i = tid; i < (int)(sizeof(Check) / sizeof(int)); i += THREADS) reinterpret_cast<int*>(&check_s)[i] = 0;
   if (warp == 1) {
     tmem_alloc(smem_u32(&tmem_slot), TMEM);
     tmem_relinquish();
@@ -753,6 +648,7 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
   tc_fence_after();
   const uint32_t taddr = tmem_slot;
   pdl_wait();
+  pdl_trigger();                                     // check_kernel may look beside this
 
   if (warp == 0) {
     if (lane == 0) {
@@ -833,8 +729,10 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
     const uint32_t tb = taddr + ((uint32_t)(q * 32) << 16) + (uint32_t)cb;
     int use = 0;
     bool ok = true;
-    const bool chains = needs_chains(g, check_s);    // beside the first K steps
-    if (chains && tid == 64) fix_s = 1;
+    if (g.look && blockIdx.x == 0) {
+      const bool chains = needs_chains(g, check_s, tid - 64);
+      if (tid == 64) *g.state = chains ? CHAINS : FINE;
+    }
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
       const int z = t % g.nz, rz = t / g.nz, mt = rz % g.mtiles, nt = rz / g.mtiles;
       const int k0 = z * g.kper, k1 = min(g.kt, k0 + g.kper);
@@ -883,7 +781,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
         }
       }
       const int row = mt * BM + q * 32 + lane, n0 = nt * BN + cb;
-      if (chains) continue;
       if (g.cs > 1) {
         // the CTA's only tile: every copy has landed and every MMA has read it,
         // so the ring holds the sums for the cluster (after a failure fail_s counts)
@@ -925,19 +822,14 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
       }
     }
   }
-  pdl_trigger();
-  __syncthreads();                                   // fix_s; the ring is free
-  const bool fix = fix_s != 0, failed = fail_s != 0;
-  if (fix && warp >= 2) run_units<BN, PAIR>(g, base, failed);
   if (g.cs > 1) {
     // one tile per CTA; CTA `rank` adds its share of the columns over the
-    // cluster (exact integers, or the FP64 chains') and rounds, or leaves the
-    // cluster's sum
+    // cluster (exact integers) and rounds, or leaves the cluster's sum
     namespace cgr = cooperative_groups;
     cgr::cluster_group cl = cgr::this_cluster();
+    cl.sync();
     const int z = (int)blockIdx.x % g.nz, rz = (int)blockIdx.x / g.nz;
     const int mt = rz % g.mtiles, nt = rz / g.mtiles, rank = (int)cl.block_rank();
-    cl.sync();
     const int share = (BN + g.cs - 1) / g.cs;
     bool bad = false;
     for (int p = 0; p < g.cs; ++p) bad = bad || *cl.map_shared_rank(&fail_s, p) != 0;
@@ -954,27 +846,18 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_kernel(const __grid_constant_
       for (int p = 0; p < kMaxSplit; ++p)
         v[p] = p < g.cs ? *cl.map_shared_rank(mine + c * BM, p) : make_longlong2(0, 0);
       long long hi = v[0].x, lo = v[0].y;
-      if (fix || bad) {
-        double sum = __longlong_as_double(hi);
 #pragma unroll
-        for (int p = 1; p < kMaxSplit; ++p)
-          if (p < g.cs) sum += __longlong_as_double(v[p].x);
-        if (bad) sum = __longlong_as_double(0x7ff8000000000000ll);
-        hi = __double_as_longlong(sum);
-        lo = LLONG_MIN;                              // marks an FP64 value
-      } else {
-#pragma unroll
-        for (int p = 1; p < kMaxSplit; ++p) {
-          hi += v[p].x;
-          lo += v[p].y;
-        }
+      for (int p = 1; p < kMaxSplit; ++p) {
+        hi += v[p].x;
+        lo += v[p].y;
       }
+      if (bad) hi = LLONG_MIN;                       // marks NaN
       if (g.nz > g.cs)
         g.part[((size_t)(z / g.cs) * g.ntiles * BN + n) * ((size_t)g.mtiles * BM) + row] =
             make_longlong2(hi, lo);
       else
         g.C[cr + c_col<PAIR>(g, n)] =
-            lo == LLONG_MIN ? __longlong_as_double(hi) : to_double(hi, lo, ea + g.eb[n] - 62);
+            hi == LLONG_MIN ? __longlong_as_double(0x7ff8000000000000ll) : to_double(hi, lo, ea + g.eb[n] - 62);
     }
     cl.sync();   // no CTA leaves while another reads its sums
   }
@@ -994,24 +877,152 @@ __global__ void __launch_bounds__(256) finish_kernel(const Args g) {
   for (i64 e = blockIdx.x * (i64)blockDim.x + threadIdx.x; e < total; e += (i64)gridDim.x * blockDim.x) {
     const int row = (int)(e % (i64)Mp), n = (int)(e / (i64)Mp);
     if (row >= g.M) continue;
-    // FP64 values (marked) where the tile was left to the FMA chains, and then
-    // in every cluster; beside a failed cluster's NaN the integers do not count
     long long hi = 0, lo = 0;
-    double sum = 0.0;
-    bool chain = false;
+    bool bad = false;
     for (int z = 0; z < g.nz / g.cs; ++z) {
       const longlong2 v = g.part[((size_t)z * Np + n) * Mp + row];
-      if (v.y == LLONG_MIN) {
-        chain = true;
-        sum += __longlong_as_double(v.x);
-      } else {
-        hi += v.x;
-        lo += v.y;
-      }
+      bad = bad || v.x == LLONG_MIN;
+      hi += v.x;
+      lo += v.y;
     }
     g.C[c_row<PAIR>(g, row) + c_col<PAIR>(g, n)] =
-        chain ? sum : to_double(hi, lo, g.ea[row] + g.eb[n] - 62);
+        bad ? __longlong_as_double(0x7ff8000000000000ll) : to_double(hi, lo, g.ea[row] + g.eb[n] - 62);
   }
+}
+
+// FP64 FMA chains of a unit, 4 NI rows x 8 NJ columns: ks warps take every ks-th k, a
+// lane rows ly + 4 i and columns lx + 8 j, and the warps' sums are added in order
+// from red (16 / ks units at once; `here`: this one exists).  Bound by the FP64 pipe,
+// as gemm_kernel of ttg_gemm.cu is: a load serves several FMAs of 64 clocks each.
+// Units this small, and K over the warps, so that a product of few rows and columns
+// keeps all SMs busy: 32 x 16 (complex 32 x 8), or 8 x 8 where those are fewer than
+// SMs (phi_left with an infinity in Phi, r = 64, n = 40, whose last product has 192 x
+// 64 results: 614 -> 395 us; FP64 kernels 311); four warps a unit where K is
+// short.
+template <class T, int NI, int NJ>
+__device__ __forceinline__ void fp64_unit(const Args& g, bool here, int r0, int c0, int ks, T* red) {
+  constexpr bool CPLX = sizeof(T) == 16;
+  constexpr int E = 32 * NI * NJ;
+  const int w16 = threadIdx.x >> 5, warp = w16 % ks, lane = threadIdx.x & 31, ly = lane >> 3, lx = lane & 7;
+  const int K = here ? g.K : 0;
+  const T *a[NI], *b[NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+    a[i] = reinterpret_cast<const T*>(g.A) + at(g.am, min(r0 + ly + 4 * i, g.rows - 1)) + (i64)warp * g.ak;
+#pragma unroll
+  for (int j = 0; j < NJ; ++j)
+    b[j] = reinterpret_cast<const T*>(g.B) + at(g.bn, min(c0 + lx + 8 * j, g.cols - 1)) + (i64)warp * g.bk;
+  T acc[NI][NJ], x[NI], y[NJ];
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) acc[i][j] = T{};
+  auto load = [&] {
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      x[i] = *a[i];
+      a[i] += ks * g.ak;
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      y[j] = *b[j];
+      b[j] += ks * g.bk;
+    }
+  };
+  constexpr bool AHEAD = !CPLX;                      // (complex: four times the FMAs per load)
+  if (AHEAD && warp < K) load();
+  for (int k = warp; k < K; k += ks) {
+    if (!AHEAD) load();
+    T u[NI], v[NJ];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) u[i] = x[i];
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) v[j] = y[j];
+    if (AHEAD && k + ks < K) load();
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) {
+        if constexpr (CPLX) {
+          const double ui = g.conjA ? -u[i].y : u[i].y, vi = g.conjB ? -v[j].y : v[j].y;
+          acc[i][j].x = fma(u[i].x, v[j].x, acc[i][j].x);
+          acc[i][j].x = fma(-ui, vi, acc[i][j].x);
+          acc[i][j].y = fma(u[i].x, vi, acc[i][j].y);
+          acc[i][j].y = fma(ui, v[j].x, acc[i][j].y);
+        } else {
+          acc[i][j] = fma(u[i], v[j], acc[i][j]);
+        }
+      }
+  }
+  __syncthreads();                                   // the unit before is read
+#pragma unroll
+  for (int i = 0; i < NI; ++i)
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) red[w16 * E + (i * NJ + j) * 32 + lane] = acc[i][j];
+  __syncthreads();
+  red += (w16 - warp) * E;
+  for (int q = warp; here && q < NI * NJ; q += ks) {
+    const int r = r0 + ly + 4 * (q / NJ), n = c0 + lx + 8 * (q % NJ);
+    if (r >= g.rows || n >= g.cols) continue;
+    T v = red[q * 32 + lane];
+    for (int w = 1; w < ks; ++w) {
+      const T t = red[w * E + q * 32 + lane];
+      if constexpr (CPLX) {
+        v.x += t.x;
+        v.y += t.y;
+      } else {
+        v += t;
+      }
+    }
+    reinterpret_cast<T*>(g.C)[at(g.cm, r) + at(g.cn, n)] = v;
+  }
+}
+
+// After the product: whether it is one for the FP64 chains, and then the chains over
+// the whole GPU.  The look is made, where the product kernel left SMs free, beside
+// that kernel; what remains when it is done is one launch (1 to 2 us).  The look and
+// the chains in the product kernel itself took 5 us more a product (time stepper d =
+// 16, n = 32: 98.5 -> 95 ms), and the chains of a K split had its few SMs alone (such
+// a product of the time stepper 180 us).  The chains take the time of the FP64
+// kernels: phi_left with an infinity in Phi, r = 82, n = 64 942 us (FP64 kernels
+// 1426), r = 256, n = 2 753 (777).
+constexpr size_t kCheckSmem = sizeof(double) * EPI_WARPS * 512;
+__global__ void __launch_bounds__(32 * EPI_WARPS, 1) check_kernel(const __grid_constant__ Args g) {
+  extern __shared__ __align__(16) unsigned char check_dyn[];
+  __shared__ Check sh;
+  __shared__ int state_s;
+  const int tid = threadIdx.x;
+  for (int i = tid; i < (int)(sizeof(Check) / sizeof(int)); i += blockDim.x) reinterpret_cast<int*>(&sh)[i] = 0;
+  // (what the split kernel wrote is there: every kernel in between has waited for it
+  // before it let this one start)
+  if (tid == 0) state_s = __ldcg(g.state);
+  __syncthreads();
+  int state = state_s;
+  if (state == UNKNOWN) {
+    state = needs_chains(g, sh, tid) ? CHAINS : FINE;
+    if (tid == 0) *(volatile int*)g.state = state;
+  }
+  pdl_wait();
+  if (state == FINE) return;
+  const int ks = g.K >= 256 ? 16 : 4, at_once = EPI_WARPS / ks, mine = (tid >> 5) / ks;
+  auto run = [&](auto t, auto ni, auto nj) {
+    using T = decltype(t);
+    constexpr int NI = decltype(ni)::value, NJ = decltype(nj)::value;
+    const int mr = (g.rows + 4 * NI - 1) / (4 * NI), nc = (g.cols + 8 * NJ - 1) / (8 * NJ);
+    const i64 units = (i64)mr * nc, steps = (units + at_once - 1) / at_once;
+    for (i64 q = steps * blockIdx.x / gridDim.x; q < steps * (blockIdx.x + 1) / gridDim.x; ++q) {
+      const i64 u = q * at_once + mine, v = u < units ? u : 0;
+      fp64_unit<T, NI, NJ>(g, u < units, (int)(v % mr) * 4 * NI, (int)(v / mr) * 8 * NJ, ks,
+                           reinterpret_cast<T*>(check_dyn));
+    }
+  };
+  using One = std::integral_constant<int, 1>;
+  using Two = std::integral_constant<int, 2>;
+  using Eight = std::integral_constant<int, 8>;
+  const bool few = (i64)((g.rows + 31) / 32) * ((g.cols + 15) / 16) < (i64)gridDim.x * at_once;
+  if (g.cplx) few ? run(double2{}, Two{}, One{}) : run(double2{}, Eight{}, One{});
+  else few ? run(double{}, Two{}, One{}) : run(double{}, Eight{}, Two{});
+  pdl_trigger();
 }
 
 constexpr int SMS = 152;
@@ -1105,7 +1116,7 @@ bool oz_fits(i64 M, i64 N, i64 K, bool cplx) {
 
 size_t oz_stat_bytes(i64 rows, i64 K, i64 groups, i64 kr) {
   using namespace oz;
-  return al(sizeof(int4) * (size_t)(rows / SROWS + 2)) + al(sizeof(short) * SLOTS * (size_t)(K + 7) * groups) +
+  return al(sizeof(int4) * (size_t)(rows / SROWS + 3)) + al(sizeof(short) * SLOTS * (size_t)(K + 7) * groups) +
          al(sizeof(short) * TPARTS * (size_t)kr);
 }
 static short* oz_tab(const OzGemm& g) {          // at the end of stat
@@ -1150,7 +1161,8 @@ void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, 
   };
   const short* tab = g.kr > 0 ? oz_tab(g) : nullptr;
   int4* bm = (int4*)g.stat;
-  short* gpart = (short*)((char*)g.stat + al(sizeof(int4) * (size_t)(((i64)g.M + g.N) / SROWS + 2)));
+  short* gpart = (short*)((char*)g.stat + al(sizeof(int4) * (size_t)(((i64)g.M + g.N) / SROWS + 3)));
+  int* state = (int*)(bm + ((i64)g.M + g.N) / SROWS + 2);
   auto stride = [](int gd) { return ((gd + SROWS - 1) / SROWS + 1 + SLOTS - 1) / SLOTS; };
   const Groups gra{g.M, g.gdA, g.gnA, stride(g.gdA), bm, gpart};
   const Groups grb{g.N, g.gdB, g.gnB, stride(g.gdB), bm + (g.M + SROWS - 1) / SROWS, gpart + (size_t)SLOTS * ((g.K + 7) & ~7) * g.gnA};
@@ -1173,6 +1185,8 @@ void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, 
     set(gemm_kernel<32, true>, 32);
     if (r == cudaSuccess)
       r = cudaFuncSetAttribute(split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kScaleSmem);
+    if (r == cudaSuccess)
+      r = cudaFuncSetAttribute(check_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCheckSmem);
     return r;
   }();
   TTG_CUDA(attr_rc);
@@ -1180,7 +1194,7 @@ void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, 
   int ky = 1;
   while (ky < kMaxCluster && (nA + nB) * ky < 2 * SMS && 2 * s.kt > 32 * ky) ky *= 2;
   launch_ex(split_kernel, dim3(nA + nB + tblocks, ky), dim3(256), dim3(ky > 1 ? 1 : 0, ky, 1), true,
-            g.kr > 0 ? split_smem(g) : 0, st, a, b, nA, nA + nB, tables, g.K, (int)s.kt);
+            g.kr > 0 ? split_smem(g) : 0, st, a, b, nA, nA + nB, tables, g.K, (int)s.kt, state);
   Args x{};
   x.Ad = Ad; x.Bd = Bd; x.ea = ea; x.eb = eb;
   x.M = (int)s.M; x.N = (int)s.N; x.K = g.K;
@@ -1189,11 +1203,10 @@ void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, 
   x.A = g.A; x.B = g.B; x.am = g.am; x.bn = g.bn; x.ak = g.ak; x.bk = g.bk;
   x.cplx = g.cplx; x.conjA = g.conjA; x.conjB = g.conjB;
   x.ga = gra; x.gb = grb;
-  // Without a K split every SM gets a CTA, for the chains' sake, unless K is so short
-  // that the CTAs without a tile would leave when the others let the next kernel in:
-  // its CTAs then crowd on the SMs that are free first (phi_left and phi_right, r =
-  // 37, n = 24: 68 us with the tiles' CTAs alone, 118 with all)
-  const int grid = z.cs > 1 ? (int)(s.mt * s.nt * nz) : (s.kt >= KCHUNK ? SMS : (int)std::min<i64>(SMS, s.mt * s.nt));
+  x.state = state; x.rows = g.M; x.cols = g.N;
+  const int grid = (int)std::min<i64>(SMS, s.mt * s.nt * nz);
+  // where the product kernel, or finish_kernel, leaves check_kernel no SM to look on
+  x.look = grid > SMS * 3 / 4 || groups > 1;
   auto kern = s.bn == 64 ? (s.dup_b ? gemm_kernel<64, true> : gemm_kernel<64, false>)
                          : (s.dup_b ? gemm_kernel<32, true> : gemm_kernel<32, false>);
   launch_ex(kern, dim3(grid), dim3(THREADS),
@@ -1202,6 +1215,7 @@ void oz_gemm(const OzGemm& g, void* ws, const OzGemm* const* later, int nlater, 
     const int fb = (int)std::min<i64>(1024, ((i64)ra * s.N + 255) / 256);
     launch_pdl(s.dup_b ? finish_kernel<true> : finish_kernel<false>, dim3(fb), dim3(256), 0, st, x);
   }
+  launch_pdl(check_kernel, dim3(SMS), dim3(32 * EPI_WARPS), kCheckSmem, st, x);
 }
 
 // A strided batched product as one split product: a batch over which one
