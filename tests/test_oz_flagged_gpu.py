@@ -1,5 +1,5 @@
-"""Split products with flagged rows (ttg_oz.cu): the tiles that meet an infinity,
-a NaN or an extreme row run as FP64 FMA chains over all SMs.
+"""Split products with flagged rows (ttg_oz.cu): a product that meets an infinity,
+a NaN or an extreme row is formed by FP64 FMA chains over all SMs.
 
 Values: against numpy in the pattern of non-finite outputs, and within the FP64
 chain's bound (K + 2) u |A| |B| beside them.  Time: a call whose every product
@@ -46,8 +46,8 @@ def test_a_flagged_call_costs_no_more_than_fp64(torch_cuda, ctx, r1, n, r2, ra):
                                    (96, 77, 5248), (1000, 129, 257)])
 @pytest.mark.parametrize("side", ["row", "column"])
 def test_tiles_beside_a_flag(torch_cuda, ctx, M, N, K, side):
-    """One extreme row (or column): tiles with it take the chains, the others the
-    tensor cores, in one tile, in K splits of one cluster and of several."""
+    """One extreme row (or column) in shapes of one tile, of K splits in one cluster
+    and in several: its elements and those beside it."""
     import ttgpu
     rng = np.random.default_rng(M + N + K)
     X, P = rng.standard_normal((M, K)), rng.standard_normal((K, N))
